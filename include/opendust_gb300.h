@@ -280,10 +280,10 @@ od_status od_set_graph(od_handle* h, int32_t enable);
  * 5: packed with one target per thread (targets_per_thread 1), 6: as 5 with every other source
  * pair on the Newton path of variant 4, 7: each unordered pair evaluated once and applied to
  * both ions (threads 256; targets_per_thread = target ions per lane: 2 or 4 with as many source
- * ions, 8 with two; jsplit = ions per tile, 1024, 2048 or 4096 (not 1024 with 8; also 512 with
- * 2), <= 0 for the default). Variants 2-7 add their sums into 64-bit fixed-point accumulators (24
+ * ions, 8 with two; jsplit = tile, 1024, 2048 or 4096 (not 1024 with 8; also 512 with 2), <= 0
+ * for the default: it caps the work a warp takes at a time). Variants 2-7 add their sums into 64-bit fixed-point accumulators (24
  * bytes per ion) with integer atomics, so results do not depend on the order of the GPU's
- * blocks. From 2^14 ions od_create selects variant 7.
+ * blocks. od_create selects variant 7.
  * jsplit <= 0 picks the source split from the SM count. Takes effect at the next step.
  * Cutoff method (force_method OD_FORCE_CUTOFF): variant 0 or 2 walks a stencil of cells per
  * target cell (scalar or packed); variant 3 (the default) sorts
@@ -298,7 +298,7 @@ od_status od_set_pair_plan(od_handle* h, int32_t threads, int32_t targets_per_th
  * cached for this (device, padded size) in the process is reused. *best_pairs_per_s receives
  * the measured rate (0 when cached). All-pairs method only. */
 od_status od_autotune(od_handle* h, int32_t use_cache, double* best_pairs_per_s);
-/* plan5 = {threads, targets_per_thread, variant, jsplit (variant 7: ions per tile), chunk} */
+/* plan5 = {threads, targets_per_thread, variant, jsplit (variant 7: tile), chunk} */
 od_status od_get_pair_plan(const od_handle* h, int32_t* plan5);
 /* FP32 FMA throughput of the device in TFLOP/s (2 flops per FMA), measured by a short probe
  * kernel: the denominator of the all-pairs kernel's roofline. */
@@ -418,8 +418,8 @@ od_status od_batch_step(od_batch* b, int64_t nsteps);
 /* Device milliseconds of the last od_batch_step (CUDA events on the batch stream). */
 od_status od_batch_last_step_ms(const od_batch* b, double* ms);
 /* The all-pairs plan a batch member with n_ions ions steps with (plan5 as od_get_pair_plan;
- * jsplit 0 = the member's default split): variant 7 with 4 x 4 ions per lane and 1024-ion
- * tiles up to 2^16 ions, 8 x 2 and 2048-ion tiles above (od_batch_set_plan changes it). A single
+ * jsplit 0 = the member's default split): variant 7 with 4 x 4 ions per lane (tile 1024) up to
+ * 2^16 ions, 8 x 2 (tile 2048) above (od_batch_set_plan changes it). A single
  * simulation given the same plan produces bitwise the same results. No
  * counterpart in the reference (it has no batching). */
 od_status od_batch_pair_plan(int64_t n_ions, int32_t* plan5);

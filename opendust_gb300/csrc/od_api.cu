@@ -365,18 +365,17 @@ static void fill_params(const od_config* c, int N, int Npad, od_dparams* p) {
   tail_consts(p);
 }
 
-// Default all-pairs plan: packed f32x2 arithmetic on SoA tiles with one target per thread
-// (variant 5, the fastest measured on GB300 from 2^16 to 2^20 ions), with enough source chunks
-// for several waves on every SM.
-// From 2^15 padded ions the default is variant 7 (each unordered pair once: 4 x 4 ions per lane
-// with 1024-ion tiles up to 2^16 ions, then 8 x 2 with 2048-ion tiles); its sums go to 24 bytes of
-// fixed-point accumulators per ion, so it always fits (the budget below only bounds the rule).
+// Directed all-pairs plan: packed f32x2 arithmetic on SoA tiles with one target per thread
+// (variant 5, the fastest directed form measured on GB300 from 2^16 to 2^20 ions), with enough
+// source chunks for several waves on every SM. Shards step with it.
+// The default is variant 7 (each unordered pair once: 4 x 4 ions per lane up to 2^16 ions, then
+// 8 x 2); its sums go to 24 bytes of fixed-point accumulators per ion, so it always fits (the
+// budget below only bounds the rule).
 static constexpr size_t OD_N3_BUDGET = (size_t)32 << 30;
 // The cutoff's tile-pair path (variant 3: 512-ion tiles with balanced group-pair lists) needs its
 // sort, boxes, tile-pair list and slot accumulators (0.3 GB at 2^20 ions); the budget bounds the
 // tile-pair list for very large N, beyond which 1024-ion tiles or the cell stencil take over.
 static constexpr size_t OD_CUTN3_BUDGET = (size_t)64 << 30;
-static bool uses_n3_default(int Npad) { return Npad >= 16384; }
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile);
 
 static od_pair_plan default_plan(int Npad, int sms) {
@@ -505,7 +504,7 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
   if (alloc_scratch_for_plan(h) != OD_OK) return bail(OD_ERR_OOM);
   if (cfg->force_method != OD_FORCE_CUTOFF && ensure_acc(h) != OD_OK) return bail(OD_ERR_OOM);
   int n3_ipt = 0, n3_tile = 0;
-  if (n3_default && cfg->force_method != OD_FORCE_CUTOFF && uses_n3_default(h->Npad))
+  if (n3_default && cfg->force_method != OD_FORCE_CUTOFF)
     n3_tile = od_n3_default(h->Npad, OD_N3_BUDGET, &n3_ipt);
   if (n3_tile && set_plan_n3(h, n3_ipt, n3_tile) != OD_OK) {
     // no each-pair-once shape for this size: stay on the directed-pair default
@@ -1114,8 +1113,9 @@ static od_status ensure_acc(od_handle* h) {
 }
 
 // Variant 7: `ions_per_lane` targets per lane (2 or 4 with as many sources, 8 with two sources),
-// `tile` ions per tile (1024, 2048, 4096; <= 0: 1024 up to 2^17 ions, else 2048). The pair
-// sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25 MB at 2^20).
+// `tile` caps the work per warp (od_n3_split_of; 1024, 2048, 4096; <= 0: 1024 up to 2^17 ions, else
+// 2048). The pair sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25
+// MB at 2^20).
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
   if (!plan_supported(256, ions_per_lane, 7))
     return fail(h, OD_ERR_INVALID, "variant 7 takes 2, 4 or 8 targets per lane");
@@ -1133,7 +1133,6 @@ static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
   od_pair_plan pl{};
   pl.nt = 256; pl.ipt = ions_per_lane; pl.variant = 7; pl.tile = tile;
   pl.jsplit = 1; pl.chunk = h->Npad;
-  OD_CK(h, od_n3_prepare(pl));
   const size_t need = od_n3_floats(h->Npad, tile);
   if (h->b.n3_len < need) {
     free_n3(h);
@@ -1590,10 +1589,8 @@ struct od_batch {
   int4* d_items = nullptr;
   int2* d_blk_corr = nullptr;
   size_t c_sims = 0, c_blk_ion = 0, c_items = 0, c_blk_corr = 0;
-  int4* d_n3_items[2] = {nullptr, nullptr};
-  size_t c_n3_items[2] = {0, 0};
-  int2* d_n3_blk = nullptr;
-  size_t c_n3_blk = 0;
+  int2* d_n3_items[OD_N3_FORMS] = {};
+  size_t c_n3_items[OD_N3_FORMS] = {};
   unsigned int* d_next = nullptr;
   uint32_t* d_err = nullptr;
   od_batchview view{};
@@ -1727,8 +1724,7 @@ static od_status batch_rebuild(od_batch* b) {
   std::vector<int2> blk_ion, blk_corr;
   struct item { int4 w; long long work; };
   std::vector<item> items;
-  std::vector<int4> n3_items[2];
-  std::vector<int2> n3_blk;
+  std::vector<int2> n3_items[OD_N3_FORMS];
   for (od_handle* h : b->members) {
     if (!h) continue;
     const int m = (int)sims.size();
@@ -1740,16 +1736,14 @@ static od_status batch_rebuild(od_batch* b) {
     const float nr = 64.0f * h->hp.rho0;
     d.newton_r2 = nr * nr;
     d.n3_tile = h->plan.variant == 7 ? h->plan.tile : 0;
+    if (d.n3_tile) d.n3 = od_n3_split_of(d.Npad, h->plan.ipt, d.n3_tile);
     sims.push_back(d);
     for (int lb = 0; lb < d.nb; lb++) blk_ion.push_back(make_int2(m, lb));
     for (int lb = 0; lb < d.nb + d.nrec; lb++) blk_corr.push_back(make_int2(m, lb));
     if (d.n3_tile) {
-      // every tile pair of this member, in the table of its instantiation
-      const int nT = (d.Npad + d.n3_tile - 1) / d.n3_tile;
-      std::vector<int4>& t = n3_items[h->plan.ipt == 4 && d.n3_tile == 1024 ? 0 : 1];
-      for (int bb = 0; bb < nT; bb++)
-        for (int aa = 0; aa <= bb; aa++) t.push_back(make_int4(m, aa, bb, nT));
-      for (int lb = 0; lb < d.nb; lb++) n3_blk.push_back(make_int2(m, lb));
+      // every block of this member's pair kernel, in the table of its form
+      std::vector<int2>& t = n3_items[od_n3_form(h->plan.ipt, sims.back().n3)];
+      for (long long k = 0; k < od_n3_blocks(sims.back().n3); k++) t.push_back(make_int2(m, (int)k));
       continue;
     }
     for (int ib = 0; ib < d.Npad / 256; ib++)
@@ -1766,10 +1760,9 @@ static od_status batch_rebuild(od_batch* b) {
   if ((st = upload_table(b, &b->d_blk_ion, &b->c_blk_ion, blk_ion)) != OD_OK) return st;
   if ((st = upload_table(b, &b->d_items, &b->c_items, w)) != OD_OK) return st;
   if ((st = upload_table(b, &b->d_blk_corr, &b->c_blk_corr, blk_corr)) != OD_OK) return st;
-  for (int k = 0; k < 2; k++)
+  for (int k = 0; k < OD_N3_FORMS; k++)
     if ((st = upload_table(b, &b->d_n3_items[k], &b->c_n3_items[k], n3_items[k])) != OD_OK)
       return st;
-  if ((st = upload_table(b, &b->d_n3_blk, &b->c_n3_blk, n3_blk)) != OD_OK) return st;
   OD_BCK(b, cudaStreamSynchronize(b->stream));
   od_batchview& v = b->view;
   v.sims = b->d_sims; v.nsims = (int)sims.size();
@@ -1778,11 +1771,10 @@ static od_status batch_rebuild(od_batch* b) {
   v.blk_corr = b->d_blk_corr; v.nblk_corr = (int)blk_corr.size();
   v.pair_grid = od_num_sms(b->device) * 4;
   v.next = b->d_next; v.err = b->d_err;
-  for (int k = 0; k < 2; k++) {
+  for (int k = 0; k < OD_N3_FORMS; k++) {
     v.n3_items[k] = b->d_n3_items[k];
     v.n3_nitems[k] = (int)n3_items[k].size();
   }
-  v.n3_blk = b->d_n3_blk; v.n3_nblk = (int)n3_blk.size();
   if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
   if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
   if (v.nsims > 0) {
@@ -1861,9 +1853,10 @@ extern "C" od_status od_batch_destroy(od_batch* b) {
     if (h) od_destroy(h);
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
-  void* ptrs[] = {b->d_sims,         b->d_blk_ion,      b->d_items,  b->d_blk_corr, b->d_next,
-                  b->d_err,          b->d_n3_items[0], b->d_n3_items[1], b->d_n3_blk};
+  void* ptrs[] = {b->d_sims, b->d_blk_ion, b->d_items, b->d_blk_corr, b->d_next, b->d_err};
   for (void* p : ptrs)
+    if (p) cudaFree(p);
+  for (int2* p : b->d_n3_items)
     if (p) cudaFree(p);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
@@ -1887,11 +1880,8 @@ extern "C" od_status od_config_device_bytes(const od_config* cfg, int64_t* bytes
     if (c512 <= OD_CUTN3_BUDGET) b += (int64_t)c512;
     else if (c1024 <= OD_CUTN3_BUDGET) b += (int64_t)c1024;
   }
-  if (cfg->force_method != OD_FORCE_CUTOFF && uses_n3_default((int)Np)) {
-    int ipt = 0;
-    const int tile = od_n3_default((int)Np, OD_N3_BUDGET, &ipt);
-    if (tile) b += (int64_t)(sizeof(float) * od_n3_floats((int)Np, tile));  // tile-pair sums
-  }
+  if (cfg->force_method != OD_FORCE_CUTOFF)
+    b += (int64_t)(sizeof(float) * od_n3_floats((int)Np, 1));  // fixed-point accumulators
   b += Np * 16 * 4;                 // pos, vel, fhi, flo
   b += Np * 12;                     // SoA copy
   b += (int64_t)pl.jsplit * Np * 32;  // partial slabs

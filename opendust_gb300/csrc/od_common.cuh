@@ -128,6 +128,9 @@ __device__ __forceinline__ void od_gauss2(uint32_t a, uint32_t b, float& g0, flo
 __device__ __forceinline__ float od_rsqrt(float x) {
   float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r;
 }
+__device__ __forceinline__ float od_sqrt(float x) {
+  float r; asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r;
+}
 __device__ __forceinline__ float od_rcp(float x) {
   float r; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r;
 }
@@ -194,6 +197,12 @@ __device__ __forceinline__ unsigned long long od_fix(float hi, float lo) {
 }
 __device__ __forceinline__ void od_fix_add(unsigned long long* a, float hi, float lo) {
   atomicAdd(a, od_fix(hi, lo));
+}
+// one FP32 value (cvt.rni.s64.f32 takes 67 cycles per warp, but on a pipe the pair kernels leave
+// idle: a split into digits on the FP32 and integer pipes is bit-identical and made the
+// all-pairs kernel 1 % and the cutoff kernel 5 % slower)
+__device__ __forceinline__ void od_fix_add1(unsigned long long* a, float v) {
+  atomicAdd(a, (unsigned long long)__float2ll_rn(v * OD_FIX_SCALE));
 }
 // accumulator (3 words, component stride `stride`) -> two-float sums, and the words cleared for
 // the next evaluation

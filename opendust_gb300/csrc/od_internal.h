@@ -15,7 +15,7 @@ struct od_pair_plan {
   int variant; // 0: shared-memory broadcast, 1: warp-shuffle broadcast, 2: packed f32x2 with
                // SoA tiles (ipt 2), 3: as 2 with Newton reciprocals for half of the targets,
                // 4-6: further packed forms, 7: each unordered pair once (od_n3.cu)
-  int tile;    // variant 7: ions per tile (1024, 2048 or 4096); ipt = targets per lane (2, 4:
+  int tile;    // variant 7: caps the work per warp (od_n3_split_of); ipt = targets per lane (2, 4:
                // as many sources; 8: two sources)
 };
 
@@ -54,9 +54,18 @@ int od_num_sms(int device);
 bool od_n3_supported(int ipt, int tile);
 int od_n3_default(int Npad, size_t budget_bytes, int* ipt);
 size_t od_n3_floats(int Npad, int tile);
-cudaError_t od_n3_prepare(const od_pair_plan& pl);  // shared-memory opt-in, current device
 cudaError_t od_launch_pairs_n3(const od_pair_plan& pl, const od_pair_io& io, int Npad, float4* ph,
                                float4* pl_lo, float rho0, cudaStream_t s, bool take = true);
+// How a variant-7 evaluation is divided: `units` units of L consecutive group pairs, or (split > 1)
+// of one group pair's lane steps in `split` parts; one unit per warp.
+struct od_n3_split {
+  long long pairs, units;  // group pairs of the upper triangle, units
+  int L, split;
+};
+od_n3_split od_n3_split_of(int Npad, int ipt, int tile);
+long long od_n3_blocks(const od_n3_split& sp);
+constexpr int OD_N3_FORMS = 5;
+int od_n3_form(int ipt, const od_n3_split& sp);  // kernel form of a batch member, < OD_N3_FORMS
 
 // One member of a batch, as the batched kernels see it.
 struct od_simdesc {
@@ -66,6 +75,7 @@ struct od_simdesc {
   int N, Npad, nb, jsplit, chunk, nrec;
   float rho0, newton_r2;
   int n3_tile;  // variant-7 tile of this member (its accumulators are b.n3), 0 otherwise
+  od_n3_split n3;  // its work split
 };
 // Device tables of one batch step.
 struct od_batchview {
@@ -80,12 +90,9 @@ struct od_batchview {
   int pair_grid;         // persistent blocks of the all-pairs stage
   unsigned int* next;    // work counter of the all-pairs stage
   uint32_t* err;
-  // members on variant 7: (member, tile a, tile b, tiles) per instantiation (0: 4 x 4 with
-  // 1024-ion tiles, 1: 8 x 2 with 2048-ion tiles), and (member, 256-ion block) row-sum blocks
-  const int4* n3_items[2];
-  int n3_nitems[2];
-  const int2* n3_blk;
-  int n3_nblk;
+  // members on variant 7: (member, block of its pair kernel) per kernel form
+  const int2* n3_items[OD_N3_FORMS];
+  int n3_nitems[OD_N3_FORMS];
 };
 cudaError_t od_launch_batch_step(const od_batchview& v, cudaStream_t s);
 // pot[k] = sum over ions i < N of exp(-r)/(r + rho0), r = |(pts[2k], 0, pts[2k+1]) - x_i|

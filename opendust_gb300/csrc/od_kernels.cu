@@ -1550,8 +1550,9 @@ __global__ void __launch_bounds__(kBlk) k_b_kick_flag(const od_simdesc* __restri
                                                       const int2* __restrict__ blk) {
   const int2 e = blk[blockIdx.x];
   const od_simdesc& d = sims[e.x];
+  // variant 7: straight from the accumulators, as a member stepped alone
   kick_flag_body(*d.dp, d.ds, d.b.pos, d.b.vel, d.b.part_hi, d.b.part_lo, d.jsplit, d.b.fhi, d.b.flo,
-                 d.b.flags, d.b.cq, e.y * kBlk + threadIdx.x);
+                 d.b.flags, d.b.cq, e.y * kBlk + threadIdx.x, d.n3_tile ? d.b.n3 : nullptr);
 }
 
 __global__ void __launch_bounds__(kCT) k_b_collect_inject(const od_simdesc* __restrict__ sims) {

@@ -7,64 +7,236 @@
 // (the reference's OpenMM CUDA nonbonded kernel also applies each pair force to both atoms).
 //
 // Decomposition
-//   * A warp owns a target group of GT = 32·MT ions (lane l holds ions l + 32k, k < MT) and
-//     visits source groups of GS = 32·MS ions. Tiles hold T = PA·8·GT ions (8 warps, PA passes).
-//   * One block per tile pair (a, b), a <= b. Warp w, pass p, holds target group ga = w + 8p of
-//     tile a in registers and sweeps the source groups of tile b in a staggered order (group
-//     s + w·NBS/8 at step s), so that at every step the eight warps touch eight different
-//     source groups and a __syncthreads() between steps makes the shared-memory updates
-//     race-free.
-//   * Inside a group pair the sources rotate around the warp: at each of the 32 lane steps every
-//     lane evaluates its MT targets against the MS sources it holds, then passes the sources —
-//     positions and their FP32 reaction sums — to the previous lane. After 32 steps every source
-//     is back in its own lane with the sum of the GT target reactions on it. The packed f32x2
-//     operations pair two sources against one target (each target duplicated in both halves)
-//     or, with 8 targets per lane, two targets against one broadcast source (n3_group_tp: half
-//     the target registers, more independent pair chains in flight).
-//   * Diagonal tiles (a == b) evaluate the source groups inside a warp's own target group as
-//     directed pairs (no reaction; the self pair contributes exactly 0) and skip source groups
-//     below it.
-//   * Per target group the per-step FP32 sums are folded into two-float accumulators; reaction
-//     sums are folded into a two-float shared-memory slice of tile b.
-//   * Output: a dense matrix S[t][y] of two-float partial sums for the ions of tile t from the
-//     ions of tile y (t < y: target side of block (t, y); t > y: reaction side of block (y, t);
-//     t == y: both). A second kernel sums row t over y in a fixed order into slab 0 of the
-//     partial-sum arrays (the all-pairs consumers then see one slab). Every result bit is
+//   * A group pair is GT = 32·MT target ions (lane l holds ions l + 32k, k < MT, each duplicated in
+//     both halves of an f32x2 register) against GS = 32·MS source ions (MS/2 packs per lane). The
+//     sources rotate around the warp: at each of 32 lane steps every lane evaluates its targets
+//     against the sources it holds, then passes the sources, their positions and their FP32
+//     reaction sums, to the previous lane.
+//   * The group pairs of the upper triangle are numbered row by row (a row: one target group
+//     against the source groups from its own on), and every warp takes L consecutive ones, or,
+//     in systems too small to fill the GPU that way, one group pair's lane steps in `split`
+//     equal parts. Warps share nothing: there is no block barrier, and a block's warps differ by
+//     at most one group pair of work.
+//   * The source groups inside a target group are evaluated as directed pairs (no reaction; the
+//     self pair contributes exactly 0).
+//   * Reactions are summed in FP32 over at most 16 lane steps, target sums over one group pair
+//     (then as two-floats in the warp's shared-memory slice when L > 1); both are then added to
+//     the ions' 64-bit fixed-point accumulators with integer atomics, so every result bit is
 //     independent of scheduling.
+//
+// What bounds it: operand fetch of the packed FP32 pipe. Measured on GB300, cycles per warp
+// instruction and sub-partition: fma.f32x2 with one, two and three distinct register operands
+// 2.1, 2.7 to 3.0 and 3.0 to 3.7; rsqrt, sqrt and rcp 8.4, ex2 4.2, shfl 4.2. At 2^18 ions the kernel
+// takes 25.3 cycles per 32 unordered pairs and sub-partition (8 x 2; 4 x 4: 26.2), and 23 with every
+// SFU operation taken out, so fewer SFU operations, or a scalar form (33), gain nothing. The pair
+// term below has the fewest packed operations (17 with the sums).
+#include <algorithm>
 #include "od_n3_pair.cuh"
 
 namespace {
 
-// (a, b) of the k-th pair of the b-major upper triangle
-__device__ __forceinline__ int2 tri_pair(int kb) {
-  int b = (int)((sqrtf(8.f * (float)kb + 1.f) - 1.f) * 0.5f);
-  while ((b + 1) * (b + 2) / 2 <= kb) b++;
-  while (b * (b + 1) / 2 > kb) b--;
-  return make_int2(kb - b * (b + 1) / 2, b);
+constexpr int kSliceWarps = 4;  // warps per block: they are independent, small blocks retire evenly
+
+// Register budget and unrolling per shape (MT targets, MS sources per lane). 2^18 ions, ms per
+// evaluation: 8 x 2 21.6 (16 warps per SM of 128 registers, two lane steps unrolled), 4 x 4 22.4 (20
+// warps of 96, four steps; with 24 warps of 80 or 16 of 128 registers 2 to 4 % slower), 2 x 2 24.4.
+// The tile-pair form this replaces (eight warps per tile pair, one barrier per source group) took
+// 23.3 (8 x 2) there, 0.928 against 0.838 now at 50021 ions (4 x 4), and 0.129 (2 x 2, its last wave
+// half empty) against 0.100 at 2^14. The registers hold the loop state only just: the split and the
+// slice length are template parameters because as variables they spilled (16384 ions 0.115 ms).
+template <int MT, int MS>
+struct slice_traits {
+  static constexpr int GT = 32 * MT, GS = 32 * MS;
+  static constexpr int R = GT / GS;  // source groups inside a target group
+  static constexpr int MIN_BLOCKS = MT == 8 ? 4 : (MT == 4 ? 5 : 8);
+  static constexpr int UNROLL = MT == 8 ? 2 : 4;
+};
+
+struct pair_consts {
+  od_u64 eps, rho, nl2e;
+};
+
+// One pack: target (X, X) against two sources. With R = r and W = 1/(r (r + rho)):
+// c = exp(-r) (1/s + 1/s^2) / r = exp(-r) (W + W (W r)), s = r + rho. One packed operation fewer
+// than the form from 1/sqrt(r^2), and more accurate (the term's rms error 0.9e-7 against 1.1e-7
+// for r < 1, 2.1e-7 against 2.9e-7 at r = 4.5).
+template <bool REACT>
+__device__ __forceinline__ void pair_once(const pair_consts& k, od_u64 X, od_u64 Y, od_u64 Z,
+                                          od_u64 QX, od_u64 QY, od_u64 QZ, od_u64& AX, od_u64& AY,
+                                          od_u64& AZ, od_u64& RX, od_u64& RY, od_u64& RZ) {
+  const od_u64 DX = sub2(X, QX), DY = sub2(Y, QY), DZ = sub2(Z, QZ);
+  od_u64 R2 = fma2(DX, DX, k.eps);
+  R2 = fma2(DY, DY, R2);
+  R2 = fma2(DZ, DZ, R2);
+  const float2 r2 = up2(R2);
+  const od_u64 R = p2(od_sqrt(r2.x), od_sqrt(r2.y));
+  const float2 rs = up2(fma2(R, k.rho, R2));
+  const od_u64 W = p2(od_rcp(rs.x), od_rcp(rs.y));
+  const float2 ea = up2(mul2(R, k.nl2e));
+  const od_u64 EX = p2(od_ex2(ea.x), od_ex2(ea.y));
+  const od_u64 C = mul2(EX, fma2(W, mul2(W, R), W));
+  AX = fma2(C, DX, AX); AY = fma2(C, DY, AY); AZ = fma2(C, DZ, AZ);
+  if (REACT) { RX = fma2(C, DX, RX); RY = fma2(C, DY, RY); RZ = fma2(C, DZ, RZ); }
 }
 
-template <int MT, int MS, int PA>
-__global__ void __launch_bounds__(kWarps * 32, (n3_traits<MT, MS, PA>::MIN_BLOCKS))
+// STEPS lane steps of one group pair
+template <int MT, int MS, bool REACT, int STEPS>
+__device__ __forceinline__ void lane_steps(const pair_consts& k, const od_u64 (&X)[MT],
+                                           const od_u64 (&Y)[MT], const od_u64 (&Z)[MT],
+                                           od_u64 (&QX)[MS / 2], od_u64 (&QY)[MS / 2],
+                                           od_u64 (&QZ)[MS / 2], od_u64 (&AX)[MT],
+                                           od_u64 (&AY)[MT], od_u64 (&AZ)[MT],
+                                           od_u64 (&RX)[MS / 2], od_u64 (&RY)[MS / 2],
+                                           od_u64 (&RZ)[MS / 2], int src) {
+  constexpr int U = slice_traits<MT, MS>::UNROLL;
+#pragma unroll U
+  for (int st = 0; st < STEPS; st++) {
+#pragma unroll
+    for (int q = 0; q < MS / 2; q++) {
+#pragma unroll
+      for (int t = 0; t < MT; t++)
+        pair_once<REACT>(k, X[t], Y[t], Z[t], QX[q], QY[q], QZ[q], AX[t], AY[t], AZ[t], RX[q],
+                         RY[q], RZ[q]);
+      QX[q] = shfl64(QX[q], src); QY[q] = shfl64(QY[q], src); QZ[q] = shfl64(QZ[q], src);
+      if (REACT) {
+        RX[q] = shfl64(RX[q], src); RY[q] = shfl64(RY[q], src); RZ[q] = shfl64(RZ[q], src);
+      }
+    }
+  }
+}
+
+// Unit `unit` of one simulation (one warp): group pairs [unit L, unit L + L) of the row-major
+// upper triangle, or (SPLIT > 1, L = 1) part unit % SPLIT of group pair unit / SPLIT.
+// h: this lane's column of the warp's shared-memory slice ([6][GT] floats, used when FOLD).
+template <int MT, int MS, int SPLIT, bool FOLD>
+__device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const float* __restrict__ sy,
+                                         const float* __restrict__ sz, int Npad,
+                                         unsigned long long* __restrict__ acc, float rho0,
+                                         long long unit, const od_n3_split& sp, float* h) {
+  using TR = slice_traits<MT, MS>;
+  constexpr int GT = TR::GT, GS = TR::GS, R = TR::R;
+  static_assert(!(FOLD && SPLIT > 1), "a split group pair is one unit");
+  const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
+  constexpr int STEPS = 32 / SPLIT;        // lane steps of a unit's group pairs
+  constexpr int PART = STEPS < 16 ? STEPS : 16;  // lane steps between two reaction flushes
+  if (unit >= sp.units) return;
+  int g, s, n;  // target group, source group, group pairs left
+  int at;       // lane whose sources this lane holds
+  {
+    const long long f = SPLIT > 1 ? unit / SPLIT : (FOLD ? unit * sp.L : unit);
+    at = SPLIT > 1 ? lane + (int)(unit % SPLIT) * STEPS : lane;
+    n = FOLD ? (int)min((long long)sp.L, sp.pairs - f) : 1;
+    // rows 0 .. g-1 hold g NS - R g (g - 1) / 2 group pairs
+    const int NS = Npad / GS;
+    const double b = NS + 0.5 * R;
+    g = (int)((b - sqrt(fmax(b * b - 2.0 * R * (double)f, 0.0))) / R);
+    auto before = [&](long long q) { return q * NS - R * (q * (q - 1) / 2); };
+    while (g > 0 && before(g) > f) g--;
+    while (before(g + 1) <= f) g++;
+    s = g * R + (int)(f - before(g));
+  }
+  pair_consts k;
+  k.eps = p2(1e-30f, 1e-30f); k.rho = p2(rho0, rho0); k.nl2e = p2(OD_NLOG2E, OD_NLOG2E);
+  for (;;) {
+    od_u64 X[MT], Y[MT], Z[MT];
+#pragma unroll
+    for (int t = 0; t < MT; t++) {
+      const int i = g * GT + lane + 32 * t;
+      X[t] = p2(sx[i], sx[i]); Y[t] = p2(sy[i], sy[i]); Z[t] = p2(sz[i], sz[i]);
+      if (FOLD)
+#pragma unroll
+        for (int c = 0; c < 6; c++) h[c * GT + 32 * t] = 0.f;
+    }
+    do {
+      od_u64 QX[MS / 2], QY[MS / 2], QZ[MS / 2], RX[MS / 2], RY[MS / 2], RZ[MS / 2];
+      od_u64 AX[MT], AY[MT], AZ[MT];
+#pragma unroll
+      for (int q = 0; q < MS / 2; q++) {
+        const int j = s * GS + (at & 31) + 64 * q;
+        QX[q] = p2(sx[j], sx[j + 32]); QY[q] = p2(sy[j], sy[j + 32]); QZ[q] = p2(sz[j], sz[j + 32]);
+      }
+#pragma unroll
+      for (int t = 0; t < MT; t++) AX[t] = AY[t] = AZ[t] = 0ull;
+      if (s >= g * R + R) {
+        // each part's reactions are added to the accumulators of the sources where they stand
+        // (the force on a source is minus the accumulated terms)
+#pragma unroll 1
+        for (int st = PART; st <= STEPS; st += PART) {
+#pragma unroll
+          for (int q = 0; q < MS / 2; q++) RX[q] = RY[q] = RZ[q] = 0ull;
+          lane_steps<MT, MS, true, PART>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src);
+#pragma unroll
+          for (int q = 0; q < MS / 2; q++) {
+            const float2 rx = up2(RX[q]), ry = up2(RY[q]), rz = up2(RZ[q]);
+            unsigned long long* e = acc + s * GS + ((at + st) & 31) + 64 * q;
+            od_fix_add1(e, -rx.x); od_fix_add1(e + 32, -rx.y);
+            e += Npad;
+            od_fix_add1(e, -ry.x); od_fix_add1(e + 32, -ry.y);
+            e += Npad;
+            od_fix_add1(e, -rz.x); od_fix_add1(e + 32, -rz.y);
+          }
+        }
+      } else {
+        lane_steps<MT, MS, false, STEPS>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src);
+      }
+      if (!FOLD) {
+#pragma unroll
+        for (int t = 0; t < MT; t++) {
+          unsigned long long* a = acc + g * GT + lane + 32 * t;
+          od_fix_add1(a, sum2(AX[t]));
+          od_fix_add1(a + Npad, sum2(AY[t]));
+          od_fix_add1(a + 2 * (size_t)Npad, sum2(AZ[t]));
+        }
+        return;
+      }
+#pragma unroll
+      for (int t = 0; t < MT; t++) {
+        od_acc2(h[32 * t], h[3 * GT + 32 * t], sum2(AX[t]));
+        od_acc2(h[GT + 32 * t], h[4 * GT + 32 * t], sum2(AY[t]));
+        od_acc2(h[2 * GT + 32 * t], h[5 * GT + 32 * t], sum2(AZ[t]));
+      }
+      n--;
+      s++;
+    } while (n > 0 && s * GS < Npad);
+#pragma unroll
+    for (int t = 0; t < MT; t++)
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        od_fix_add(acc + (size_t)c * Npad + g * GT + lane + 32 * t, h[c * GT + 32 * t],
+                   h[(3 + c) * GT + 32 * t]);
+    if (n <= 0) return;
+    g++;
+    s = g * R;
+  }
+}
+
+template <int MT, int MS, int SPLIT, bool FOLD>
+__global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_BLOCKS))
     k_pairs_n3(const float* __restrict__ sx, const float* __restrict__ sy,
                const float* __restrict__ sz, int Npad, unsigned long long* __restrict__ acc,
-               float rho0) {
-  extern __shared__ float sm[];
-  const int2 ab = tri_pair(blockIdx.x);
-  n3_tile_pair<MT, MS, PA, 0, false>(sx, sy, sz, Npad, acc, (size_t)Npad,
-                                     n3_cut{rho0, 0.f, 0.f, 0.f}, ab.x, ab.y, sm);
+               float rho0, const __grid_constant__ od_n3_split sp) {
+  __shared__ float sm[FOLD ? kSliceWarps * 6 * slice_traits<MT, MS>::GT : 1];
+  const int w = threadIdx.x >> 5;
+  n3_slice<MT, MS, SPLIT, FOLD>(sx, sy, sz, Npad, acc, rho0,
+                                (long long)blockIdx.x * kSliceWarps + w, sp,
+                                sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT + (threadIdx.x & 31)
+                                           : 0));
 }
 
-// Batched form: block k takes work item k = (simulation, tile a, tile b) of a table that lists
-// every tile pair of every simulation using this instantiation.
-template <int MT, int MS, int PA>
-__global__ void __launch_bounds__(kWarps * 32, (n3_traits<MT, MS, PA>::MIN_BLOCKS))
-    k_b_pairs_n3(const od_simdesc* __restrict__ sims, const int4* __restrict__ items) {
-  extern __shared__ float sm[];
-  const int4 w = items[blockIdx.x];
-  const od_simdesc& d = sims[w.x];
+// Batched form: block k takes block items[k].y of member items[k].x; the table lists every block of
+// every member using this form.
+template <int MT, int MS, int SPLIT, bool FOLD>
+__global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_BLOCKS))
+    k_b_pairs_n3(const od_simdesc* __restrict__ sims, const int2* __restrict__ items) {
+  __shared__ float sm[FOLD ? kSliceWarps * 6 * slice_traits<MT, MS>::GT : 1];
+  const int2 it = items[blockIdx.x];
+  const od_simdesc& d = sims[it.x];
   if (!od_evaluates(d.dp->force_every, d.ds->step)) return;  // force interval: no evaluation
-  n3_tile_pair<MT, MS, PA, 0, false>(d.b.sx, d.b.sy, d.b.sz, d.Npad, d.b.n3, (size_t)d.Npad,
-                                     n3_cut{d.rho0, 0.f, 0.f, 0.f}, w.y, w.z, sm);
+  const int w = threadIdx.x >> 5;
+  n3_slice<MT, MS, SPLIT, FOLD>(d.b.sx, d.b.sy, d.b.sz, d.Npad, d.b.n3, d.rho0,
+                                (long long)it.y * kSliceWarps + w, d.n3,
+                                sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT + (threadIdx.x & 31)
+                                           : 0));
 }
 
 // Accumulators -> slab 0 of (ph, pl) as two-float sums, and cleared for the next evaluation.
@@ -78,90 +250,72 @@ __global__ void k_n3_take(unsigned long long* __restrict__ acc, int Npad, float4
   pl[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
 }
 
-// Batched form: block k covers 256 ions of the simulation in blk[k] (those using variant 7).
-__global__ void k_b_n3_take(const od_simdesc* __restrict__ sims, const int2* __restrict__ blk) {
-  const int2 e = blk[blockIdx.x];
-  const od_simdesc& d = sims[e.x];
-  if (!od_evaluates(d.dp->force_every, d.ds->step)) return;
-  const int i = e.y * 256 + threadIdx.x;
-  if (i >= d.Npad) return;
-  float3 hi, lo;
-  od_fix_take(d.b.n3 + i, (size_t)d.Npad, hi, lo);
-  d.b.part_hi[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
-  d.b.part_lo[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
-}
-
-template <int MT, int MS, int PA>
-cudaError_t launch_n3(const od_pair_io& io, int Npad, unsigned long long* acc, float4* ph,
-                      float4* pl, float rho0, cudaStream_t s, bool take) {
-  using TR = n3_traits<MT, MS, PA>;
-  const int nT = (Npad + TR::T - 1) / TR::T;
-  const long long nblk = (long long)nT * (nT + 1) / 2;
-  k_pairs_n3<MT, MS, PA><<<(unsigned)nblk, kWarps * 32, TR::SMEM, s>>>(io.sx, io.sy, io.sz, Npad,
-                                                                      acc, rho0);
-  if (take) k_n3_take<<<(Npad + 255) / 256, 256, 0, s>>>(acc, Npad, ph, pl);
-  return cudaGetLastError();
-}
-
-template <int MT, int MS, int PA>
-cudaError_t prepare_n3() {
-  const int smem = (int)n3_traits<MT, MS, PA>::SMEM;
-  cudaError_t e = cudaFuncSetAttribute(k_pairs_n3<MT, MS, PA>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_b_pairs_n3<MT, MS, PA>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+template <int MT, int MS, int SPLIT, bool FOLD>
+void launch_n3(const od_pair_io& io, int Npad, float rho0, const od_n3_split& sp, cudaStream_t s) {
+  k_pairs_n3<MT, MS, SPLIT, FOLD><<<(unsigned)od_n3_blocks(sp), kSliceWarps * 32, 0, s>>>(
+      io.sx, io.sy, io.sz, Npad, io.n3, rho0, sp);
 }
 
 }  // namespace
 
-
-// (plan ipt, tile) -> instantiation: ipt 2 and 4 take as many sources as targets per lane,
-// ipt 8 takes 8 targets and 2 sources per lane.
-#define OD_N3_CASES(CALL)                                                  \
-  case 20512: return CALL(2, 2, 1);                                        \
-  case 21024: return CALL(2, 2, 2); case 22048: return CALL(2, 2, 4);      \
-  case 24096: return CALL(2, 2, 8); case 41024: return CALL(4, 4, 1);      \
-  case 42048: return CALL(4, 4, 2); case 44096: return CALL(4, 4, 4);      \
-  case 82048: return CALL(8, 2, 1); case 84096: return CALL(8, 2, 2);
-
 bool od_n3_supported(int ipt, int tile) {
-#define OD_N3_YES(a, b, c) true
-  switch (ipt * 10000 + tile) { OD_N3_CASES(OD_N3_YES) }
-#undef OD_N3_YES
+  switch (ipt * 10000 + tile) {
+    case 20512: case 21024: case 22048: case 24096: case 41024: case 42048: case 44096:
+    case 82048: case 84096:
+      return true;
+  }
   return false;
 }
 
-cudaError_t od_n3_prepare(const od_pair_plan& pl) {
-#define OD_N3_PREP(a, b, c) prepare_n3<a, b, c>()
-  switch (pl.ipt * 10000 + pl.tile) { OD_N3_CASES(OD_N3_PREP) }
-#undef OD_N3_PREP
-  return cudaErrorInvalidValue;
+long long od_n3_blocks(const od_n3_split& sp) { return (sp.units + kSliceWarps - 1) / kSliceWarps; }
+
+// Work split of (ipt targets per lane, tile) for Npad ions, the same on every GPU so that results
+// do not depend on the device.
+//   * 4 x 4: one group pair (128 x 128 ions, 512 pair terms per lane) per warp. 50021 ions 0.838 ms,
+//     against 0.848 and 0.859 with 4 and 8 per warp (a longer last wave; the flush of the target
+//     sums that longer slices save is small). Below 12288 ions the group pairs leave warp slots
+//     empty (3040 on 152 SMs; 4656 group pairs at 12000) and a single warp's dependency chain sets
+//     the time, so they are split by lane steps: 8192 ions 32.8 us in 2 parts (36.9 whole, 34.0 in
+//     4), 4096 and below in 4 (2048 ions 8.2 against 16.4 us whole).
+//   * 8 x 2 (256 x 64 ions) and 2 x 2: a tile names how many group pairs a slice may hold (tile / 64),
+//     at least 16 slices per resident warp. 8 x 2 at 2^18 ions: 21.6 ms with 8 or 16, 22.3 with 1.
+od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
+  const long long GT = 32 * ipt, GS = ipt == 8 ? 64 : GT, R = GT / GS, NG = Npad / GT, NS = Npad / GS;
+  od_n3_split sp{};
+  sp.pairs = NG * NS - R * (NG * (NG - 1) / 2);
+  sp.split = 1;
+  long long L = 1;
+  if (ipt == 4) {
+    if (Npad <= 12288) sp.split = Npad <= 4096 ? 4 : 2;
+  } else {
+    const long long warps = 152ll * kSliceWarps * (ipt == 8 ? 4 : 8);
+    L = std::max(1ll, std::min<long long>(tile / 64, sp.pairs / (warps * 16)));
+  }
+  while (sp.pairs / L / kSliceWarps >= 0x7fffffff) L *= 2;  // the grid holds 2^31 - 1 blocks
+  sp.L = (int)L;
+  sp.units = sp.split > 1 ? sp.pairs * sp.split : (sp.pairs + L - 1) / L;
+  return sp;
 }
 
 cudaError_t od_launch_pairs_n3(const od_pair_plan& pl, const od_pair_io& io, int Npad, float4* ph,
                                float4* plo, float rho0, cudaStream_t s, bool take) {
-  if (!io.n3) return cudaErrorInvalidValue;
-#define OD_N3_LAUNCH(a, b, c) launch_n3<a, b, c>(io, Npad, io.n3, ph, plo, rho0, s, take)
-  switch (pl.ipt * 10000 + pl.tile) { OD_N3_CASES(OD_N3_LAUNCH) }
-#undef OD_N3_LAUNCH
-  return cudaErrorInvalidValue;
+  if (!io.n3 || !od_n3_supported(pl.ipt, pl.tile)) return cudaErrorInvalidValue;
+  const od_n3_split sp = od_n3_split_of(Npad, pl.ipt, pl.tile);
+  if (pl.ipt == 2) launch_n3<2, 2, 1, true>(io, Npad, rho0, sp, s);
+  else if (pl.ipt == 8) launch_n3<8, 2, 1, true>(io, Npad, rho0, sp, s);
+  else if (sp.split == 4) launch_n3<4, 4, 4, false>(io, Npad, rho0, sp, s);
+  else if (sp.split == 2) launch_n3<4, 4, 2, false>(io, Npad, rho0, sp, s);
+  else if (sp.L > 1) launch_n3<4, 4, 1, true>(io, Npad, rho0, sp, s);
+  else launch_n3<4, 4, 1, false>(io, Npad, rho0, sp, s);
+  if (take) k_n3_take<<<(Npad + 255) / 256, 256, 0, s>>>(io.n3, Npad, ph, plo);
+  return cudaGetLastError();
 }
 
 int od_n3_default(int Npad, size_t budget_bytes, int* ipt) {
-  // 2 x 2 with 512-ion tiles up to 2^15 ions (2.04e12 pair terms/s at 2^14 against 1.77e12 for
-  // the directed-pair kernel and 1.70e12 for 4 x 4 with 1024-ion tiles, which leave SMs idle:
-  // 136 tile pairs; 2.50e12 at 2^15 against 2.39e12), 4 x 4 with 1024-ion tiles up to 2^16
-  // (2.93e12 against 2.62e12 for 2 x 2 and 2.51e12 for 8 x 2), then 8 x 2 with 2048-ion tiles
-  // (2.91e12 at 2^17, 2.99e12 at 2^18, 3.05e12 at 2^20), then 4 x 4 with 4096-ion tiles: the
-  // first whose accumulators fit the budget (always: 24 bytes per ion)
-  const int cand[4][2] = {{2, 512}, {4, 1024}, {8, 2048}, {4, 4096}};
-  for (int c = Npad <= (1 << 15) ? 0 : (Npad <= (1 << 16) ? 1 : 2); c < 4; c++)
-    if (sizeof(float) * od_n3_floats(Npad, cand[c][1]) <= budget_bytes) {
-      *ipt = cand[c][0];
-      return cand[c][1];
-    }
-  return 0;
+  // 4 x 4 up to 2^16 ions, 8 x 2 above: 100000 ions 3.33 and 3.22 ms, 50021 ions 0.838 and 0.824 ms,
+  // 16384 ions 0.100 and 0.102 ms (the accumulators fit any budget that holds the ions: 24 bytes
+  // per ion)
+  return od_n3_batch_plan(Npad, budget_bytes, ipt);
 }
 
 size_t od_n3_floats(int Npad, int T) {
@@ -170,23 +324,29 @@ size_t od_n3_floats(int Npad, int T) {
   return 6 * (size_t)Npad;
 }
 
+int od_n3_form(int ipt, const od_n3_split& sp) {
+  if (ipt == 8) return 3;
+  return sp.split == 4 ? 2 : (sp.split == 2 ? 1 : (sp.L > 1 ? 4 : 0));
+}
+
 cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, cudaStream_t s) {
-  // the two instantiations batch members use (od_n3_batch_plan)
-  if (v.n3_nitems[0] > 0)
-    k_b_pairs_n3<4, 4, 1><<<v.n3_nitems[0], kWarps * 32, n3_traits<4, 4, 1>::SMEM, s>>>(
-        v.sims, v.n3_items[0]);
-  if (v.n3_nitems[1] > 0)
-    k_b_pairs_n3<8, 2, 1><<<v.n3_nitems[1], kWarps * 32, n3_traits<8, 2, 1>::SMEM, s>>>(
-        v.sims, v.n3_items[1]);
-  if (v.n3_nblk > 0) k_b_n3_take<<<v.n3_nblk, 256, 0, s>>>(v.sims, v.n3_blk);
+  // the forms batch members use (od_n3_batch_plan, od_n3_form)
+#define OD_B_N3(f, MT, MS, SPLIT, FOLD)                                                      \
+  if (v.n3_nitems[f] > 0)                                                                    \
+  k_b_pairs_n3<MT, MS, SPLIT, FOLD><<<v.n3_nitems[f], kSliceWarps * 32, 0, s>>>(v.sims,      \
+                                                                                v.n3_items[f])
+  OD_B_N3(3, 8, 2, 1, true);
+  OD_B_N3(0, 4, 4, 1, false);
+  OD_B_N3(1, 4, 4, 2, false);
+  OD_B_N3(2, 4, 4, 4, false);
+  OD_B_N3(4, 4, 4, 1, true);
+#undef OD_B_N3
   return cudaGetLastError();
 }
 
 int od_n3_batch_plan(int Npad, size_t budget_bytes, int* ipt) {
-  // batch members: 4 x 4 with 1024-ion tiles up to 2^16 ions (also below 2^15, where the tile
-  // pairs of the other members fill the GPU), 8 x 2 with 2048-ion tiles above, as a member
-  // stepped alone; 0 when the matrix does not fit (the member then takes the directed-pair
-  // kernel)
+  // batch members: 4 x 4 ions per lane up to 2^16 ions, 8 x 2 above; 0 when the accumulators do not
+  // fit (the member then takes the directed-pair kernel)
   const int T = Npad <= (1 << 16) ? 1024 : 2048;
   if (sizeof(float) * od_n3_floats(Npad, T) > budget_bytes) return 0;
   *ipt = T == 1024 ? 4 : 8;
