@@ -286,11 +286,10 @@ od_status od_set_graph(od_handle* h, int32_t enable);
  * blocks. od_create selects variant 7.
  * jsplit <= 0 picks the source split from the SM count. Takes effect at the next step.
  * Cutoff method (force_method OD_FORCE_CUTOFF): variant 0 or 2 walks a stencil of cells per
- * target cell (scalar or packed); variant 3 (the default) sorts
- * the ions along a Hilbert curve and evaluates each pair inside the cutoff once over tile
- * pairs whose bounding boxes come within it — targets_per_thread 2 with 512-ion tiles
- * (balanced group-pair lists) or 4 with 1024-ion tiles; a positive jsplit must name that tile
- * size; 24 bytes of accumulators per ion slot. */
+ * target cell (scalar or packed); variant 3 (the default) sorts the ions along a Hilbert curve and
+ * evaluates each pair inside the cutoff once over pairs of 32-ion blocks whose bounding boxes come
+ * within it — targets_per_thread 2 pads the sorted slots to a multiple of 512, 4 to one of 1024 (a
+ * positive jsplit must name that number); 24 bytes of accumulators per slot. */
 od_status od_set_pair_plan(od_handle* h, int32_t threads, int32_t targets_per_thread,
                            int32_t variant, int32_t jsplit);
 /* Autotuner: times every supported (threads, targets_per_thread, variant) and three source

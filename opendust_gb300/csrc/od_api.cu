@@ -372,9 +372,8 @@ static void fill_params(const od_config* c, int N, int Npad, od_dparams* p) {
 // 8 x 2); its sums go to 24 bytes of fixed-point accumulators per ion, so it always fits (the
 // budget below only bounds the rule).
 static constexpr size_t OD_N3_BUDGET = (size_t)32 << 30;
-// The cutoff's tile-pair path (variant 3: 512-ion tiles with balanced group-pair lists) needs its
-// sort, boxes, tile-pair list and slot accumulators (0.3 GB at 2^20 ions); the budget bounds the
-// tile-pair list for very large N, beyond which 1024-ion tiles or the cell stencil take over.
+// The cutoff's sorted path (variant 3) needs its sort, boxes and slot accumulators (45 bytes per
+// ion); beyond the budget the cell stencil takes over.
 static constexpr size_t OD_CUTN3_BUDGET = (size_t)64 << 30;
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile);
 
@@ -1014,19 +1013,18 @@ static void free_cutn3(od_handle* h) {
   od_cutn3* L = h->cut.n3;
   if (!L) return;
   void* ptrs[] = {L->cell_of, L->count, L->fill, L->start, L->perm, L->xs, L->ys, L->zs,
-                  L->box, L->gbox, L->adj, L->rowptr, L->pairs, L->acc};
+                  L->tbox, L->bbox, L->next, L->acc};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete L;
   h->cut.n3 = nullptr;
 }
 
-// Cutoff variant 3: Hilbert-sorted tiles of T ions (ipt 4: 1024, ipt 2: 512) and the per-slot
+// Cutoff variant 3: Hilbert-sorted slots, padded to a multiple of T (ipt 4: 1024, ipt 2: 512), and the per-slot
 // fixed-point accumulators (24 bytes per slot).
 static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
   free_cutn3(h);
   OD_CK(h, cudaSetDevice(h->device));
-  OD_CK(h, od_cutn3_prepare(ipt, T));
   od_cutn3* L = new (std::nothrow) od_cutn3();
   if (!L) return fail(h, OD_ERR_OOM, "host allocation");
   h->cut.n3 = L;
@@ -1043,12 +1041,10 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
   L->inv_s = (float)(G / g.side);
   L->T = T; L->ipt = ipt;
   L->rc_d = h->cfg.cutoff / h->cfg.r_D_e;
-  L->nT = (N + T - 1) / T;
-  L->nslots = L->nT * T;
-  L->nwords = (L->nT + 31) / 32;
-  L->grid = od_num_sms(h->device) * od_cutn3_blocks_per_sm(ipt, T, false);
-  L->grid_hard = od_num_sms(h->device) * od_cutn3_blocks_per_sm(ipt, T, true);
-  const size_t nT = L->nT, ns = L->nslots, nc = L->ncells;
+  L->nslots = (N + T - 1) / T * T;
+  L->grid = od_num_sms(h->device) * od_cutn3_blocks_per_sm(false);
+  L->grid_hard = od_num_sms(h->device) * od_cutn3_blocks_per_sm(true);
+  const size_t ns = L->nslots, nc = L->ncells;
   auto al = [&](auto** p, size_t n) {
     return cudaMalloc((void**)p, sizeof(**p) * std::max<size_t>(n, 1));
   };
@@ -1060,27 +1056,15 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
   if (e == cudaSuccess) e = al(&L->xs, ns);
   if (e == cudaSuccess) e = al(&L->ys, ns);
   if (e == cudaSuccess) e = al(&L->zs, ns);
-  if (e == cudaSuccess) e = al(&L->box, nT * 6);
-  if (e == cudaSuccess) e = al(&L->gbox, (ns / 64) * 6);
-  if (e == cudaSuccess) e = al(&L->adj, nT * L->nwords);
-  if (e == cudaSuccess) e = al(&L->rowptr, nT + 1);
-  if (e == cudaSuccess) e = al(&L->pairs, nT * (nT + 1) / 2);
+  if (e == cudaSuccess) e = al(&L->tbox, ns / 512 * 2);
+  if (e == cudaSuccess) e = al(&L->bbox, ns / 32 * 2);
+  if (e == cudaSuccess) e = al(&L->next, 1);
   if (e == cudaSuccess) e = al(&L->acc, 3 * ns);
   if (e == cudaSuccess) e = cudaMemset(L->acc, 0, sizeof(unsigned long long) * 3 * ns);
   if (e != cudaSuccess) {
     cudaGetLastError();
     free_cutn3(h);
     return fail(h, OD_ERR_OOM, "no device memory for the tile-pair cutoff");
-  }
-  // tail slots: far-away sentinels that no ion owns
-  if (ns > (size_t)N) {
-    std::vector<float> sent(ns - N, OD_SENTINEL);
-    std::vector<int32_t> none(ns - N, -1);
-    OD_CK(h, cudaMemcpy(L->xs + N, sent.data(), sizeof(float) * (ns - N), cudaMemcpyHostToDevice));
-    OD_CK(h, cudaMemcpy(L->ys + N, sent.data(), sizeof(float) * (ns - N), cudaMemcpyHostToDevice));
-    OD_CK(h, cudaMemcpy(L->zs + N, sent.data(), sizeof(float) * (ns - N), cudaMemcpyHostToDevice));
-    OD_CK(h, cudaMemcpy(L->perm + N, none.data(), sizeof(int32_t) * (ns - N),
-                        cudaMemcpyHostToDevice));
   }
   return OD_OK;
 }

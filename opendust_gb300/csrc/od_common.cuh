@@ -161,7 +161,9 @@ __device__ __forceinline__ od_u64 mul2(od_u64 a, od_u64 b) {
   od_u64 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d;
 }
 
-
+__device__ __forceinline__ od_u64 shfl64(od_u64 v, int src) {
+  return __shfl_sync(0xffffffffu, v, src);
+}
 __device__ __forceinline__ float sum2(od_u64 v) {
   const float2 f = up2(v);
   return f.x + f.y;

@@ -1,21 +1,37 @@
-// od_cutn3.cu — ion–ion forces within a cutoff over tile pairs (cutoff variant 3): ions sorted
-// along a Hilbert curve of a cell grid, 512- or 1024-ion tiles of consecutive sorted ions, the tile
-// pairs whose bounding boxes come within the cutoff listed, each unordered pair inside the cutoff
-// evaluated once (od_n3_pair.cuh) with 64-ion group pairs beyond it skipped, and the sums added
-// as 64-bit fixed point with integer atomics (per-ion words in shared memory, then per-slot
-// accumulators). Every result bit is independent of scheduling.
+// od_cutn3.cu — ion–ion forces within a cutoff (cutoff variant 3): ions sorted along a Hilbert curve
+// of a cell grid, blocks of 32 consecutive sorted ions with their bounding boxes, each unordered
+// pair inside the cutoff evaluated once, and the sums added as 64-bit fixed point with integer
+// atomics to per-slot accumulators. Every result bit is independent of scheduling.
+//
+// A warp works alone: it takes a source group of 64 slots (two blocks) and a run of 512-slot tiles
+// at or above it, lists the target blocks of those tiles whose boxes come within the cutoff
+// (tile boxes first, then block boxes, one lane per box and a ballot), and evaluates them four
+// blocks at a time: 4 targets and 2 sources per lane, the sources rotating around the warp as in
+// the all-pairs kernel (od_n3.cu). Blocks wholly inside the switching radius (hard cutoff: the
+// cutoff) take the plain screened term, the others the switched one.
+//
+// What bounds it: as the all-pairs kernel, operand fetch of the packed FP32 pipe (17 packed
+// operations per pair of pairs for the plain term, 27 with switching), plus the pairs of the
+// listed blocks that lie beyond the cutoff. field_chain (2^19 ions, 2 lambda): 1.63 pairs
+// evaluated per pair inside, 22.7 ms per evaluation. The tile-pair form this replaces (512-ion
+// tile pairs, 64 x 64 group lists built by one warp between two block barriers, 2 x 2 ions per
+// lane, sums in shared memory with compare-and-swap atomics) took 32.2 ms there; 65536 ions in
+// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.82 ms, 20011 ions at 2 lambda 0.197 -> 0.120 ms.
 #include "od_hilbert.h"
-#include "od_n3_pair.cuh"
+#include "od_internal.h"
+#include <algorithm>
+#include <cmath>
 
 namespace {
 
-// ------------------------------------------------------------------ cutoff over tile pairs
 // Cell grid of G^3 cells over the cube [lo, lo + G/inv_s)^3; a cell's key is its index along
 // a Hilbert curve (od_hilbert.h), so that the ions sorted by key fill tiles and 64-ion groups
-// with compact bounding boxes: at 2^19 ions in the 3 x 6 lambda cylinder the group boxes keep
-// 1.73x the pairs inside a 2 lambda cutoff, against 1.94x in Morton order.
-__global__ void k_mc_clear(int ncells, int32_t* __restrict__ count, int32_t* __restrict__ fill) {
+// with compact bounding boxes: at 2^19 ions in the 3 x 6 lambda cylinder the boxes of 64-ion
+// groups keep 1.73x the pairs inside a 2 lambda cutoff, against 1.94x in Morton order.
+__global__ void k_mc_clear(int ncells, int32_t* __restrict__ count, int32_t* __restrict__ fill,
+                           unsigned long long* __restrict__ next) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0) *next = 0ull;  // the pair kernel's work counter
   if (c < ncells) { count[c] = 0; fill[c] = 0; }
 }
 
@@ -125,319 +141,361 @@ __global__ void __launch_bounds__(128) k_mc_sort(const int32_t* __restrict__ cou
   }
 }
 
-// bounding boxes of every 64-slot group of tile t (real ions only; a group without ions gets
-// an inverted box that is never within range) and of the tile itself
-__global__ void __launch_bounds__(256) k_tile_box(int n, int T, const float* __restrict__ xs,
-                                                  const float* __restrict__ ys,
-                                                  const float* __restrict__ zs,
-                                                  float* __restrict__ gbox, float* __restrict__ box) {
-  __shared__ float tb[8][6];
+// Bounding boxes of the 16 blocks of every 512-slot tile and of the tile itself: (min x, min y,
+// min z, max x) and (max y, max z, -, -). Real ions only: a block without ions gets an inverted
+// box that is never within range. Slots past the ions become far-away sentinels that no ion owns.
+constexpr int kTile = 512, kBlk = 32, kTB = kTile / kBlk;
+__global__ void __launch_bounds__(kTile) k_tile_box(int n, float* __restrict__ xs,
+                                                    float* __restrict__ ys, float* __restrict__ zs,
+                                                    int32_t* __restrict__ perm,
+                                                    float4* __restrict__ bbox,
+                                                    float4* __restrict__ tbox) {
+  __shared__ float tb[kTB][6];
   const int t = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  float um[6] = {3e38f, 3e38f, 3e38f, -3e38f, -3e38f, -3e38f};  // this warp's union
-  for (int g = w; g < T / 64; g += 8) {
-    float mn[3] = {3e38f, 3e38f, 3e38f}, mx[3] = {-3e38f, -3e38f, -3e38f};
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int i = t * T + g * 64 + h * 32 + lane;
-      if (i < n) {
-        const float v[3] = {xs[i], ys[i], zs[i]};
-#pragma unroll
-        for (int d = 0; d < 3; d++) { mn[d] = fminf(mn[d], v[d]); mx[d] = fmaxf(mx[d], v[d]); }
-      }
-    }
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        mn[d] = fminf(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-        mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-      }
-    if (lane < 6) gbox[((size_t)t * (T / 64) + g) * 6 + lane] = lane < 3 ? mn[lane] : mx[lane - 3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) { um[d] = fminf(um[d], mn[d]); um[3 + d] = fmaxf(um[3 + d], mx[d]); }
+  const int i = t * kTile + threadIdx.x;
+  float b[6] = {3e38f, 3e38f, 3e38f, -3e38f, -3e38f, -3e38f};
+  if (i < n) {
+    b[0] = b[3] = xs[i]; b[1] = b[4] = ys[i]; b[2] = b[5] = zs[i];
+  } else {
+    xs[i] = ys[i] = zs[i] = OD_SENTINEL;
+    perm[i] = -1;
   }
-  if (lane == 0)
-    for (int d = 0; d < 6; d++) tb[w][d] = um[d];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      b[d] = fminf(b[d], __shfl_xor_sync(0xffffffffu, b[d], o));
+      b[3 + d] = fmaxf(b[3 + d], __shfl_xor_sync(0xffffffffu, b[3 + d], o));
+    }
+  if (lane == 0) {
+    bbox[2 * (t * kTB + w)] = make_float4(b[0], b[1], b[2], b[3]);
+    bbox[2 * (t * kTB + w) + 1] = make_float4(b[4], b[5], 0.f, 0.f);
+#pragma unroll
+    for (int d = 0; d < 6; d++) tb[w][d] = b[d];
+  }
   __syncthreads();
   if (threadIdx.x < 6) {
     float v = tb[0][threadIdx.x];
-    for (int k = 1; k < 8; k++)
+    for (int k = 1; k < kTB; k++)
       v = threadIdx.x < 3 ? fminf(v, tb[k][threadIdx.x]) : fmaxf(v, tb[k][threadIdx.x]);
-    box[t * 6 + threadIdx.x] = v;
+    reinterpret_cast<float*>(tbox + 2 * t)[threadIdx.x] = v;
   }
 }
 
-// row a of the tile-pair bitmap: b >= a whose box comes within the cutoff (box distance in
-// FP32 with a relative margin of 1e-5, so that no pair inside r_c is dropped by rounding)
-__global__ void __launch_bounds__(128) k_tile_adj(int nT, int nwords, const float* __restrict__ box,
-                                                  float rc2m, uint32_t* __restrict__ adj,
-                                                  int32_t* __restrict__ rowcnt) {
-  __shared__ int s_cnt;
-  const int a = blockIdx.x;
-  uint32_t* row = adj + (size_t)a * nwords;
-  for (int w = threadIdx.x; w < nwords; w += 128) row[w] = 0u;
-  if (threadIdx.x == 0) s_cnt = 0;
-  __syncthreads();
-  const float* A = box + a * 6;
-  int cnt = 0;
-  for (int b = a + threadIdx.x; b < nT; b += 128) {
-    const float* B = box + b * 6;
-    float d2 = 0.f;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      const float g = fmaxf(fmaxf(B[d] - A[3 + d], A[d] - B[3 + d]), 0.f);
-      d2 = fmaf(g, g, d2);
-    }
-    if (d2 < rc2m) { atomicOr(&row[b >> 5], 1u << (b & 31)); cnt++; }
-  }
-  atomicAdd(&s_cnt, cnt);
-  __syncthreads();
-  if (threadIdx.x == 0) rowcnt[a] = s_cnt;
-}
-
-// listed pairs of row a in increasing b (one thread per row: at most nT bits)
-__global__ void k_tile_list(int nT, int nwords, const uint32_t* __restrict__ adj,
-                            const int32_t* __restrict__ rowptr, int2* __restrict__ pairs) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= nT) return;
-  const uint32_t* row = adj + (size_t)a * nwords;
-  int k = rowptr[a];
-  for (int w = a >> 5; w < nwords; w++) {
-    uint32_t bits = row[w];
-    while (bits) {
-      const int j = __ffs(bits) - 1;
-      bits &= bits - 1;
-      pairs[k++] = make_int2(a, w * 32 + j);
-    }
-  }
-}
-
-// Balanced tile pair of the cutoff path: 512-ion tiles, NBT target groups of GT = 32·MT ions
-// and NBS source groups of GS = 32·MS ions per tile (MT targets and MS sources per lane). The
-// group pairs whose boxes come within the cutoff form a list in (target group, source group)
-// order, and warp w takes the contiguous slice [w·n/8, (w+1)·n/8) of it, so that the warps
-// evaluate the same number of group pairs (± 1) whatever the culling left and no barrier
-// separates them. Every listed group pair adds its FP32 target and reaction sums, converted to
-// 64-bit fixed point (od_fix), into per-ion words in shared memory with integer atomics, so
-// the block's sums do not depend on which warp ran what, or when; the block then adds each
-// ion's words to its global accumulators. A group pair whose farthest box distance is below the
-// switching radius (hard cutoff: the cutoff) is marked inner and takes the plain screened term:
-// the switching factor is exactly 1 for all its pairs.
-template <int MT, int MS>
-struct cut_traits {
-  static constexpr int GT = 32 * MT, GS = 32 * MS;    // target and source group sizes
-  static constexpr int T = 512;                       // ions per tile
-  static constexpr int NBT = T / GT, NBS = T / GS;    // groups per tile
-  static constexpr int NI = NBT * NBS;                // group pairs per tile pair (<= 64)
-  // [3][T] fixed-point words of tile a's ions and [3][T] of tile b's, then the list
-  static constexpr size_t SMEM = sizeof(unsigned long long) * 6 * T + 256;
+// ------------------------------------------------------------------ pair terms
+// CUT = 0: the plain screened term (blocks inside the switching radius); 1: OpenMM's switching
+// polynomial on the energy, S = (1-x)^3 (1 + 3x + 6x^2), x = (r - r_s)/(r_c - r_s) clamped to
+// [0, 1], so that pairs beyond r_c contribute exactly 0 (opendust.py:481-485); 2: hard cutoff.
+struct cut_args {
+  float rho0, rc2, rs, inv_w;
+  float in2;    // blocks closer than sqrt(in2) throughout take CUT = 0
+  float cull2;  // blocks farther than sqrt(cull2) are skipped
+  double rcd;   // hard cutoff: r_c (lambda) in FP64
 };
-
-// group pair (ga, gb) of a diagonal tile: 2 each pair once, 1 directed (the sources lie in the
-// target group), 0 skipped (counted from the other side)
-template <int GT, int GS>
-__device__ __forceinline__ int cut_diag_mode(int ga, int gb) {
-  const int t0 = ga * GT, s0 = gb * GS;
-  return s0 >= t0 + GT ? 2 : (s0 >= t0 ? 1 : 0);
+struct cut_consts {
+  od_u64 eps, rho, nl2e, one, three, six, w30, rc2;
+  float invw, nrsw, rc2f, skip2, band;
+};
+__device__ __forceinline__ cut_consts make_consts(const cut_args& c) {
+  cut_consts k;
+  k.eps = p2(1e-30f, 1e-30f);
+  k.rho = p2(c.rho0, c.rho0);
+  k.nl2e = p2(OD_NLOG2E, OD_NLOG2E);
+  k.one = p2(1.f, 1.f); k.three = p2(3.f, 3.f); k.six = p2(6.f, 6.f);
+  k.w30 = p2(30.f * c.inv_w, 30.f * c.inv_w);
+  k.rc2 = p2(c.rc2, c.rc2);
+  k.invw = c.inv_w;
+  k.nrsw = -c.rs * c.inv_w;
+  k.rc2f = c.rc2;
+  // (1 + 2e-5) rc^2: beyond it the clamped switching variable is 1 in FP32 and the switched term
+  // exactly zero (the hard cutoff is exactly zero from rc^2 on)
+  k.skip2 = c.rc2 * 1.00002f;
+  // the FP32 r^2 of a pair is within 4e-7 of its exact value on the same float positions
+  k.band = c.rc2 * 2e-6f;
+  return k;
+}
+__device__ __forceinline__ float fma_sat(float a, float b, float c) {
+  float r; asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r;
 }
 
-constexpr int kItem = 63, kInner = 128;  // list entry: group pair index | inner flag
-
-template <int MT, int MS, int CUT, bool COUNT>
-__device__ __forceinline__ unsigned int cut_tile_pair(const float* __restrict__ sx,
-                                                         const float* __restrict__ sy,
-                                                         const float* __restrict__ sz,
-                                                         unsigned long long* __restrict__ acc,
-                                                         size_t stride, const n3_consts& k, int a,
-                                                         int b, float* sm,
-                                                         const float* __restrict__ gbox,
-                                                         float cull2, float k_in2) {
-  using CT = cut_traits<MT, MS>;
-  constexpr int GT = CT::GT, GS = CT::GS, T = CT::T, NBT = CT::NBT, NBS = CT::NBS, NI = CT::NI;
-  constexpr int MS2 = MS / 2;
-  static_assert(NI % 32 == 0 && NI <= 64, "list of at most 64 group pairs");
-  // [3][T] fixed-point sums of tile a's ions, then [3][T] of tile b's (unused when a == b)
-  unsigned long long* const fa = reinterpret_cast<unsigned long long*>(sm);
-  unsigned long long* const fb = fa + 3 * T;
-  unsigned char* const items = reinterpret_cast<unsigned char*>(fb + 3 * T);  // ga·NBS + gb
-  int* const s_n = reinterpret_cast<int*>(items + 64);
-  const bool diag = a == b;
-  unsigned long long* const fs = diag ? fa : fb;  // where the reactions go
-  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, src = (lane + 1) & 31;
-
-  // 1. the list (warp 0): group pairs within range; on a diagonal tile the source groups
-  // inside a target group (directed) and those above it
-  if (w == 0) {
-    int n = 0;
-    for (int r = 0; r < NI / 32; r++) {
-      const int c = r * 32 + lane, ga = c / NBS, gb = c % NBS;
-      const int mode = diag ? cut_diag_mode<GT, GS>(ga, gb) : 2;
-      bool keep = mode == 1, inner = false;
-      if (mode != 0) {
-        float ta[6], tb[6];
-        group_box(gbox, (a * NBT + ga) * (GT / 64), GT / 64, ta);
-        group_box(gbox, (b * NBS + gb) * (GS / 64), GS / 64, tb);
-        float d2 = 0.f, f2 = 0.f;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-          const float gap = fmaxf(fmaxf(tb[d] - ta[3 + d], ta[d] - tb[3 + d]), 0.f);
-          const float far = fmaxf(tb[3 + d] - ta[d], ta[3 + d] - tb[d]);
-          d2 = fmaf(gap, gap, d2);
-          f2 = fmaf(far, far, f2);
-        }
-        if (mode == 2) keep = d2 < cull2;
-        inner = f2 < k_in2;
-      }
-      const unsigned int bal = __ballot_sync(0xffffffffu, keep);
-      const int pos = n + __popc(bal & ((1u << lane) - 1u));
-      if (keep) items[pos] = (unsigned char)(c | (inner ? kInner : 0));
-      n += __popc(bal);
-    }
-    if (lane == 0) *s_n = n;
-  }
-  __syncthreads();
-
-  // 2. this warp's slice of the list; sums into the shared fixed-point words
-  const int n = *s_n, i0 = (w * n) >> 3, i1 = ((w + 1) * n) >> 3;
-  unsigned int cnt = 0;
-  od_u64 X[MT], Y[MT], Z[MT];
-  int cur = -1;
-  for (int i = i0; i < i1; i++) {
-    const int c = items[i] & kItem, ga = c / NBS, gb = c % NBS;
-    const bool inner = (items[i] & kInner) != 0;
-    if (ga != cur) {
-#pragma unroll
-      for (int kt = 0; kt < MT; kt++) {
-        const int j = (a * NBT + ga) * GT + lane + 32 * kt;
-        const float x = sx[j], y = sy[j], z = sz[j];
-        X[kt] = p2(x, x); Y[kt] = p2(y, y); Z[kt] = p2(z, z);
-      }
-      cur = ga;
-    }
-    od_u64 QX[MS2], QY[MS2], QZ[MS2], RX[MS2], RY[MS2], RZ[MS2], AX[MT], AY[MT], AZ[MT];
-#pragma unroll
-    for (int q = 0; q < MS2; q++) {
-      const int j = (b * NBS + gb) * GS + lane + 64 * q;
-      QX[q] = p2(sx[j], sx[j + 32]);
-      QY[q] = p2(sy[j], sy[j + 32]);
-      QZ[q] = p2(sz[j], sz[j + 32]);
-      RX[q] = RY[q] = RZ[q] = 0ull;
-    }
-#pragma unroll
-    for (int kt = 0; kt < MT; kt++) AX[kt] = AY[kt] = AZ[kt] = 0ull;
-    const bool react = !(diag && cut_diag_mode<GT, GS>(ga, gb) == 1);
-    if (!react) {
-      if (inner)
-        n3_group<MT, MS, 0, false, COUNT>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src,
-                                          cnt);
-      else
-        n3_group<MT, MS, CUT, false, COUNT>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src,
-                                            cnt);
-    } else {
-      if (inner)
-        n3_group<MT, MS, 0, true, COUNT>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src,
-                                         cnt);
-      else
-        n3_group<MT, MS, CUT, true, COUNT>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src,
-                                           cnt);
-      // the force on the sources is minus the accumulated terms
-#pragma unroll
-      for (int q = 0; q < MS2; q++) {
-        const int e = gb * GS + lane + 64 * q;
-        const float2 rx = up2(RX[q]), ry = up2(RY[q]), rz = up2(RZ[q]);
-        atomicAdd(fs + e, od_fix(-rx.x, 0.f));
-        atomicAdd(fs + e + 32, od_fix(-rx.y, 0.f));
-        atomicAdd(fs + T + e, od_fix(-ry.x, 0.f));
-        atomicAdd(fs + T + e + 32, od_fix(-ry.y, 0.f));
-        atomicAdd(fs + 2 * T + e, od_fix(-rz.x, 0.f));
-        atomicAdd(fs + 2 * T + e + 32, od_fix(-rz.y, 0.f));
-      }
-    }
-#pragma unroll
-    for (int kt = 0; kt < MT; kt++) {
-      const int e = ga * GT + lane + 32 * kt;
-      atomicAdd(fa + e, od_fix(sum2(AX[kt]), 0.f));
-      atomicAdd(fa + T + e, od_fix(sum2(AY[kt]), 0.f));
-      atomicAdd(fa + 2 * T + e, od_fix(sum2(AZ[kt]), 0.f));
-    }
-  }
-  __syncthreads();
-
-  // 3. the block's words into the ions' global accumulators, and cleared for the next tile pair
-  for (int e = tid; e < T; e += kWarps * 32) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      const unsigned long long va = fa[c * T + e];
-      if (va) atomicAdd(acc + c * stride + (size_t)a * T + e, va);
-      fa[c * T + e] = 0ull;
-      if (!diag) {
-        const unsigned long long vb = fb[c * T + e];
-        if (vb) atomicAdd(acc + c * stride + (size_t)b * T + e, vb);
-        fb[c * T + e] = 0ull;
-      }
-    }
-  }
-  __syncthreads();  // the next tile pair rewrites the list and the words
-  return cnt;
+// Is the pair of float positions t, s inside the cutoff as the FP64 reference decides it:
+// sqrt((dx^2 + dy^2) + dz^2) < r_c with the differences taken exactly in FP64 and every
+// operation rounded once (the oracle's pair_factor).
+__device__ __noinline__ bool inside_exact(float tx, float ty, float tz, float sx, float sy,
+                                          float sz, double rcd) {
+  const double dx = __dsub_rn((double)tx, (double)sx), dy = __dsub_rn((double)ty, (double)sy),
+               dz = __dsub_rn((double)tz, (double)sz);
+  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+  return __dsqrt_rn(r2) < rcd;
 }
 
-// ions per tile of the staggered tile pair, or of the balanced list (BAL)
-template <bool BAL, int MT, int MS, int PA>
-struct cutn3_tile {
-  static constexpr int T = n3_traits<MT, MS, PA>::T;
-};
-template <int MT, int MS, int PA>
-struct cutn3_tile<true, MT, MS, PA> {
-  static constexpr int T = cut_traits<MT, MS>::T;
-};
-
-// every listed tile pair, each unordered ion pair once (static assignment: pair k to block
-// k mod grid), group pairs beyond the cutoff skipped. BAL: the balanced list routine above
-// (512-ion tiles); otherwise the staggered tile-pair routine.
-// blocks per SM the registers of the balanced tile pair are budgeted for. Measured on GB300 at
-// 2^19 ions (field_chain), ms per step: with switching 32.9 (4 blocks of at most 64 registers),
-// 34.2 (3 blocks), 35.8 with per-item slots in shared memory summed in a fixed order (74 KB per
-// block, 3 blocks); hard cutoff 30.6 (3 blocks), 31.6 (4 blocks: its exact-decision branch
-// spills at 64 registers), 31.9 with the slots.
-template <int CUT>
-struct cut_blocks {
-  static constexpr int value = CUT == 2 ? 3 : 4;
-};
-
-template <int MT, int MS, int PA, int CUT, bool COUNT, bool BAL>
-__global__ void __launch_bounds__(kWarps * 32, (BAL ? cut_blocks<CUT>::value
-                                                                : n3_traits<MT, MS, PA>::MIN_BLOCKS))
-    k_pairs_cutn3(const float* __restrict__ xs, const float* __restrict__ ys,
-                  const float* __restrict__ zs, int nslots, int nT,
-                  const int2* __restrict__ pairs, const int32_t* __restrict__ npairs,
-                  unsigned long long* __restrict__ acc, n3_cut cut,
-                  const float* __restrict__ gbox, float cull2,
-                  unsigned long long* __restrict__ pair_count) {
-  extern __shared__ float sm[];
-  static_assert(!BAL || PA == 1, "balanced list: one pass");
-  const int np = *npairs;
-  unsigned int cnt = 0;
-  if constexpr (BAL) {
-    const n3_consts kc = make_consts(cut);
-    unsigned long long* const f = reinterpret_cast<unsigned long long*>(sm);
-    for (int e = threadIdx.x; e < 6 * cut_traits<MT, MS>::T; e += kWarps * 32) f[e] = 0ull;
-    __syncthreads();
-    for (int k = blockIdx.x; k < np; k += gridDim.x) {
-      const int2 ab = pairs[k];
-      cnt += cut_tile_pair<MT, MS, CUT, COUNT>(xs, ys, zs, acc, (size_t)nslots, kc, ab.x,
-                                                  ab.y, sm, gbox, cull2, cut.in2);
-    }
+// One pack: a target (in both halves) against two sources, as od_n3.cu's pair_once with R = r and
+// W = 1/(r (r + rho)). Switching, with u = exp(-r)/s: c = exp(-r) W [(1 + 1/s) S + 30 x^2 (1-x)^2
+// /(r_c - r_s)] = exp(-r) W (1-x)^2 [(1 + W r)(1-x)(1 + 3x + 6x^2) + 30 x^2/(r_c - r_s)] (no
+// cancellation as x -> 1; x by a saturating fma, so that neither x nor 1 - x needs a clamp). A pack
+// whose 64 pairs all lie beyond the cutoff is skipped (a warp vote: 22.7 ms with it at field_chain,
+// 25.5 without; a second vote that skips the switching part where no pair needs it made the
+// kernel 5 % slower). Hard cutoff: pairs more than `band` inside count here, pairs within it are
+// left to the exact pass; near keeps the smallest |r^2 - r_c^2|. COUNT adds the pairs inside.
+template <int CUT, bool REACT, bool COUNT>
+__device__ __forceinline__ void cut_pair(const cut_consts& k, od_u64 X, od_u64 Y, od_u64 Z, od_u64 QX,
+                                         od_u64 QY, od_u64 QZ, od_u64& AX, od_u64& AY, od_u64& AZ,
+                                         od_u64& RX, od_u64& RY, od_u64& RZ, float& near,
+                                         unsigned int& cnt) {
+  const od_u64 DX = sub2(X, QX), DY = sub2(Y, QY), DZ = sub2(Z, QZ);
+  od_u64 R2 = fma2(DX, DX, k.eps);
+  R2 = fma2(DY, DY, R2);
+  R2 = fma2(DZ, DZ, R2);
+  const float2 r2 = up2(R2);
+  if (CUT != 0 && __all_sync(0xffffffffu, fminf(r2.x, r2.y) >= k.skip2)) return;
+  const od_u64 R = p2(od_sqrt(r2.x), od_sqrt(r2.y));
+  const float2 rs = up2(fma2(R, k.rho, R2));
+  const od_u64 W = p2(od_rcp(rs.x), od_rcp(rs.y));
+  const float2 ea = up2(mul2(R, k.nl2e));
+  const od_u64 EX = p2(od_ex2(ea.x), od_ex2(ea.y));
+  const od_u64 SI = mul2(W, R);
+  od_u64 C;
+  if (CUT == 0) {
+    C = mul2(EX, fma2(W, SI, W));
+  } else if (CUT == 1) {
+    const float2 r = up2(R);
+    const od_u64 x = p2(fma_sat(r.x, k.invw, k.nrsw), fma_sat(r.y, k.invw, k.nrsw));
+    const od_u64 om = sub2(k.one, x);
+    const od_u64 P = mul2(om, fma2(x, fma2(k.six, x, k.three), k.one));
+    const od_u64 V = fma2(mul2(x, x), k.w30, fma2(SI, P, P));
+    C = mul2(mul2(W, mul2(om, om)), mul2(EX, V));
   } else {
-    for (int k = blockIdx.x; k < np; k += gridDim.x) {
-      const int2 ab = pairs[k];
-      cnt += n3_tile_pair<MT, MS, PA, CUT, COUNT, true>(xs, ys, zs, nslots, acc, (size_t)nslots,
-                                                        cut, ab.x, ab.y, sm, gbox, cull2);
+    const float2 c = up2(mul2(EX, fma2(W, SI, W)));
+    const float2 e = up2(sub2(R2, k.rc2));
+    near = fminf(near, fminf(fabsf(e.x), fabsf(e.y)));
+    C = p2(e.x < -k.band ? c.x : 0.f, e.y < -k.band ? c.y : 0.f);
+  }
+  if (COUNT) {
+    const float lim = CUT == 2 ? -k.band : 0.f;
+    cnt += (REACT ? 2u : 1u) * ((unsigned)(r2.x - k.rc2f < lim && r2.x > 1e-29f) +
+                                (unsigned)(r2.y - k.rc2f < lim && r2.y > 1e-29f));
+  }
+  AX = fma2(C, DX, AX); AY = fma2(C, DY, AY); AZ = fma2(C, DZ, AZ);
+  if (REACT) { RX = fma2(C, DX, RX); RY = fma2(C, DY, RY); RZ = fma2(C, DZ, RZ); }
+}
+
+// Hard cutoff, the exact pass of a batch: pairs whose FP32 r^2 lies within `band` of r_c^2 are
+// decided as the FP64 reference decides them and added straight to the accumulators, so that both
+// include the same pairs (rare: about 1 batch in 25 at field_chain has such a pair).
+template <int MT, bool REACT, bool COUNT>
+__device__ __noinline__ void exact_pass(const float* __restrict__ xs, const float* __restrict__ ys,
+                                        const float* __restrict__ zs, size_t ns,
+                                        unsigned long long* __restrict__ acc, const cut_args& cut,
+                                        int sg, const unsigned int* tb, int nb, unsigned int& cnt) {
+  const int lane = threadIdx.x & 31;
+  const float band = cut.rc2 * 2e-6f;
+  for (int t = 0; t < nb; t++) {
+    const int ti = (int)tb[t] * kBlk + lane;
+    const float px = xs[ti], py = ys[ti], pz = zs[ti];
+    for (int j = 0; j < 64; j++) {
+      const int sj = sg * 64 + (j & 32) + ((lane + j) & 31);
+      const float sx = xs[sj], sy = ys[sj], sz = zs[sj];
+      const float dx = px - sx, dy = py - sy, dz = pz - sz;
+      const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
+      const float e = r2 - cut.rc2;
+      if (!(e < -band) && e <= band && inside_exact(px, py, pz, sx, sy, sz, cut.rcd)) {
+        const float c = od_pair_c(r2, cut.rho0);
+        od_fix_add1(acc + ti, c * dx); od_fix_add1(acc + ns + ti, c * dy);
+        od_fix_add1(acc + 2 * ns + ti, c * dz);
+        if (REACT) {
+          od_fix_add1(acc + sj, -c * dx); od_fix_add1(acc + ns + sj, -c * dy);
+          od_fix_add1(acc + 2 * ns + sj, -c * dz);
+        }
+        if (COUNT) cnt += REACT ? 2u : 1u;
+      }
+    }
+  }
+}
+
+// MT target blocks tb[0 .. nb) (nb <= MT, the rest empty) against the 64 slots of source group sg.
+// Reactions are summed in FP32 over 16 lane steps and added to the accumulators of the sources where
+// they stand (shorter chains than the 32 steps they could take: at 2^19 ions the median per-ion
+// error is 0.8 of that and the kernel 1 % slower).
+template <int MT, int CUT, bool REACT, bool COUNT, int UNROLL>
+__device__ __forceinline__ void cut_batch(const cut_consts& k, const float* __restrict__ xs,
+                                          const float* __restrict__ ys,
+                                          const float* __restrict__ zs, size_t ns,
+                                          unsigned long long* __restrict__ acc,
+                                          const cut_args& cut, int sg, const unsigned int* tb,
+                                          int nb, unsigned int& cnt) {
+  const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
+  od_u64 X[MT], Y[MT], Z[MT], AX[MT], AY[MT], AZ[MT];
+#pragma unroll
+  for (int t = 0; t < MT; t++) {
+    float x = OD_SENTINEL, y = OD_SENTINEL, z = OD_SENTINEL;
+    if (t < nb) {
+      const int i = (int)tb[t] * kBlk + lane;
+      x = xs[i]; y = ys[i]; z = zs[i];
+    }
+    X[t] = p2(x, x); Y[t] = p2(y, y); Z[t] = p2(z, z);
+    AX[t] = AY[t] = AZ[t] = 0ull;
+  }
+  const int j = sg * 64 + lane;
+  od_u64 QX = p2(xs[j], xs[j + 32]), QY = p2(ys[j], ys[j + 32]), QZ = p2(zs[j], zs[j + 32]);
+  float near = 3e38f;
+#pragma unroll 1
+  for (int part = 16; part <= 32; part += 16) {
+    od_u64 RX = 0ull, RY = 0ull, RZ = 0ull;
+#pragma unroll UNROLL
+    for (int st = 0; st < 16; st++) {
+#pragma unroll
+      for (int t = 0; t < MT; t++)
+        cut_pair<CUT, REACT, COUNT>(k, X[t], Y[t], Z[t], QX, QY, QZ, AX[t], AY[t], AZ[t], RX, RY,
+                                    RZ, near, cnt);
+      QX = shfl64(QX, src); QY = shfl64(QY, src); QZ = shfl64(QZ, src);
+      if (REACT) { RX = shfl64(RX, src); RY = shfl64(RY, src); RZ = shfl64(RZ, src); }
+    }
+    if (REACT) {  // the force on the sources is minus the accumulated terms
+      const float2 rx = up2(RX), ry = up2(RY), rz = up2(RZ);
+      unsigned long long* a = acc + sg * 64 + ((lane + part) & 31);
+      od_fix_add1(a, -rx.x); od_fix_add1(a + 32, -rx.y);
+      od_fix_add1(a + ns, -ry.x); od_fix_add1(a + ns + 32, -ry.y);
+      od_fix_add1(a + 2 * ns, -rz.x); od_fix_add1(a + 2 * ns + 32, -rz.y);
+    }
+  }
+  if (CUT == 2 && __any_sync(0xffffffffu, near <= k.band))
+    exact_pass<MT, REACT, COUNT>(xs, ys, zs, ns, acc, cut, sg, tb, nb, cnt);
+#pragma unroll
+  for (int t = 0; t < MT; t++)
+    if (t < nb) {
+      unsigned long long* a = acc + (int)tb[t] * kBlk + lane;
+      od_fix_add1(a, sum2(AX[t]));
+      od_fix_add1(a + ns, sum2(AY[t]));
+      od_fix_add1(a + 2 * ns, sum2(AZ[t]));
+    }
+}
+
+// squared nearest and farthest distance of a box from box a (min xyz, max xyz)
+__device__ __forceinline__ void box_dist(const float4* __restrict__ box, int i, const float (&a)[6],
+                                         float& d2, float& f2) {
+  const float4 u = box[2 * i], v = box[2 * i + 1];
+  const float lo[3] = {u.x, u.y, u.z}, hi[3] = {u.w, v.x, v.y};
+  d2 = 0.f;
+  f2 = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const float gap = fmaxf(fmaxf(lo[d] - a[3 + d], a[d] - hi[d]), 0.f);
+    const float far = fmaxf(hi[d] - a[d], a[3 + d] - lo[d]);
+    d2 = fmaf(gap, gap, d2);
+    f2 = fmaf(far, far, f2);
+  }
+}
+
+// Units: source group sg (row a = sg / 8) and its c-th run of B tiles from tile a on, numbered run by
+// run over the groups, c = 0 first. Units before run c: 8 (c nT - B c (c - 1) / 2).
+__host__ __device__ __forceinline__ long long units_before(long long c, int nT, int B) {
+  return 8 * (c * nT - B * (c * (c - 1) / 2));
+}
+
+// registers: warps per SM and unrolling. field_chain, ms per evaluation: switching 22.8 with 20 warps
+// and two steps, 22.7 with 24 and one or two, 24.5 with 16; 20011 ions 0.120, 0.130, 0.124; hard cutoff
+// 21.8 with 24 warps and one step, 22.6 with 20 and 23.4 with 16 (without the vote).
+template <int CUT>
+struct cut_traits {
+  static constexpr int WARPS = 4;  // per block; they share nothing
+  static constexpr int MIN_BLOCKS = CUT == 2 ? 6 : 5;
+  static constexpr int UNROLL = CUT == 2 ? 1 : 2;
+};
+
+template <int CUT, bool COUNT>
+__global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::MIN_BLOCKS)
+    k_pairs_cutn3(const float* __restrict__ xs, const float* __restrict__ ys,
+                  const float* __restrict__ zs, int nslots, int nT, int B, long long nunits,
+                  unsigned long long* __restrict__ next, unsigned long long* __restrict__ acc,
+                  const __grid_constant__ cut_args cut, const float4* __restrict__ tbox,
+                  const float4* __restrict__ bbox, unsigned long long* __restrict__ pair_count) {
+  constexpr int WARPS = cut_traits<CUT>::WARPS, UNROLL = cut_traits<CUT>::UNROLL;
+  // per warp: target blocks waiting, those that need the cutoff term and the inner ones (at most 3
+  // left over plus the 32 of one round)
+  __shared__ unsigned int s_list[WARPS][2][40];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  unsigned int* const qo = s_list[w][0];
+  unsigned int* const qi = s_list[w][1];
+  const cut_consts k = make_consts(cut);
+  unsigned int cnt = 0;
+  for (;;) {
+    unsigned long long u = 0;
+    if (lane == 0) u = atomicAdd(next, 1ull);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    if (u >= (unsigned long long)nunits) break;
+    int sg, b0, b1;
+    {
+      const float h = (float)nT + 0.5f * (float)B;
+      int c = (int)((h - sqrtf(fmaxf(h * h - 0.25f * (float)B * (float)u, 0.f))) / (float)B);
+      while (c > 0 && units_before(c, nT, B) > (long long)u) c--;
+      while (units_before(c + 1, nT, B) <= (long long)u) c++;
+      sg = (int)((long long)u - units_before(c, nT, B));
+      b0 = (sg >> 3) + c * B;
+      b1 = min(b0 + B, nT);
+    }
+    float sb[6];  // box of the source group
+    {
+      const float4 p = bbox[4 * sg], q = bbox[4 * sg + 1], r = bbox[4 * sg + 2], s = bbox[4 * sg + 3];
+      sb[0] = fminf(p.x, r.x); sb[1] = fminf(p.y, r.y); sb[2] = fminf(p.z, r.z);
+      sb[3] = fmaxf(p.w, r.w); sb[4] = fmaxf(q.x, s.x); sb[5] = fmaxf(q.y, s.y);
+    }
+    unsigned int tiles;
+    {
+      float d2 = 3e38f, f2;
+      if (b0 + lane < b1) box_dist(tbox, b0 + lane, sb, d2, f2);
+      tiles = __ballot_sync(0xffffffffu, d2 < cut.cull2);
+    }
+    if (b0 == sg >> 3) {  // the group itself: directed
+      if (lane < 2) qo[lane] = 2 * sg + lane;
+      __syncwarp();
+      cut_batch<2, CUT, false, COUNT, 1>(k, xs, ys, zs, nslots, acc, cut, sg, qo, 2, cnt);
+      __syncwarp();
+    }
+    int no = 0, ni = 0;
+    while (tiles) {
+      // two tiles a round: lanes 0-15 the blocks of the first, 16-31 of the second
+      const int t1 = __ffs(tiles) - 1;
+      tiles &= tiles - 1;
+      const int t2 = tiles ? __ffs(tiles) - 1 : -1;
+      if (tiles) tiles &= tiles - 1;
+      const int tl = lane < 16 ? t1 : t2;
+      const int blk = (b0 + tl) * kTB + (lane & 15);
+      float d2 = 3e38f, f2 = 3e38f;
+      if (tl >= 0 && blk > 2 * sg + 1) box_dist(bbox, blk, sb, d2, f2);
+      const bool keep = d2 < cut.cull2, inner = keep && f2 < cut.in2;
+      const unsigned int mi = __ballot_sync(0xffffffffu, inner),
+                         mo = __ballot_sync(0xffffffffu, keep && !inner);
+      const unsigned int below = (1u << lane) - 1u;
+      if (inner) qi[ni + __popc(mi & below)] = blk;
+      else if (keep) qo[no + __popc(mo & below)] = blk;
+      ni += __popc(mi);
+      no += __popc(mo);
+      __syncwarp();
+      const bool last = tiles == 0;
+      if (last) {  // the inner blocks that fill no batch join the others
+        const int r = ni & 3;
+        if (lane < r) qo[no + lane] = qi[ni - r + lane];
+        no += r;
+        ni -= r;
+        __syncwarp();
+      }
+      for (; ni >= 4; ni -= 4)
+        cut_batch<4, 0, true, COUNT, UNROLL>(k, xs, ys, zs, nslots, acc, cut, sg, qi + ni - 4, 4,
+                                             cnt);
+      for (; no >= 4; no -= 4)
+        cut_batch<4, CUT, true, COUNT, UNROLL>(k, xs, ys, zs, nslots, acc, cut, sg, qo + no - 4, 4,
+                                               cnt);
+      if (last && no > 2)
+        cut_batch<4, CUT, true, COUNT, UNROLL>(k, xs, ys, zs, nslots, acc, cut, sg, qo, no, cnt);
+      else if (last && no > 0)
+        cut_batch<2, CUT, true, COUNT, 1>(k, xs, ys, zs, nslots, acc, cut, sg, qo, no, cnt);
+      __syncwarp();
     }
   }
   if (COUNT) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(pair_count, (unsigned long long)cnt);
+    if (lane == 0 && cnt) atomicAdd(pair_count, (unsigned long long)cnt);
   }
 }
 
@@ -473,102 +531,61 @@ od_cgrid od_cutn3_grid(int N, double R, double H) {
 }
 
 size_t od_cutn3_bytes(int N, int T, int ncells) {
-  const size_t nT = (size_t)((N + T - 1) / T), ns = nT * T, nc = (size_t)ncells;
-  const size_t nw = (nT + 31) / 32;
-  return sizeof(unsigned long long) * 3 * ns                 // accumulators
-         + sizeof(int2) * nT * (nT + 1) / 2                   // pairs
-         + sizeof(uint32_t) * nT * nw                         // bitmap
-         + sizeof(float) * (3 * ns + 6 * nT + 6 * (ns / 64))  // sorted positions, boxes
-         + sizeof(int32_t) * (ns + N + 3 * nc + nT + 4);
-}
-
-// cutoff tile-pair shapes: (ipt, T) = (2, 512) the balanced list with 2 x 2 targets x sources
-// per lane, (4, 1024) the staggered tile pair with 4 x 4. Measured on GB300 at 2^19 ions
-// (field_chain), ms per step: 32.9 with (2, 512); the balanced list at 4 x 2 (128-ion target
-// groups: more arithmetic per shuffle, but coarser culling) 33.2 with 3 blocks per SM and 34.3
-// with 4 (it spills at 64 registers); the staggered (4, 1024) 55.7 in an earlier form.
-template <int MT, int MS, bool BAL>
-cudaError_t prepare_cutn3(int smem) {
-  void* fn[4] = {(void*)k_pairs_cutn3<MT, MS, 1, 1, false, BAL>,
-                 (void*)k_pairs_cutn3<MT, MS, 1, 1, true, BAL>,
-                 (void*)k_pairs_cutn3<MT, MS, 1, 2, false, BAL>,
-                 (void*)k_pairs_cutn3<MT, MS, 1, 2, true, BAL>};
-  for (int q = 0; q < 4; q++) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(fn[q], cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  const size_t ns = (size_t)((N + T - 1) / T) * T, nc = (size_t)ncells;
+  return sizeof(unsigned long long) * (3 * ns + 1)                    // accumulators, work counter
+         + sizeof(float4) * 2 * (ns / kBlk + ns / kTile)              // boxes
+         + sizeof(float) * 3 * ns                                     // sorted positions
+         + sizeof(int32_t) * (ns + N + 3 * nc + 1);
 }
 
 bool od_cutn3_supported(int ipt, int T) {
   return (ipt == 2 && T == 512) || (ipt == 4 && T == 1024);
 }
 
-// dynamic shared memory of the balanced tile pair
-constexpr size_t kCutBalSmem = cut_traits<2, 2>::SMEM;
-
-// resident blocks per SM of the production pair kernel (the persistent grid is this times the
-// SM count)
-int od_cutn3_blocks_per_sm(int ipt, int T, bool hard) {
+// resident blocks per SM of the pair kernel (the persistent grid is this times the SM count)
+int od_cutn3_blocks_per_sm(bool hard) {
   int nb = 0;
-  cudaError_t e = cudaErrorInvalidValue;
-  if (ipt == 2 && T == 512)
-    e = hard ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                   &nb, k_pairs_cutn3<2, 2, 1, 2, false, true>, kWarps * 32, kCutBalSmem)
-             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                   &nb, k_pairs_cutn3<2, 2, 1, 1, false, true>, kWarps * 32, kCutBalSmem);
-  else if (ipt == 4 && T == 1024)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_cutn3<4, 4, 1, 1, false, false>,
-                                                      kWarps * 32, n3_traits<4, 4, 1>::SMEM);
+  const cudaError_t e =
+      hard ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_cutn3<2, false>,
+                                                           cut_traits<2>::WARPS * 32, 0)
+           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_pairs_cutn3<1, false>,
+                                                           cut_traits<1>::WARPS * 32, 0);
   if (e != cudaSuccess) cudaGetLastError();
-  return e == cudaSuccess && nb > 0 ? nb : 3;
-}
-
-cudaError_t od_cutn3_prepare(int ipt, int T) {
-  if (ipt == 2 && T == 512) return prepare_cutn3<2, 2, true>((int)kCutBalSmem);
-  if (ipt == 4 && T == 1024)
-    return prepare_cutn3<4, 4, false>((int)n3_traits<4, 4, 1>::SMEM);
-  return cudaErrorInvalidValue;
+  return e == cudaSuccess && nb > 0 ? nb : 5;
 }
 
 cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, float4* part_hi,
                                 float4* part_lo, float rho0, float rc, float rs, uint32_t* err,
                                 unsigned long long* pair_count, cudaStream_t s) {
-  k_mc_clear<<<(L.ncells + 255) / 256, 256, 0, s>>>(L.ncells, L.count, L.fill);
+  k_mc_clear<<<(L.ncells + 255) / 256, 256, 0, s>>>(L.ncells, L.count, L.fill, L.next);
   k_mc_count<<<(n + 255) / 256, 256, 0, s>>>(n, pos, L.lo, L.lo_z, L.inv_s, L.G, L.nb,
                                               L.cell_of, L.count);
   k_scan_excl<<<1, 1024, 0, s>>>(L.ncells, L.count, L.start);
   k_mc_scatter<<<(n + 255) / 256, 256, 0, s>>>(n, L.cell_of, L.start, L.fill, L.perm);
   k_mc_sort<<<L.ncells, 128, 0, s>>>(L.count, L.start, pos, L.perm, L.xs, L.ys, L.zs, err);
-  k_tile_box<<<L.nT, 256, 0, s>>>(n, L.T, L.xs, L.ys, L.zs, L.gbox, L.box);
-  const float rc2m = rc * rc * 1.00001f;
-  k_tile_adj<<<L.nT, 128, 0, s>>>(L.nT, L.nwords, L.box, rc2m, L.adj, L.rowptr);
-  k_scan_excl<<<1, 1024, 0, s>>>(L.nT, L.rowptr, L.rowptr);
-  k_tile_list<<<(L.nT + 127) / 128, 128, 0, s>>>(L.nT, L.nwords, L.adj, L.rowptr, L.pairs);
+  const int nT = L.nslots / kTile;
+  k_tile_box<<<nT, kTile, 0, s>>>(n, L.xs, L.ys, L.zs, L.perm, L.bbox, L.tbox);
   const bool sw = rs < rc;
-  // group pairs whose farthest box distance is below the switching radius (hard cutoff: the
-  // cutoff), with a relative margin of 1e-5 against rounding, skip the switching polynomial
+  // blocks whose farthest box distance is below the switching radius (hard cutoff: the cutoff), with a
+  // relative margin of 1e-5 against rounding, skip the switching polynomial; blocks whose nearest box
+  // distance is beyond the cutoff, with the same margin, are skipped
   const float rin = (sw ? rs : rc) * (1.0f - 1e-5f);
-  const n3_cut cut{rho0, rc * rc, rs, sw ? 1.0f / (rc - rs) : 0.0f, rin * rin, L.rc_d};
-  const int32_t* np = L.rowptr + L.nT;
-#define OD_CUTN3(MT, MS, BAL, SM)                                                             \
-  do {                                                                                        \
-    if (sw) {                                                                                 \
-      if (pair_count) OD_CUTN3L(MT, MS, 1, true, BAL, SM);                                    \
-      else OD_CUTN3L(MT, MS, 1, false, BAL, SM);                                              \
-    } else {                                                                                  \
-      if (pair_count) OD_CUTN3L(MT, MS, 2, true, BAL, SM);                                    \
-      else OD_CUTN3L(MT, MS, 2, false, BAL, SM);                                              \
-    }                                                                                         \
-  } while (0)
-#define OD_CUTN3L(MT, MS, CUT, CNT, BAL, SM)                                                  \
-  k_pairs_cutn3<MT, MS, 1, CUT, CNT, BAL><<<sw ? L.grid : L.grid_hard, kWarps * 32, SM, s>>>( \
-      L.xs, L.ys, L.zs, L.nslots, L.nT, L.pairs, np, L.acc, cut, L.gbox, rc2m, pair_count)
-  if (L.ipt == 2 && L.T == 512) OD_CUTN3(2, 2, true, kCutBalSmem);
-  else if (L.ipt == 4 && L.T == 1024) OD_CUTN3(4, 4, false, (n3_traits<4, 4, 1>::SMEM));
-  else return cudaErrorInvalidValue;
-#undef OD_CUTN3L
+  const cut_args cut{rho0, rc * rc, rs, sw ? 1.0f / (rc - rs) : 0.0f, rin * rin,
+                     rc * rc * 1.00001f, L.rc_d};
+  // tiles per unit: one up to 256 tiles (65536 ions 0.82 ms, 0.89 with two), then more so that the
+  // units, most of them empty, stay few beside the work (2^19 ions: no difference from 4 to 16)
+  const int B = std::min(32, std::max(1, nT / 128));
+  const long long nunits = units_before((nT + B - 1) / B, nT, B);
+#define OD_CUTN3(CUT, CNT)                                                                      \
+  k_pairs_cutn3<CUT, CNT><<<CUT == 2 ? L.grid_hard : L.grid, cut_traits<CUT>::WARPS * 32, 0, s>>>( \
+      L.xs, L.ys, L.zs, L.nslots, nT, B, nunits, L.next, L.acc, cut, L.tbox, L.bbox, pair_count)
+  if (sw) {
+    if (pair_count) OD_CUTN3(1, true);
+    else OD_CUTN3(1, false);
+  } else {
+    if (pair_count) OD_CUTN3(2, true);
+    else OD_CUTN3(2, false);
+  }
 #undef OD_CUTN3
   k_slot_take<<<(L.nslots + 255) / 256, 256, 0, s>>>(L.nslots, L.acc, L.perm, part_hi, part_lo);
   return cudaGetLastError();

@@ -109,23 +109,19 @@ struct od_cellgeom {
   float c, inv_c, lox, loy, loz;
 };
 // Device cell list of the cutoff path.
-// Cutoff over tile pairs (cutoff variant 3, od_cutn3.cu): ions sorted along a Hilbert curve of a
-// G^3 cell grid, tiles of T consecutive sorted ions, and every tile pair whose bounding boxes
-// come within the cutoff evaluated with each unordered pair once (64-ion group pairs farther
-// apart than the cutoff skipped).
+// Cutoff variant 3 (od_cutn3.cu): ions sorted along a Hilbert curve of a G^3 cell grid, every pair
+// of 32-ion blocks whose bounding boxes come within the cutoff evaluated with each unordered pair
+// once.
 struct od_cutn3 {
   int G, bits, nb, ncells;          // cells per cube axis (power of two), key bits per axis,
                                     // cubes along z, nb * G^3
   float lo, lo_z, inv_s;            // grid origin (x and y, z) and 1 / cell side (lambda)
-  int T, ipt, nT, nslots, nwords;   // tile, targets per lane, tiles, nT*T slots, bitmap words
+  int T, ipt, nslots;               // plan (the slots are padded to a multiple of T), slots
   int32_t *cell_of, *count, *fill, *start;  // [N], [ncells], [ncells], [ncells + 1]
   int32_t* perm;                    // [nslots] ion of each sorted slot, -1 for sentinels
   float *xs, *ys, *zs;              // [nslots] sorted positions; sentinels in the tail
-  float* box;                       // [nT][6] min xyz, max xyz
-  float* gbox;                      // [nslots / 64][6] boxes of 64-slot groups
-  uint32_t* adj;                    // [nT][nwords] tile pairs (a, b >= a) within the cutoff
-  int32_t* rowptr;                  // [nT + 1] pair counts, then their exclusive prefix
-  int2* pairs;                      // [nT (nT + 1) / 2] listed pairs, row-major
+  float4 *tbox, *bbox;              // [nslots / 512][2], [nslots / 32][2] boxes
+  unsigned long long* next;         // work counter of the pair kernel
   unsigned long long* acc;          // [3][nslots] fixed-point ion–ion sums per sorted slot
   double rc_d;                      // cutoff / r_D_e in FP64 (the hard cutoff's exact test)
   int grid, grid_hard;              // persistent blocks of the pair kernel (switching, hard)
@@ -136,8 +132,7 @@ struct od_cgrid { int G, nb, ncells; double side; };
 od_cgrid od_cutn3_grid(int N, double R, double H);
 size_t od_cutn3_bytes(int N, int T, int ncells);
 bool od_cutn3_supported(int ipt, int T);
-cudaError_t od_cutn3_prepare(int ipt, int T);
-int od_cutn3_blocks_per_sm(int ipt, int T, bool hard);  // after od_cutn3_prepare
+int od_cutn3_blocks_per_sm(bool hard);
 cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, float4* part_hi,
                                 float4* part_lo, float rho0, float rc, float rs, uint32_t* err,
                                 unsigned long long* pair_count, cudaStream_t s);

@@ -31,7 +31,7 @@
 // SFU operation taken out, so fewer SFU operations, or a scalar form (33), gain nothing. The pair
 // term below has the fewest packed operations (17 with the sums).
 #include <algorithm>
-#include "od_n3_pair.cuh"
+#include "od_internal.h"
 
 namespace {
 
