@@ -7,6 +7,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <unistd.h>
 #include <algorithm>
 #include <cstddef>
 #include <cstdlib>
@@ -33,9 +34,13 @@ struct od_handle {
   bool has_cut = false;
   od_cutlist cut{};
   unsigned long long* d_pairs = nullptr;  // pairs inside the cutoff, counted in timing mode
+  // one allocation for the state, the lists and the series, one for the cell-stencil cutoff
+  void *arena = nullptr, *cut_arena = nullptr;
+  int slabs = 0;  // partial-sum slabs at b.part_hi (b.part_lo follows them)
   // snapshot scratch (allocated on first use)
-  float4 *snap_pos = nullptr, *snap_hi = nullptr, *snap_lo = nullptr;
+  float4* snap_pos = nullptr;
   double* snap_counts = nullptr;
+  double* stage = nullptr;  // FP64 staging of a shard (other handles use the list block)
   // CUDA graph of one step (production path)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -396,6 +401,31 @@ static cudaError_t dalloc(T** p, size_t n) {
   return cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(n, 1));
 }
 
+// Several buffers in one allocation (a cudaMalloc takes about 20 us): a layout function calls
+// take() for each buffer, once to add up the size and once to hand out the addresses.
+struct od_carver {
+  char* base = nullptr;
+  size_t off = 0;
+  template <typename T>
+  void take(T*& p, size_t n) {
+    off = (off + 255) & ~(size_t)255;
+    if (base) p = reinterpret_cast<T*>(base + off);
+    off += sizeof(T) * std::max<size_t>(n, 1);
+  }
+};
+template <typename F>
+static cudaError_t carve(void** block, size_t* bytes, F layout) {
+  od_carver c;
+  layout(c);
+  if (bytes) *bytes = c.off;
+  const cudaError_t e = cudaMalloc(block, c.off);
+  if (e != cudaSuccess) return e;
+  od_carver d;
+  d.base = (char*)*block;
+  layout(d);
+  return cudaSuccess;
+}
+
 static void free_timing(od_handle* h) {
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   h->ev_pool.clear();
@@ -412,24 +442,26 @@ static void free_all(od_handle* h) {
   if (h->graph_exec_nf) { cudaGraphExecDestroy(h->graph_exec_nf); h->graph_exec_nf = nullptr; }
   if (h->graph_nf) { cudaGraphDestroy(h->graph_nf); h->graph_nf = nullptr; }
   free_timing(h);
-  void* ptrs[] = {h->dp, h->ds, h->b.pos, h->b.rel, h->b.vel, h->b.fhi, h->b.flo, h->b.part_hi, h->b.part_lo,
-                  h->b.flags, h->b.list, h->b.list_bits, h->b.list_old, h->b.list_new, h->b.list_v,
-                  h->b.orbit_part, h->b.s_q, h->b.s_orbit, h->b.s_collect, h->b.s_dust,
-                  h->b.s_field, h->b.cq, h->snap_pos, h->snap_hi, h->snap_lo, h->snap_counts,
-                  h->b.sx, h->b.sy, h->b.sz, h->cut.cell_of, h->cut.count, h->cut.fill,
-                  h->cut.start, h->cut.chunk_prefix, h->cut.perm, h->cut.ox, h->cut.oy, h->cut.oz,
-                  h->cut.stencil, h->d_pairs, h->cut.chunk_prefix2, h->b.n3, h->ssx, h->ssy,
-                  h->ssz, h->g_idx, h->g_bits, h->g_old, h->g_new, h->g_v, h->g_orbit};
+  void* ptrs[] = {h->arena, h->cut_arena, h->b.part_hi, h->snap_pos, h->snap_counts, h->stage,
+                  h->b.n3, h->ssx, h->ssy, h->ssz, h->g_idx, h->g_bits, h->g_old, h->g_new, h->g_v,
+                  h->g_orbit};
   for (void* p : ptrs)
     if (p) cudaFree(p);
 }
 
-static od_status alloc_scratch_for_plan(od_handle* h) {
-  if (h->b.part_hi) { cudaFree(h->b.part_hi); h->b.part_hi = nullptr; }
-  if (h->b.part_lo) { cudaFree(h->b.part_lo); h->b.part_lo = nullptr; }
-  size_t n = (size_t)h->plan.jsplit * h->Npad;
-  OD_CK(h, dalloc(&h->b.part_hi, n));
-  OD_CK(h, dalloc(&h->b.part_lo, n));
+// Partial-sum slabs: one (the consumers' view of the sums), or jsplit of them for the plans that
+// write each source chunk's sums apart (the scalar variants 0 and 1, and batch members on the
+// directed kernel).
+static int slabs_of(const od_pair_plan& pl) { return pl.variant <= 1 ? pl.jsplit : 1; }
+static od_status ensure_slabs(od_handle* h, int slabs) {
+  if (h->slabs >= slabs) return OD_OK;
+  if (h->b.part_hi) cudaFree(h->b.part_hi);
+  h->b.part_hi = h->b.part_lo = nullptr;
+  h->slabs = 0;
+  const size_t n = (size_t)slabs * h->Npad;
+  OD_CK(h, dalloc(&h->b.part_hi, 2 * n));
+  h->b.part_lo = h->b.part_hi + n;
+  h->slabs = slabs;
   return OD_OK;
 }
 
@@ -477,30 +509,29 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
   fill_params(cfg, h->N, h->Npad, &h->hp);
   h->plan = default_plan(h->Npad, od_num_sms(device));
   const size_t Np = h->Npad, P = std::max(h->P, 1), ns = cfg->n_steps;
-  OD_CKC(dalloc(&h->dp, 1));
-  OD_CKC(dalloc(&h->ds, 1));
-  OD_CKC(dalloc(&h->b.pos, Np));
-  OD_CKC(dalloc(&h->b.rel, Np));
-  OD_CKC(dalloc(&h->b.vel, Np));
-  OD_CKC(dalloc(&h->b.fhi, Np));
-  OD_CKC(dalloc(&h->b.flo, Np));
-  OD_CKC(dalloc(&h->b.flags, Np / 32));
-  OD_CKC(dalloc(&h->b.list, Np));
-  OD_CKC(dalloc(&h->b.list_bits, Np));
-  OD_CKC(dalloc(&h->b.list_old, Np));
-  OD_CKC(dalloc(&h->b.list_new, Np));
-  OD_CKC(dalloc(&h->b.list_v, Np));
-  OD_CKC(dalloc(&h->b.orbit_part, (size_t)h->nb * P * 3));
-  OD_CKC(dalloc(&h->b.s_q, ns * P));
-  OD_CKC(dalloc(&h->b.s_orbit, ns * P * 3));
-  OD_CKC(dalloc(&h->b.s_collect, ns * P * 3));
-  OD_CKC(dalloc(&h->b.s_dust, ns * P * 3));
-  OD_CKC(dalloc(&h->b.s_field, ns * P * 3));
-  OD_CKC(dalloc(&h->b.cq, OD_MAX_GRAINS));
-  OD_CKC(dalloc(&h->b.sx, Np));
-  OD_CKC(dalloc(&h->b.sy, Np));
-  OD_CKC(dalloc(&h->b.sz, Np));
-  if (alloc_scratch_for_plan(h) != OD_OK) return bail(OD_ERR_OOM);
+  size_t arena_bytes = 0;
+  OD_CKC(carve(&h->arena, &arena_bytes, [&](od_carver& c) {
+    c.take(h->dp, 1);
+    c.take(h->ds, 1);
+    c.take(h->b.pos, Np);
+    c.take(h->b.rel, Np);
+    c.take(h->b.vel, Np);
+    c.take(h->b.fhi, Np);
+    c.take(h->b.flo, Np);
+    c.take(h->b.flags, Np / 32);
+    c.take(h->b.list, Np);
+    c.take(h->b.list_bits, Np);
+    c.take(h->b.list_old, 3 * Np);
+    c.take(h->b.orbit_part, (size_t)h->nb * P * 3);
+    c.take(h->b.series, ns * P * 13);
+    c.take(h->b.cq, OD_MAX_GRAINS);
+    c.take(h->b.sx, Np);
+    c.take(h->b.sy, Np);
+    c.take(h->b.sz, Np);
+  }));
+  h->b.list_new = h->b.list_old + Np;
+  h->b.list_v = h->b.list_new + Np;
+  if (ensure_slabs(h, 1) != OD_OK) return bail(OD_ERR_OOM);
   if (cfg->force_method != OD_FORCE_CUTOFF && ensure_acc(h) != OD_OK) return bail(OD_ERR_OOM);
   int n3_ipt = 0, n3_tile = 0;
   if (n3_default && cfg->force_method != OD_FORCE_CUTOFF)
@@ -539,24 +570,27 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
     h->cut.nstencil = (int)st.size();
     h->cut.cap = h->Npad + 8 * g.ncells;
     const size_t nc = g.ncells;
-    OD_CKC(dalloc(&h->cut.cell_of, Np));
-    OD_CKC(dalloc(&h->cut.count, nc));
-    OD_CKC(dalloc(&h->cut.fill, nc));
-    OD_CKC(dalloc(&h->cut.start, nc + 1));
-    OD_CKC(dalloc(&h->cut.chunk_prefix, nc + 1));
-    OD_CKC(dalloc(&h->cut.chunk_prefix2, nc + 1));
     h->cut.packed = true;
-    OD_CKC(dalloc(&h->cut.perm, h->cut.cap));
-    OD_CKC(dalloc(&h->cut.ox, h->cut.cap));
-    OD_CKC(dalloc(&h->cut.oy, h->cut.cap));
-    OD_CKC(dalloc(&h->cut.oz, h->cut.cap));
-    OD_CKC(dalloc(&h->cut.stencil, st.size()));
-    OD_CKC(dalloc(&h->d_pairs, 1));
-    OD_CKC(cudaMemcpy(h->cut.stencil, st.data(), sizeof(int4) * st.size(), cudaMemcpyHostToDevice));
-    OD_CKC(cudaMemset(h->d_pairs, 0, sizeof(unsigned long long)));
+    OD_CKC(carve(&h->cut_arena, nullptr, [&](od_carver& c) {
+      c.take(h->cut.cell_of, Np);
+      c.take(h->cut.count, nc);
+      c.take(h->cut.fill, nc);
+      c.take(h->cut.start, nc + 1);
+      c.take(h->cut.chunk_prefix, nc + 1);
+      c.take(h->cut.chunk_prefix2, nc + 1);
+      c.take(h->cut.perm, h->cut.cap);
+      c.take(h->cut.ox, h->cut.cap);
+      c.take(h->cut.oy, h->cut.cap);
+      c.take(h->cut.oz, h->cut.cap);
+      c.take(h->cut.stencil, st.size());
+      c.take(h->d_pairs, 1);
+    }));
+    OD_CKC(cudaMemcpyAsync(h->cut.stencil, st.data(), sizeof(int4) * st.size(),
+                           cudaMemcpyHostToDevice, h->stream));
+    OD_CKC(cudaMemsetAsync(h->d_pairs, 0, sizeof(unsigned long long), h->stream));
     h->has_cut = true;
-    // default: tile pairs with each pair once (512-ion tiles, else 1024) when their memory
-    // fits the budget; the cell-stencil kernel otherwise
+    // default: the Hilbert-sorted kernel (variant 3) when its memory fits the budget; the
+    // cell-stencil kernel otherwise
     const int nc3 = od_cutn3_grid(h->N, h->hp.Rh, h->hp.Hh).ncells;
     const int cut_ipt = od_cutn3_bytes(h->N, 512, nc3) <= OD_CUTN3_BUDGET ? 2
                         : (od_cutn3_bytes(h->N, 1024, nc3) <= OD_CUTN3_BUDGET ? 4 : 0);
@@ -565,20 +599,13 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
       h->err.clear();
     }
   }
+  OD_CKC(cudaMemsetAsync(h->arena, 0, arena_bytes, h->stream));
   OD_CKC(cudaMemcpyAsync(h->dp, &h->hp, sizeof(od_dparams), cudaMemcpyHostToDevice, h->stream));
   od_dstate s0{};
   for (int g = 0; g < h->P; g++) s0.q_param[g] = cfg->grain_q0[g];
   OD_CKC(cudaMemcpyAsync(h->ds, &s0, sizeof(s0), cudaMemcpyHostToDevice, h->stream));
-  // padded slots: far-away sources, zero velocity
-  std::vector<float4> pad(Np, make_float4(OD_SENTINEL, OD_SENTINEL, OD_SENTINEL, 0.f));
-  OD_CKC(cudaMemcpy(h->b.pos, pad.data(), sizeof(float4) * Np, cudaMemcpyHostToDevice));
-  OD_CKC(cudaMemset(h->b.rel, 0, sizeof(float4) * Np));
-  OD_CKC(od_launch_aos_to_soa(h->b.pos, h->Npad, h->b.sx, h->b.sy, h->b.sz, h->stream));
-  OD_CKC(cudaMemset(h->b.vel, 0, sizeof(float4) * Np));
-  OD_CKC(cudaMemset(h->b.fhi, 0, sizeof(float4) * Np));
-  OD_CKC(cudaMemset(h->b.flo, 0, sizeof(float4) * Np));
-  OD_CKC(cudaMemset(h->b.s_q, 0, sizeof(double) * ns * P));
-  OD_CKC(cudaMemset(h->b.s_field, 0, sizeof(double) * ns * P * 3));
+  // every slot a far-away source until a state is set, the padded ones for good; zero velocity
+  OD_CKC(od_launch_clear_state(h->Npad, h->b, h->stream));
   OD_CKC(od_launch_set_charges(h->dp, h->ds, h->b.cq, h->P, h->stream));
   OD_CKC(cudaStreamSynchronize(h->stream));
 #undef OD_CKC
@@ -614,21 +641,36 @@ static void to_device_units(const od_handle* h, const double* pos, const double*
 }
 
 static od_status check_device_err(od_handle* h) {
-  od_dstate s;
-  OD_CK(h, cudaMemcpyAsync(&s, h->ds, sizeof(s), cudaMemcpyDeviceToHost, h->stream));
+  uint32_t err = 0;
+  OD_CK(h, cudaMemcpyAsync(&err, &h->ds->err, sizeof(err), cudaMemcpyDeviceToHost, h->stream));
   OD_CK(h, cudaStreamSynchronize(h->stream));
-  if (s.err & OD_DERR_TIMEOUT) return fail(h, OD_ERR_TIMEOUT, "a bounded device wait ran out");
-  if (s.err & OD_DERR_CELL)
+  if (err & OD_DERR_TIMEOUT) return fail(h, OD_ERR_TIMEOUT, "a bounded device wait ran out");
+  if (err & OD_DERR_CELL)
     return fail(h, OD_ERR_CAPACITY, "a cutoff cell holds more than 4096 ions (density too high)");
-  if (s.err) return fail(h, OD_ERR_STATE, "device error word set");
+  if (err) return fail(h, OD_ERR_STATE, "device error word set");
+  return OD_OK;
+}
+
+// Touches the pages of an output array before a device copy writes it: fresh pages that the copy
+// engine faults in one by one cost 30 ms for the 50 MB of a 2^20-ion state, from the host 5 ms.
+static void touch_pages(void* p, size_t bytes) {
+  static const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
+  volatile char* c = (volatile char*)p;
+  for (size_t k = 0; k < bytes; k += page) c[k] = 0;
+  if (bytes) c[bytes - 1] = 0;
+}
+
+// FP64 staging of state copies: 6 doubles per ion. Between steps the lists of re-injected ions are
+// free (48 bytes per ion); a shard's list outlives its calls, so a shard has its own.
+static od_status staging(od_handle* h, double** p) {
+  if (h->shard && !h->stage) OD_CK(h, dalloc(&h->stage, (size_t)h->Npad * 6));
+  *p = h->shard ? h->stage : reinterpret_cast<double*>(h->b.list_old);
   return OD_OK;
 }
 
 // ion–ion sums of the current positions into fhi/flo (the force the first half kick uses)
+// (b.sx, b.sy, b.sz hold the SoA copies of b.pos)
 static od_status refresh_forces(od_handle* h) {
-  const float rho0 = h->hp.rho0;
-  OD_CK(h, od_launch_aos_to_soa(h->b.pos, h->Npad, h->b.sx, h->b.sy, h->b.sz, h->stream));
-  (void)rho0;
   OD_CK(h, od_launch_force(force_ctx(h, false), od_pair_io{h->b.pos, h->b.sx, h->b.sy, h->b.sz, h->b.n3}, h->N,
                            h->Npad, h->b.part_hi, h->b.part_lo, &h->ds->err, h->stream));
   OD_CK(h, od_launch_reduce(h->dp, h->Npad, force_jsplit(h), h->b.part_hi, h->b.part_lo, h->b.fhi,
@@ -672,16 +714,21 @@ extern "C" od_status od_set_state(od_handle* h, const double* pos, const double*
   if (!h) return fail(nullptr, OD_ERR_INVALID, "handle is NULL");
   if (!pos || !vel) return fail(h, OD_ERR_INVALID, "pos/vel is NULL");
   if (n != h->N) return fail(h, OD_ERR_INVALID, "n must equal the configured n_ions");
-  if (!all_finite(pos, 3 * n) || !all_finite(vel, 3 * n))
-    return fail(h, OD_ERR_INVALID, "a position or velocity is not finite");
   OD_CK(h, cudaSetDevice(h->device));
-  std::vector<float4> xp, vp, rel;
-  to_device_units(h, nullptr, vel, n, xp, &vp);
-  to_rel_state(h, pos, n, rel, xp);
-  OD_CK(h, cudaMemcpyAsync(h->b.rel, rel.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, h->stream));
-  OD_CK(h, cudaMemcpyAsync(h->b.pos, xp.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, h->stream));
-  OD_CK(h, cudaMemcpyAsync(h->b.vel, vp.data(), sizeof(float4) * n, cudaMemcpyHostToDevice, h->stream));
-  od_status st = refresh_forces(h);
+  double* st64 = nullptr;
+  od_status st = staging(h, &st64);
+  if (st != OD_OK) return st;
+  const size_t bytes = sizeof(double) * 3 * n;
+  OD_CK(h, cudaMemcpyAsync(st64, pos, bytes, cudaMemcpyHostToDevice, h->stream));
+  OD_CK(h, cudaMemcpyAsync(st64 + 3 * n, vel, bytes, cudaMemcpyHostToDevice, h->stream));
+  OD_CK(h, cudaMemsetAsync(&h->ds->bad, 0, sizeof(uint32_t), h->stream));
+  OD_CK(h, od_launch_state_check(st64, 6 * n, &h->ds->bad, h->stream));
+  uint32_t bad = 0;
+  OD_CK(h, cudaMemcpyAsync(&bad, &h->ds->bad, sizeof(bad), cudaMemcpyDeviceToHost, h->stream));
+  OD_CK(h, cudaStreamSynchronize(h->stream));
+  if (bad) return fail(h, OD_ERR_INVALID, "a position or velocity is not finite");
+  OD_CK(h, od_launch_state_in(h->dp, h->N, st64, st64 + 3 * n, h->b, h->stream));
+  st = refresh_forces(h);
   if (st != OD_OK) return st;
   OD_CK(h, cudaStreamSynchronize(h->stream));
   h->state_set = true;
@@ -706,8 +753,7 @@ extern "C" od_status od_init_state(od_handle* h, const double* vz_v, const doubl
     OD_CK(h, cudaMemcpy(d_v, v.data(), sizeof(float) * vz_n, cudaMemcpyHostToDevice));
     OD_CK(h, cudaMemcpy(d_x, vz_cdf, sizeof(double) * vz_n, cudaMemcpyHostToDevice));
   }
-  cudaError_t e = od_launch_init_state(h->dp, h->N, h->b.rel, h->b.pos, h->b.vel, d_v, d_x, vz_n,
-                                       &h->ds->err, h->stream);
+  cudaError_t e = od_launch_init_state(h->dp, h->N, h->b, d_v, d_x, vz_n, &h->ds->err, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (d_v) cudaFree(d_v);
   if (d_x) cudaFree(d_x);
@@ -805,15 +851,8 @@ extern "C" od_status od_set_grains(od_handle* h, const double* x, const double* 
 extern "C" od_status od_begin_window(od_handle* h) {
   if (!h) return fail(nullptr, OD_ERR_INVALID, "handle is NULL");
   OD_CK(h, cudaSetDevice(h->device));
-  od_dstate s;
-  OD_CK(h, cudaMemcpyAsync(&s, h->ds, sizeof(s), cudaMemcpyDeviceToHost, h->stream));
-  OD_CK(h, cudaStreamSynchronize(h->stream));
-  s.rng_base += s.step;
-  s.step = 0;
-  memset(s.avg, 0, sizeof(s.avg));
-  s.n_avg = 0;
-  OD_CK(h, cudaMemcpyAsync(h->ds, &s, sizeof(s), cudaMemcpyHostToDevice, h->stream));
-  OD_CK(h, cudaStreamSynchronize(h->stream));
+  OD_CK(h, od_launch_begin_window(h->ds, h->stream));
+  OD_CK(h, cudaStreamSynchronize(h->stream));  // a batch member steps on the batch's stream
   h->step = 0;
   return OD_OK;
 }
@@ -822,23 +861,17 @@ extern "C" od_status od_get_state(od_handle* h, double* pos, double* vel, int64_
   if (!h) return fail(nullptr, OD_ERR_INVALID, "handle is NULL");
   if (n != h->N) return fail(h, OD_ERR_INVALID, "n must equal the configured n_ions");
   OD_CK(h, cudaSetDevice(h->device));
-  std::vector<float4> rp(n), vp(n);
-  OD_CK(h, cudaMemcpyAsync(rp.data(), h->b.rel, sizeof(float4) * n, cudaMemcpyDeviceToHost, h->stream));
-  OD_CK(h, cudaMemcpyAsync(vp.data(), h->b.vel, sizeof(float4) * n, cudaMemcpyDeviceToHost, h->stream));
+  double* st64 = nullptr;
+  od_status st = staging(h, &st64);
+  if (st != OD_OK) return st;
+  const size_t bytes = sizeof(double) * 3 * n;
+  OD_CK(h, od_launch_state_out(h->dp, h->N, h->b, pos ? st64 : nullptr, vel ? st64 + 3 * n : nullptr,
+                               h->stream));
+  if (pos) touch_pages(pos, bytes);
+  if (vel) touch_pages(vel, bytes);
+  if (pos) OD_CK(h, cudaMemcpyAsync(pos, st64, bytes, cudaMemcpyDeviceToHost, h->stream));
+  if (vel) OD_CK(h, cudaMemcpyAsync(vel, st64 + 3 * n, bytes, cudaMemcpyDeviceToHost, h->stream));
   OD_CK(h, cudaStreamSynchronize(h->stream));
-  const double lam = h->hp.lam, vunit = h->hp.vunit, s = h->hp.rel_s;
-  for (int64_t i = 0; i < n; i++) {
-    if (pos) {  // the cell-relative state, exactly (c s + offset is exact in FP64)
-      int key;
-      memcpy(&key, &rp[i].w, sizeof(key));
-      const double c[3] = {(double)((key & 1023) - OD_REL_BIAS), (double)(((key >> 10) & 1023) - OD_REL_BIAS),
-                           (double)(((key >> 20) & 1023) - OD_REL_BIAS)};
-      pos[3 * i] = (c[0] * s + rp[i].x) * lam;
-      pos[3 * i + 1] = (c[1] * s + rp[i].y) * lam;
-      pos[3 * i + 2] = (c[2] * s + rp[i].z) * lam;
-    }
-    if (vel) { vel[3 * i] = vp[i].x * vunit; vel[3 * i + 1] = vp[i].y * vunit; vel[3 * i + 2] = vp[i].z * vunit; }
-  }
   return OD_OK;
 }
 
@@ -1012,10 +1045,7 @@ static bool plan_supported(int nt, int ipt, int variant) {
 static void free_cutn3(od_handle* h) {
   od_cutn3* L = h->cut.n3;
   if (!L) return;
-  void* ptrs[] = {L->cell_of, L->count, L->fill, L->start, L->perm, L->xs, L->ys, L->zs,
-                  L->tbox, L->bbox, L->next, L->acc};
-  for (void* p : ptrs)
-    if (p) cudaFree(p);
+  if (L->block) cudaFree(L->block);
   delete L;
   h->cut.n3 = nullptr;
 }
@@ -1045,26 +1075,26 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
   L->grid = od_num_sms(h->device) * od_cutn3_blocks_per_sm(false);
   L->grid_hard = od_num_sms(h->device) * od_cutn3_blocks_per_sm(true);
   const size_t ns = L->nslots, nc = L->ncells;
-  auto al = [&](auto** p, size_t n) {
-    return cudaMalloc((void**)p, sizeof(**p) * std::max<size_t>(n, 1));
-  };
-  cudaError_t e = al(&L->cell_of, (size_t)N);
-  if (e == cudaSuccess) e = al(&L->count, nc);
-  if (e == cudaSuccess) e = al(&L->fill, nc);
-  if (e == cudaSuccess) e = al(&L->start, nc + 1);
-  if (e == cudaSuccess) e = al(&L->perm, ns);
-  if (e == cudaSuccess) e = al(&L->xs, ns);
-  if (e == cudaSuccess) e = al(&L->ys, ns);
-  if (e == cudaSuccess) e = al(&L->zs, ns);
-  if (e == cudaSuccess) e = al(&L->tbox, ns / 512 * 2);
-  if (e == cudaSuccess) e = al(&L->bbox, ns / 32 * 2);
-  if (e == cudaSuccess) e = al(&L->next, 1);
-  if (e == cudaSuccess) e = al(&L->acc, 3 * ns);
-  if (e == cudaSuccess) e = cudaMemset(L->acc, 0, sizeof(unsigned long long) * 3 * ns);
+  cudaError_t e = carve(&L->block, nullptr, [&](od_carver& c) {
+    c.take(L->cell_of, (size_t)N);
+    c.take(L->count, nc);
+    c.take(L->fill, nc);
+    c.take(L->start, nc + 1);
+    c.take(L->perm, ns);
+    c.take(L->xs, ns);
+    c.take(L->ys, ns);
+    c.take(L->zs, ns);
+    c.take(L->tbox, ns / 512 * 2);
+    c.take(L->bbox, ns / 32 * 2);
+    c.take(L->next, 1);
+    c.take(L->acc, 3 * ns);
+  });
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(L->acc, 0, sizeof(unsigned long long) * 3 * ns, h->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     free_cutn3(h);
-    return fail(h, OD_ERR_OOM, "no device memory for the tile-pair cutoff");
+    return fail(h, OD_ERR_OOM, "no device memory for the sorted cutoff");
   }
   return OD_OK;
 }
@@ -1092,7 +1122,7 @@ static od_status ensure_acc(od_handle* h) {
     return fail(h, OD_ERR_OOM, "no device memory for the ion–ion accumulators");
   }
   h->b.n3_len = need;
-  OD_CK(h, cudaMemset(h->b.n3, 0, sizeof(float) * need));
+  OD_CK(h, cudaMemsetAsync(h->b.n3, 0, sizeof(float) * need, h->stream));
   return OD_OK;
 }
 
@@ -1127,7 +1157,7 @@ static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
     }
     h->b.n3_len = need;
     // the accumulators start at zero; every evaluation clears them after reading them
-    OD_CK(h, cudaMemset(h->b.n3, 0, sizeof(float) * need));
+    OD_CK(h, cudaMemsetAsync(h->b.n3, 0, sizeof(float) * need, h->stream));
   }
   h->plan = pl;  // one partial slab: part_hi/part_lo always hold at least one
   drop_graph(h);
@@ -1184,9 +1214,8 @@ extern "C" od_status od_set_pair_plan(od_handle* h, int32_t threads, int32_t tar
   chunk = ((chunk + OD_TJ - 1) / OD_TJ) * OD_TJ;
   pl.chunk = chunk;
   pl.jsplit = (h->Npad + chunk - 1) / chunk;
-  const bool grow = pl.jsplit > h->plan.jsplit;
+  if (ensure_slabs(h, slabs_of(pl)) != OD_OK) return OD_ERR_OOM;
   h->plan = pl;
-  if (grow && alloc_scratch_for_plan(h) != OD_OK) return OD_ERR_OOM;
   if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
   if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
   if (h->graph_exec_nf) { cudaGraphExecDestroy(h->graph_exec_nf); h->graph_exec_nf = nullptr; }
@@ -1344,14 +1373,29 @@ extern "C" od_status od_get_series(od_handle* h, int64_t first, int64_t count, d
     return fail(h, OD_ERR_INVALID, "requested steps have not been taken");
   if (count == 0) return OD_OK;
   OD_CK(h, cudaSetDevice(h->device));
-  const size_t P = h->P;
-  const size_t o1 = first * P, n1 = count * P;
-  if (q) OD_CK(h, cudaMemcpyAsync(q, h->b.s_q + o1, n1 * 8, cudaMemcpyDeviceToHost, h->stream));
-  if (f_orbit) OD_CK(h, cudaMemcpyAsync(f_orbit, h->b.s_orbit + 3 * o1, 3 * n1 * 8, cudaMemcpyDeviceToHost, h->stream));
-  if (f_collect) OD_CK(h, cudaMemcpyAsync(f_collect, h->b.s_collect + 3 * o1, 3 * n1 * 8, cudaMemcpyDeviceToHost, h->stream));
-  if (f_dust) OD_CK(h, cudaMemcpyAsync(f_dust, h->b.s_dust + 3 * o1, 3 * n1 * 8, cudaMemcpyDeviceToHost, h->stream));
-  if (f_field) OD_CK(h, cudaMemcpyAsync(f_field, h->b.s_field + 3 * o1, 3 * n1 * 8, cudaMemcpyDeviceToHost, h->stream));
-  OD_CK(h, cudaStreamSynchronize(h->stream));
+  const size_t P = h->P, row = 13 * P;
+  if (P == 0) return OD_OK;
+  double* out[5] = {q, f_orbit, f_collect, f_dust, f_field};
+  const double* src = h->b.series + first * row;
+  const bool whole = sizeof(double) * row * count <= (256 << 10);
+  std::vector<double> rows;
+  if (whole) {  // one copy of the rows (each copy takes about 9 us), split on the host
+    rows.resize((size_t)count * row);
+    OD_CK(h, cudaMemcpyAsync(rows.data(), src, sizeof(double) * rows.size(),
+                             cudaMemcpyDeviceToHost, h->stream));
+    OD_CK(h, cudaStreamSynchronize(h->stream));
+  }
+  for (int m = 0; m < 5; m++) {
+    if (!out[m]) continue;
+    const size_t w = m ? 3 * P : P, at = m ? P + 3 * P * (m - 1) : 0;
+    if (whole)
+      for (int64_t k = 0; k < count; k++)
+        memcpy(out[m] + (size_t)k * w, rows.data() + (size_t)k * row + at, sizeof(double) * w);
+    else
+      OD_CK(h, cudaMemcpy2DAsync(out[m], sizeof(double) * w, src + at, sizeof(double) * row,
+                                 sizeof(double) * w, (size_t)count, cudaMemcpyDeviceToHost, h->stream));
+  }
+  if (!whole) OD_CK(h, cudaStreamSynchronize(h->stream));
   return OD_OK;
 }
 
@@ -1368,23 +1412,19 @@ extern "C" od_status od_get_averages(od_handle* h, double* out, int64_t* n_avg) 
   return OD_OK;
 }
 
-static od_status ensure_snapshot(od_handle* h) {
-  if (h->snap_pos) return OD_OK;
-  OD_CK(h, dalloc(&h->snap_pos, h->Npad));
-  OD_CK(h, dalloc(&h->snap_hi, h->Npad));
-  OD_CK(h, dalloc(&h->snap_lo, h->Npad));
-  OD_CK(h, dalloc(&h->snap_counts, OD_MAX_GRAINS + 1));
-  return OD_OK;
-}
-
-static od_status upload_snapshot(od_handle* h, const double* pos, int64_t n) {
-  od_status st = ensure_snapshot(h);
+// a snapshot's positions into snap_pos and, with soa, into the SoA source buffers (od_step rewrites
+// them before its next use)
+static od_status upload_snapshot(od_handle* h, const double* pos, int64_t n, bool soa) {
+  if (!h->snap_pos) {
+    OD_CK(h, dalloc(&h->snap_pos, h->Npad));
+    OD_CK(h, dalloc(&h->snap_counts, OD_MAX_GRAINS + 1));
+  }
+  double* st64 = nullptr;
+  const od_status st = staging(h, &st64);
   if (st != OD_OK) return st;
-  std::vector<float4> xp;
-  to_device_units(h, pos, nullptr, n, xp, nullptr);
-  xp.resize(h->Npad, make_float4(OD_SENTINEL, OD_SENTINEL, OD_SENTINEL, 0.f));
-  OD_CK(h, cudaMemcpyAsync(h->snap_pos, xp.data(), sizeof(float4) * h->Npad, cudaMemcpyHostToDevice, h->stream));
-  OD_CK(h, cudaStreamSynchronize(h->stream));
+  OD_CK(h, cudaMemcpyAsync(st64, pos, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, h->stream));
+  OD_CK(h, od_launch_snapshot_in((int)n, h->Npad, st64, h->hp.lam, h->snap_pos, soa ? h->b.sx : nullptr,
+                                 h->b.sy, h->b.sz, h->stream));
   return OD_OK;
 }
 
@@ -1393,27 +1433,20 @@ extern "C" od_status od_force_snapshot(od_handle* h, const double* pos, int64_t 
   if (!pos || !force) return fail(h, OD_ERR_INVALID, "NULL argument");
   if (n < 1 || n > h->N) return fail(h, OD_ERR_INVALID, "n must be in [1, n_ions]");
   OD_CK(h, cudaSetDevice(h->device));
-  od_status st = upload_snapshot(h, pos, n);
+  od_status st = upload_snapshot(h, pos, n, true);
   if (st != OD_OK) return st;
-  // the snapshot borrows the SoA source buffers; od_step rewrites them before its next use
-  OD_CK(h, od_launch_aos_to_soa(h->snap_pos, h->Npad, h->b.sx, h->b.sy, h->b.sz, h->stream));
-  OD_CK(h, od_launch_force(force_ctx(h, false), od_pair_io{h->snap_pos, h->b.sx, h->b.sy, h->b.sz, h->b.n3},
-                           (int)n, h->Npad, h->b.part_hi, h->b.part_lo, &h->ds->err, h->stream));
-  OD_CK(h, od_launch_reduce(h->dp, h->Npad, force_jsplit(h), h->b.part_hi, h->b.part_lo, h->snap_hi,
-                            h->snap_lo, h->stream));
-  std::vector<float4> hi(n), lo(n);
-  OD_CK(h, cudaMemcpyAsync(hi.data(), h->snap_hi, sizeof(float4) * n, cudaMemcpyDeviceToHost, h->stream));
-  OD_CK(h, cudaMemcpyAsync(lo.data(), h->snap_lo, sizeof(float4) * n, cudaMemcpyDeviceToHost, h->stream));
-  OD_CK(h, cudaStreamSynchronize(h->stream));
-  st = check_device_err(h);
+  const od_force_ctx fc = force_ctx(h, false);
+  OD_CK(h, od_launch_force(fc, od_pair_io{h->snap_pos, h->b.sx, h->b.sy, h->b.sz, h->b.n3}, (int)n,
+                           h->Npad, h->b.part_hi, h->b.part_lo, &h->ds->err, h->stream, !fc.acc));
+  double* out = nullptr;
+  st = staging(h, &out);
   if (st != OD_OK) return st;
   const double F = h->hp.k * h->hp.q_s * h->hp.q_s / (h->hp.lam * h->hp.lam);
-  for (int64_t i = 0; i < n; i++) {
-    force[3 * i] = F * ((double)hi[i].x + (double)lo[i].x);
-    force[3 * i + 1] = F * ((double)hi[i].y + (double)lo[i].y);
-    force[3 * i + 2] = F * ((double)hi[i].z + (double)lo[i].z);
-  }
-  return OD_OK;
+  OD_CK(h, od_launch_snapshot_out((int)n, h->Npad, force_jsplit(h), h->b.part_hi, h->b.part_lo,
+                                  fc.acc, F, out, h->stream));
+  touch_pages(force, sizeof(double) * 3 * n);  // while the kernels run
+  OD_CK(h, cudaMemcpyAsync(force, out, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream));
+  return check_device_err(h);
 }
 
 extern "C" od_status od_snapshot_positions(od_handle* h, const double* pos, int64_t n, double* pos_dev) {
@@ -1434,7 +1467,7 @@ extern "C" od_status od_collect_flags(od_handle* h, const double* pos, int64_t n
   if (!pos || !count || (cap > 0 && !idx_out)) return fail(h, OD_ERR_INVALID, "NULL argument");
   if (n < 1 || n > h->N) return fail(h, OD_ERR_INVALID, "n must be in [1, n_ions]");
   OD_CK(h, cudaSetDevice(h->device));
-  od_status st = upload_snapshot(h, pos, n);
+  od_status st = upload_snapshot(h, pos, n, false);
   if (st != OD_OK) return st;
   OD_CK(h, od_launch_snapshot_flags(h->dp, (int)n, h->Npad, h->snap_pos, h->b.flags, h->b.list,
                                     h->b.list_bits, h->snap_counts, h->stream));
@@ -1641,6 +1674,7 @@ extern "C" od_status od_batch_add(od_batch* b, const od_config* cfg, const doubl
   if (st != OD_OK) {
     cudaGetLastError();
     st = od_set_pair_plan(h, 256, 1, 5, 0);
+    if (st == OD_OK) st = ensure_slabs(h, h->plan.jsplit);  // the batched directed kernel's
     if (st != OD_OK) { std::string m = h->err; od_destroy(h); return bfail(b, st, m); }
   }
   st = pos ? od_set_state(h, pos, vel, cfg->n_ions) : od_init_state(h, nullptr, nullptr, 0);
@@ -1793,18 +1827,21 @@ extern "C" od_status od_batch_step(od_batch* b, int64_t nsteps) {
   OD_BCK(b, cudaEventRecord(b->ev0, b->stream));
   for (int64_t s = 0; s < nsteps; s++) OD_BCK(b, cudaGraphLaunch(b->exec, b->stream));
   OD_BCK(b, cudaEventRecord(b->ev1, b->stream));
+  OD_BCK(b, od_launch_batch_errors(b->view, b->stream));
+  uint32_t berr = 0;
+  OD_BCK(b, cudaMemcpyAsync(&berr, b->d_err, sizeof(berr), cudaMemcpyDeviceToHost, b->stream));
   OD_BCK(b, cudaStreamSynchronize(b->stream));
   float ms = 0;
   OD_BCK(b, cudaEventElapsedTime(&ms, b->ev0, b->ev1));
   b->last_ms = ms;
-  uint32_t berr = 0;
-  OD_BCK(b, cudaMemcpy(&berr, b->d_err, sizeof(berr), cudaMemcpyDeviceToHost));
-  for (od_handle* h : b->members) {
-    if (!h) continue;
-    h->step += nsteps;
-    od_status st = check_device_err(h);
-    if (st != OD_OK) return bfail(b, st, h->err);
-  }
+  for (od_handle* h : b->members)
+    if (h) h->step += nsteps;
+  if (berr)  // some member's error word, or the batch's own
+    for (od_handle* h : b->members) {
+      if (!h) continue;
+      od_status st = check_device_err(h);
+      if (st != OD_OK) return bfail(b, st, h->err);
+    }
   if (berr & OD_DERR_TIMEOUT) return bfail(b, OD_ERR_TIMEOUT, "a bounded device wait ran out");
   return OD_OK;
 }
@@ -1854,7 +1891,6 @@ extern "C" od_status od_config_device_bytes(const od_config* cfg, int64_t* bytes
   od_status st = validate(cfg);
   if (st != OD_OK) return st;
   const int64_t Np = ((cfg->n_ions + OD_PAD - 1) / OD_PAD) * OD_PAD;
-  const od_pair_plan pl = default_plan((int)Np, 152);
   const int64_t P = std::max(cfg->n_grains, 1);
   int64_t b = 0;
   if (cfg->force_method == OD_FORCE_CUTOFF) {  // tile-pair cutoff, as od_create chooses it
@@ -1866,9 +1902,9 @@ extern "C" od_status od_config_device_bytes(const od_config* cfg, int64_t* bytes
   }
   if (cfg->force_method != OD_FORCE_CUTOFF)
     b += (int64_t)(sizeof(float) * od_n3_floats((int)Np, 1));  // fixed-point accumulators
-  b += Np * 16 * 4;                 // pos, vel, fhi, flo
+  b += Np * 16 * 5;                 // pos, rel, vel, fhi, flo
   b += Np * 12;                     // SoA copy
-  b += (int64_t)pl.jsplit * Np * 32;  // partial slabs
+  b += Np * 32;                     // partial slab
   b += Np / 32 * 4 + Np * (4 + 4 + 48);  // flags, list, list bits, list positions/velocities
   b += (Np / 256) * P * 3 * 8;      // orbit partials
   b += cfg->n_steps * P * 13 * 8;   // result series
@@ -1954,8 +1990,7 @@ extern "C" od_status od_shard_create(const od_config* cfg, int64_t first, int64_
     g_err = m;
     return r;
   };
-  if (alloc_scratch_for_plan(h) != OD_OK) return bad("no device memory for the partial sums");
-  const size_t nt = (size_t)h->Npad_total, P = std::max(h->P, 1);
+    const size_t nt = (size_t)h->Npad_total, P = std::max(h->P, 1);
   if (dalloc(&h->ssx, nt) || dalloc(&h->ssy, nt) || dalloc(&h->ssz, nt) ||
       dalloc(&h->g_idx, (size_t)Nt) || dalloc(&h->g_bits, (size_t)Nt) ||
       dalloc(&h->g_old, (size_t)Nt) || dalloc(&h->g_new, (size_t)Nt) ||

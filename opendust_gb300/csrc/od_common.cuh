@@ -91,6 +91,7 @@ struct od_dstate {
   int64_t n_avg;
   int64_t n_inj_total;
   uint32_t ticket;                    // orbit blocks of K5 done this step (0 between steps)
+  uint32_t bad;                       // a non-finite value in the state being set
 };
 
 // ------------------------------------------------------------------ Philox4x32-10

@@ -36,9 +36,11 @@ struct od_dbufs {
   uint32_t* flags;                      // [nwords] ballot words
   int32_t* list;                        // [Npad] flagged ion indices, increasing
   int32_t* list_bits;                   // [Npad] flag bits of each entry
-  float4 *list_old, *list_new, *list_v; // [Npad] pre/post re-injection positions, velocities
+  float4 *list_old, *list_new, *list_v; // [Npad] pre/post re-injection positions, velocities: one
+                                        // block, between steps the FP64 staging of state copies
   double* orbit_part;                   // [nb_corr][P][3]
-  double *s_q, *s_orbit, *s_collect, *s_dust, *s_field;  // result series
+  // result series: row r of 13 P doubles holds q [P], then orbit, collect, dust, field [P][3]
+  double* series;
   float* cq;                            // [P] A_id * q_param, FP32 copy for the ion kernels
   float *sx, *sy, *sz;                  // [Npad] SoA copy of positions (all-pairs sources)
   unsigned long long* n3;               // variant 7 fixed-point accumulators [3][Npad] (or NULL)
@@ -123,6 +125,7 @@ struct od_cutn3 {
   float4 *tbox, *bbox;              // [nslots / 512][2], [nslots / 32][2] boxes
   unsigned long long* next;         // work counter of the pair kernel
   unsigned long long* acc;          // [3][nslots] fixed-point ion–ion sums per sorted slot
+  void* block;                      // the allocation that holds all of these
   double rc_d;                      // cutoff / r_D_e in FP64 (the hard cutoff's exact test)
   int grid, grid_hard;              // persistent blocks of the pair kernel (switching, hard)
 };
@@ -168,9 +171,29 @@ cudaError_t od_launch_pairs(const od_pair_plan& pl, const od_pair_io& io, int Np
 cudaError_t od_launch_pairs_probe(const od_pair_plan& pl, const od_pair_io& io, int Npad,
                                   int gridx_limit, float4* part_hi, float4* part_lo, float rho0,
                                   uint32_t* err, cudaStream_t s);
-cudaError_t od_launch_init_state(const od_dparams* dp, int N, float4* rel, float4* pos, float4* vel,
-                                 const float* vz_v, const double* vz_cdf, int vz_n, uint32_t* err,
-                                 cudaStream_t s);
+cudaError_t od_launch_init_state(const od_dparams* dp, int N, const od_dbufs& b, const float* vz_v,
+                                 const double* vz_cdf, int vz_n, uint32_t* err, cudaStream_t s);
+// FP64 host representations on the device (SI, n x 3): a non-finite entry of a sets *flag; positions
+// and velocities -> cell-relative state, absolute positions (float4 and SoA), velocities; the state
+// -> positions and velocities; a snapshot's positions -> device units (padded with sentinels up to
+// Npad; SoA copies when sx != NULL); ion–ion sums (accumulators acc, cleared, or jsplit slabs) ->
+// forces scale * sum.
+cudaError_t od_launch_state_check(const double* a, int64_t n, uint32_t* flag, cudaStream_t s);
+cudaError_t od_launch_state_in(const od_dparams* dp, int N, const double* pos, const double* vel,
+                               const od_dbufs& b, cudaStream_t s);
+cudaError_t od_launch_state_out(const od_dparams* dp, int N, const od_dbufs& b, double* pos,
+                                double* vel, cudaStream_t s);
+cudaError_t od_launch_snapshot_in(int n, int Npad, const double* pos, double lam, float4* x,
+                                  float* sx, float* sy, float* sz, cudaStream_t s);
+cudaError_t od_launch_snapshot_out(int n, int Npad, int jsplit, const float4* ph, const float4* pl,
+                                   unsigned long long* acc, double scale, double* force,
+                                   cudaStream_t s);
+// empty state of a new handle: every position a far-away sentinel
+cudaError_t od_launch_clear_state(int Npad, const od_dbufs& b, cudaStream_t s);
+// series row 0 next, averages restarted, the Philox step counter running on (od_begin_window)
+cudaError_t od_launch_begin_window(od_dstate* ds, cudaStream_t s);
+// *err |= the members' error words
+cudaError_t od_launch_batch_errors(const od_batchview& v, cudaStream_t s);
 cudaError_t od_launch_aos_to_soa(const float4* pos, int Npad, float* sx, float* sy, float* sz,
                                  cudaStream_t s);
 cudaError_t od_launch_reduce(const od_dparams* dp, int Npad, int jsplit, const float4* part_hi,

@@ -1019,10 +1019,7 @@ __device__ __forceinline__ double charge_update(const od_dparams& p, int g, doub
 // grain forces, from the host-precomputed constants.
 __device__ __forceinline__ void tail_body(const od_dparams& p, od_dstate* __restrict__ ds,
                                           const double* __restrict__ orbit_part, int nb,
-                                          double* __restrict__ s_q, double* __restrict__ s_orbit,
-                                          double* __restrict__ s_collect,
-                                          double* __restrict__ s_dust,
-                                          double* __restrict__ s_field, float* __restrict__ cq) {
+                                          double* __restrict__ series, float* __restrict__ cq) {
   __shared__ double s_red[kBlk / 32][OD_MAX_GRAINS * 3];
   __shared__ double S[OD_MAX_GRAINS * 3];
   __shared__ double qn[OD_MAX_GRAINS];
@@ -1074,14 +1071,10 @@ __device__ __forceinline__ void tail_body(const od_dparams& p, od_dstate* __rest
       vals[7 + d] = qn[g] * fd[d];
       vals[10 + d] = d == 2 ? qn[g] * p.gfield[g] : 0.0;
     }
-    const size_t r = (size_t)step * P + g;
-    s_q[r] = vals[0];
-    for (int d = 0; d < 3; d++) {
-      s_orbit[r * 3 + d] = vals[1 + d];
-      s_collect[r * 3 + d] = vals[4 + d];
-      s_dust[r * 3 + d] = vals[7 + d];
-      s_field[r * 3 + d] = vals[10 + d];
-    }
+    double* const row = series + (size_t)step * 13 * P;
+    row[g] = vals[0];
+    for (int m = 0; m < 4; m++)
+      for (int d = 0; d < 3; d++) row[P + 3 * (m * P + g) + d] = vals[1 + 3 * m + d];
     if (avg)
       for (int m = 0; m < 13; m++) ds->avg[g][m] += vals[m];
     ds->q_param[g] = qn[g];
@@ -1098,11 +1091,8 @@ __device__ __forceinline__ void tail_body(const od_dparams& p, od_dstate* __rest
 __global__ void __launch_bounds__(kBlk) k_tail(const od_dparams* __restrict__ dp,
                                                od_dstate* __restrict__ ds,
                                                const double* __restrict__ orbit_part, int nb,
-                                               double* __restrict__ s_q, double* __restrict__ s_orbit,
-                                               double* __restrict__ s_collect,
-                                               double* __restrict__ s_dust,
-                                               double* __restrict__ s_field, float* __restrict__ cq) {
-  tail_body(*dp, ds, orbit_part, nb, s_q, s_orbit, s_collect, s_dust, s_field, cq);
+                                               double* __restrict__ series, float* __restrict__ cq) {
+  tail_body(*dp, ds, orbit_part, nb, series, cq);
 }
 
 // K5 + K6: the last of the nb orbit blocks to finish (a ticket taken after its partials are
@@ -1112,9 +1102,7 @@ __global__ void __launch_bounds__(kBlk) k_correct_orbit_tail(
     const float4* __restrict__ pos, float4* __restrict__ fhi, float4* __restrict__ flo,
     const uint32_t* __restrict__ flags, const int32_t* __restrict__ list,
     const float4* __restrict__ list_old, const float4* __restrict__ list_new,
-    double* __restrict__ orbit_part, int nb, double* __restrict__ s_q,
-    double* __restrict__ s_orbit, double* __restrict__ s_collect, double* __restrict__ s_dust,
-    double* __restrict__ s_field, float* __restrict__ cq) {
+    double* __restrict__ orbit_part, int nb, double* __restrict__ series, float* __restrict__ cq) {
   od_pdl_wait();
   correct_orbit_body(*dp, ds, pos, fhi, flo, flags, list, list_old, list_new, orbit_part, nb,
                      blockIdx.x, gridDim.x - nb);
@@ -1128,7 +1116,7 @@ __global__ void __launch_bounds__(kBlk) k_correct_orbit_tail(
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  tail_body(*dp, ds, orbit_part, nb, s_q, s_orbit, s_collect, s_dust, s_field, cq);
+  tail_body(*dp, ds, orbit_part, nb, series, cq);
   if (threadIdx.x == 0) ds->ticket = 0u;
 }
 
@@ -1190,6 +1178,8 @@ __global__ void __launch_bounds__(kBlk) k_init_state(const od_dparams* __restric
                                                      float4* __restrict__ rel,
                                                      float4* __restrict__ pos,
                                                      float4* __restrict__ vel,
+                                                     float* __restrict__ sx, float* __restrict__ sy,
+                                                     float* __restrict__ sz,
                                                      const float* __restrict__ vz_v,
                                                      const double* __restrict__ vz_cdf, int vz_n,
                                                      uint32_t* __restrict__ err) {
@@ -1228,16 +1218,18 @@ __global__ void __launch_bounds__(kBlk) k_init_state(const od_dparams* __restric
   }
   const float4 r = od_rel_encode(p, x.x, x.y, x.z);
   rel[i] = r;
-  pos[i] = od_rel_abs(p, r);
+  x = od_rel_abs(p, r);
+  pos[i] = x;
+  sx[i] = x.x; sy[i] = x.y; sz[i] = x.z;
   vel[i] = make_float4(p.vT * gx, p.vT * gy, vz, 0.f);
 }
 
 }  // namespace
 
-cudaError_t od_launch_init_state(const od_dparams* dp, int N, float4* rel, float4* pos,
-                                 float4* vel, const float* vz_v, const double* vz_cdf, int vz_n,
-                                 uint32_t* err, cudaStream_t s) {
-  k_init_state<<<(N + kBlk - 1) / kBlk, kBlk, 0, s>>>(dp, rel, pos, vel, vz_v, vz_cdf, vz_n, err);
+cudaError_t od_launch_init_state(const od_dparams* dp, int N, const od_dbufs& b, const float* vz_v,
+                                 const double* vz_cdf, int vz_n, uint32_t* err, cudaStream_t s) {
+  k_init_state<<<(N + kBlk - 1) / kBlk, kBlk, 0, s>>>(dp, b.rel, b.pos, b.vel, b.sx, b.sy, b.sz, vz_v,
+                                                      vz_cdf, vz_n, err);
   return cudaGetLastError();
 }
 
@@ -1377,8 +1369,7 @@ cudaError_t od_launch_step_part(int part, const od_dparams* dp, od_dstate* ds, c
     e = od_launch_pdl(k_correct_orbit_tail, dim3(nb + nrec), dim3(kBlk), s, dp, ds,
                       (const float4*)b.pos, b.fhi, b.flo, (const uint32_t*)b.flags,
                       (const int32_t*)b.list, (const float4*)b.list_old,
-                      (const float4*)b.list_new, b.orbit_part, nb, b.s_q, b.s_orbit,
-                      b.s_collect, b.s_dust, b.s_field, b.cq);
+                      (const float4*)b.list_new, b.orbit_part, nb, b.series, b.cq);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
@@ -1571,8 +1562,7 @@ __global__ void __launch_bounds__(kBlk) k_b_correct_orbit(const od_simdesc* __re
 
 __global__ void __launch_bounds__(kBlk) k_b_tail(const od_simdesc* __restrict__ sims) {
   const od_simdesc& d = sims[blockIdx.x];
-  tail_body(*d.dp, d.ds, d.b.orbit_part, d.nb, d.b.s_q, d.b.s_orbit, d.b.s_collect, d.b.s_dust,
-            d.b.s_field, d.b.cq);
+  tail_body(*d.dp, d.ds, d.b.orbit_part, d.nb, d.b.series, d.b.cq);
 }
 
 }  // namespace
@@ -1621,6 +1611,167 @@ cudaError_t od_launch_batch_step(const od_batchview& v, cudaStream_t s) {
   k_b_collect_inject<<<v.nsims, kCT, 0, s>>>(v.sims);
   k_b_correct_orbit<<<v.nblk_corr, kBlk, 0, s>>>(v.sims, v.blk_corr);
   k_b_tail<<<v.nsims, kBlk, 0, s>>>(v.sims);
+  return cudaGetLastError();
+}
+
+// ============================================================== host representations
+// The FP64 SI arrays of the C ABI to and from the device state, one thread per ion. Bound by
+// memory: 48 B per ion over the host link (about 180 GB/s) and 96 B in HBM. On the host the same
+// conversions took most of a small call: 70001 ions, snapshot without its pair kernel 0.45 ms,
+// now 0.1 ms. Every operation is rounded as the host code (-ffp-contract=off) rounds it.
+namespace {
+__global__ void __launch_bounds__(kBlk) k_state_check(const double* __restrict__ a, int64_t n,
+                                                      uint32_t* __restrict__ flag) {
+  const int64_t i = blockIdx.x * (int64_t)kBlk + threadIdx.x;
+  if (i < n && !isfinite(a[i])) atomicOr(flag, 1u);
+}
+
+// Cell-relative state (od_common.cuh) of positions in metres, and the absolute FP32 positions
+// derived from it: per axis, c = floor(x / s) and the offset x - c s rounded once to FP32 (from
+// the FP64 position, so nothing is lost to an FP32 absolute first).
+__global__ void __launch_bounds__(kBlk) k_state_in(const od_dparams* __restrict__ dp,
+                                                   const double* __restrict__ pos,
+                                                   const double* __restrict__ vel,
+                                                   float4* __restrict__ rel, float4* __restrict__ x,
+                                                   float4* __restrict__ v, float* __restrict__ sx,
+                                                   float* __restrict__ sy, float* __restrict__ sz) {
+  const int i = blockIdx.x * kBlk + threadIdx.x;
+  if (i >= dp->N) return;
+  const double lam = dp->lam, vu = dp->vunit, s = dp->rel_s, inv = dp->rel_inv;
+  int c[3];
+  float o[3], a[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const double u = __ddiv_rn(pos[3 * (size_t)i + d], lam);
+    c[d] = od_rel_clamp((int)fmax(fmin(floor(__dmul_rn(u, inv)), 1e9), -1e9));
+    o[d] = __double2float_rn(__dsub_rn(u, __dmul_rn((double)c[d], s)));
+    if (o[d] == (float)s && c[d] < OD_REL_BIAS - 1) { c[d] += 1; o[d] = 0.f; }
+    a[d] = __double2float_rn(__fma_rn((double)c[d], s, (double)o[d]));  // exact, then rounded once
+  }
+  rel[i] = make_float4(o[0], o[1], o[2], __int_as_float(od_rel_pack(c[0], c[1], c[2])));
+  x[i] = make_float4(a[0], a[1], a[2], 0.f);
+  sx[i] = a[0]; sy[i] = a[1]; sz[i] = a[2];
+  v[i] = make_float4(__double2float_rn(__ddiv_rn(vel[3 * (size_t)i], vu)),
+                     __double2float_rn(__ddiv_rn(vel[3 * (size_t)i + 1], vu)),
+                     __double2float_rn(__ddiv_rn(vel[3 * (size_t)i + 2], vu)), 0.f);
+}
+
+__global__ void __launch_bounds__(kBlk) k_state_out(const od_dparams* __restrict__ dp,
+                                                    const float4* __restrict__ rel,
+                                                    const float4* __restrict__ v,
+                                                    double* __restrict__ pos,
+                                                    double* __restrict__ vel) {
+  const int i = blockIdx.x * kBlk + threadIdx.x;
+  if (i >= dp->N) return;
+  const double lam = dp->lam, vu = dp->vunit, s = dp->rel_s;
+  if (pos) {  // the cell-relative state, exactly (c s + offset is exact in FP64)
+    const float4 r = rel[i];
+    const int3 c = od_rel_cells(r.w);
+    pos[3 * (size_t)i] = __dmul_rn(__dadd_rn(__dmul_rn((double)c.x, s), (double)r.x), lam);
+    pos[3 * (size_t)i + 1] = __dmul_rn(__dadd_rn(__dmul_rn((double)c.y, s), (double)r.y), lam);
+    pos[3 * (size_t)i + 2] = __dmul_rn(__dadd_rn(__dmul_rn((double)c.z, s), (double)r.z), lam);
+  }
+  if (vel) {
+    const float4 u = v[i];
+    vel[3 * (size_t)i] = __dmul_rn((double)u.x, vu);
+    vel[3 * (size_t)i + 1] = __dmul_rn((double)u.y, vu);
+    vel[3 * (size_t)i + 2] = __dmul_rn((double)u.z, vu);
+  }
+}
+
+__global__ void __launch_bounds__(kBlk) k_snapshot_in(int n, int Npad,
+                                                      const double* __restrict__ pos, double lam,
+                                                      float4* __restrict__ x, float* __restrict__ sx,
+                                                      float* __restrict__ sy, float* __restrict__ sz) {
+  const int i = blockIdx.x * kBlk + threadIdx.x;
+  if (i >= Npad) return;
+  float4 q = make_float4(OD_SENTINEL, OD_SENTINEL, OD_SENTINEL, 0.f);
+  if (i < n)
+    q = make_float4(__double2float_rn(__ddiv_rn(pos[3 * (size_t)i], lam)),
+                    __double2float_rn(__ddiv_rn(pos[3 * (size_t)i + 1], lam)),
+                    __double2float_rn(__ddiv_rn(pos[3 * (size_t)i + 2], lam)), 0.f);
+  x[i] = q;
+  if (sx) { sx[i] = q.x; sy[i] = q.y; sz[i] = q.z; }
+}
+
+__global__ void __launch_bounds__(kBlk) k_snapshot_out(int n, int Npad, int jsplit,
+                                                       const float4* __restrict__ ph,
+                                                       const float4* __restrict__ pl,
+                                                       unsigned long long* __restrict__ acc,
+                                                       double scale, double* __restrict__ force) {
+  const int i = blockIdx.x * kBlk + threadIdx.x;
+  if (i >= Npad) return;
+  float3 hi, lo;
+  if (acc) od_fix_take(acc + i, (size_t)Npad, hi, lo);
+  else if (i < n) reduce_parts(ph, pl, Npad, jsplit, i, hi, lo);
+  if (i >= n) return;
+  force[3 * (size_t)i] = __dmul_rn(scale, __dadd_rn((double)hi.x, (double)lo.x));
+  force[3 * (size_t)i + 1] = __dmul_rn(scale, __dadd_rn((double)hi.y, (double)lo.y));
+  force[3 * (size_t)i + 2] = __dmul_rn(scale, __dadd_rn((double)hi.z, (double)lo.z));
+}
+
+__global__ void __launch_bounds__(kBlk) k_clear_state(int Npad, float4* __restrict__ x,
+                                                      float* __restrict__ sx,
+                                                      float* __restrict__ sy,
+                                                      float* __restrict__ sz) {
+  const int i = blockIdx.x * kBlk + threadIdx.x;
+  if (i >= Npad) return;
+  x[i] = make_float4(OD_SENTINEL, OD_SENTINEL, OD_SENTINEL, 0.f);
+  sx[i] = sy[i] = sz[i] = OD_SENTINEL;
+}
+
+__global__ void k_begin_window(od_dstate* __restrict__ ds) {
+  if (threadIdx.x == 0) {
+    ds->rng_base += ds->step;
+    ds->step = 0;
+    ds->n_avg = 0;
+  }
+  for (int k = threadIdx.x; k < OD_MAX_GRAINS * 13; k += blockDim.x) (&ds->avg[0][0])[k] = 0.0;
+}
+
+__global__ void k_b_errors(const od_simdesc* __restrict__ sims, int n, uint32_t* __restrict__ err) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m < n && sims[m].ds->err) atomicOr(err, sims[m].ds->err);
+}
+}  // namespace
+
+static unsigned blocks_of(int64_t n) { return (unsigned)((n + kBlk - 1) / kBlk); }
+
+cudaError_t od_launch_state_check(const double* a, int64_t n, uint32_t* flag, cudaStream_t s) {
+  k_state_check<<<blocks_of(n), kBlk, 0, s>>>(a, n, flag);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_state_in(const od_dparams* dp, int N, const double* pos, const double* vel,
+                               const od_dbufs& b, cudaStream_t s) {
+  k_state_in<<<blocks_of(N), kBlk, 0, s>>>(dp, pos, vel, b.rel, b.pos, b.vel, b.sx, b.sy, b.sz);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_state_out(const od_dparams* dp, int N, const od_dbufs& b, double* pos,
+                                double* vel, cudaStream_t s) {
+  k_state_out<<<blocks_of(N), kBlk, 0, s>>>(dp, b.rel, b.vel, pos, vel);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_snapshot_in(int n, int Npad, const double* pos, double lam, float4* x,
+                                  float* sx, float* sy, float* sz, cudaStream_t s) {
+  k_snapshot_in<<<blocks_of(Npad), kBlk, 0, s>>>(n, Npad, pos, lam, x, sx, sy, sz);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_snapshot_out(int n, int Npad, int jsplit, const float4* ph, const float4* pl,
+                                   unsigned long long* acc, double scale, double* force,
+                                   cudaStream_t s) {
+  k_snapshot_out<<<blocks_of(Npad), kBlk, 0, s>>>(n, Npad, jsplit, ph, pl, acc, scale, force);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_clear_state(int Npad, const od_dbufs& b, cudaStream_t s) {
+  k_clear_state<<<blocks_of(Npad), kBlk, 0, s>>>(Npad, b.pos, b.sx, b.sy, b.sz);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_begin_window(od_dstate* ds, cudaStream_t s) {
+  k_begin_window<<<1, 256, 0, s>>>(ds);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_batch_errors(const od_batchview& v, cudaStream_t s) {
+  k_b_errors<<<(v.nsims + 255) / 256, 256, 0, s>>>(v.sims, v.nsims, v.err);
   return cudaGetLastError();
 }
 
@@ -1730,8 +1881,7 @@ cudaError_t od_launch_shard_correct(const od_dparams* dp, const od_dstate* ds, c
 
 cudaError_t od_launch_shard_tail(const od_dparams* dp, od_dstate* ds, const od_dbufs& b,
                                  const double* orbit_all, int nb_all, cudaStream_t s) {
-  k_tail<<<1, kBlk, 0, s>>>(dp, ds, orbit_all, nb_all, b.s_q, b.s_orbit, b.s_collect, b.s_dust,
-                           b.s_field, b.cq);
+  k_tail<<<1, kBlk, 0, s>>>(dp, ds, orbit_all, nb_all, b.series, b.cq);
   return cudaGetLastError();
 }
 
