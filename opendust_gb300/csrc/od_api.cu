@@ -1088,6 +1088,11 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
     c.take(L->bbox, ns / 32 * 2);
     c.take(L->next, 1);
     c.take(L->acc, 3 * ns);
+    if (od_cutn3_listed(ns)) {
+      c.take(L->rows, ns / 64 * (ns / 32));
+      c.take(L->counts, ns / 64);
+      c.take(L->prefix, ns / 64 + 1);
+    }
   });
   if (e == cudaSuccess)
     e = cudaMemsetAsync(L->acc, 0, sizeof(unsigned long long) * 3 * ns, h->stream);

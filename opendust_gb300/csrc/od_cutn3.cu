@@ -13,10 +13,10 @@
 // What bounds it: as the all-pairs kernel, operand fetch of the packed FP32 pipe (17 packed
 // operations per pair of pairs for the plain term, 27 with switching), plus the pairs of the
 // listed blocks that lie beyond the cutoff. field_chain (2^19 ions, 2 lambda): 1.63 pairs
-// evaluated per pair inside, 22.7 ms per evaluation. The tile-pair form this replaces (512-ion
+// evaluated per pair inside, 22.6 ms per evaluation. The tile-pair form this replaces (512-ion
 // tile pairs, 64 x 64 group lists built by one warp between two block barriers, 2 x 2 ions per
 // lane, sums in shared memory with compare-and-swap atomics) took 32.2 ms there; 65536 ions in
-// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.82 ms, 20011 ions at 2 lambda 0.197 -> 0.120 ms.
+// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.79 ms, 20011 ions at 2 lambda 0.197 -> 0.105 ms.
 #include "od_hilbert.h"
 #include "od_internal.h"
 #include <algorithm>
@@ -279,21 +279,22 @@ __device__ __forceinline__ void cut_pair(const cut_consts& k, od_u64 X, od_u64 Y
   if (REACT) { RX = fma2(C, DX, RX); RY = fma2(C, DY, RY); RZ = fma2(C, DZ, RZ); }
 }
 
-// Hard cutoff, the exact pass of a batch: pairs whose FP32 r^2 lies within `band` of r_c^2 are
+// Hard cutoff, the exact pass of half a batch: pairs whose FP32 r^2 lies within `band` of r_c^2 are
 // decided as the FP64 reference decides them and added straight to the accumulators, so that both
-// include the same pairs (rare: about 1 batch in 25 at field_chain has such a pair).
-template <int MT, bool REACT, bool COUNT>
+// include the same pairs (rare: about 1 half in 50 at field_chain has such a pair).
+template <bool REACT, bool COUNT>
 __device__ __noinline__ void exact_pass(const float* __restrict__ xs, const float* __restrict__ ys,
                                         const float* __restrict__ zs, size_t ns,
                                         unsigned long long* __restrict__ acc, const cut_args& cut,
-                                        int sg, const unsigned int* tb, int nb, unsigned int& cnt) {
+                                        int sg, const unsigned int* tb, int nb, int half,
+                                        unsigned int& cnt) {
   const int lane = threadIdx.x & 31;
   const float band = cut.rc2 * 2e-6f;
   for (int t = 0; t < nb; t++) {
     const int ti = (int)tb[t] * kBlk + lane;
     const float px = xs[ti], py = ys[ti], pz = zs[ti];
-    for (int j = 0; j < 64; j++) {
-      const int sj = sg * 64 + (j & 32) + ((lane + j) & 31);
+    for (int j = 0; j < 32; j++) {  // 16 lane steps, two sources each
+      const int sj = sg * 64 + 2 * (j & 16) + ((lane + 16 * half + (j & 15)) & 31);
       const float sx = xs[sj], sy = ys[sj], sz = zs[sj];
       const float dx = px - sx, dy = py - sy, dz = pz - sz;
       const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
@@ -312,8 +313,8 @@ __device__ __noinline__ void exact_pass(const float* __restrict__ xs, const floa
   }
 }
 
-// MT target blocks tb[0 .. nb) (nb <= MT, the rest empty) against the 64 slots of source group sg.
-// Reactions are summed in FP32 over 16 lane steps and added to the accumulators of the sources where
+// MT target blocks tb[0 .. nb) (nb <= MT, the rest empty) against the 64 slots of source group sg:
+// halves [h0, h1) of the 32 lane steps. Reactions are summed in FP32 over 16 lane steps and added to the accumulators of the sources where
 // they stand (shorter chains than the 32 steps they could take: at 2^19 ions the median per-ion
 // error is 0.8 of that and the kernel 1 % slower).
 template <int MT, int CUT, bool REACT, bool COUNT, int UNROLL>
@@ -322,7 +323,7 @@ __device__ __forceinline__ void cut_batch(const cut_consts& k, const float* __re
                                           const float* __restrict__ zs, size_t ns,
                                           unsigned long long* __restrict__ acc,
                                           const cut_args& cut, int sg, const unsigned int* tb,
-                                          int nb, unsigned int& cnt) {
+                                          int nb, unsigned int& cnt, int h0 = 0, int h1 = 2) {
   const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
   od_u64 X[MT], Y[MT], Z[MT], AX[MT], AY[MT], AZ[MT];
 #pragma unroll
@@ -335,12 +336,12 @@ __device__ __forceinline__ void cut_batch(const cut_consts& k, const float* __re
     X[t] = p2(x, x); Y[t] = p2(y, y); Z[t] = p2(z, z);
     AX[t] = AY[t] = AZ[t] = 0ull;
   }
-  const int j = sg * 64 + lane;
+  const int j = sg * 64 + ((lane + 16 * h0) & 31);
   od_u64 QX = p2(xs[j], xs[j + 32]), QY = p2(ys[j], ys[j + 32]), QZ = p2(zs[j], zs[j + 32]);
-  float near = 3e38f;
 #pragma unroll 1
-  for (int part = 16; part <= 32; part += 16) {
+  for (int h = h0; h < h1; h++) {
     od_u64 RX = 0ull, RY = 0ull, RZ = 0ull;
+    float near = 3e38f;
 #pragma unroll UNROLL
     for (int st = 0; st < 16; st++) {
 #pragma unroll
@@ -352,14 +353,14 @@ __device__ __forceinline__ void cut_batch(const cut_consts& k, const float* __re
     }
     if (REACT) {  // the force on the sources is minus the accumulated terms
       const float2 rx = up2(RX), ry = up2(RY), rz = up2(RZ);
-      unsigned long long* a = acc + sg * 64 + ((lane + part) & 31);
+      unsigned long long* a = acc + sg * 64 + ((lane + 16 * h + 16) & 31);
       od_fix_add1(a, -rx.x); od_fix_add1(a + 32, -rx.y);
       od_fix_add1(a + ns, -ry.x); od_fix_add1(a + ns + 32, -ry.y);
       od_fix_add1(a + 2 * ns, -rz.x); od_fix_add1(a + 2 * ns + 32, -rz.y);
     }
+    if (CUT == 2 && __any_sync(0xffffffffu, near <= k.band))
+      exact_pass<REACT, COUNT>(xs, ys, zs, ns, acc, cut, sg, tb, nb, h, cnt);
   }
-  if (CUT == 2 && __any_sync(0xffffffffu, near <= k.band))
-    exact_pass<MT, REACT, COUNT>(xs, ys, zs, ns, acc, cut, sg, tb, nb, cnt);
 #pragma unroll
   for (int t = 0; t < MT; t++)
     if (t < nb) {
@@ -386,19 +387,26 @@ __device__ __forceinline__ void box_dist(const float4* __restrict__ box, int i, 
   }
 }
 
+// box of source group sg
+__device__ __forceinline__ void group_box(const float4* __restrict__ bbox, int sg, float (&b)[6]) {
+  const float4 p = bbox[4 * sg], q = bbox[4 * sg + 1], r = bbox[4 * sg + 2], s = bbox[4 * sg + 3];
+  b[0] = fminf(p.x, r.x); b[1] = fminf(p.y, r.y); b[2] = fminf(p.z, r.z);
+  b[3] = fmaxf(p.w, r.w); b[4] = fmaxf(q.x, s.x); b[5] = fmaxf(q.y, s.y);
+}
+
 // Units: source group sg (row a = sg / 8) and its c-th run of B tiles from tile a on, numbered run by
 // run over the groups, c = 0 first. Units before run c: 8 (c nT - B c (c - 1) / 2).
 __host__ __device__ __forceinline__ long long units_before(long long c, int nT, int B) {
   return 8 * (c * nT - B * (c * (c - 1) / 2));
 }
 
-// registers: warps per SM and unrolling. field_chain, ms per evaluation: switching 22.8 with 20 warps
-// and two steps, 22.7 with 24 and one or two, 24.5 with 16; 20011 ions 0.120, 0.130, 0.124; hard cutoff
-// 21.8 with 24 warps and one step, 22.6 with 20 and 23.4 with 16 (without the vote).
+// Registers: resident warps and unrolling. field_chain, ms per evaluation: switching 22.6 with 24 warps per
+// SM and two lane steps (22.9 with 20, 22.5 with 28 and one step, 24.5 with 16), hard cutoff 20.5 with 20
+// and one step (21.2 with 24 and two); 65536 ions at 2 lambda 0.594 and 0.548 ms.
 template <int CUT>
 struct cut_traits {
   static constexpr int WARPS = 4;  // per block; they share nothing
-  static constexpr int MIN_BLOCKS = CUT == 2 ? 6 : 5;
+  static constexpr int MIN_BLOCKS = CUT == 2 ? 5 : 6;
   static constexpr int UNROLL = CUT == 2 ? 1 : 2;
 };
 
@@ -433,12 +441,8 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
       b0 = (sg >> 3) + c * B;
       b1 = min(b0 + B, nT);
     }
-    float sb[6];  // box of the source group
-    {
-      const float4 p = bbox[4 * sg], q = bbox[4 * sg + 1], r = bbox[4 * sg + 2], s = bbox[4 * sg + 3];
-      sb[0] = fminf(p.x, r.x); sb[1] = fminf(p.y, r.y); sb[2] = fminf(p.z, r.z);
-      sb[3] = fmaxf(p.w, r.w); sb[4] = fmaxf(q.x, s.x); sb[5] = fmaxf(q.y, s.y);
-    }
+    float sb[6];
+    group_box(bbox, sg, sb);
     unsigned int tiles;
     {
       float d2 = 3e38f, f2;
@@ -499,6 +503,159 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
   }
 }
 
+// ------------------------------------------------------------------ small systems: listed work
+// Up to kListBlocks blocks the units above are too coarse: a warp gets a few batches, and the last ones
+// run alone (force chain of 8192 ions at 2 lambda 0.132 ms). Here one warp per source group lists its
+// target blocks first (inner ones from the front of its row, the others from the back), the last block to
+// finish takes the prefix over the groups, and the warps of the pair kernel draw runs of equal length from
+// it: half batches where there are fewer than four per warp (8192 ions 0.069 ms; whole batches 0.077), else
+// whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635 with the units).
+constexpr int kListBlocks = 4096;
+__global__ void __launch_bounds__(256) k_cut_lists(int nsg, int nT, const cut_args cut,
+                                                   const float4* __restrict__ tbox,
+                                                   const float4* __restrict__ bbox,
+                                                   uint16_t* __restrict__ rows,
+                                                   int2* __restrict__ cnt, int* __restrict__ prefix,
+                                                   unsigned long long* __restrict__ ticket) {
+  __shared__ int s_w[8];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int sg = blockIdx.x * 8 + w, nB = nT * kTB;
+  if (sg < nsg) {
+    float sb[6];
+    group_box(bbox, sg, sb);
+    uint16_t* const row = rows + (size_t)sg * nB;
+    int ni = 0, no = 0;
+    for (int b0 = sg >> 3; b0 < nT; b0 += 32) {
+      float d2 = 3e38f, f2;
+      if (b0 + lane < nT) box_dist(tbox, b0 + lane, sb, d2, f2);
+      unsigned int tiles = __ballot_sync(0xffffffffu, d2 < cut.cull2);
+      while (tiles) {
+        const int t1 = __ffs(tiles) - 1;
+        tiles &= tiles - 1;
+        const int t2 = tiles ? __ffs(tiles) - 1 : -1;
+        if (tiles) tiles &= tiles - 1;
+        const int tl = lane < 16 ? t1 : t2;
+        const int blk = (b0 + tl) * kTB + (lane & 15);
+        d2 = f2 = 3e38f;
+        if (tl >= 0 && blk > 2 * sg + 1) box_dist(bbox, blk, sb, d2, f2);
+        const bool keep = d2 < cut.cull2, inner = keep && f2 < cut.in2;
+        const unsigned int mi = __ballot_sync(0xffffffffu, inner),
+                           mo = __ballot_sync(0xffffffffu, keep && !inner);
+        const unsigned int below = (1u << lane) - 1u;
+        if (inner) row[ni + __popc(mi & below)] = (uint16_t)blk;
+        else if (keep) row[nB - 1 - no - __popc(mo & below)] = (uint16_t)blk;
+        ni += __popc(mi);
+        no += __popc(mo);
+      }
+    }
+    if (lane == 0) cnt[sg] = make_int2(ni, no);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *ticket = 0ull;  // the pair kernel's work counter from here on
+  // half batches of each group: the group itself, the inner fours, the rest
+  const int per = (nsg + 255) / 256, g0 = min((int)threadIdx.x * per, nsg), g1 = min(g0 + per, nsg);
+  int sum = 0;
+  for (int g = g0; g < g1; g++) {
+    const int2 c = __ldcg(cnt + g);
+    sum += 2 * (1 + c.x / 4 + (c.y + (c.x & 3) + 3) / 4);
+  }
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_w[w] = incl;
+  __syncthreads();
+  int off = incl - sum;
+  for (int k = 0; k < w; k++) off += s_w[k];
+  for (int g = g0; g < g1; g++) {
+    const int2 c = __ldcg(cnt + g);
+    prefix[g] = off;
+    off += 2 * (1 + c.x / 4 + (c.y + (c.x & 3) + 3) / 4);
+  }
+  if (g1 == nsg && g0 < nsg) prefix[nsg] = off;
+}
+
+template <int CUT, bool COUNT>
+__global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::MIN_BLOCKS)
+    k_pairs_cutlist(const float* __restrict__ xs, const float* __restrict__ ys,
+                    const float* __restrict__ zs, int nslots, unsigned long long* __restrict__ acc,
+                    const __grid_constant__ cut_args cut, const uint16_t* __restrict__ rows,
+                    const int2* __restrict__ counts, const int* __restrict__ prefix,
+                    unsigned int* __restrict__ next,
+                    unsigned long long* __restrict__ pair_count) {
+  constexpr int WARPS = cut_traits<CUT>::WARPS, UNROLL = cut_traits<CUT>::UNROLL;
+  __shared__ int s_prefix[kListBlocks / 2 + 1];
+  __shared__ unsigned int s_tb[WARPS][4];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nsg = nslots / 64, nB = nslots / kBlk;
+  for (int g = threadIdx.x; g <= nsg; g += WARPS * 32) s_prefix[g] = prefix[g];
+  __syncthreads();
+  unsigned int* const tb = s_tb[w];
+  const cut_consts k = make_consts(cut);
+  unsigned int cnt = 0;
+  const int Q = s_prefix[nsg], W = gridDim.x * WARPS;
+  const int run = Q < 4 * W ? 1 : max(2, (Q / (W * 32)) & ~1);
+  for (;;) {
+    int q = 0;
+    if (lane == 0) q = (int)min(atomicAdd(next, 1u), (unsigned)Q) * run;
+    q = __shfl_sync(0xffffffffu, q, 0);
+    if (q >= Q) break;
+    const int q1 = min(q + run, Q);
+    int sg = 0;
+    for (int hi = nsg; hi - sg > 1;) {  // the group whose range holds q
+      const int mid = (sg + hi) >> 1;
+      if (s_prefix[mid] <= q) sg = mid;
+      else hi = mid;
+    }
+    while (q < q1) {
+      while (s_prefix[sg + 1] <= q) sg++;
+      const int r = q - s_prefix[sg], b = r >> 1, h0 = r & 1;
+      const int h1 = min(2, h0 + q1 - q);
+      const int2 c = counts[sg];
+      const int fours = c.x >> 2, rest = c.x & 3;
+      const uint16_t* const row = rows + (size_t)sg * nB;
+      int nb = 4;
+      __syncwarp();
+      if (b == 0) {  // the group itself
+        nb = 2;
+        if (lane < 2) tb[lane] = 2 * sg + lane;
+      } else if (b <= fours) {
+        if (lane < 4) tb[lane] = row[4 * (b - 1) + lane];
+      } else {  // the inner blocks that fill no batch, then the others
+        const int at = 4 * (b - 1 - fours);
+        nb = min(4, c.y + rest - at);
+        if (lane < nb)
+          tb[lane] = at + lane < rest ? row[4 * fours + at + lane] : row[nB - 1 - (at + lane - rest)];
+      }
+      __syncwarp();
+      if (b == 0)
+        cut_batch<2, CUT, false, COUNT, 1>(k, xs, ys, zs, nslots, acc, cut, sg, tb, 2, cnt, h0, h1);
+      else if (b <= fours)
+        cut_batch<4, 0, true, COUNT, UNROLL>(k, xs, ys, zs, nslots, acc, cut, sg, tb, 4, cnt, h0, h1);
+      else if (nb > 2)
+        cut_batch<4, CUT, true, COUNT, UNROLL>(k, xs, ys, zs, nslots, acc, cut, sg, tb, nb, cnt, h0,
+                                               h1);
+      else
+        cut_batch<2, CUT, true, COUNT, 1>(k, xs, ys, zs, nslots, acc, cut, sg, tb, nb, cnt, h0, h1);
+      q += h1 - h0;
+    }
+  }
+  if (COUNT) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
+    if (lane == 0 && cnt) atomicAdd(pair_count, (unsigned long long)cnt);
+  }
+}
+
 // Slot accumulators -> the ions' entries of (ph, pl) as two-float sums (slot s holds ion
 // perm[s], -1 for the sentinels in the tail), every slot cleared for the next evaluation.
 __global__ void __launch_bounds__(256) k_slot_take(int nslots, unsigned long long* __restrict__ acc,
@@ -530,10 +687,18 @@ od_cgrid od_cutn3_grid(int N, double R, double H) {
   return g;
 }
 
+bool od_cutn3_listed(size_t nslots) { return nslots / kBlk <= kListBlocks; }
+static size_t od_cutn3_list_bytes(size_t ns) {
+  const size_t nsg = ns / 64, nB = ns / kBlk;
+  return od_cutn3_listed(ns) ? sizeof(uint16_t) * nsg * nB + sizeof(int2) * nsg + sizeof(int) * (nsg + 1)
+                             : 0;
+}
+
 size_t od_cutn3_bytes(int N, int T, int ncells) {
   const size_t ns = (size_t)((N + T - 1) / T) * T, nc = (size_t)ncells;
   return sizeof(unsigned long long) * (3 * ns + 1)                    // accumulators, work counter
          + sizeof(float4) * 2 * (ns / kBlk + ns / kTile)              // boxes
+         + od_cutn3_list_bytes(ns)
          + sizeof(float) * 3 * ns                                     // sorted positions
          + sizeof(int32_t) * (ns + N + 3 * nc + 1);
 }
@@ -554,6 +719,17 @@ int od_cutn3_blocks_per_sm(bool hard) {
   return e == cudaSuccess && nb > 0 ? nb : 5;
 }
 
+#define OD_CUTN3_FORMS()                       \
+  do {                                         \
+    if (sw) {                                  \
+      if (pair_count) OD_CUTN3(1, true);       \
+      else OD_CUTN3(1, false);                 \
+    } else {                                   \
+      if (pair_count) OD_CUTN3(2, true);       \
+      else OD_CUTN3(2, false);                 \
+    }                                          \
+  } while (0)
+
 cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, float4* part_hi,
                                 float4* part_lo, float rho0, float rc, float rs, uint32_t* err,
                                 unsigned long long* pair_count, cudaStream_t s) {
@@ -572,21 +748,27 @@ cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, flo
   const float rin = (sw ? rs : rc) * (1.0f - 1e-5f);
   const cut_args cut{rho0, rc * rc, rs, sw ? 1.0f / (rc - rs) : 0.0f, rin * rin,
                      rc * rc * 1.00001f, L.rc_d};
-  // tiles per unit: one up to 256 tiles (65536 ions 0.82 ms, 0.89 with two), then more so that the
-  // units, most of them empty, stay few beside the work (2^19 ions: no difference from 4 to 16)
-  const int B = std::min(32, std::max(1, nT / 128));
-  const long long nunits = units_before((nT + B - 1) / B, nT, B);
-#define OD_CUTN3(CUT, CNT)                                                                      \
-  k_pairs_cutn3<CUT, CNT><<<CUT == 2 ? L.grid_hard : L.grid, cut_traits<CUT>::WARPS * 32, 0, s>>>( \
-      L.xs, L.ys, L.zs, L.nslots, nT, B, nunits, L.next, L.acc, cut, L.tbox, L.bbox, pair_count)
-  if (sw) {
-    if (pair_count) OD_CUTN3(1, true);
-    else OD_CUTN3(1, false);
-  } else {
-    if (pair_count) OD_CUTN3(2, true);
-    else OD_CUTN3(2, false);
-  }
+  const int grid = sw ? L.grid : L.grid_hard;
+  if (L.rows) {
+    const int nsg = L.nslots / 64;
+    k_cut_lists<<<(nsg + 7) / 8, 256, 0, s>>>(nsg, nT, cut, L.tbox, L.bbox, L.rows, L.counts, L.prefix,
+                                              L.next);
+#define OD_CUTN3(CUT, CNT)                                                              \
+  k_pairs_cutlist<CUT, CNT><<<grid, cut_traits<CUT>::WARPS * 32, 0, s>>>(               \
+      L.xs, L.ys, L.zs, L.nslots, L.acc, cut, L.rows, L.counts, L.prefix, (unsigned int*)L.next, pair_count)
+    OD_CUTN3_FORMS();
 #undef OD_CUTN3
+  } else {
+    // tiles per unit: more in larger systems, so that the units, most of them empty, stay few beside
+    // the work (2^19 ions: no difference from 4 to 16)
+    const int B = std::min(32, std::max(1, nT / 128));
+    const long long nunits = units_before((nT + B - 1) / B, nT, B);
+#define OD_CUTN3(CUT, CNT)                                                              \
+  k_pairs_cutn3<CUT, CNT><<<grid, cut_traits<CUT>::WARPS * 32, 0, s>>>(                 \
+      L.xs, L.ys, L.zs, L.nslots, nT, B, nunits, L.next, L.acc, cut, L.tbox, L.bbox, pair_count)
+    OD_CUTN3_FORMS();
+#undef OD_CUTN3
+  }
   k_slot_take<<<(L.nslots + 255) / 256, 256, 0, s>>>(L.nslots, L.acc, L.perm, part_hi, part_lo);
   return cudaGetLastError();
 }

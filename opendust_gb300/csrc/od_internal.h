@@ -123,7 +123,12 @@ struct od_cutn3 {
   int32_t* perm;                    // [nslots] ion of each sorted slot, -1 for sentinels
   float *xs, *ys, *zs;              // [nslots] sorted positions; sentinels in the tail
   float4 *tbox, *bbox;              // [nslots / 512][2], [nslots / 32][2] boxes
-  unsigned long long* next;         // work counter of the pair kernel
+  unsigned long long* next;         // work counter of the pair kernel (lists: finished blocks)
+  // listed work of small systems (od_cutn3_listed, else NULL): target blocks per source group
+  // [nslots / 64][nslots / 32], (inner, other) counts, prefix of half batches
+  uint16_t* rows;
+  int2* counts;
+  int* prefix;
   unsigned long long* acc;          // [3][nslots] fixed-point ion–ion sums per sorted slot
   void* block;                      // the allocation that holds all of these
   double rc_d;                      // cutoff / r_D_e in FP64 (the hard cutoff's exact test)
@@ -134,6 +139,7 @@ struct od_cutn3 {
 struct od_cgrid { int G, nb, ncells; double side; };
 od_cgrid od_cutn3_grid(int N, double R, double H);
 size_t od_cutn3_bytes(int N, int T, int ncells);
+bool od_cutn3_listed(size_t nslots);
 bool od_cutn3_supported(int ipt, int T);
 int od_cutn3_blocks_per_sm(bool hard);
 cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, float4* part_hi,
