@@ -26,7 +26,7 @@ struct od_handle {
   od_dparams* dp = nullptr;
   od_dstate* ds = nullptr;
   od_dbufs b{};
-  int N = 0, Npad = 0, P = 0, nb = 0, nrec = 32;
+  int N = 0, Npad = 0, P = 0, nb = 0, nrec = 0;
   int64_t step = 0;
   bool state_set = false;
   od_pair_plan plan{};
@@ -492,6 +492,7 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
   h->Npad = (int)(((cfg->n_ions + OD_PAD - 1) / OD_PAD) * OD_PAD);
   h->P = cfg->n_grains;
   h->nb = h->Npad / 256;
+  h->nrec = std::min(304, std::max(32, h->nb));  // 304: two blocks per SM
   auto bail = [&](od_status s) {
     g_err = h->err;
     free_all(h);
@@ -1762,7 +1763,6 @@ static od_status batch_rebuild(od_batch* b) {
     if (d.n3_tile) d.n3 = od_n3_split_of(d.Npad, h->plan.ipt, d.n3_tile);
     sims.push_back(d);
     for (int lb = 0; lb < d.nb; lb++) blk_ion.push_back(make_int2(m, lb));
-    for (int lb = 0; lb < d.nb + d.nrec; lb++) blk_corr.push_back(make_int2(m, lb));
     if (d.n3_tile) {
       // every block of this member's pair kernel, in the table of its form
       std::vector<int2>& t = n3_items[od_n3_form(h->plan.ipt, sims.back().n3)];
@@ -1775,6 +1775,10 @@ static od_status batch_rebuild(od_batch* b) {
         if (j1 > j0) items.push_back({make_int4(m, ib, j0, j1), (long long)(j1 - j0)});
       }
   }
+  // K5: the tails first (they take longest), then every member's correction blocks
+  for (int m = 0; m < (int)sims.size(); m++) blk_corr.push_back(make_int2(m, -1));
+  for (int m = 0; m < (int)sims.size(); m++)
+    for (int lb = 0; lb < sims[m].nrec + sims[m].nb; lb++) blk_corr.push_back(make_int2(m, lb));
   std::stable_sort(items.begin(), items.end(), [](const item& a, const item& c) { return a.work > c.work; });
   std::vector<int4> w(items.size());
   for (size_t k = 0; k < items.size(); k++) w[k] = items[k].w;

@@ -90,7 +90,6 @@ struct od_dstate {
   double avg[OD_MAX_GRAINS][13];      // running sums over the averaging window
   int64_t n_avg;
   int64_t n_inj_total;
-  uint32_t ticket;                    // orbit blocks of K5 done this step (0 between steps)
   uint32_t bad;                       // a non-finite value in the state being set
 };
 

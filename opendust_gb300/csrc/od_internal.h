@@ -38,7 +38,7 @@ struct od_dbufs {
   int32_t* list_bits;                   // [Npad] flag bits of each entry
   float4 *list_old, *list_new, *list_v; // [Npad] pre/post re-injection positions, velocities: one
                                         // block, between steps the FP64 staging of state copies
-  double* orbit_part;                   // [nb_corr][P][3]
+  double* orbit_part;                   // [Npad / 256][P][3] orbit sums of 256-ion blocks
   // result series: row r of 13 P doubles holds q [P], then orbit, collect, dust, field [P][3]
   double* series;
   float* cq;                            // [P] A_id * q_param, FP32 copy for the ion kernels
@@ -87,7 +87,7 @@ struct od_batchview {
   int nblk_ion;
   const int4* items;     // (member, 256-target block, j0, j1) all-pairs work items
   int nitems;
-  const int2* blk_corr;  // (member, local block in [0, nb + nrec)) for correction/orbit sums
+  const int2* blk_corr;  // (member, local block in [0, nrec + nb), or -1: its tail) for K5
   int nblk_corr;
   int pair_grid;         // persistent blocks of the all-pairs stage
   unsigned int* next;    // work counter of the all-pairs stage
@@ -224,8 +224,8 @@ cudaError_t od_launch_step_part(int part, const od_dparams* dp, od_dstate* ds, c
 cudaError_t od_run_fp32_probe(int device, double* tflops);
 // shards of one simulation (od_kernels.cu): K1 (part 0, positions also into the sources) or
 // K3 + K4 (part 1); the ion–ion sums of the shard's ions over all sources (directed variants
-// 2-6); the whole run's re-injection list -> grain sums and sources; correction and orbit sums
-// of the shard's ions; the tail over all shards' orbit partials
+// 2-6); the whole run's re-injection list -> grain sums and sources; correction of the shard's
+// ions; the tail over all shards' orbit partials
 cudaError_t od_launch_shard_part(int part, const od_dparams* dp, od_dstate* ds, const od_dbufs& b,
                                  int N, int Npad, int jsplit, float* sx, float* sy, float* sz,
                                  cudaStream_t s);
@@ -241,7 +241,7 @@ cudaError_t od_launch_shard_correct(const od_dparams* dp, const od_dstate* ds, c
                                     const float4* gold, const float4* gnew, const float* sx,
                                     const float* sy, const float* sz, int nsrc, cudaStream_t s);
 cudaError_t od_launch_shard_tail(const od_dparams* dp, od_dstate* ds, const od_dbufs& b,
-                                 const double* orbit_all, int nb_all, cudaStream_t s);
+                                 double* orbit_all, int nb_all, cudaStream_t s);
 // one-thread mbarrier wait that gives up after `limit` polls unless `arrive` (self test)
 cudaError_t od_launch_wait_selftest(uint32_t* err, uint32_t limit, int arrive, cudaStream_t s);
 cudaError_t od_launch_snapshot_flags(const od_dparams* dp, int n, int Npad, const float4* pos,

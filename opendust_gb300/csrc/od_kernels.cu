@@ -3,10 +3,11 @@
 // One step of the reference program (opendust.py:839-1037 + host tail :1117-1383) runs as
 //   K1 kick_drift      collisions, v += a/2 with forces at the current positions, x += v
 //   K2 pairs           ion–ion sums at the drifted positions (all pairs, N^2)
-//   K3 kick_flag       reduce K2 partials, v += a/2, grain/domain flags -> warp ballots
-//   K4 collect_inject  ordered compaction of flagged ions, per-grain sums, re-injection
-//   K5 correct_orbit   ion–ion sums moved to the re-injected positions, orbit-force sums
-//   K6 tail            FP64 charge update, grain forces, result series, averages
+//   K3 kick_flag       take K2's sums, v += a/2, grain/domain flags -> warp ballots
+//   K4 collect_inject  ordered compaction of flagged ions, per-grain sums, re-injection in the first
+//                      block; orbit-force sums of the ions that stay in the others
+//   K5 correct         ion–ion sums moved to the re-injected positions; in its first block the FP64
+//                      tail: orbit sums, charge update, grain forces, result series, averages
 // The reference evaluates ion–ion forces twice per step (after the drift and again after
 // re-injection, because OpenMM re-evaluates forces whenever positions change). Only the few
 // re-injected ions move between those two evaluations, so K5 applies their O(N*K) difference
@@ -728,6 +729,199 @@ __device__ __forceinline__ void list_sums(const od_dparams& p, od_dstate* __rest
   }
 }
 
+// ============================================================== orbit-force sums
+// orbit term of grain g from an ion at x (opendust.py:977-1037): exp(-r)(x_p - x)(1/r^3 + 1/r^2),
+// lambda units
+__device__ __forceinline__ float3 orbit_term(const od_dparams& p, int g, const float4& x) {
+  const float dx = (p.gxh[g] - x.x) + p.gxl[g];
+  const float dy = (p.gyh[g] - x.y) + p.gyl[g];
+  const float dz = (p.gzh[g] - x.z) + p.gzl[g];
+  const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+  const float ri = rsqrtf(r2);
+  const float r = r2 * ri;
+  const float e = od_ex2(r * OD_NLOG2E);
+  const float t = e * ri * ri * (ri + 1.0f);
+  return make_float3(dx * t, dy * t, dz * t);
+}
+
+// FP64 sums of three values over a warp in a fixed order: a in lane 0, b in lane 16, c in lane 8. Six
+// additions instead of fifteen (an FP64 instruction takes a GB300 SM 16 cycles per warp): the first
+// two exchanges split the values between the halves.
+__device__ __forceinline__ double warp_sum3(double a, double b, double c) {
+  const int lane = threadIdx.x & 31;
+  const double give = lane < 16 ? b : a;
+  double ab = (lane < 16 ? a : b) + __shfl_xor_sync(0xffffffffu, give, 16);
+  c += __shfl_xor_sync(0xffffffffu, c, 16);
+  const bool up = lane & 8;
+  double v = (up ? c : ab) + __shfl_xor_sync(0xffffffffu, up ? ab : c, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// the lane that holds component d of warp_sum3, as d of the lane (or -1)
+__device__ __forceinline__ int sum3_component(int lane) {
+  return lane == 0 ? 0 : (lane == 16 ? 1 : (lane == 8 ? 2 : -1));
+}
+
+// orbit sums of `per` (1 or 4) 256-ion blocks, of the ions that stay, by a block of kCT threads: FP64
+// sums of warps, then a 256-ion block's warps in order. Each 256 threads take a block of their own
+// (per = 4, b is theirs) or every fourth grain of the one block (per = 1). An SM adds two FP64 values
+// per clock, so few blocks are spread over the SMs (2048 ions: 4.2 us, with four a block 6.1); many
+// fill them better four a block, as one thread block is resident (9 10^5 ions in a batch: 14.6 us,
+// else 19.9). The limit is two 256-ion blocks per SM.
+__device__ __forceinline__ void orbit_body(const od_dparams& p, const float4* pos,
+                                           const uint32_t* __restrict__ flags, int per, bool on,
+                                           int b, double* orbit_part) {
+  __shared__ double s_orb[kCT / 32][OD_MAX_GRAINS * 3];
+  const int tid = threadIdx.x, lane = tid & 31, t = tid & (kBlk - 1), q = tid / kBlk;
+  const int i = b * kBlk + t, d = sum3_component(lane);
+  const int g0 = per == 1 ? q : 0, dg = per == 1 ? kCT / kBlk : 1;
+  double(*const mine)[OD_MAX_GRAINS * 3] = s_orb + (per == 1 ? 0 : q * (kBlk / 32));
+  if (on && g0 < p.P) {
+    const bool live = i < p.N && !((flags[i >> 5] >> (i & 31)) & 1u);
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) x = pos[i];
+    for (int g = g0; g < p.P; g += dg) {
+      const float3 o = live ? orbit_term(p, g, x) : make_float3(0.f, 0.f, 0.f);
+      const double v = warp_sum3(o.x, o.y, o.z);
+      if (d >= 0) mine[t >> 5][3 * g + d] = v;
+    }
+  }
+  __syncthreads();
+  if (on && (per == 4 || q == 0) && t < 3 * p.P) {
+    double v = 0;
+    for (int k = 0; k < kBlk / 32; k++) v += mine[k][t];
+    orbit_part[(size_t)b * p.P * 3 + t] = v;
+  }
+}
+inline int orbit_per(int nb) { return nb > 2 * 152 ? 4 : 1; }
+
+// ============================================================== FP64 host-tail on device
+// opendust.py:1117-1202 (charge), :1205-1235 (dust–dust), :1237-1331 (orbit + out-of-domain),
+// :1333-1365 (collect), :1367-1383 (field); one 256-thread block, the first of K5, so that its FP64
+// latency (3.5 us: an FP64 instruction takes a GB300 SM 16 cycles per warp, and the chains are short
+// and dependent) passes while the other blocks correct the forces. In the last block of K5 to finish,
+// with the orbit sums before it, it held up every step by 8 us (2048 ions: K3 to K5 19.5 us, now 14).
+//
+// charge of grain g after a step with dN collected ions (opendust.py:1117-1202), from the
+// host-precomputed constants of tail_consts
+__device__ __forceinline__ double charge_update(const od_dparams& p, int g, double q_prev,
+                                                double dN) {
+  const double ge = p.ge_pref[g] * exp(p.ge_arg[g] * q_prev);
+  if (p.gmethod[g] == OD_CHARGE_CONSISTENT) return q_prev + (dN * p.q_s + ge);
+  if (p.gmethod[g] == OD_CHARGE_OML) return q_prev + (fma(p.oml_b[g], q_prev, p.oml_a[g]) + ge);
+  return q_prev;
+}
+
+struct tail_smem {
+  double part[kCT / 32][OD_MAX_GRAINS * 3];  // orbit sums of the blocks' partials, per warp
+  double S[OD_MAX_GRAINS * 3];
+  double q[OD_MAX_GRAINS];
+};
+static_assert(OD_MAX_GRAINS <= 32, "the tail has one lane per grain");
+
+// The K re-injected ions' orbit terms join the partials of their 256-ion blocks: the list is in ion
+// order, so one thread per grain takes a block's entries in turn.
+__device__ __forceinline__ void orbit_reinjected(const od_dparams& p, int tid, int nt, int K,
+                                                 const int32_t* __restrict__ list,
+                                                 const float4* __restrict__ list_new,
+                                                 double* orbit_part) {
+  for (int64_t e = tid; e < (int64_t)K * p.P; e += nt) {
+    const int k0 = (int)(e / p.P), g = (int)(e % p.P), b = list[k0] / kBlk;
+    if (k0 > 0 && list[k0 - 1] / kBlk == b) continue;
+    double v[3] = {0, 0, 0};
+    for (int k = k0; k < K && list[k] / kBlk == b; k++) {
+      const float3 t = orbit_term(p, g, list_new[k]);
+      v[0] += t.x; v[1] += t.y; v[2] += t.z;
+    }
+    double* o = orbit_part + ((size_t)b * p.P + g) * 3;
+#pragma unroll
+    for (int m = 0; m < 3; m++) o[m] += v[m];
+  }
+}
+
+// The tail of one handle. Warp 0 computes what needs no orbit sum, one grain per lane; the others add
+// the re-injected ions' orbit terms (list; NULL: all are in the partials) and sum the nb blocks'
+// partials.
+__device__ __forceinline__ void tail_body(const od_dparams& p, od_dstate* __restrict__ ds,
+                                          const int32_t* __restrict__ list,
+                                          const float4* __restrict__ list_new, double* orbit_part,
+                                          int nb, double* __restrict__ series,
+                                          float* __restrict__ cq) {
+  __shared__ tail_smem sm;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, P = p.P, nc = 3 * P;
+  const int K = ds->nlist;
+  const int nw = min(kCT / 32 - 1, (nb + 31) / 32);
+  const int64_t step = ds->step;
+  double vals[13] = {}, so = 0;
+  if (w == 0) {
+    const int g = lane;
+    const double qn = g >= P ? 0.0
+                      : step > 0 ? charge_update(p, g, ds->q_param[g], ds->dN[g]) : ds->q_param[g];
+    if (g < P) sm.q[g] = qn;
+    __syncwarp();
+    if (g < P) {
+      double fd[3] = {0, 0, 0};
+      for (int j = 0; j < P; j++) {
+        if (j == g) continue;
+        fd[0] = fma(sm.q[j], p.dd[g][j][0], fd[0]);
+        fd[1] = fma(sm.q[j], p.dd[g][j][1], fd[1]);
+        fd[2] = fma(sm.q[j], p.dd[g][j][2], fd[2]);
+      }
+      so = qn * p.k * p.q_s / (p.lam * p.lam);
+      const double sc = p.vunit * p.m_s / p.dt;
+      vals[0] = qn;
+      for (int m = 0; m < 3; m++) {
+        vals[1 + m] = qn * p.gout[g][m];
+        vals[4 + m] = ds->M[g][m] * sc;
+        vals[7 + m] = qn * fd[m];
+        vals[10 + m] = m == 2 ? qn * p.gfield[g] : 0.0;
+      }
+    }
+  } else {
+    if (list && K > 0) {
+      orbit_reinjected(p, tid - 32, kCT - 32, K, list, list_new, orbit_part);
+      asm volatile("bar.sync 1, %0;" ::"n"(kCT - 32) : "memory");
+    }
+    const int d = sum3_component(lane);
+    if (w <= nw)
+      for (int g = 0; g < P; g++) {
+        double v[3] = {0, 0, 0};
+        for (int b = tid - 32; b < nb; b += nw * 32) {
+          const double* o = orbit_part + (size_t)b * nc + 3 * g;
+          const double a0 = __ldcg(o), a1 = __ldcg(o + 1), a2 = __ldcg(o + 2);
+          v[0] += a0; v[1] += a1; v[2] += a2;
+        }
+        const double t = warp_sum3(v[0], v[1], v[2]);
+        if (d >= 0) sm.part[w - 1][3 * g + d] = t;
+      }
+  }
+  __syncthreads();
+  if (tid < nc) {
+    double v = 0;
+    for (int k = 0; k < nw; k++) v += sm.part[k][tid];
+    sm.S[tid] = v;
+  }
+  __syncthreads();
+  if (tid < P) {
+    const int g = tid;
+    for (int m = 0; m < 3; m++) vals[1 + m] = sm.S[g * 3 + m] * so + vals[1 + m];
+    double* const row = series + (size_t)step * 13 * P;
+    row[g] = vals[0];
+    for (int m = 0; m < 4; m++)
+      for (int e = 0; e < 3; e++) row[P + 3 * (m * P + g) + e] = vals[1 + 3 * m + e];
+    if (step >= p.avg_start)
+      for (int m = 0; m < 13; m++) ds->avg[g][m] += vals[m];
+    ds->q_param[g] = vals[0];
+    cq[g] = (float)(p.A_id_d * vals[0]);
+  }
+  if (tid == 0) {
+    if (step >= p.avg_start) ds->n_avg += 1;
+    ds->n_inj_total += K;
+    ds->step = step + 1;
+  }
+}
+
 __device__ __forceinline__ void collect_inject_body(
     const od_dparams& p, od_dstate* __restrict__ ds, float4* __restrict__ rel,
     float4* __restrict__ pos, float4* __restrict__ vel, const uint32_t* __restrict__ flags,
@@ -746,19 +940,26 @@ __device__ __forceinline__ void collect_inject_body(
   }
   __syncthreads();
   // warp 0 sums the grains' collected counts and momenta while warps 1.. re-inject
-  list_sums(p, ds, K, list_bits, list_v);
-  if (tid < 32) return;
+  if (tid < 32) list_sums(p, ds, K, list_bits, list_v);
   const uint32_t step = (uint32_t)(ds->step + ds->rng_base);
-  if (p.dist == OD_DIST_MATTHEWS) {
-    // the fork (chains/matthews.py:653-682): ions past |z| = H/2 or inside a grain re-enter
-    // through the top face; ions past the side wall keep their position and have the radial
-    // velocity component reversed, with the normal taken before any re-injection
-    const int grains = (1 << p.P) - 1;
-    for (int k = tid - 32; k < K; k += kCT - 32) {
-      const int i = list[k];
+  const bool reflect = p.dist == OD_DIST_MATTHEWS;
+  const int grains = (1 << p.P) - 1;
+  for (int k = tid - 32; tid >= 32 && k < K; k += kCT - 32) {
+    const int i = list[k];
+    float4 x, v;
+    if (!reflect) {
+      inject_one(p, (uint32_t)(p.ion0 + i), step, x, v);
+      const float4 r = od_rel_encode(p, x.x, x.y, x.z);
+      x = od_rel_abs(p, r);
+      rel[i] = r;
+    } else {
+      // the fork (chains/matthews.py:653-682): ions past |z| = H/2 or inside a grain re-enter
+      // through the top face; ions past the side wall keep their position and have the radial
+      // velocity component reversed, with the normal taken before any re-injection
       const int bits = list_bits[k];
       const float4 xo = list_old[k];
-      float4 x = xo, v = list_v[k];
+      x = xo;
+      v = list_v[k];
       if (bits & (grains | (1 << 29))) {
         inject_one(p, (uint32_t)(p.ion0 + i), step, x, v);
         const float4 r = od_rel_encode(p, x.x, x.y, x.z);
@@ -773,19 +974,7 @@ __device__ __forceinline__ void collect_inject_body(
         v.x = fmaf(-vn, nx, vt * ny);
         v.y = fmaf(-vn, ny, -vt * nx);
       }
-      pos[i] = x;
-      vel[i] = v;
-      list_new[k] = x;
     }
-    return;
-  }
-  for (int k = tid - 32; k < K; k += kCT - 32) {
-    const int i = list[k];
-    float4 x, v;
-    inject_one(p, (uint32_t)(p.ion0 + i), step, x, v);
-    const float4 r = od_rel_encode(p, x.x, x.y, x.z);
-    x = od_rel_abs(p, r);
-    rel[i] = r;
     pos[i] = x;
     vel[i] = v;
     list_new[k] = x;
@@ -796,9 +985,15 @@ __global__ void __launch_bounds__(kCT) k_collect_inject(
     const od_dparams* __restrict__ dp, od_dstate* __restrict__ ds, float4* __restrict__ rel,
     float4* __restrict__ pos, float4* __restrict__ vel, const uint32_t* __restrict__ flags,
     int32_t* __restrict__ list, int32_t* __restrict__ list_bits, float4* __restrict__ list_old,
-    float4* __restrict__ list_new, float4* __restrict__ list_v) {
+    float4* __restrict__ list_new, float4* __restrict__ list_v,
+    double* __restrict__ orbit_part, int nb, int per) {
   od_pdl_wait();
   od_pdl_trigger();
+  if (blockIdx.x > 0) {
+    const int b = (blockIdx.x - 1) * per + (per == 4 ? threadIdx.x / kBlk : 0);
+    orbit_body(*dp, pos, flags, per, b < nb, b, orbit_part);
+    return;
+  }
   collect_inject_body(*dp, ds, rel, pos, vel, flags, list, list_bits, list_old, list_new, list_v);
 }
 
@@ -826,28 +1021,19 @@ __global__ void __launch_bounds__(kCT) k_list_only(const od_dparams* __restrict_
   if (tid == 0) counts[OD_MAX_GRAINS] = K;
 }
 
-// ============================================================== K5: correction + orbit sums
-__device__ __forceinline__ double block_sum_256(double v, double* s_red) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) s_red[wid] = v;
-  __syncthreads();
-  double r = 0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < kBlk / 32; w++) r += s_red[w];
-  __syncthreads();
-  return r;  // valid in thread 0
-}
-
-// block blk of nb + nrec: blocks [0, nb) correct and sum orbit terms, the rest recompute the
-// re-injected ions' sums
-__device__ __forceinline__ void correct_orbit_body(
+// ============================================================== K5: correction
+// Block blk of nrec + nb, kCT threads: blocks [0, nrec) recompute the re-injected ions' sums, the rest
+// correct the 256 ions of a block that stay, kCorrLanes lanes to an ion. Bound by latency (a few dozen
+// sums of N terms each, on 152 SMs), so a sum is spread over all of a block's threads and up to 304
+// blocks take one each: 30000 ions 8.6 us (256 threads and 32 blocks: 18, with the orbit sums), 65536
+// with a cutoff 16 (33).
+constexpr int kCorrLanes = kCT / kBlk;
+__device__ __forceinline__ void correct_body(
     const od_dparams& p, const od_dstate* __restrict__ ds,
     const float4* __restrict__ pos, float4* __restrict__ fhi, float4* __restrict__ flo,
     const uint32_t* __restrict__ flags, const int32_t* __restrict__ list,
-    const float4* __restrict__ list_old, const float4* __restrict__ list_new,
-    double* __restrict__ orbit_part, int nb, int blk, int nrec,
+    const float4* __restrict__ list_old, const float4* __restrict__ list_new, int blk,
+    int nrec,
     const float* __restrict__ ssx = nullptr, const float* __restrict__ ssy = nullptr,
     const float* __restrict__ ssz = nullptr, int nsrc = 0) {
   // ssx..ssz (a shard of a larger run): the list holds the re-injected ions of every shard by
@@ -855,67 +1041,46 @@ __device__ __forceinline__ void correct_orbit_body(
   // (all shards' ions, re-injected ones at their new positions), and only this shard's own
   // entries (global index - p.ion0 in [0, p.N)) are written
   const int K = ds->nlist;
+  if (K == 0) return;
   const int tid = threadIdx.x;
-  if (blk < nb) {
-    const int i = blk * kBlk + tid;
-    const bool live = i < p.N;
+  if (blk >= nrec) {
+    // move the ion–ion sums of unflagged ions to the re-injected positions: kCorrLanes lanes share
+    // an ion, each takes every kCorrLanes-th entry in list order (loaded kU at a time so that their
+    // loads overlap)
+    const int i = (blk - nrec) * kBlk + tid / kCorrLanes, part = tid % kCorrLanes;
+    const bool live = i < p.N && !((flags[i >> 5] >> (i & 31)) & 1u);
+    if (!__any_sync(0xffffffffu, live)) return;
     const float4 x = live ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    // orbit sums (opendust.py:977-1037): exp(-r)(x_p - x)(1/r^3 + 1/r^2), lambda units; FP64
-    // warp trees for every component, then the 8 warps in order
-    __shared__ double s_orb[kBlk / 32][OD_MAX_GRAINS * 3];
-    const int lane = tid & 31, w = tid >> 5;
-    for (int g = 0; g < p.P; g++) {
-      float tx = 0.f, ty = 0.f, tz = 0.f;
-      if (live) {
-        const float dx = (p.gxh[g] - x.x) + p.gxl[g];
-        const float dy = (p.gyh[g] - x.y) + p.gyl[g];
-        const float dz = (p.gzh[g] - x.z) + p.gzl[g];
-        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-        const float ri = rsqrtf(r2);
-        const float r = r2 * ri;
-        const float e = od_ex2(r * OD_NLOG2E);
-        const float t = e * ri * ri * (ri + 1.0f);
-        tx = dx * t; ty = dy * t; tz = dz * t;
-      }
-      double sx = tx, sy = ty, sz = tz;
+    float gx = 0.f, gy = 0.f, gz = 0.f;
+    const bool cut = p.method == OD_FORCE_CUTOFF;
+    constexpr int kU = 4;
+    for (int k0 = part; k0 < K; k0 += kU * kCorrLanes) {
+      float4 qn[kU], qo[kU];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        sx += __shfl_xor_sync(0xffffffffu, sx, o);
-        sy += __shfl_xor_sync(0xffffffffu, sy, o);
-        sz += __shfl_xor_sync(0xffffffffu, sz, o);
+      for (int u = 0; u < kU; u++) {
+        const int k = k0 + u * kCorrLanes;
+        if (k < K) { qn[u] = list_new[k]; qo[u] = list_old[k]; }
       }
-      if (lane == 0) { s_orb[w][3 * g] = sx; s_orb[w][3 * g + 1] = sy; s_orb[w][3 * g + 2] = sz; }
+#pragma unroll
+      for (int u = 0; u < kU; u++) {
+        if (k0 + u * kCorrLanes >= K) break;
+        float dx = x.x - qn[u].x, dy = x.y - qn[u].y, dz = x.z - qn[u].z;
+        float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
+        float c = cut ? od_pair_c_cut(r2, p) : od_pair_c(r2, p.rho0);
+        gx = fmaf(c, dx, gx); gy = fmaf(c, dy, gy); gz = fmaf(c, dz, gz);
+        dx = x.x - qo[u].x; dy = x.y - qo[u].y; dz = x.z - qo[u].z;
+        r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
+        c = cut ? od_pair_c_cut(r2, p) : od_pair_c(r2, p.rho0);
+        gx = fmaf(-c, dx, gx); gy = fmaf(-c, dy, gy); gz = fmaf(-c, dz, gz);
+      }
     }
-    __syncthreads();
-    if (tid < 3 * p.P) {
-      double v = 0;
-      for (int k = 0; k < kBlk / 32; k++) v += s_orb[k][tid];
-      orbit_part[(size_t)blk * p.P * 3 + tid] = v;
+#pragma unroll
+    for (int o = 1; o < kCorrLanes; o <<= 1) {
+      gx += __shfl_xor_sync(0xffffffffu, gx, o);
+      gy += __shfl_xor_sync(0xffffffffu, gy, o);
+      gz += __shfl_xor_sync(0xffffffffu, gz, o);
     }
-    // move the ion–ion sums of unflagged ions to the re-injected positions (the entries are
-    // loaded kU at a time so that their loads overlap; the terms are added in list order)
-    if (K > 0 && live && !((flags[i >> 5] >> (i & 31)) & 1u)) {
-      float gx = 0.f, gy = 0.f, gz = 0.f;
-      const bool cut = p.method == OD_FORCE_CUTOFF;
-      constexpr int kU = 4;
-      for (int k0 = 0; k0 < K; k0 += kU) {
-        float4 qn[kU], qo[kU];
-#pragma unroll
-        for (int u = 0; u < kU; u++)
-          if (k0 + u < K) { qn[u] = list_new[k0 + u]; qo[u] = list_old[k0 + u]; }
-#pragma unroll
-        for (int u = 0; u < kU; u++) {
-          if (k0 + u >= K) break;
-          float dx = x.x - qn[u].x, dy = x.y - qn[u].y, dz = x.z - qn[u].z;
-          float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
-          float c = cut ? od_pair_c_cut(r2, p) : od_pair_c(r2, p.rho0);
-          gx = fmaf(c, dx, gx); gy = fmaf(c, dy, gy); gz = fmaf(c, dz, gz);
-          dx = x.x - qo[u].x; dy = x.y - qo[u].y; dz = x.z - qo[u].z;
-          r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
-          c = cut ? od_pair_c_cut(r2, p) : od_pair_c(r2, p.rho0);
-          gx = fmaf(-c, dx, gx); gy = fmaf(-c, dy, gy); gz = fmaf(-c, dz, gz);
-        }
-      }
+    if (live && part == 0) {
       float4 h = fhi[i], l = flo[i];
       od_acc2(h.x, l.x, gx); od_acc2(h.y, l.y, gy); od_acc2(h.z, l.z, gz);
       fhi[i] = h;
@@ -923,9 +1088,9 @@ __device__ __forceinline__ void correct_orbit_body(
     }
   } else {
     // full ion–ion sums of the re-injected ions at their new positions
-    __shared__ float s_h[3][kBlk], s_l[3][kBlk];
+    __shared__ float s_h[3][kCT / 32], s_l[3][kCT / 32];
     const bool cut = p.method == OD_FORCE_CUTOFF;
-    for (int k = blk - nb; k < K; k += nrec) {
+    for (int k = blk; k < K; k += nrec) {
       const int i = ssx ? list[k] - p.ion0 : list[k];
       if (ssx && (i < 0 || i >= p.N)) continue;  // another shard's ion (uniform per block)
       const float4 xi = list_new[k];
@@ -933,19 +1098,19 @@ __device__ __forceinline__ void correct_orbit_body(
       float ax = 0.f, ay = 0.f, az = 0.f;
       int cnt = 0;
       const int nj = ssx ? nsrc : p.N;
-      // sources j = tid, tid + kBlk, ... in that order, loaded kU at a time so that their loads
+      // sources j = tid, tid + kCT, ... in that order, loaded kU at a time so that their loads
       // overlap (a load per iteration waited the full memory latency each time)
       constexpr int kU = 8;
-      for (int j0 = tid; j0 < nj; j0 += kU * kBlk) {
+      for (int j0 = tid; j0 < nj; j0 += kU * kCT) {
         float4 q[kU];
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-          const int j = j0 + u * kBlk;
+          const int j = j0 + u * kCT;
           if (j < nj) q[u] = ssx ? make_float4(ssx[j], ssy[j], ssz[j], 0.f) : pos[j];
         }
 #pragma unroll
         for (int u = 0; u < kU; u++) {
-          if (j0 + u * kBlk >= nj) break;
+          if (j0 + u * kCT >= nj) break;
           const float dx = xi.x - q[u].x, dy = xi.y - q[u].y, dz = xi.z - q[u].z;
           const float r2 = fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, 1e-30f)));
           const float c = cut ? od_pair_c_cut(r2, p) : od_pair_c(r2, p.rho0);
@@ -958,7 +1123,7 @@ __device__ __forceinline__ void correct_orbit_body(
         }
       }
       od_acc2(hx, lx, ax); od_acc2(hy, ly, ay); od_acc2(hz, lz, az);
-      // two-float warp trees (fixed order), then the 8 warps in order
+      // two-float warp trees (fixed order), then the warps in order
       const int lane = tid & 31, w = tid >> 5;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -977,7 +1142,7 @@ __device__ __forceinline__ void correct_orbit_body(
       __syncthreads();
       if (tid < 3) {
         float h = 0.f, l = 0.f;
-        for (int u = 0; u < kBlk / 32; u++) { od_acc2(h, l, s_h[tid][u]); l += s_l[tid][u]; }
+        for (int u = 0; u < kCT / 32; u++) { od_acc2(h, l, s_h[tid][u]); l += s_l[tid][u]; }
         s_h[tid][0] = h;
         s_l[tid][0] = l;
       }
@@ -991,135 +1156,28 @@ __device__ __forceinline__ void correct_orbit_body(
   }
 }
 
-__global__ void __launch_bounds__(kBlk) k_correct_orbit(
+__global__ void __launch_bounds__(kCT) k_correct(
     const od_dparams* __restrict__ dp, od_dstate* __restrict__ ds,
     const float4* __restrict__ pos, float4* __restrict__ fhi, float4* __restrict__ flo,
     const uint32_t* __restrict__ flags, const int32_t* __restrict__ list,
     const float4* __restrict__ list_old, const float4* __restrict__ list_new,
-    double* __restrict__ orbit_part, int nb) {
-  correct_orbit_body(*dp, ds, pos, fhi, flo, flags, list, list_old, list_new, orbit_part, nb,
-                     blockIdx.x, gridDim.x - nb);
-}
-
-// ============================================================== K6: FP64 host-tail on device
-// opendust.py:1117-1202 (charge), :1205-1235 (dust–dust), :1237-1331 (orbit + out-of-domain),
-// :1333-1365 (collect), :1367-1383 (field)
-// charge of grain g after a step with dN collected ions (opendust.py:1117-1202), from the
-// host-precomputed constants of tail_consts
-__device__ __forceinline__ double charge_update(const od_dparams& p, int g, double q_prev,
-                                                double dN) {
-  const double ge = p.ge_pref[g] * exp(p.ge_arg[g] * q_prev);
-  if (p.gmethod[g] == OD_CHARGE_CONSISTENT) return q_prev + (dN * p.q_s + ge);
-  if (p.gmethod[g] == OD_CHARGE_OML) return q_prev + (fma(p.oml_b[g], q_prev, p.oml_a[g]) + ge);
-  return q_prev;
-}
-
-// FP64 tail of one step (opendust.py:1117-1383): orbit sums over the blocks' partials in a fixed
-// order (all components at once), then one thread per grain for the charge update and the
-// grain forces, from the host-precomputed constants.
-__device__ __forceinline__ void tail_body(const od_dparams& p, od_dstate* __restrict__ ds,
-                                          const double* __restrict__ orbit_part, int nb,
-                                          double* __restrict__ series, float* __restrict__ cq) {
-  __shared__ double s_red[kBlk / 32][OD_MAX_GRAINS * 3];
-  __shared__ double S[OD_MAX_GRAINS * 3];
-  __shared__ double qn[OD_MAX_GRAINS];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int P = p.P, nc = P * 3;
-  for (int g = 0; g < P; g++) {
-    double v[3] = {0, 0, 0};
-    // L2 loads: the partials may come from other blocks of the same launch (fused tail); the
-    // three components of a grain are loaded together so that their latencies overlap
-    for (int b = tid; b < nb; b += kBlk) {
-      const double* o = orbit_part + (size_t)b * nc + 3 * g;
-      const double a0 = __ldcg(o), a1 = __ldcg(o + 1), a2 = __ldcg(o + 2);
-      v[0] += a0; v[1] += a1; v[2] += a2;
-    }
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[d] += __shfl_xor_sync(0xffffffffu, v[d], o);
-      if (lane == 0) s_red[w][3 * g + d] = v[d];
-    }
-  }
-  const int64_t step = ds->step;
-  if (tid < P)
-    qn[tid] = step > 0 ? charge_update(p, tid, ds->q_param[tid], ds->dN[tid]) : ds->q_param[tid];
-  __syncthreads();
-  if (tid < nc) {
-    double v = 0;
-    for (int k = 0; k < kBlk / 32; k++) v += s_red[k][tid];
-    S[tid] = v;
-  }
-  __syncthreads();
-  const bool avg = step >= p.avg_start;
-  if (tid < P) {
-    const int g = tid;
-    double fd[3] = {0, 0, 0};
-    for (int j = 0; j < P; j++) {
-      if (j == g) continue;
-      fd[0] = fma(qn[j], p.dd[g][j][0], fd[0]);
-      fd[1] = fma(qn[j], p.dd[g][j][1], fd[1]);
-      fd[2] = fma(qn[j], p.dd[g][j][2], fd[2]);
-    }
-    const double so = qn[g] * p.k * p.q_s / (p.lam * p.lam);
-    const double sc = p.vunit * p.m_s / p.dt;
-    double vals[13];
-    vals[0] = qn[g];
-    for (int d = 0; d < 3; d++) {
-      vals[1 + d] = S[g * 3 + d] * so + qn[g] * p.gout[g][d];
-      vals[4 + d] = ds->M[g][d] * sc;
-      vals[7 + d] = qn[g] * fd[d];
-      vals[10 + d] = d == 2 ? qn[g] * p.gfield[g] : 0.0;
-    }
-    double* const row = series + (size_t)step * 13 * P;
-    row[g] = vals[0];
-    for (int m = 0; m < 4; m++)
-      for (int d = 0; d < 3; d++) row[P + 3 * (m * P + g) + d] = vals[1 + 3 * m + d];
-    if (avg)
-      for (int m = 0; m < 13; m++) ds->avg[g][m] += vals[m];
-    ds->q_param[g] = qn[g];
-    cq[g] = (float)(p.A_id_d * qn[g]);
-  }
-  __syncthreads();  // every grain has read ds->step
-  if (tid == 0) {
-    if (avg) ds->n_avg += 1;
-    ds->n_inj_total += ds->nlist;
-    ds->step = step + 1;
-  }
-}
-
-__global__ void __launch_bounds__(kBlk) k_tail(const od_dparams* __restrict__ dp,
-                                               od_dstate* __restrict__ ds,
-                                               const double* __restrict__ orbit_part, int nb,
-                                               double* __restrict__ series, float* __restrict__ cq) {
-  tail_body(*dp, ds, orbit_part, nb, series, cq);
-}
-
-// K5 + K6: the last of the nb orbit blocks to finish (a ticket taken after its partials are
-// fenced) runs the FP64 tail over all partials, so the tail needs no launch of its own.
-__global__ void __launch_bounds__(kBlk) k_correct_orbit_tail(
-    const od_dparams* __restrict__ dp, od_dstate* __restrict__ ds,
-    const float4* __restrict__ pos, float4* __restrict__ fhi, float4* __restrict__ flo,
-    const uint32_t* __restrict__ flags, const int32_t* __restrict__ list,
-    const float4* __restrict__ list_old, const float4* __restrict__ list_new,
-    double* __restrict__ orbit_part, int nb, double* __restrict__ series, float* __restrict__ cq) {
+    double* orbit_part, int nb, double* __restrict__ series, float* __restrict__ cq) {
   od_pdl_wait();
-  correct_orbit_body(*dp, ds, pos, fhi, flo, flags, list, list_old, list_new, orbit_part, nb,
-                     blockIdx.x, gridDim.x - nb);
-  if ((int)blockIdx.x >= nb) return;  // re-injected ions' sums: the tail does not read them
-  __shared__ bool s_last;
-  __syncthreads();                    // this block's partials are written
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(&ds->ticket, 1u) == (unsigned)nb - 1u;
+  if (blockIdx.x == 0) {
+    tail_body(*dp, ds, list, list_new, orbit_part, nb, series, cq);
+    return;
   }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  tail_body(*dp, ds, orbit_part, nb, series, cq);
-  if (threadIdx.x == 0) ds->ticket = 0u;
+  correct_body(*dp, ds, pos, fhi, flo, flags, list, list_old, list_new, blockIdx.x - 1,
+               gridDim.x - 1 - nb);
 }
 
+// The tail of a sharded run, over every shard's orbit partials.
+__global__ void __launch_bounds__(kCT) k_tail(const od_dparams* __restrict__ dp,
+                                               od_dstate* __restrict__ ds,
+                                               double* __restrict__ orbit_part, int nb,
+                                               double* __restrict__ series, float* __restrict__ cq) {
+  tail_body(*dp, ds, nullptr, nullptr, orbit_part, nb, series, cq);
+}
 
 __global__ void k_set_charges(const od_dparams* __restrict__ dp, const od_dstate* __restrict__ ds,
                               float* __restrict__ cq, int P) {
@@ -1356,17 +1414,18 @@ cudaError_t od_launch_step_part(int part, const od_dparams* dp, od_dstate* ds, c
     return od_launch_force(fc, od_pair_io{b.pos, b.sx, b.sy, b.sz, b.n3}, N, Npad, b.part_hi, b.part_lo,
                            &ds->err, s, fc.acc == nullptr);
   const int jsplit = fc.cut ? 1 : fc.plan.jsplit;
+  const int per = orbit_per(nb);
   // K3, K4 and K5 with programmatic dependent launch: each starts launching while its
   // predecessor runs and waits in od_pdl_wait for the predecessor's results
   cudaError_t e = od_launch_pdl(k_kick_flag, dim3(nb), dim3(kBlk), s, dp, ds, b.pos, b.vel,
                                 (const float4*)b.part_hi, (const float4*)b.part_lo, jsplit, b.fhi,
                                 b.flo, b.flags, (const float*)b.cq, fc.acc);
   if (e == cudaSuccess)
-    e = od_launch_pdl(k_collect_inject, dim3(1), dim3(kCT), s, dp, ds, b.rel, b.pos, b.vel,
-                      (const uint32_t*)b.flags, b.list, b.list_bits, b.list_old, b.list_new,
-                      b.list_v);
+    e = od_launch_pdl(k_collect_inject, dim3(1 + (nb + per - 1) / per), dim3(kCT), s, dp, ds, b.rel, b.pos,
+                      b.vel, (const uint32_t*)b.flags, b.list, b.list_bits, b.list_old, b.list_new,
+                      b.list_v, b.orbit_part, nb, per);
   if (e == cudaSuccess)
-    e = od_launch_pdl(k_correct_orbit_tail, dim3(nb + nrec), dim3(kBlk), s, dp, ds,
+    e = od_launch_pdl(k_correct, dim3(1 + nrec + nb), dim3(kCT), s, dp, ds,
                       (const float4*)b.pos, b.fhi, b.flo, (const uint32_t*)b.flags,
                       (const int32_t*)b.list, (const float4*)b.list_old,
                       (const float4*)b.list_new, b.orbit_part, nb, b.series, b.cq);
@@ -1503,7 +1562,7 @@ cudaError_t od_launch_static_forces(const od_static_view& v, const double* pos, 
 // the whole batch. Blocks of the ion-parallel stages look up (simulation, local block) in a
 // table; the all-pairs stage is one persistent launch whose blocks take work items
 // (simulation, 256-target block, source range) from a device counter, largest items first;
-// compaction/re-injection and the FP64 tail run one block per simulation. Each simulation
+// compaction and re-injection run one block per simulation, the FP64 tails as K5's first blocks. Each simulation
 // keeps its own buffers, source split and partial slabs, so its results are bitwise the
 // results of the same simulation stepped alone.
 namespace {
@@ -1546,23 +1605,31 @@ __global__ void __launch_bounds__(kBlk) k_b_kick_flag(const od_simdesc* __restri
                  d.b.flags, d.b.cq, e.y * kBlk + threadIdx.x, d.n3_tile ? d.b.n3 : nullptr);
 }
 
-__global__ void __launch_bounds__(kCT) k_b_collect_inject(const od_simdesc* __restrict__ sims) {
+__global__ void __launch_bounds__(kCT) k_b_collect_inject(const od_simdesc* __restrict__ sims,
+                                                          int nsims, int per,
+                                                          const int2* __restrict__ blk, int nblk) {
+  if ((int)blockIdx.x >= nsims) {
+    const int k = (blockIdx.x - nsims) * per + (per == 4 ? threadIdx.x / kBlk : 0);
+    const int2 e = blk[min(k, nblk - 1)];
+    const od_simdesc& d = sims[e.x];
+    orbit_body(*d.dp, d.b.pos, d.b.flags, per, k < nblk, e.y, d.b.orbit_part);
+    return;
+  }
   const od_simdesc& d = sims[blockIdx.x];
   collect_inject_body(*d.dp, d.ds, d.b.rel, d.b.pos, d.b.vel, d.b.flags, d.b.list, d.b.list_bits,
                       d.b.list_old, d.b.list_new, d.b.list_v);
 }
 
-__global__ void __launch_bounds__(kBlk) k_b_correct_orbit(const od_simdesc* __restrict__ sims,
-                                                          const int2* __restrict__ blk) {
+__global__ void __launch_bounds__(kCT) k_b_correct(const od_simdesc* __restrict__ sims,
+                                                    const int2* __restrict__ blk) {
   const int2 e = blk[blockIdx.x];
   const od_simdesc& d = sims[e.x];
-  correct_orbit_body(*d.dp, d.ds, d.b.pos, d.b.fhi, d.b.flo, d.b.flags, d.b.list, d.b.list_old,
-                     d.b.list_new, d.b.orbit_part, d.nb, e.y, d.nrec);
-}
-
-__global__ void __launch_bounds__(kBlk) k_b_tail(const od_simdesc* __restrict__ sims) {
-  const od_simdesc& d = sims[blockIdx.x];
-  tail_body(*d.dp, d.ds, d.b.orbit_part, d.nb, d.b.series, d.b.cq);
+  if (e.y < 0) {
+    tail_body(*d.dp, d.ds, d.b.list, d.b.list_new, d.b.orbit_part, d.nb, d.b.series, d.b.cq);
+    return;
+  }
+  correct_body(*d.dp, d.ds, d.b.pos, d.b.fhi, d.b.flo, d.b.flags, d.b.list, d.b.list_old,
+               d.b.list_new, e.y, d.nrec);
 }
 
 }  // namespace
@@ -1608,9 +1675,10 @@ cudaError_t od_launch_batch_step(const od_batchview& v, cudaStream_t s) {
   cudaError_t e = od_launch_batch_pairs_n3(v, s);
   if (e != cudaSuccess) return e;
   k_b_kick_flag<<<v.nblk_ion, kBlk, 0, s>>>(v.sims, v.blk_ion);
-  k_b_collect_inject<<<v.nsims, kCT, 0, s>>>(v.sims);
-  k_b_correct_orbit<<<v.nblk_corr, kBlk, 0, s>>>(v.sims, v.blk_corr);
-  k_b_tail<<<v.nsims, kBlk, 0, s>>>(v.sims);
+  const int per = orbit_per(v.nblk_ion);
+  k_b_collect_inject<<<v.nsims + (v.nblk_ion + per - 1) / per, kCT, 0, s>>>(v.sims, v.nsims, per,
+                                                                            v.blk_ion, v.nblk_ion);
+  k_b_correct<<<v.nblk_corr, kCT, 0, s>>>(v.sims, v.blk_corr);
   return cudaGetLastError();
 }
 
@@ -1803,15 +1871,24 @@ __global__ void __launch_bounds__(kCT) k_shard_list(const od_dparams* __restrict
   }
 }
 
-__global__ void __launch_bounds__(kBlk) k_shard_correct_orbit(
+// own re-injected ions' orbit terms, before the list becomes the whole run's
+__global__ void __launch_bounds__(kBlk) k_shard_orbit(const od_dparams* __restrict__ dp,
+                                                      const od_dstate* __restrict__ ds,
+                                                      const int32_t* __restrict__ list,
+                                                      const float4* __restrict__ list_new,
+                                                      double* orbit_part) {
+  orbit_reinjected(*dp, threadIdx.x, kBlk, ds->nlist, list, list_new, orbit_part);
+}
+
+__global__ void __launch_bounds__(kCT) k_shard_correct(
     const od_dparams* __restrict__ dp, const od_dstate* __restrict__ ds,
     const float4* __restrict__ pos, float4* __restrict__ fhi, float4* __restrict__ flo,
     const uint32_t* __restrict__ flags, const int32_t* __restrict__ gidx,
-    const float4* __restrict__ gold, const float4* __restrict__ gnew,
-    double* __restrict__ orbit_part, int nb, const float* __restrict__ sx,
-    const float* __restrict__ sy, const float* __restrict__ sz, int nsrc) {
-  correct_orbit_body(*dp, ds, pos, fhi, flo, flags, gidx, gold, gnew, orbit_part, nb, blockIdx.x,
-                     gridDim.x - nb, sx, sy, sz, nsrc);
+    const float4* __restrict__ gold, const float4* __restrict__ gnew, int nb,
+    const float* __restrict__ sx, const float* __restrict__ sy, const float* __restrict__ sz,
+    int nsrc) {
+  correct_body(*dp, ds, pos, fhi, flo, flags, gidx, gold, gnew, blockIdx.x, gridDim.x - nb, sx,
+               sy, sz, nsrc);
 }
 
 // directed ion–ion sums of a shard's ions (sources tgt_off .. tgt_off + Npad_local of the
@@ -1874,14 +1951,14 @@ cudaError_t od_launch_shard_correct(const od_dparams* dp, const od_dstate* ds, c
                                     const float4* gold, const float4* gnew, const float* sx,
                                     const float* sy, const float* sz, int nsrc, cudaStream_t s) {
   const int nb = Npad_local / kBlk;
-  k_shard_correct_orbit<<<nb + nrec, kBlk, 0, s>>>(dp, ds, b.pos, b.fhi, b.flo, b.flags, gidx,
-                                                   gold, gnew, b.orbit_part, nb, sx, sy, sz, nsrc);
+  k_shard_correct<<<nrec + nb, kCT, 0, s>>>(dp, ds, b.pos, b.fhi, b.flo, b.flags, gidx, gold, gnew,
+                                            nb, sx, sy, sz, nsrc);
   return cudaGetLastError();
 }
 
 cudaError_t od_launch_shard_tail(const od_dparams* dp, od_dstate* ds, const od_dbufs& b,
-                                 const double* orbit_all, int nb_all, cudaStream_t s) {
-  k_tail<<<1, kBlk, 0, s>>>(dp, ds, orbit_all, nb_all, b.series, b.cq);
+                                 double* orbit_all, int nb_all, cudaStream_t s) {
+  k_tail<<<1, kCT, 0, s>>>(dp, ds, orbit_all, nb_all, b.series, b.cq);
   return cudaGetLastError();
 }
 
@@ -1896,8 +1973,10 @@ cudaError_t od_launch_shard_part(int part, const od_dparams* dp, od_dstate* ds, 
   }
   k_kick_flag<<<Npad / kBlk, kBlk, 0, s>>>(dp, ds, b.pos, b.vel, b.part_hi, b.part_lo, jsplit,
                                           b.fhi, b.flo, b.flags, b.cq, b.n3);
-  k_collect_inject<<<1, kCT, 0, s>>>(dp, ds, b.rel, b.pos, b.vel, b.flags, b.list, b.list_bits,
-                                     b.list_old, b.list_new, b.list_v);
+  const int nb = Npad / kBlk;
+  k_collect_inject<<<1 + nb, kCT, 0, s>>>(dp, ds, b.rel, b.pos, b.vel, b.flags, b.list, b.list_bits,
+                                          b.list_old, b.list_new, b.list_v, b.orbit_part, nb, 1);
+  k_shard_orbit<<<1, kBlk, 0, s>>>(dp, ds, b.list, b.list_new, b.orbit_part);
   return cudaGetLastError();
 }
 
