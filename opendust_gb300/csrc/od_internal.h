@@ -252,6 +252,24 @@ cudaError_t od_launch_set_charges(const od_dparams* dp, od_dstate* ds, float* cq
 cudaError_t od_launch_trap(double Rh, double Hh, int n_r, int n_h, int64_t n_points, uint64_t seed,
                            double* part, int nchunks, cudaStream_t s);
 
+// launch with programmatic stream serialization (the kernel calls od_pdl_wait before
+// it touches anything that an earlier kernel wrote or reads)
+template <typename... KArgs, typename... Args>
+inline cudaError_t od_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                                 Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = 0;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Record msg as the last error of calls without a handle (od_last_error(NULL)); returns st.
 od_status od_fail_nohandle(od_status st, const std::string& msg);
 

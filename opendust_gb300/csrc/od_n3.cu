@@ -137,6 +137,7 @@ __device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const flo
   }
   pair_consts k;
   k.eps = p2(1e-30f, 1e-30f); k.rho = p2(rho0, rho0); k.nl2e = p2(OD_NLOG2E, OD_NLOG2E);
+  od_pdl_wait();  // the unit is found while the kernel that writes the positions still runs
   for (;;) {
     od_u64 X[MT], Y[MT], Z[MT];
 #pragma unroll
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_B
                float rho0, const __grid_constant__ od_n3_split sp) {
   __shared__ float sm[FOLD ? kSliceWarps * 6 * slice_traits<MT, MS>::GT : 1];
   const int w = threadIdx.x >> 5;
+  od_pdl_trigger();
   n3_slice<MT, MS, SPLIT, FOLD>(sx, sy, sz, Npad, acc, rho0,
                                 (long long)blockIdx.x * kSliceWarps + w, sp,
                                 sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT + (threadIdx.x & 31)
@@ -229,9 +231,13 @@ template <int MT, int MS, int SPLIT, bool FOLD>
 __global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_BLOCKS))
     k_b_pairs_n3(const od_simdesc* __restrict__ sims, const int2* __restrict__ items) {
   __shared__ float sm[FOLD ? kSliceWarps * 6 * slice_traits<MT, MS>::GT : 1];
+  od_pdl_trigger();
   const int2 it = items[blockIdx.x];
   const od_simdesc& d = sims[it.x];
-  if (!od_evaluates(d.dp->force_every, d.ds->step)) return;  // force interval: no evaluation
+  if (!od_evaluates(d.dp->force_every, d.ds->step)) {  // force interval: no evaluation
+    od_pdl_wait();  // the next kernel may start when this grid is done: it needs the one before too
+    return;
+  }
   const int w = threadIdx.x >> 5;
   n3_slice<MT, MS, SPLIT, FOLD>(d.b.sx, d.b.sy, d.b.sz, d.Npad, d.b.n3, d.rho0,
                                 (long long)it.y * kSliceWarps + w, d.n3,
@@ -251,9 +257,10 @@ __global__ void k_n3_take(unsigned long long* __restrict__ acc, int Npad, float4
 }
 
 template <int MT, int MS, int SPLIT, bool FOLD>
-void launch_n3(const od_pair_io& io, int Npad, float rho0, const od_n3_split& sp, cudaStream_t s) {
-  k_pairs_n3<MT, MS, SPLIT, FOLD><<<(unsigned)od_n3_blocks(sp), kSliceWarps * 32, 0, s>>>(
-      io.sx, io.sy, io.sz, Npad, io.n3, rho0, sp);
+cudaError_t launch_n3(const od_pair_io& io, int Npad, float rho0, const od_n3_split& sp,
+                      cudaStream_t s) {
+  return od_launch_pdl(k_pairs_n3<MT, MS, SPLIT, FOLD>, dim3((unsigned)od_n3_blocks(sp)),
+                       dim3(kSliceWarps * 32), s, io.sx, io.sy, io.sz, Npad, io.n3, rho0, sp);
 }
 
 }  // namespace
@@ -301,12 +308,14 @@ cudaError_t od_launch_pairs_n3(const od_pair_plan& pl, const od_pair_io& io, int
                                float4* plo, float rho0, cudaStream_t s, bool take) {
   if (!io.n3 || !od_n3_supported(pl.ipt, pl.tile)) return cudaErrorInvalidValue;
   const od_n3_split sp = od_n3_split_of(Npad, pl.ipt, pl.tile);
-  if (pl.ipt == 2) launch_n3<2, 2, 1, true>(io, Npad, rho0, sp, s);
-  else if (pl.ipt == 8) launch_n3<8, 2, 1, true>(io, Npad, rho0, sp, s);
-  else if (sp.split == 4) launch_n3<4, 4, 4, false>(io, Npad, rho0, sp, s);
-  else if (sp.split == 2) launch_n3<4, 4, 2, false>(io, Npad, rho0, sp, s);
-  else if (sp.L > 1) launch_n3<4, 4, 1, true>(io, Npad, rho0, sp, s);
-  else launch_n3<4, 4, 1, false>(io, Npad, rho0, sp, s);
+  cudaError_t e;
+  if (pl.ipt == 2) e = launch_n3<2, 2, 1, true>(io, Npad, rho0, sp, s);
+  else if (pl.ipt == 8) e = launch_n3<8, 2, 1, true>(io, Npad, rho0, sp, s);
+  else if (sp.split == 4) e = launch_n3<4, 4, 4, false>(io, Npad, rho0, sp, s);
+  else if (sp.split == 2) e = launch_n3<4, 4, 2, false>(io, Npad, rho0, sp, s);
+  else if (sp.L > 1) e = launch_n3<4, 4, 1, true>(io, Npad, rho0, sp, s);
+  else e = launch_n3<4, 4, 1, false>(io, Npad, rho0, sp, s);
+  if (e != cudaSuccess) return e;
   if (take) k_n3_take<<<(Npad + 255) / 256, 256, 0, s>>>(io.n3, Npad, ph, plo);
   return cudaGetLastError();
 }
@@ -331,17 +340,18 @@ int od_n3_form(int ipt, const od_n3_split& sp) {
 
 cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, cudaStream_t s) {
   // the forms batch members use (od_n3_batch_plan, od_n3_form)
+  cudaError_t e = cudaSuccess;
 #define OD_B_N3(f, MT, MS, SPLIT, FOLD)                                                      \
-  if (v.n3_nitems[f] > 0)                                                                    \
-  k_b_pairs_n3<MT, MS, SPLIT, FOLD><<<v.n3_nitems[f], kSliceWarps * 32, 0, s>>>(v.sims,      \
-                                                                                v.n3_items[f])
+  if (v.n3_nitems[f] > 0 && e == cudaSuccess)                                                \
+  e = od_launch_pdl(k_b_pairs_n3<MT, MS, SPLIT, FOLD>, dim3(v.n3_nitems[f]),                 \
+                    dim3(kSliceWarps * 32), s, v.sims, (const int2*)v.n3_items[f])
   OD_B_N3(3, 8, 2, 1, true);
   OD_B_N3(0, 4, 4, 1, false);
   OD_B_N3(1, 4, 4, 2, false);
   OD_B_N3(2, 4, 4, 4, false);
   OD_B_N3(4, 4, 4, 1, true);
 #undef OD_B_N3
-  return cudaGetLastError();
+  return e;
 }
 
 int od_n3_batch_plan(int Npad, size_t budget_bytes, int* ipt) {
