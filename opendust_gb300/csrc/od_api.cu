@@ -1527,14 +1527,14 @@ extern "C" od_status od_trap_potential(double Rh, double Hh, int32_t n_r, int32_
 // cudaMalloc after start-up, or plug-ins whose host framework owns every device buffer and
 // hands them only pointers. od_ion_forces_static serves them: the caller passes device
 // arrays for the positions and the forces, and every scratch byte the kernels need (a padded
-// SoA copy of the positions, the partial sums of the source split, and an error word) lives
+// SoA copy of the positions and the partial sums of the source split) lives
 // in the file-scope array below, which each GPU that loads this library holds until the
 // process exits.
 #define OD_STATIC_MAX_IONS 32768
 #define OD_STATIC_MAX_SPLIT 8
 static constexpr size_t kStaticSoA = (size_t)OD_STATIC_MAX_IONS * sizeof(float);
 static constexpr size_t kStaticSlab = (size_t)OD_STATIC_MAX_SPLIT * OD_STATIC_MAX_IONS * sizeof(float4);
-static constexpr size_t kStaticBytes = 256 + 3 * kStaticSoA + 2 * kStaticSlab;  // about 8.8 MB
+static constexpr size_t kStaticBytes = 3 * kStaticSoA + 2 * kStaticSlab;  // about 8.8 MB
 static __device__ __align__(256) unsigned char od_static_scratch[kStaticBytes];
 
 // Device address of od_static_scratch on each device. In host code the array's name is only a
@@ -1576,25 +1576,18 @@ extern "C" od_status od_ion_forces_static(const double* pos_dev, int64_t n, doub
   e = static_scratch_addr(dev, &base);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaGetSymbolAddress(od_static_scratch)");
   od_static_view v{};
-  v.err = (uint32_t*)base;
-  v.sx = (float*)(base + 256);
-  v.sy = (float*)(base + 256 + kStaticSoA);
-  v.sz = (float*)(base + 256 + 2 * kStaticSoA);
-  v.part_hi = (float4*)(base + 256 + 3 * kStaticSoA);
-  v.part_lo = (float4*)(base + 256 + 3 * kStaticSoA + kStaticSlab);
-  v.max_split = OD_STATIC_MAX_SPLIT;
+  v.sx = (float*)base;
+  v.sy = (float*)(base + kStaticSoA);
+  v.sz = (float*)(base + 2 * kStaticSoA);
+  v.part_hi = (float4*)(base + 3 * kStaticSoA);
+  v.part_lo = (float4*)(base + 3 * kStaticSoA + kStaticSlab);
+  v.slab_ions = OD_STATIC_MAX_SPLIT * OD_STATIC_MAX_IONS;
   cudaStream_t s = (cudaStream_t)stream;
-  // the error word keeps the previous call's value: clear it
-  e = cudaMemsetAsync(v.err, 0, sizeof(uint32_t), s);
-  if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaMemsetAsync(error word)");
   const double scale = kq_sq_s / (r_D_e * r_D_e);
   e = od_launch_static_forces(v, pos_dev, (int)n, r_D_e, r_0, scale, force_dev, s);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "all-pairs launch");
-  uint32_t err = 0;
-  e = cudaMemcpyAsync(&err, v.err, sizeof(err), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "od_ion_forces_static");
-  if (err & OD_DERR_TIMEOUT) return fail(nullptr, OD_ERR_TIMEOUT, "a bounded device wait ran out");
   return OD_OK;
 }
 

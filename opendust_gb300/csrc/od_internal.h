@@ -162,10 +162,9 @@ cudaError_t od_launch_cutoff(const od_cutlist& L, const float4* pos, int n, int 
 
 // Pointers into the allocation-free scratch array of od_ion_forces_static.
 struct od_static_view {
-  uint32_t* err;
   float *sx, *sy, *sz;
-  float4 *part_hi, *part_lo;
-  int max_split;
+  float4 *part_hi, *part_lo;  // slab_ions entries each: source chunks times padded ions
+  int slab_ions;
 };
 cudaError_t od_launch_static_forces(const od_static_view& v, const double* pos, int n, double lam,
                                     double r0, double scale, double* force, cudaStream_t s);

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "od_internal.h"
+#include <algorithm>
 
 namespace {
 
@@ -1494,12 +1495,13 @@ cudaError_t od_launch_trap(double Rh, double Hh, int n_r, int n_h, int64_t n_poi
 }
 
 // ============================================================== scratch-array variant
-// Kernels behind od_ion_forces_static: the same packed all-pairs kernel, reading positions
-// and writing partial sums in a caller-independent scratch region (see od_api.cu).
+// Kernels behind od_ion_forces_static, with their positions and partial sums in a
+// caller-independent scratch region (see od_api.cu).
 namespace {
 __global__ void k_static_pack(const double* __restrict__ pos, int n, int Npad, double inv_lam,
                               float* __restrict__ sx, float* __restrict__ sy,
                               float* __restrict__ sz) {
+  od_pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Npad) return;
   if (i < n) {
@@ -1511,35 +1513,101 @@ __global__ void k_static_pack(const double* __restrict__ pos, int n, int Npad, d
   }
 }
 
-__global__ void k_static_finish(const float4* __restrict__ ph, const float4* __restrict__ pl,
-                                int n, int Npad, int jsplit, double scale,
-                                double* __restrict__ force) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float3 hi, lo;
-  reduce_parts(ph, pl, Npad, jsplit, i, hi, lo);
-  force[3 * i] = scale * ((double)hi.x + (double)lo.x);
-  force[3 * i + 1] = scale * ((double)hi.y + (double)lo.y);
-  force[3 * i + 2] = scale * ((double)hi.z + (double)lo.z);
+// Sums of a thread's target over a chunk of sources, two sources to a packed operation, the sources
+// staged in shared memory; 64 sources are one FP32 chain, longer chunks add them to two-float sums.
+// Bound by the SFU (three operations per pair, 21 cycles per 32 pairs and sub-partition) and, below
+// 4000 ions, by launches. Directed, not each pair once: the caller's positions may be anywhere, and
+// fixed-point sums would not keep the relative accuracy of a far ion's small force.
+// One call, 700 ions: 18 us (44.5 with up to 8 source chunks and an error word read back), 3001: 24
+// (57), 8000: 59 (87), 32768: 641 (763). Two targets per thread: 20.6, 27.1, 62, 758.
+constexpr int kStaticThreads = 256, kStaticTile = 256;
+__global__ void __launch_bounds__(kStaticThreads) k_static_pairs(
+    const float* __restrict__ sx, const float* __restrict__ sy, const float* __restrict__ sz,
+    int Npad, int chunk, float rho0, float4* __restrict__ ph, float4* __restrict__ pl) {
+  __shared__ __align__(16) float q[3][kStaticTile];
+  od_pdl_trigger();
+  od_pdl_wait();
+  const int tid = threadIdx.x, i = blockIdx.x * kStaticThreads + tid;
+  const int j0 = blockIdx.y * chunk, j1 = min(j0 + chunk, Npad);
+  const od_u64 eps = p2(1e-30f, 1e-30f), rho = p2(rho0, rho0), nl2e = p2(OD_NLOG2E, OD_NLOG2E);
+  od_u64 X = 0ull, Y = 0ull, Z = 0ull;
+  if (i < Npad) { X = p2(sx[i], sx[i]); Y = p2(sy[i], sy[i]); Z = p2(sz[i], sz[i]); }
+  float3 hi = make_float3(0.f, 0.f, 0.f), lo = hi;
+  for (int jt = j0; jt < j1; jt += kStaticTile) {
+    const int m = min(kStaticTile, j1 - jt);
+    __syncthreads();
+    if (tid < m) { q[0][tid] = sx[jt + tid]; q[1][tid] = sy[jt + tid]; q[2][tid] = sz[jt + tid]; }
+    __syncthreads();
+    for (int k0 = 0; k0 < m; k0 += 64) {
+      od_u64 AX = 0ull, AY = 0ull, AZ = 0ull;
+#pragma unroll 4
+      for (int k = k0; k < k0 + 64; k += 2) {
+        const od_u64 DX = sub2(X, *(const od_u64*)(q[0] + k)), DY = sub2(Y, *(const od_u64*)(q[1] + k)),
+                     DZ = sub2(Z, *(const od_u64*)(q[2] + k));
+        const od_u64 C = od_pair_c2(fma2(DZ, DZ, fma2(DY, DY, fma2(DX, DX, eps))), rho, nl2e);
+        AX = fma2(C, DX, AX); AY = fma2(C, DY, AY); AZ = fma2(C, DZ, AZ);
+      }
+      od_acc2(hi.x, lo.x, sum2(AX)); od_acc2(hi.y, lo.y, sum2(AY)); od_acc2(hi.z, lo.z, sum2(AZ));
+    }
+  }
+  if (i >= Npad) return;
+  const size_t e = (size_t)blockIdx.y * Npad + i;
+  ph[e] = make_float4(hi.x, hi.y, hi.z, 0.f);
+  pl[e] = make_float4(lo.x, lo.y, lo.z, 0.f);
+}
+
+// four lanes to an ion: each sums every fourth slab, then two-float sums over the four
+__global__ void __launch_bounds__(kBlk) k_static_finish(const float4* ph, const float4* pl, int n,
+                                                        int Npad, int jsplit, double scale,
+                                                        double* __restrict__ force) {
+  od_pdl_wait();
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e >> 2;
+  float3 hi = make_float3(0.f, 0.f, 0.f), lo = hi;
+  if (i < n)
+    for (int s = e & 3; s < jsplit; s += 4) {
+      const float4 a = ph[(size_t)s * Npad + i], b = pl[(size_t)s * Npad + i];
+      od_acc2(hi.x, lo.x, a.x); lo.x += b.x;
+      od_acc2(hi.y, lo.y, a.y); lo.y += b.y;
+      od_acc2(hi.z, lo.z, a.z); lo.z += b.z;
+    }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    float t;
+    t = __shfl_xor_sync(0xffffffffu, hi.x, o); lo.x += __shfl_xor_sync(0xffffffffu, lo.x, o);
+    od_acc2(hi.x, lo.x, t);
+    t = __shfl_xor_sync(0xffffffffu, hi.y, o); lo.y += __shfl_xor_sync(0xffffffffu, lo.y, o);
+    od_acc2(hi.y, lo.y, t);
+    t = __shfl_xor_sync(0xffffffffu, hi.z, o); lo.z += __shfl_xor_sync(0xffffffffu, lo.z, o);
+    od_acc2(hi.z, lo.z, t);
+  }
+  if (i >= n || (e & 3) == 3) return;
+  const int c = e & 3;
+  const float h = c == 0 ? hi.x : (c == 1 ? hi.y : hi.z), l = c == 0 ? lo.x : (c == 1 ? lo.y : lo.z);
+  force[3 * (size_t)i + c] = scale * ((double)h + (double)l);
 }
 }  // namespace
 
 cudaError_t od_launch_static_forces(const od_static_view& v, const double* pos, int n, double lam,
                                     double r0, double scale, double* force, cudaStream_t s) {
   const int Npad = ((n + OD_PAD - 1) / OD_PAD) * OD_PAD;
-  int jsplit = v.max_split < Npad / OD_TJ ? v.max_split : Npad / OD_TJ;
-  int chunk = (Npad + jsplit - 1) / jsplit;
-  chunk = ((chunk + OD_TJ - 1) / OD_TJ) * OD_TJ;
+  // Source chunks: about four blocks per SM, of 128 sources at least (64 below 2048 ions, where the
+  // chain of a chunk is the time); from 76 target tiles on eight, as four would leave a third of the
+  // SMs a block short (32768 ions 781 us with 512 blocks, 659 with 1024; 15000 162 with 600, 169 with
+  // 1200). The scratch holds slab_ions sums.
+  const int tiles = Npad / kStaticThreads, least = Npad < 2048 ? 64 : 128;
+  const int most = std::min(Npad / least, v.slab_ions / Npad);
+  int jsplit = std::max(1, std::min(most, (tiles <= 76 ? 608 : 1216) / tiles));
+  const int chunk = (Npad / 64 + jsplit - 1) / jsplit * 64;
   jsplit = (Npad + chunk - 1) / chunk;
   k_static_pack<<<(Npad + kBlk - 1) / kBlk, kBlk, 0, s>>>(pos, n, Npad, 1.0 / lam, v.sx, v.sy, v.sz);
-  const float rho0 = (float)(r0 / lam);
-  const float nr = 64.0f * rho0;
-  dim3 grid(Npad / 512, jsplit);
-  k_pairs_x2<256, 0><<<grid, 256, 0, s>>>(v.sx, v.sy, v.sz, Npad, chunk, v.part_hi, v.part_lo,
-                                          rho0, nr * nr, v.err, nullptr);  // partial slabs
-  k_static_finish<<<(n + kBlk - 1) / kBlk, kBlk, 0, s>>>(v.part_hi, v.part_lo, n, Npad, jsplit,
-                                                        scale, force);
-  return cudaGetLastError();
+  cudaError_t e = od_launch_pdl(k_static_pairs, dim3(tiles, jsplit), dim3(kStaticThreads), s,
+                                (const float*)v.sx, (const float*)v.sy, (const float*)v.sz, Npad,
+                                chunk, (float)(r0 / lam), v.part_hi, v.part_lo);
+  if (e != cudaSuccess) return e;
+  e = od_launch_pdl(k_static_finish, dim3((4 * n + kBlk - 1) / kBlk), dim3(kBlk), s,
+                    (const float4*)v.part_hi, (const float4*)v.part_lo, n, Npad, jsplit, scale,
+                    force);
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // ============================================================== batched step
@@ -1672,7 +1740,7 @@ cudaError_t od_launch_batch_step(const od_batchview& v, cudaStream_t s) {
                       v.sims, v.nsims, per, v.blk_ion, v.nblk_ion);
   if (e == cudaSuccess)
     e = od_launch_pdl(k_b_correct, dim3(v.nblk_corr), dim3(kCT), s, v.sims, v.blk_corr);
-  return e;
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // ============================================================== host representations

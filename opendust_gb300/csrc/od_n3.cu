@@ -56,10 +56,7 @@ struct pair_consts {
   od_u64 eps, rho, nl2e;
 };
 
-// One pack: target (X, X) against two sources. With R = r and W = 1/(r (r + rho)):
-// c = exp(-r) (1/s + 1/s^2) / r = exp(-r) (W + W (W r)), s = r + rho. One packed operation fewer
-// than the form from 1/sqrt(r^2), and more accurate (the term's rms error 0.9e-7 against 1.1e-7
-// for r < 1, 2.1e-7 against 2.9e-7 at r = 4.5).
+// One pack: target (X, X) against two sources.
 template <bool REACT>
 __device__ __forceinline__ void pair_once(const pair_consts& k, od_u64 X, od_u64 Y, od_u64 Z,
                                           od_u64 QX, od_u64 QY, od_u64 QZ, od_u64& AX, od_u64& AY,
@@ -68,13 +65,7 @@ __device__ __forceinline__ void pair_once(const pair_consts& k, od_u64 X, od_u64
   od_u64 R2 = fma2(DX, DX, k.eps);
   R2 = fma2(DY, DY, R2);
   R2 = fma2(DZ, DZ, R2);
-  const float2 r2 = up2(R2);
-  const od_u64 R = p2(od_sqrt(r2.x), od_sqrt(r2.y));
-  const float2 rs = up2(fma2(R, k.rho, R2));
-  const od_u64 W = p2(od_rcp(rs.x), od_rcp(rs.y));
-  const float2 ea = up2(mul2(R, k.nl2e));
-  const od_u64 EX = p2(od_ex2(ea.x), od_ex2(ea.y));
-  const od_u64 C = mul2(EX, fma2(W, mul2(W, R), W));
+  const od_u64 C = od_pair_c2(R2, k.rho, k.nl2e);
   AX = fma2(C, DX, AX); AY = fma2(C, DY, AY); AZ = fma2(C, DZ, AZ);
   if (REACT) { RX = fma2(C, DX, RX); RY = fma2(C, DY, RY); RZ = fma2(C, DZ, RZ); }
 }
@@ -351,7 +342,7 @@ cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, cudaStream_t s) {
   OD_B_N3(2, 4, 4, 4, false);
   OD_B_N3(4, 4, 4, 1, true);
 #undef OD_B_N3
-  return e;
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 int od_n3_batch_plan(int Npad, size_t budget_bytes, int* ipt) {
