@@ -1504,20 +1504,16 @@ extern "C" od_status od_trap_potential(double Rh, double Hh, int32_t n_r, int32_
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaSetDevice");
   const int nn = n_r * n_h;
-  const int nchunks = std::max(1, (int)std::min<int64_t>(od_num_sms(device) * 4, (n_points + 4095) / 4096));
+  const int nchunks = od_trap_chunks(nn, n_points, od_num_sms(device));
   double* part = nullptr;
-  e = cudaMalloc(&part, sizeof(double) * nn * nchunks);
+  e = cudaMalloc(&part, sizeof(double) * nn * ((size_t)nchunks + 1));
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaMalloc");
-  e = od_launch_trap(Rh, Hh, n_r, n_h, n_points, seed, part, nchunks, 0);
-  std::vector<double> hpart((size_t)nn * nchunks);
-  if (e == cudaSuccess) e = cudaMemcpy(hpart.data(), part, sizeof(double) * nn * nchunks, cudaMemcpyDeviceToHost);
+  double* const sum = part + (size_t)nn * nchunks;
+  e = od_launch_trap(Rh, Hh, n_r, n_h, n_points, seed, part, nchunks, sum, 0);
+  if (e == cudaSuccess) e = cudaMemcpy(pot, sum, sizeof(double) * nn, cudaMemcpyDeviceToHost);
   cudaFree(part);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "trap potential");
-  for (int i = 0; i < nn; i++) {
-    double s = 0;
-    for (int c = 0; c < nchunks; c++) s += hpart[(size_t)c * nn + i];
-    pot[i] = s / (double)n_points;
-  }
+  for (int i = 0; i < nn; i++) pot[i] /= (double)n_points;
   return OD_OK;
 }
 

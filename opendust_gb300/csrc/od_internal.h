@@ -249,7 +249,8 @@ cudaError_t od_launch_snapshot_flags(const od_dparams* dp, int n, int Npad, cons
 cudaError_t od_launch_set_charges(const od_dparams* dp, od_dstate* ds, float* cq, int P,
                                   cudaStream_t s);
 cudaError_t od_launch_trap(double Rh, double Hh, int n_r, int n_h, int64_t n_points, uint64_t seed,
-                           double* part, int nchunks, cudaStream_t s);
+                           double* part, int nchunks, double* sum, cudaStream_t s);
+int od_trap_chunks(int nn, int64_t n_points, int sms);  // chunks of the points (part: [chunks][nn])
 
 // launch with programmatic stream serialization (the kernel calls od_pdl_wait before
 // it touches anything that an earlier kernel wrote or reads)

@@ -1188,12 +1188,19 @@ __global__ void k_set_charges(const od_dparams* __restrict__ dp, const od_dstate
 }
 
 // ============================================================== trap-fit potential grid
-constexpr int kTrapPts = 2048;
-__global__ void __launch_bounds__(kBlk) k_trap(double Rh, double Hh, int n_r, int n_h,
-                                               int64_t n_points, int64_t pts_per_block,
-                                               uint32_t k0, uint32_t k1,
-                                               double* __restrict__ part) {
-  __shared__ float4 s_pts[kTrapPts];
+// Thread: one node; block: 256 nodes and a chunk of points, which it draws into shared memory 2048 at a
+// time. exp(-r)/(r + 0.001) over four points at once, on one common denominator, so that a point costs
+// two and a quarter SFU operations (14.7 cycles per 32 and sub-partition) instead of three (21), and the
+// FP32 chain has 128 additions instead of 2048. The chunks fill the GPU once (six blocks per
+// SM), where a fixed size of 4096 points left a second wave of a few blocks. 900 nodes and 1.36e6
+// points: a call 1.23 -> 0.77 ms (the chunk sums no longer copied to the host); 3600 nodes and 1.1e7
+// points 25.3 -> 17.3 ms.
+constexpr int kTrapPts = 2048, kTrapBlocks = 6;
+__global__ void __launch_bounds__(kBlk, kTrapBlocks) k_trap(double Rh, double Hh, int n_r, int n_h,
+                                                            int64_t n_points, int64_t pts_per_block,
+                                                            uint32_t k0, uint32_t k1,
+                                                            double* __restrict__ part) {
+  __shared__ __align__(16) float s_x[kTrapPts], s_y[kTrapPts], s_z[kTrapPts];
   const int node = blockIdx.x * kBlk + threadIdx.x;
   const int nn = n_r * n_h;
   float gr = 0.f, gh = 0.f;
@@ -1202,33 +1209,59 @@ __global__ void __launch_bounds__(kBlk) k_trap(double Rh, double Hh, int n_r, in
     gr = (float)((i == n_r - 1) ? Rh : i * (Rh / (n_r - 1)));
     gh = (float)((j == n_h - 1) ? Hh / 2.0 : j * ((Hh / 2.0) / (n_h - 1)));
   }
+  const od_u64 GR = p2(gr, gr), GH = p2(gh, gh), eps = p2(1e-30f, 1e-30f);
+  const od_u64 nl2e = p2(OD_NLOG2E, OD_NLOG2E), r0 = p2(0.001f, 0.001f), one = p2(1.f, 1.f);
   const int64_t p0 = blockIdx.y * pts_per_block;
   const int64_t p1 = min(p0 + pts_per_block, n_points);
   double acc = 0.0;
   for (int64_t t0 = p0; t0 < p1; t0 += kTrapPts) {
-    const int cnt = (int)min((int64_t)kTrapPts, p1 - t0);
+    const int cnt = (int)min((int64_t)kTrapPts, p1 - t0), cnt4 = (cnt + 3) & ~3;
     __syncthreads();
-    for (int q = threadIdx.x; q < cnt; q += kBlk) {
+    for (int q = threadIdx.x; q < cnt4; q += kBlk) {
       od_u4 w = od_philox((uint32_t)(t0 + q), 0u, OD_RNG_TRAP, 0u, k0, k1);
       const float r = sqrtf(od_u01(w.x));
       float s, c;
       sincospif(2.0f * od_u01(w.y), &s, &c);
-      s_pts[q] = make_float4((float)Rh * r * c, (float)Rh * r * s,
-                             (float)Hh * od_u01(w.z) - (float)Hh * 0.5f, 0.f);
+      const bool real = q < cnt;  // the others are too far away to add anything
+      s_x[q] = real ? (float)Rh * r * c : 1e6f;
+      s_y[q] = real ? (float)Rh * r * s : 1e6f;
+      s_z[q] = real ? (float)Hh * od_u01(w.z) - (float)Hh * 0.5f : 1e6f;
     }
     __syncthreads();
-    float a = 0.f;
-    for (int q = 0; q < cnt; q++) {
-      const float4 pt = s_pts[q];
-      const float dx = gr - pt.x, dy = pt.y, dz = gh - pt.z;
-      const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-      const float ri = od_rsqrt(fmaxf(r2, 1e-30f));
-      const float r = r2 * ri;
-      a += od_ex2(r * OD_NLOG2E) * od_rcp(r + 0.001f);
+    for (int q0 = 0; q0 < cnt4; q0 += 512) {
+      float a = 0.f;
+      const int q1 = min(q0 + 512, cnt4);
+#pragma unroll 4
+      for (int q = q0; q < q1; q += 4) {
+        const ulonglong2 x = *(const ulonglong2*)(s_x + q), y = *(const ulonglong2*)(s_y + q),
+                         z = *(const ulonglong2*)(s_z + q);
+        float num[2], den[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const od_u64 DX = sub2(GR, h ? x.y : x.x), DY = h ? y.y : y.x, DZ = sub2(GH, h ? z.y : z.x);
+          const float2 r2 = up2(fma2(DX, DX, fma2(DY, DY, fma2(DZ, DZ, eps))));
+          const od_u64 R = p2(od_sqrt(r2.x), od_sqrt(r2.y));
+          const float2 ea = up2(mul2(R, nl2e)), sr = up2(fma2(R, one, r0));
+          num[h] = fmaf(od_ex2(ea.x), sr.y, od_ex2(ea.y) * sr.x);
+          den[h] = sr.x * sr.y;
+        }
+        a = fmaf(fmaf(num[0], den[1], num[1] * den[0]), od_rcp(den[0] * den[1]), a);
+      }
+      acc += a;
     }
-    acc += a;
   }
   if (node < nn) part[(size_t)blockIdx.y * nn + node] = acc;
+}
+
+// sums over the chunks, in their order
+__global__ void __launch_bounds__(kBlk) k_trap_sum(const double* __restrict__ part, int nn,
+                                                   int nchunks, double* __restrict__ sum) {
+  const int node = blockIdx.x * kBlk + threadIdx.x;
+  if (node >= nn) return;
+  double s = 0;
+#pragma unroll 8
+  for (int c = 0; c < nchunks; c++) s += part[(size_t)c * nn + node];
+  sum[node] = s;
 }
 
 // ============================================================== initial state on the device
@@ -1484,13 +1517,19 @@ cudaError_t od_launch_set_charges(const od_dparams* dp, od_dstate* ds, float* cq
   return cudaGetLastError();
 }
 
+int od_trap_chunks(int nn, int64_t n_points, int sms) {
+  const int64_t fill = (int64_t)sms * kTrapBlocks / ((nn + kBlk - 1) / kBlk);
+  return (int)std::max<int64_t>(1, std::min<int64_t>(fill, (n_points + 255) / 256));
+}
+
 cudaError_t od_launch_trap(double Rh, double Hh, int n_r, int n_h, int64_t n_points, uint64_t seed,
-                           double* part, int nchunks, cudaStream_t s) {
-  const int nn = n_r * n_h;
+                           double* part, int nchunks, double* sum, cudaStream_t s) {
+  const int nn = n_r * n_h, nb = (nn + kBlk - 1) / kBlk;
   const int64_t per = (n_points + nchunks - 1) / nchunks;
-  dim3 grid((nn + kBlk - 1) / kBlk, nchunks);
-  k_trap<<<grid, kBlk, 0, s>>>(Rh, Hh, n_r, n_h, n_points, per, (uint32_t)(seed & 0xffffffffu),
-                               (uint32_t)(seed >> 32), part);
+  k_trap<<<dim3(nb, nchunks), kBlk, 0, s>>>(Rh, Hh, n_r, n_h, n_points, per,
+                                            (uint32_t)(seed & 0xffffffffu), (uint32_t)(seed >> 32),
+                                            part);
+  k_trap_sum<<<nb, kBlk, 0, s>>>(part, nn, nchunks, sum);
   return cudaGetLastError();
 }
 
