@@ -1078,8 +1078,9 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
   const size_t ns = L->nslots, nc = L->ncells;
   cudaError_t e = carve(&L->block, nullptr, [&](od_carver& c) {
     c.take(L->cell_of, (size_t)N);
+    c.take(L->rank_of, (size_t)N);
+    c.take(L->unsorted, (size_t)N);
     c.take(L->count, nc);
-    c.take(L->fill, nc);
     c.take(L->start, nc + 1);
     c.take(L->perm, ns);
     c.take(L->xs, ns);
@@ -1092,11 +1093,11 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
     if (od_cutn3_listed(ns)) {
       c.take(L->rows, ns / 64 * (ns / 32));
       c.take(L->counts, ns / 64);
-      c.take(L->prefix, ns / 64 + 1);
     }
   });
   if (e == cudaSuccess)
     e = cudaMemsetAsync(L->acc, 0, sizeof(unsigned long long) * 3 * ns, h->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(L->count, 0, sizeof(int32_t) * nc, h->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
     free_cutn3(h);

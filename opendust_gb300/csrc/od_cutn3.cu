@@ -13,10 +13,10 @@
 // What bounds it: as the all-pairs kernel, operand fetch of the packed FP32 pipe (17 packed
 // operations per pair of pairs for the plain term, 27 with switching), plus the pairs of the
 // listed blocks that lie beyond the cutoff. field_chain (2^19 ions, 2 lambda): 1.63 pairs
-// evaluated per pair inside, 22.6 ms per evaluation. The tile-pair form this replaces (512-ion
+// evaluated per pair inside, 22.2 ms per evaluation. The tile-pair form this replaces (512-ion
 // tile pairs, 64 x 64 group lists built by one warp between two block barriers, 2 x 2 ions per
 // lane, sums in shared memory with compare-and-swap atomics) took 32.2 ms there; 65536 ions in
-// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.79 ms, 20011 ions at 2 lambda 0.197 -> 0.105 ms.
+// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.74 ms, 20011 ions at 2 lambda 0.197 -> 0.077 ms.
 #include "od_hilbert.h"
 #include "od_internal.h"
 #include <algorithm>
@@ -28,23 +28,18 @@ namespace {
 // a Hilbert curve (od_hilbert.h), so that the ions sorted by key fill tiles and 64-ion groups
 // with compact bounding boxes: at 2^19 ions in the 3 x 6 lambda cylinder the boxes of 64-ion
 // groups keep 1.73x the pairs inside a 2 lambda cutoff, against 1.94x in Morton order.
-__global__ void k_mc_clear(int ncells, int32_t* __restrict__ count, int32_t* __restrict__ fill,
+//
+// Cubes of G^3 cells stacked nb deep along z (nb = 1 for a compact domain); a cell's key is its
+// cube's index times G^3 plus its index along the cube's Hilbert curve. The counts are zero between
+// evaluations (k_mc_sort clears them); an ion's rank is the count that it found.
+__global__ void k_mc_count(int n, const float4* __restrict__ pos, float lo, float lo_z,
+                           float inv_s, int G, int nb, int32_t* __restrict__ cell_of,
+                           int32_t* __restrict__ rank_of, int32_t* __restrict__ count,
                            unsigned long long* __restrict__ next) {
   od_pdl_wait();
   od_pdl_trigger();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c == 0) *next = 0ull;  // the pair kernel's work counter
-  if (c < ncells) { count[c] = 0; fill[c] = 0; }
-}
-
-// Cubes of G^3 cells stacked nb deep along z (nb = 1 for a compact domain); a cell's key is its
-// cube's index times G^3 plus its index along the cube's Hilbert curve.
-__global__ void k_mc_count(int n, const float4* __restrict__ pos, float lo, float lo_z,
-                           float inv_s, int G, int nb, int32_t* __restrict__ cell_of,
-                           int32_t* __restrict__ count) {
-  od_pdl_wait();
-  od_pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *next = 0ull;  // the pair kernel's work counter
   if (i >= n) return;
   const float4 p = pos[i];
   const int bits = 31 - __clz(G);
@@ -54,20 +49,29 @@ __global__ void k_mc_count(int n, const float4* __restrict__ pos, float lo, floa
   const int c = ((cz >> bits) << (3 * bits)) +
                 (int)od_hilbert3((uint32_t)cx, (uint32_t)cy, (uint32_t)(cz & (G - 1)), bits);
   cell_of[i] = c;
-  atomicAdd(&count[c], 1);
+  rank_of[i] = atomicAdd(&count[c], 1);
 }
 
-// exclusive scan of in[0..n) into out[0..n], out[n] = total (one 1024-thread block; in and out
-// may be the same array: every thread reads each of its entries before writing it)
+// exclusive scan of in[0..n) into out[0..n], out[n] = total (one 1024-thread block, four entries to a
+// load where the threads' runs allow it)
 __global__ void __launch_bounds__(1024) k_scan_excl(int n, const int32_t* in, int32_t* out) {
+  __shared__ int s_w[32];
   od_pdl_wait();
   od_pdl_trigger();
-  __shared__ int s_w[32];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int per = (n + 1023) / 1024;
+  const bool quads = n % 4096 == 0;
   const int c0 = min(tid * per, n), c1 = min(c0 + per, n);
   int a = 0;
-  for (int c = c0; c < c1; c++) a += in[c];
+  if (quads) {
+#pragma unroll 8
+    for (int c = c0; c < c1; c += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(in + c);
+      a += (v.x + v.y) + (v.z + v.w);
+    }
+  } else {
+    for (int c = c0; c < c1; c++) a += in[c];
+  }
   int ia = a;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -88,67 +92,113 @@ __global__ void __launch_bounds__(1024) k_scan_excl(int n, const int32_t* in, in
   }
   __syncthreads();
   int off = s_w[wid] + ia - a;
-  for (int c = c0; c < c1; c++) {
-    const int v = in[c];
-    out[c] = off;
-    off += v;
+  if (quads) {
+#pragma unroll 8
+    for (int c = c0; c < c1; c += 4) {
+      const int4 v = *reinterpret_cast<const int4*>(in + c);
+      *reinterpret_cast<int4*>(out + c) = make_int4(off, off + v.x, off + v.x + v.y,
+                                                    off + v.x + v.y + v.z);
+      off += (v.x + v.y) + (v.z + v.w);
+    }
+  } else {
+    for (int c = c0; c < c1; c++) {
+      const int v = in[c];
+      out[c] = off;
+      off += v;
+    }
   }
   if (tid == 1023) out[n] = off;
 }
 
 __global__ void k_mc_scatter(int n, const int32_t* __restrict__ cell_of,
-                             const int32_t* __restrict__ start, int32_t* __restrict__ fill,
-                             int32_t* __restrict__ perm) {
+                             const int32_t* __restrict__ rank_of,
+                             const int32_t* __restrict__ start,
+                             int32_t* __restrict__ unsorted) {
   od_pdl_wait();
   od_pdl_trigger();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int c = cell_of[i];
-  perm[start[c] + atomicAdd(&fill[c], 1)] = i;
+  unsorted[start[cell_of[i]] + rank_of[i]] = i;
 }
 
-// One block per cell: sort the cell's ions by index (bitonic in shared memory; the order of
-// the atomic scatter is not reproducible, the sorted order is) and write their positions.
-constexpr int kCellMax = 2048;
-__global__ void __launch_bounds__(128) k_mc_sort(const int32_t* count,
-                                                 const int32_t* __restrict__ start,
-                                                 const float4* __restrict__ pos,
-                                                 int32_t* __restrict__ perm, float* __restrict__ xs,
-                                                 float* __restrict__ ys, float* __restrict__ zs,
-                                                 uint32_t* __restrict__ err) {
+// The same with the scan: up to kScanCells cells every block scans the counts for itself (16 KB at 4096
+// cells, from L2), which takes less than the launch of a scan of its own (20011 ions: 4.8 + 2.5 us ->
+// 4.1, the ranks of k_mc_count instead of a second round of atomics included). A multiple of 512 cells.
+constexpr int kScanCells = 8192;
+__global__ void __launch_bounds__(256) k_mc_scan_scatter(int n, int ncells,
+                                                         const int32_t* __restrict__ cell_of,
+                                                         const int32_t* __restrict__ rank_of,
+                                                         const int32_t* count,
+                                                         int32_t* __restrict__ start,
+                                                         int32_t* __restrict__ unsorted) {
+  extern __shared__ int32_t s_start[];  // cell c at c + c / 16, so that a thread's run has no conflicts
+  __shared__ int s_w[8];
   od_pdl_wait();
   od_pdl_trigger();
-  __shared__ int32_t key[kCellMax];
-  const int c = blockIdx.x;
-  const int n0 = count[c];
-  if (n0 == 0) return;
-  if (n0 > kCellMax) {
-    if (threadIdx.x == 0) atomicOr(err, OD_DERR_CELL);
-    return;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, per = ncells / 256, c0 = tid * per;
+  int sum = 0;
+  for (int c = 0; c < per; c += 2) {
+    const int2 v = *reinterpret_cast<const int2*>(count + c0 + c);
+    s_start[c0 + c + ((c0 + c) >> 4)] = v.x;
+    s_start[c0 + c + 1 + ((c0 + c + 1) >> 4)] = v.y;
+    sum += v.x + v.y;
   }
-  const int s0 = start[c];
-  int m = 1;
-  while (m < n0) m <<= 1;
-  for (int k = threadIdx.x; k < m; k += 128) key[k] = k < n0 ? perm[s0 + k] : 0x7fffffff;
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) s_w[w] = incl;
   __syncthreads();
-  for (int size = 2; size <= m; size <<= 1)
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int k = threadIdx.x; k < m; k += 128) {
-        const int l = k ^ stride;
-        if (l > k) {
-          const bool up = (k & size) == 0;
-          const int a = key[k], b = key[l];
-          if ((a > b) == up) { key[k] = b; key[l] = a; }
-        }
-      }
-      __syncthreads();
-    }
-  for (int k = threadIdx.x; k < n0; k += 128) {
-    const int i = key[k];
-    const float4 p = pos[i];
-    perm[s0 + k] = i;
-    xs[s0 + k] = p.x; ys[s0 + k] = p.y; zs[s0 + k] = p.z;
+  int off = incl - sum;
+  for (int k = 0; k < w; k++) off += s_w[k];
+  for (int c = c0; c < c0 + per; c++) {
+    const int v = s_start[c + (c >> 4)];
+    s_start[c + (c >> 4)] = off;
+    off += v;
   }
+  __syncthreads();
+  if (blockIdx.x == 0) {
+    for (int c = tid; c < ncells; c += 256) start[c] = s_start[c + (c >> 4)];
+    if (tid == 0) start[ncells] = n;
+  }
+  const int i = blockIdx.x * 256 + tid;
+  if (i >= n) return;
+  const int c = cell_of[i];
+  unsorted[s_start[c + (c >> 4)] + rank_of[i]] = i;
+}
+
+// Sorts every cell's ions by index (the order of the atomic ranks is not reproducible, the sorted
+// order is) and writes their positions; the counts are cleared for the next evaluation. A
+// thread takes an unsorted slot and counts the smaller indices in its cell: neighbouring threads read
+// the same few entries, and the work does not depend on the number of cells (20011 ions 6.0 -> 3.5 us
+// against a block per cell with a bitonic sort).
+constexpr int kCellMax = 2048;
+__global__ void __launch_bounds__(256) k_mc_sort(int n, const int32_t* __restrict__ cell_of,
+                                                 const int32_t* __restrict__ start,
+                                                 const int32_t* __restrict__ unsorted,
+                                                 const float4* __restrict__ pos, int32_t* count,
+                                                 int32_t* __restrict__ perm,
+                                                 float* __restrict__ xs, float* __restrict__ ys,
+                                                 float* __restrict__ zs, uint32_t* __restrict__ err) {
+  od_pdl_wait();
+  od_pdl_trigger();
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= n) return;
+  const int i = unsorted[s], c = cell_of[i], s0 = start[c], n0 = start[c + 1] - s0;
+  const float4 p = pos[i];
+  int slot = s0;
+  if (n0 <= kCellMax) {
+#pragma unroll 4
+    for (int k = 0; k < n0; k++) slot += unsorted[s0 + k] < i;
+  } else {  // left unsorted, with an error
+    slot = s;
+    if (s == s0) atomicOr(err, OD_DERR_CELL);
+  }
+  if (s == s0) count[c] = 0;
+  perm[slot] = i;
+  xs[slot] = p.x; ys[slot] = p.y; zs[slot] = p.z;
 }
 
 // Bounding boxes of the 16 blocks of every 512-slot tile and of the tile itself: (min x, min y,
@@ -520,21 +570,17 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
 // ------------------------------------------------------------------ small systems: listed work
 // Up to kListBlocks blocks the units above are too coarse: a warp gets a few batches, and the last ones
 // run alone (force chain of 8192 ions at 2 lambda 0.132 ms). Here one warp per source group lists its
-// target blocks first (inner ones from the front of its row, the others from the back), the last block to
-// finish takes the prefix over the groups, and the warps of the pair kernel draw runs of equal length from
-// it: half batches where there are fewer than four per warp (8192 ions 0.069 ms; whole batches 0.077), else
+// target blocks first (inner ones from the front of its row, the others from the back), every block of the
+// pair kernel takes the prefix over the groups, and its warps draw runs of equal length from it: half batches where there are fewer than four per warp (8192 ions 0.069 ms; whole batches 0.077), else
 // whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635 with the units).
 constexpr int kListBlocks = 4096;
 __global__ void __launch_bounds__(256) k_cut_lists(int nsg, int nT, const cut_args cut,
                                                    const float4* __restrict__ tbox,
                                                    const float4* __restrict__ bbox,
                                                    uint16_t* __restrict__ rows,
-                                                   int2* __restrict__ cnt, int* __restrict__ prefix,
-                                                   unsigned long long* __restrict__ ticket) {
+                                                   int2* __restrict__ cnt) {
   od_pdl_wait();
   od_pdl_trigger();
-  __shared__ int s_w[8];
-  __shared__ bool s_last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int sg = blockIdx.x * 8 + w, nB = nT * kTB;
   if (sg < nsg) {
@@ -547,58 +593,36 @@ __global__ void __launch_bounds__(256) k_cut_lists(int nsg, int nT, const cut_ar
       if (b0 + lane < nT) box_dist(tbox, b0 + lane, sb, d2, f2);
       unsigned int tiles = __ballot_sync(0xffffffffu, d2 < cut.cull2);
       while (tiles) {
-        const int t1 = __ffs(tiles) - 1;
-        tiles &= tiles - 1;
-        const int t2 = tiles ? __ffs(tiles) - 1 : -1;
-        if (tiles) tiles &= tiles - 1;
-        const int tl = lane < 16 ? t1 : t2;
-        const int blk = (b0 + tl) * kTB + (lane & 15);
-        d2 = f2 = 3e38f;
-        if (tl >= 0 && blk > 2 * sg + 1) box_dist(bbox, blk, sb, d2, f2);
-        const bool keep = d2 < cut.cull2, inner = keep && f2 < cut.in2;
-        const unsigned int mi = __ballot_sync(0xffffffffu, inner),
-                           mo = __ballot_sync(0xffffffffu, keep && !inner);
-        const unsigned int below = (1u << lane) - 1u;
-        if (inner) row[ni + __popc(mi & below)] = (uint16_t)blk;
-        else if (keep) row[nB - 1 - no - __popc(mo & below)] = (uint16_t)blk;
-        ni += __popc(mi);
-        no += __popc(mo);
+        // eight tiles a round, two at a time, so that their loads overlap (20011 ions: 10.3 us with
+        // two a round)
+        int blk[4];
+        float near2[4], far2[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const int t1 = __ffs(tiles) - 1;  // -1: none left
+          tiles &= tiles - 1;
+          const int t2 = __ffs(tiles) - 1;
+          tiles &= tiles - 1;
+          const int tl = lane < 16 ? t1 : t2;
+          blk[r] = (b0 + tl) * kTB + (lane & 15);
+          near2[r] = far2[r] = 3e38f;
+          if (tl >= 0 && blk[r] > 2 * sg + 1) box_dist(bbox, blk[r], sb, near2[r], far2[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const bool keep = near2[r] < cut.cull2, inner = keep && far2[r] < cut.in2;
+          const unsigned int mi = __ballot_sync(0xffffffffu, inner),
+                             mo = __ballot_sync(0xffffffffu, keep && !inner);
+          const unsigned int below = (1u << lane) - 1u;
+          if (inner) row[ni + __popc(mi & below)] = (uint16_t)blk[r];
+          else if (keep) row[nB - 1 - no - __popc(mo & below)] = (uint16_t)blk[r];
+          ni += __popc(mi);
+          no += __popc(mo);
+        }
       }
     }
     if (lane == 0) cnt[sg] = make_int2(ni, no);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  if (threadIdx.x == 0) *ticket = 0ull;  // the pair kernel's work counter from here on
-  // half batches of each group: the group itself, the inner fours, the rest
-  const int per = (nsg + 255) / 256, g0 = min((int)threadIdx.x * per, nsg), g1 = min(g0 + per, nsg);
-  int sum = 0;
-  for (int g = g0; g < g1; g++) {
-    const int2 c = __ldcg(cnt + g);
-    sum += 2 * (1 + c.x / 4 + (c.y + (c.x & 3) + 3) / 4);
-  }
-  int incl = sum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) s_w[w] = incl;
-  __syncthreads();
-  int off = incl - sum;
-  for (int k = 0; k < w; k++) off += s_w[k];
-  for (int g = g0; g < g1; g++) {
-    const int2 c = __ldcg(cnt + g);
-    prefix[g] = off;
-    off += 2 * (1 + c.x / 4 + (c.y + (c.x & 3) + 3) / 4);
-  }
-  if (g1 == nsg && g0 < nsg) prefix[nsg] = off;
 }
 
 template <int CUT, bool COUNT>
@@ -606,8 +630,7 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
     k_pairs_cutlist(const float* __restrict__ xs, const float* __restrict__ ys,
                     const float* __restrict__ zs, int nslots, unsigned long long* __restrict__ acc,
                     const __grid_constant__ cut_args cut, const uint16_t* __restrict__ rows,
-                    const int2* __restrict__ counts, const int* __restrict__ prefix,
-                    unsigned int* __restrict__ next,
+                    const int2* __restrict__ counts, unsigned int* __restrict__ next,
                     unsigned long long* __restrict__ pair_count) {
   od_pdl_wait();
   od_pdl_trigger();
@@ -615,8 +638,36 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
   __shared__ int s_prefix[kListBlocks / 2 + 1];
   __shared__ unsigned int s_tb[WARPS][4];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nsg = nslots / 64, nB = nslots / kBlk;
-  for (int g = threadIdx.x; g <= nsg; g += WARPS * 32) s_prefix[g] = prefix[g];
-  __syncthreads();
+  {  // prefix of the groups' half batches: the group itself, the inner fours, the rest
+    __shared__ int s_w[WARPS];
+    const int per = (nsg + WARPS * 32 - 1) / (WARPS * 32);
+    const int g0 = min((int)threadIdx.x * per, nsg), g1 = min(g0 + per, nsg);
+    int sum = 0;
+#pragma unroll 4
+    for (int g = g0; g < g1; g++) {
+      const int2 c = counts[g];
+      const int q = 2 * (1 + c.x / 4 + (c.y + (c.x & 3) + 3) / 4);
+      s_prefix[g] = q;
+      sum += q;
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_w[w] = incl;
+    __syncthreads();
+    int off = incl - sum;
+    for (int v = 0; v < w; v++) off += s_w[v];
+    for (int g = g0; g < g1; g++) {
+      const int q = s_prefix[g];
+      s_prefix[g] = off;
+      off += q;
+    }
+    if (threadIdx.x == WARPS * 32 - 1) s_prefix[nsg] = off;
+    __syncthreads();
+  }
   unsigned int* const tb = s_tb[w];
   const cut_consts k = make_consts(cut);
   unsigned int cnt = 0;
@@ -699,10 +750,12 @@ od_cgrid od_cutn3_grid(int N, double R, double H) {
   // wide as the domain, so that the cells keep their size whatever the aspect ratio
   g.nb = H <= 3.0 * R ? 1 : (int)std::ceil(H / (2.0 * R));
   g.side = (g.nb == 1 ? std::max(2.0 * R, H) : 2.0 * R) * 1.02;
-  // about 16 ions per cell: G the smallest power of two with G^3 >= (N / nb) / 22, 8 <= G <= 128
+  // 1.4 to 11 ions per cell of a cube: the sort's order inside a cell is arbitrary, so smaller cells give
+  // tighter blocks. Against 2.8 to 22 and, before, up to 128 per cell, us per step: 20011 ions 128, 128,
+  // 137; 40000 298, 298, 328; 65536 606, 616, 616; 131072 1870, 1870, 1968; 2^19 22270, 22710, 22710
   const double per = (double)N / g.nb;
   g.G = 8;
-  while (g.G < 128 && (double)g.G * g.G * g.G * 8.0 * 16.0 < per * 1.4142) g.G <<= 1;
+  while (g.G < 128 && (double)g.G * g.G * g.G * 8.0 * 2.0 < per * 1.4142) g.G <<= 1;
   g.ncells = g.nb * g.G * g.G * g.G;
   return g;
 }
@@ -710,7 +763,7 @@ od_cgrid od_cutn3_grid(int N, double R, double H) {
 bool od_cutn3_listed(size_t nslots) { return nslots / kBlk <= kListBlocks; }
 static size_t od_cutn3_list_bytes(size_t ns) {
   const size_t nsg = ns / 64, nB = ns / kBlk;
-  return od_cutn3_listed(ns) ? sizeof(uint16_t) * nsg * nB + sizeof(int2) * nsg + sizeof(int) * (nsg + 1)
+  return od_cutn3_listed(ns) ? sizeof(uint16_t) * nsg * nB + sizeof(int2) * nsg
                              : 0;
 }
 
@@ -720,7 +773,7 @@ size_t od_cutn3_bytes(int N, int T, int ncells) {
          + sizeof(float4) * 2 * (ns / kBlk + ns / kTile)              // boxes
          + od_cutn3_list_bytes(ns)
          + sizeof(float) * 3 * ns                                     // sorted positions
-         + sizeof(int32_t) * (ns + N + 3 * nc + 1);
+         + sizeof(int32_t) * (ns + 3 * (size_t)N + 2 * nc + 1);
 }
 
 bool od_cutn3_supported(int ipt, int T) {
@@ -753,24 +806,30 @@ int od_cutn3_blocks_per_sm(bool hard) {
 cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, float4* part_hi,
                                 float4* part_lo, float rho0, float rc, float rs, uint32_t* err,
                                 unsigned long long* pair_count, cudaStream_t s) {
-  cudaError_t e = od_launch_pdl(k_mc_clear, dim3((L.ncells + 255) / 256), dim3(256), s, L.ncells, L.count,
-                                L.fill, L.next);
   // every kernel of the chain with programmatic dependent launch, the next one let in only after the
   // wait (8192 ions 72.0 -> 68.7 us per step, 20011 140 -> 137; let in before it, the waiting blocks of
   // two kernels on, the pair kernel's among them, hold the SMs: 142)
   const dim3 nb((n + 255) / 256), nt(256);
   const int nT = L.nslots / kTile;
+  cudaError_t e = od_launch_pdl(k_mc_count, nb, nt, s, n, pos, L.lo, L.lo_z, L.inv_s, L.G, L.nb,
+                                L.cell_of, L.rank_of, L.count, L.next);
+  if (L.ncells <= kScanCells) {
+    if (e == cudaSuccess)
+      e = od_launch_pdl_smem(k_mc_scan_scatter, nb, nt, sizeof(int32_t) * (L.ncells + L.ncells / 16), s,
+                             n, L.ncells, (const int32_t*)L.cell_of, (const int32_t*)L.rank_of,
+                             (const int32_t*)L.count, L.start, L.unsorted);
+  } else {
+    if (e == cudaSuccess)
+      e = od_launch_pdl(k_scan_excl, dim3(1), dim3(1024), s, L.ncells, (const int32_t*)L.count,
+                        L.start);
+    if (e == cudaSuccess)
+      e = od_launch_pdl(k_mc_scatter, nb, nt, s, n, (const int32_t*)L.cell_of,
+                        (const int32_t*)L.rank_of, (const int32_t*)L.start, L.unsorted);
+  }
   if (e == cudaSuccess)
-    e = od_launch_pdl(k_mc_count, nb, nt, s, n, pos, L.lo, L.lo_z, L.inv_s, L.G, L.nb, L.cell_of,
-                      L.count);
-  if (e == cudaSuccess)
-    e = od_launch_pdl(k_scan_excl, dim3(1), dim3(1024), s, L.ncells, (const int32_t*)L.count, L.start);
-  if (e == cudaSuccess)
-    e = od_launch_pdl(k_mc_scatter, nb, nt, s, n, (const int32_t*)L.cell_of, (const int32_t*)L.start,
-                      L.fill, L.perm);
-  if (e == cudaSuccess)
-    e = od_launch_pdl(k_mc_sort, dim3(L.ncells), dim3(128), s, (const int32_t*)L.count,
-                      (const int32_t*)L.start, pos, L.perm, L.xs, L.ys, L.zs, err);
+    e = od_launch_pdl(k_mc_sort, nb, nt, s, n, (const int32_t*)L.cell_of, (const int32_t*)L.start,
+                      (const int32_t*)L.unsorted, pos, L.count, L.perm, L.xs, L.ys, L.zs,
+                      err);
   if (e == cudaSuccess)
     e = od_launch_pdl(k_tile_box, dim3(nT), dim3(kTile), s, n, L.xs, L.ys, L.zs, L.perm, L.bbox,
                       L.tbox);
@@ -786,13 +845,13 @@ cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, flo
   if (L.rows) {
     const int nsg = L.nslots / 64;
     e = od_launch_pdl(k_cut_lists, dim3((nsg + 7) / 8), nt, s, nsg, nT, cut, (const float4*)L.tbox,
-                      (const float4*)L.bbox, L.rows, L.counts, L.prefix, L.next);
+                      (const float4*)L.bbox, L.rows, L.counts);
     if (e != cudaSuccess) return e;
 #define OD_CUTN3(CUT, CNT)                                                                       \
   e = od_launch_pdl(k_pairs_cutlist<CUT, CNT>, dim3(grid), dim3(cut_traits<CUT>::WARPS * 32), s, \
                     (const float*)L.xs, (const float*)L.ys, (const float*)L.zs, L.nslots, L.acc, \
-                    cut, (const uint16_t*)L.rows, (const int2*)L.counts, (const int*)L.prefix,   \
-                    (unsigned int*)L.next, pair_count)
+                    cut, (const uint16_t*)L.rows, (const int2*)L.counts, (unsigned int*)L.next,  \
+                    pair_count)
     OD_CUTN3_FORMS();
 #undef OD_CUTN3
   } else {

@@ -119,16 +119,16 @@ struct od_cutn3 {
                                     // cubes along z, nb * G^3
   float lo, lo_z, inv_s;            // grid origin (x and y, z) and 1 / cell side (lambda)
   int T, ipt, nslots;               // plan (the slots are padded to a multiple of T), slots
-  int32_t *cell_of, *count, *fill, *start;  // [N], [ncells], [ncells], [ncells + 1]
+  int32_t *cell_of, *rank_of, *unsorted;  // [N] cell of each ion, rank in it, ions by cell
+  int32_t *count, *start;           // [ncells] (zero between evaluations), [ncells + 1]
   int32_t* perm;                    // [nslots] ion of each sorted slot, -1 for sentinels
   float *xs, *ys, *zs;              // [nslots] sorted positions; sentinels in the tail
   float4 *tbox, *bbox;              // [nslots / 512][2], [nslots / 32][2] boxes
-  unsigned long long* next;         // work counter of the pair kernel (lists: finished blocks)
+  unsigned long long* next;         // work counter of the pair kernel
   // listed work of small systems (od_cutn3_listed, else NULL): target blocks per source group
-  // [nslots / 64][nslots / 32], (inner, other) counts, prefix of half batches
+  // [nslots / 64][nslots / 32], (inner, other) counts
   uint16_t* rows;
   int2* counts;
-  int* prefix;
   unsigned long long* acc;          // [3][nslots] fixed-point ion–ion sums per sorted slot
   void* block;                      // the allocation that holds all of these
   double rc_d;                      // cutoff / r_D_e in FP64 (the hard cutoff's exact test)
@@ -255,12 +255,12 @@ int od_trap_chunks(int nn, int64_t n_points, int sms);  // chunks of the points 
 // launch with programmatic stream serialization (the kernel calls od_pdl_wait before
 // it touches anything that an earlier kernel wrote or reads)
 template <typename... KArgs, typename... Args>
-inline cudaError_t od_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
-                                 Args... args) {
+inline cudaError_t od_launch_pdl_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                      cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -268,6 +268,11 @@ inline cudaError_t od_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block
   cfg.attrs = at;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t od_launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
+                                 Args... args) {
+  return od_launch_pdl_smem(kernel, grid, block, 0, s, args...);
 }
 
 // Record msg as the last error of calls without a handle (od_last_error(NULL)); returns st.

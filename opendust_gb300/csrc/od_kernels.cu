@@ -1253,15 +1253,16 @@ __global__ void __launch_bounds__(kBlk, kTrapBlocks) k_trap(double Rh, double Hh
   if (node < nn) part[(size_t)blockIdx.y * nn + node] = acc;
 }
 
-// sums over the chunks, in their order
+// sums over the chunks: a warp per node, lanes in steps of 32, then the lanes in a fixed order
 __global__ void __launch_bounds__(kBlk) k_trap_sum(const double* __restrict__ part, int nn,
                                                    int nchunks, double* __restrict__ sum) {
-  const int node = blockIdx.x * kBlk + threadIdx.x;
+  const int node = (blockIdx.x * kBlk + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (node >= nn) return;
   double s = 0;
-#pragma unroll 8
-  for (int c = 0; c < nchunks; c++) s += part[(size_t)c * nn + node];
-  sum[node] = s;
+  for (int c = lane; c < nchunks; c += 32) s += part[(size_t)c * nn + node];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) sum[node] = s;
 }
 
 // ============================================================== initial state on the device
@@ -1529,7 +1530,7 @@ cudaError_t od_launch_trap(double Rh, double Hh, int n_r, int n_h, int64_t n_poi
   k_trap<<<dim3(nb, nchunks), kBlk, 0, s>>>(Rh, Hh, n_r, n_h, n_points, per,
                                             (uint32_t)(seed & 0xffffffffu), (uint32_t)(seed >> 32),
                                             part);
-  k_trap_sum<<<nb, kBlk, 0, s>>>(part, nn, nchunks, sum);
+  k_trap_sum<<<(nn + kBlk / 32 - 1) / (kBlk / 32), kBlk, 0, s>>>(part, nn, nchunks, sum);
   return cudaGetLastError();
 }
 
