@@ -48,6 +48,7 @@ struct od_handle {
   cudaGraph_t graph_nf = nullptr;
   cudaGraphExec_t graph_exec_nf = nullptr;
   bool use_graph = true;
+  int64_t steps_made = 0;  // by od_step, in all windows
   // device timing (events on the handle's stream)
   bool timing = false;
   bool count_pairs = false;  // timing mode 1: the cutoff kernel also counts its pairs
@@ -968,6 +969,18 @@ static od_status ensure_graph(od_handle* h) {
   return capture_step(h, false, &h->graph_nf, &h->graph_exec_nf);
 }
 
+// A step's launches cost the host 4.4 us each. A graph costs it one, but 40 to 60 us once, and its first
+// kernel waits for the last one of the step before instead of following by programmatic launch. So:
+// graphs where launches take as long as what they launch (all pairs up to 4096 ions: 2048 21.1 us per
+// step, 22.0 launched; the cutoff's chain of small kernels: ten steps of 20011 ions 1.306 ms, 1.331
+// launched), from the handle's 32nd step on (the first ten steps of 2048 ions: 0.46 ms with the graph,
+// 0.24 without); single launches for the others (8192 ions 44.5 us per step, in graphs 45.8). Steps
+// without an ion-ion evaluation (force interval) are short at any size.
+static bool wants_graph(const od_handle* h, int64_t nsteps) {
+  if (h->graph_exec || h->cfg.force_every > 1) return true;
+  return (h->has_cut || h->N <= 4096) && h->steps_made + nsteps >= 32;
+}
+
 extern "C" od_status od_step(od_handle* h, int64_t nsteps) {
   if (!h) return fail(nullptr, OD_ERR_INVALID, "handle is NULL");
   if (!h->state_set) return fail(h, OD_ERR_STATE, "od_set_state has not been called");
@@ -978,7 +991,7 @@ extern "C" od_status od_step(od_handle* h, int64_t nsteps) {
   if (h->timing) {
     od_status st = step_timed(h, nsteps);
     if (st != OD_OK) return st;
-  } else if (h->use_graph) {
+  } else if (h->use_graph && wants_graph(h, nsteps)) {
     od_status st = ensure_graph(h);
     if (st != OD_OK) return st;
     for (int64_t s = 0; s < nsteps; s++)
@@ -989,6 +1002,7 @@ extern "C" od_status od_step(od_handle* h, int64_t nsteps) {
       OD_CK(h, launch_step_parts(h, force_ctx(h, false), step_evaluates(h, h->step + s)));
   }
   h->step += nsteps;
+  h->steps_made += nsteps;
   return check_device_err(h);
 }
 

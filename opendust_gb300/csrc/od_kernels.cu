@@ -508,6 +508,7 @@ __global__ void __launch_bounds__(kBlk) k_kick_drift(const od_dparams* __restric
                                                      float* __restrict__ sx, float* __restrict__ sy,
                                                      float* __restrict__ sz) {
   od_pdl_trigger();
+  od_pdl_wait();
   kick_drift_body(*dp, ds, rel, pos, vel, fhi, flo, cq, sx, sy, sz,
                   blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -1164,6 +1165,7 @@ __global__ void __launch_bounds__(kCT) k_correct(
     const uint32_t* __restrict__ flags, const int32_t* __restrict__ list,
     const float4* __restrict__ list_old, const float4* __restrict__ list_new,
     double* orbit_part, int nb, double* __restrict__ series, float* __restrict__ cq) {
+  od_pdl_trigger();
   od_pdl_wait();
   if (blockIdx.x == 0) {
     tail_body(*dp, ds, list, list_new, orbit_part, nb, series, cq);
@@ -1424,9 +1426,9 @@ cudaError_t od_launch_step_part(int part, const od_dparams* dp, od_dstate* ds, c
   (void)P;
   const int nb = Npad / kBlk;
   if (part == 0) {
-    k_kick_drift<<<(N + kBlk - 1) / kBlk, kBlk, 0, s>>>(dp, ds, b.rel, b.pos, b.vel, b.fhi, b.flo, b.cq,
-                                                        b.sx, b.sy, b.sz);
-    return cudaGetLastError();
+    return od_launch_pdl(k_kick_drift, dim3((N + kBlk - 1) / kBlk), dim3(kBlk), s, dp,
+                         (const od_dstate*)ds, b.rel, b.pos, b.vel, (const float4*)b.fhi,
+                         (const float4*)b.flo, (const float*)b.cq, b.sx, b.sy, b.sz);
   }
   // with accumulators (fc.acc) K3 takes the ion–ion sums from them
   if (part == 1)
@@ -1434,7 +1436,7 @@ cudaError_t od_launch_step_part(int part, const od_dparams* dp, od_dstate* ds, c
                            &ds->err, s, fc.acc == nullptr);
   const int jsplit = fc.cut ? 1 : fc.plan.jsplit;
   const int per = orbit_per(nb);
-  // K2 to K5 with programmatic dependent launch: each starts launching while its predecessor runs
+  // K1 to K5 with programmatic dependent launch: each starts launching while its predecessor runs
   // and waits in od_pdl_wait for the predecessor's end (K2 on its positions only after it has found
   // its unit: 2048 ions 24.2 -> 22.8 us per step)
   cudaError_t e = od_launch_pdl(k_kick_flag, dim3(nb), dim3(kBlk), s, dp, ds, b.pos, b.vel,
@@ -1765,13 +1767,15 @@ cudaError_t od_launch_grid_potential(const float4* pos, int N, const double* pts
 }
 
 cudaError_t od_launch_batch_step(const od_batchview& v, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
+  // K1 waits for the step before in full: six members 1042 us per step, 1048 let in early
   k_b_kick_drift<<<v.nblk_ion, kBlk, 0, s>>>(v.sims, v.blk_ion);
   if (v.nitems > 0) {  // members on the directed-pair kernel
-    cudaError_t e = cudaMemsetAsync(v.next, 0, sizeof(unsigned int), s);
+    e = cudaMemsetAsync(v.next, 0, sizeof(unsigned int), s);
     if (e != cudaSuccess) return e;
     k_b_pairs<<<v.pair_grid, 256, 0, s>>>(v.sims, v.items, v.nitems, v.next, v.err);
   }
-  cudaError_t e = od_launch_batch_pairs_n3(v, s);
+  e = od_launch_batch_pairs_n3(v, s);
   if (e != cudaSuccess) return e;
   e = od_launch_pdl(k_b_kick_flag, dim3(v.nblk_ion), dim3(kBlk), s, v.sims, v.blk_ion);
   const int per = orbit_per(v.nblk_ion);
