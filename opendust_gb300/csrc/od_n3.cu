@@ -271,10 +271,12 @@ long long od_n3_blocks(const od_n3_split& sp) { return (sp.units + kSliceWarps -
 // do not depend on the device.
 //   * 4 x 4: one group pair (128 x 128 ions, 512 pair terms per lane) per warp. 50021 ions 0.838 ms,
 //     against 0.848 and 0.859 with 4 and 8 per warp (a longer last wave; the flush of the target
-//     sums that longer slices save is small). Below 12288 ions the group pairs leave warp slots
+//     sums that longer slices save is small). In small systems the group pairs leave warp slots
 //     empty (3040 on 152 SMs; 4656 group pairs at 12000) and a single warp's dependency chain sets
-//     the time, so they are split by lane steps: 8192 ions 32.8 us in 2 parts (36.9 whole, 34.0 in
-//     4), 4096 and below in 4 (2048 ions 8.2 against 16.4 us whole).
+//     the time, so they are split by lane steps. Steps of 2048, 4096, 5000, 7680, 8192 and 14000
+//     ions in us: whole 29.0, 31.1, 52.4, 54.7, 55.3, 94.5; two parts 24.4, 28.9, 37.5, 44.7, 44.4,
+//     90.7; four 22.8, 27.0, 30.1, 42.6, 46.0, 97.5. Two parts still gain 1.5 % at 2^14, but there
+//     batches would run them apart from their larger members, with a last wave of their own.
 //   * 8 x 2 (256 x 64 ions) and 2 x 2: a tile names how many group pairs a slice may hold (tile / 64),
 //     at least 16 slices per resident warp. 8 x 2 at 2^18 ions: 21.6 ms with 8 or 16, 22.3 with 1.
 od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
@@ -284,7 +286,7 @@ od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
   sp.split = 1;
   long long L = 1;
   if (ipt == 4) {
-    if (Npad <= 12288) sp.split = Npad <= 4096 ? 4 : 2;
+    if (Npad < 16384) sp.split = Npad <= 7680 ? 4 : 2;
   } else {
     const long long warps = 152ll * kSliceWarps * (ipt == 8 ? 4 : 8);
     L = std::max(1ll, std::min<long long>(tile / 64, sp.pairs / (warps * 16)));

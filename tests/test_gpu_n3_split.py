@@ -32,3 +32,9 @@ def test_split_boundaries(gpu_lib, N, plan):
     err = rel_err_per_ion(f[idx], oracle.force_targets(holder, pos, idx, round32=True))
     print(f"N={N} plan {plan}: per-ion rel err max {err.max():.3e}")
     assert err.max() <= 1e-5
+
+
+@pytest.mark.parametrize("N", [7680, 7681, 15872, 15873])
+def test_part_boundaries(gpu_lib, N):
+    """group pairs in 4 parts up to 7680 padded ions, in 2 below 2^14"""
+    test_split_boundaries(gpu_lib, N, None)
