@@ -249,6 +249,8 @@ static void out_domain_per_charge(const od_dparams& p, double x, double y, doubl
 // constants and the grains of p; called again when grains move.
 static void tail_consts(od_dparams* p) {
   const double pi = OD_PI_D;
+  p->orbit_pref = p->k * p->q_s / (p->lam * p->lam);
+  p->collect_pref = p->vunit * p->m_s / p->dt;
   for (int g = 0; g < p->P; g++) {
     const double r = p->grs[g], S = r * r * 4.0 * pi;
     // gamma_e dt S e with gamma_e = n_inf sqrt(T_e k_B / pi / m_e / 2) exp(-e k q / r / T_e / k_B)

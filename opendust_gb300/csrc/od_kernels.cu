@@ -871,12 +871,11 @@ __device__ __forceinline__ void tail_body(const od_dparams& p, od_dstate* __rest
         fd[1] = fma(sm.q[j], p.dd[g][j][1], fd[1]);
         fd[2] = fma(sm.q[j], p.dd[g][j][2], fd[2]);
       }
-      so = qn * p.k * p.q_s / (p.lam * p.lam);
-      const double sc = p.vunit * p.m_s / p.dt;
+      so = qn * p.orbit_pref;
       vals[0] = qn;
       for (int m = 0; m < 3; m++) {
         vals[1 + m] = qn * p.gout[g][m];
-        vals[4 + m] = ds->M[g][m] * sc;
+        vals[4 + m] = ds->M[g][m] * p.collect_pref;
         vals[7 + m] = qn * fd[m];
         vals[10 + m] = m == 2 ? qn * p.gfield[g] : 0.0;
       }
