@@ -1606,8 +1606,8 @@ extern "C" od_status od_ion_forces_static(const double* pos_dev, int64_t n, doub
 
 // ============================================================== batches of simulations
 // A batch owns member handles (ordinary od_handle objects) and steps all of them with one set
-// of batch-wide launches per step (od_launch_batch_step), replayed from a CUDA graph that is
-// rebuilt whenever members join or leave.
+// of batch-wide launches per step (od_launch_batch_step), replayed from a CUDA graph for each set of
+// pair launches that a step needs; the graphs are dropped whenever members join or leave.
 struct od_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -1623,8 +1623,9 @@ struct od_batch {
   unsigned int* d_next = nullptr;
   uint32_t* d_err = nullptr;
   od_batchview view{};
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  // step graphs by the set of pair launches they hold: bit f form f of variant 7, bit OD_N3_FORMS the
+  // directed kernel
+  cudaGraphExec_t exec[2 << OD_N3_FORMS] = {};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   double last_ms = 0;
   std::string err;
@@ -1749,6 +1750,11 @@ static od_status upload_table(od_batch* b, T** dptr, size_t* cap, const std::vec
   return OD_OK;
 }
 
+static void drop_batch_graphs(od_batch* b) {
+  for (cudaGraphExec_t& g : b->exec)
+    if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+}
+
 static od_status batch_rebuild(od_batch* b) {
   std::vector<od_simdesc> sims;
   std::vector<int2> blk_ion, blk_corr;
@@ -1808,22 +1814,35 @@ static od_status batch_rebuild(od_batch* b) {
     v.n3_items[k] = b->d_n3_items[k];
     v.n3_nitems[k] = (int)n3_items[k].size();
   }
-  if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
-  if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-  if (v.nsims > 0) {
-    OD_BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = od_launch_batch_step(v, b->stream);
-    cudaGraph_t g = nullptr;
-    cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
-      if (g) cudaGraphDestroy(g);
-      return bfail(b, OD_ERR_CUDA, std::string("batch step capture: ") +
-                                       cudaGetErrorString(e != cudaSuccess ? e : e2));
-    }
-    b->graph = g;
-    OD_BCK(b, cudaGraphInstantiate(&b->exec, g, 0));
-  }
+  drop_batch_graphs(b);
   b->dirty = false;
+  return OD_OK;
+}
+
+// The pair launches of the batch's step s from now: those with a member that evaluates in it. With a
+// force interval of 16 the pair kernels' blocks, which would find nothing to do and leave, took 126 us
+// of a 230 us step (seven members, 4.5 10^5 ions).
+static unsigned batch_pair_mask(const od_batch* b, int64_t s) {
+  unsigned mask = 0;
+  for (const od_handle* h : b->members)
+    if (h && step_evaluates(h, h->step + s))
+      mask |= 1u << (h->plan.variant == 7
+                         ? od_n3_form(h->plan.ipt, od_n3_split_of(h->Npad, h->plan.ipt, h->plan.tile))
+                         : OD_N3_FORMS);
+  return mask;
+}
+
+static od_status batch_graph(od_batch* b, unsigned mask) {
+  if (b->exec[mask]) return OD_OK;
+  OD_BCK(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+  cudaError_t e = od_launch_batch_step(b->view, mask, b->stream);
+  cudaGraph_t g = nullptr;
+  cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
+  if (e == cudaSuccess) e = e2;
+  if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec[mask], g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (e != cudaSuccess)
+    return bfail(b, OD_ERR_CUDA, std::string("batch step capture: ") + cudaGetErrorString(e));
   return OD_OK;
 }
 
@@ -1838,9 +1857,14 @@ extern "C" od_status od_batch_step(od_batch* b, int64_t nsteps) {
     od_status st = batch_rebuild(b);
     if (st != OD_OK) return st;
   }
-  if (!b->exec || nsteps == 0) { b->last_ms = 0; return OD_OK; }
+  if (b->view.nsims == 0 || nsteps == 0) { b->last_ms = 0; return OD_OK; }
   OD_BCK(b, cudaEventRecord(b->ev0, b->stream));
-  for (int64_t s = 0; s < nsteps; s++) OD_BCK(b, cudaGraphLaunch(b->exec, b->stream));
+  for (int64_t s = 0; s < nsteps; s++) {
+    const unsigned mask = batch_pair_mask(b, s);
+    od_status st = batch_graph(b, mask);
+    if (st != OD_OK) return st;
+    OD_BCK(b, cudaGraphLaunch(b->exec[mask], b->stream));
+  }
   OD_BCK(b, cudaEventRecord(b->ev1, b->stream));
   OD_BCK(b, od_launch_batch_errors(b->view, b->stream));
   uint32_t berr = 0;
@@ -1887,8 +1911,7 @@ extern "C" od_status od_batch_destroy(od_batch* b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   for (od_handle* h : b->members)
     if (h) od_destroy(h);
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
+  drop_batch_graphs(b);
   void* ptrs[] = {b->d_sims, b->d_blk_ion, b->d_items, b->d_blk_corr, b->d_next, b->d_err};
   for (void* p : ptrs)
     if (p) cudaFree(p);

@@ -1765,16 +1765,16 @@ cudaError_t od_launch_grid_potential(const float4* pos, int N, const double* pts
   return cudaGetLastError();
 }
 
-cudaError_t od_launch_batch_step(const od_batchview& v, cudaStream_t s) {
+cudaError_t od_launch_batch_step(const od_batchview& v, unsigned pairs, cudaStream_t s) {
   cudaError_t e = cudaSuccess;
   // K1 waits for the step before in full: six members 1042 us per step, 1048 let in early
   k_b_kick_drift<<<v.nblk_ion, kBlk, 0, s>>>(v.sims, v.blk_ion);
-  if (v.nitems > 0) {  // members on the directed-pair kernel
+  if (v.nitems > 0 && (pairs >> OD_N3_FORMS & 1)) {  // members on the directed-pair kernel
     e = cudaMemsetAsync(v.next, 0, sizeof(unsigned int), s);
     if (e != cudaSuccess) return e;
     k_b_pairs<<<v.pair_grid, 256, 0, s>>>(v.sims, v.items, v.nitems, v.next, v.err);
   }
-  e = od_launch_batch_pairs_n3(v, s);
+  e = od_launch_batch_pairs_n3(v, pairs, s);
   if (e != cudaSuccess) return e;
   e = od_launch_pdl(k_b_kick_flag, dim3(v.nblk_ion), dim3(kBlk), s, v.sims, v.blk_ion);
   const int per = orbit_per(v.nblk_ion);

@@ -331,11 +331,11 @@ int od_n3_form(int ipt, const od_n3_split& sp) {
   return sp.split == 4 ? 2 : (sp.split == 2 ? 1 : (sp.L > 1 ? 4 : 0));
 }
 
-cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, cudaStream_t s) {
+cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, unsigned pairs, cudaStream_t s) {
   // the forms batch members use (od_n3_batch_plan, od_n3_form)
   cudaError_t e = cudaSuccess;
 #define OD_B_N3(f, MT, MS, SPLIT, FOLD)                                                      \
-  if (v.n3_nitems[f] > 0 && e == cudaSuccess)                                                \
+  if (v.n3_nitems[f] > 0 && (pairs >> f & 1) && e == cudaSuccess)                            \
   e = od_launch_pdl(k_b_pairs_n3<MT, MS, SPLIT, FOLD>, dim3(v.n3_nitems[f]),                 \
                     dim3(kSliceWarps * 32), s, v.sims, (const int2*)v.n3_items[f])
   OD_B_N3(3, 8, 2, 1, true);

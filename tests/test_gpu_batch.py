@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from opendust_gb300 import _lib, build_simulation, setup_host, workloads
+from tests._util import case
 
 pytestmark = pytest.mark.gpu
 
@@ -123,3 +124,35 @@ def test_batch_member_plan_can_be_set(gpu_lib):
         same(ref, (m.series(0, 8), *m.get_state()))
         with pytest.raises(_lib.OpenDustError):
             b.set_plan(s, 4, 2048)
+
+
+def test_batch_step_without_evaluations(gpu_lib):
+    """Members whose evaluations fall on different steps, in different kernel forms, with steps in
+    which no member evaluates: bitwise the members stepped alone, in one call and one step at a time."""
+    sizes = [(3000, 4, 0), (9000, 4, 1), (66000, 8, 0), (17000, 1, 0)]
+    for subset in (sizes[:3], sizes):
+        alone, holders = [], []
+        for n, k, ahead in subset:
+            holder, pos, vel, *_ = case(N=n, n=40, seed=n, trap=np.zeros(15), force_every=k)
+            holders.append((holder, pos, vel, ahead))
+            with _lib.Engine(holder) as eng:
+                eng.set_pair_plan(*_lib.batch_pair_plan(n))
+                eng.set_state(pos, vel)
+                eng.step(ahead + 17)
+                alone.append((eng.get_state(), eng.series(0, ahead + 17)))
+        for chunks in ([17], [1] * 17):
+            batch = _lib.Batch(0)
+            try:
+                slots = [batch.add(h, p, v) for h, p, v, _ in holders]
+                for s, (*_, ahead) in zip(slots, holders):
+                    if ahead:
+                        batch.member(s).step(ahead)
+                for c in chunks:
+                    batch.step(c)
+                for s, (*_, ahead), ((p, v), ser) in zip(slots, holders, alone):
+                    m = batch.member(s)
+                    pm, vm = m.get_state()
+                    assert np.array_equal(pm, p) and np.array_equal(vm, v)
+                    assert all(np.array_equal(m.series(0, ahead + 17)[k], ser[k]) for k in ser)
+            finally:
+                batch.close()
