@@ -14,9 +14,9 @@ kick, flags, ordered compaction, re-injection, grain sums, FP64 tail).
              that step (device->host), then od_get_state (device->host); wall clock.
   roofline   the all-pairs force evaluation: N(N-1) directed pair interactions x 25 FP32 flops
              per launch over its CUDA-event duration, against the larger of the FP32 FMA probe
-             and the SMs' FP32 rate at the sampled clock. The default kernel from 2^14 ions
-             (variant 7) evaluates each unordered pair once and applies it to both ions, so it
-             does about half those flops (executed_frac). Cutoff workloads credit the pairs
+             and the SMs' FP32 rate at the sampled clock. The default kernel (variant 7)
+             evaluates each unordered pair once and applies it to both ions, so it does about
+             half those flops (executed_frac). Cutoff workloads credit the pairs
              inside r_c, counted by one more, untimed step.
 Other workloads (--workload): small_plain (C1, 16384 ions), field_chain (C3, 2^19 ions, 2 lambda
 cutoff; --hard-cutoff without the switching function), cutoff_scaling (the reference's cutoff
@@ -49,11 +49,24 @@ sys.path.insert(0, ROOT)
 
 FLOPS_PER_PAIR = 25
 KERNELS_PER_STEP = 5          # all pairs: kick/drift, pairs, kick/flag (takes the fixed-point
-                              # sums), collect/inject, correct/orbit (its last block runs the
-                              # FP64 tail)
+                              # sums), collect/inject (with the orbit sums), correct (its first
+                              # block runs the FP64 tail)
 KERNELS_PER_STEP_CUTOFF = 11  # + cell clear, count, scan, scatter, sort, chunk scan
-KERNELS_PER_STEP_CUTOFF_TILES = 15  # + clear, count, scan, scatter, sort, boxes, pairs,
-                                    # scan, list, tile-pair kernel, slot take (cutoff variant 3)
+
+
+def kernels_per_step_sorted_cutoff(n_ions: int, R: float, H: float) -> int:
+    """Launches per step of cutoff variant 3 in a cylinder of radius R and height H: the four of
+    all pairs without its pair kernel; count, scatter (scanning the counts itself up to 8192
+    cells, else a scan of one or two kernels before it), sort, boxes, lists (up to 131072 slots),
+    pairs, slot take."""
+    cubes = 1 if H <= 3.0 * R else -int(-H // (2.0 * R))
+    side = 8
+    while side < 128 and side**3 * 16 < n_ions / cubes * 1.4142:
+        side *= 2
+    slots = -(-n_ions // 512) * 512
+    cells = cubes * side**3
+    scans = 0 if cells <= 8192 else (2 if cells % 4096 == 0 else 1)
+    return 4 + 6 + scans + (slots <= 131072)
 
 
 def parse():
@@ -197,7 +210,7 @@ def describe(name, sim, ext):
     cut = "cutoff_distance" in ext or ext.get("cutOff", False)
     force = "all-pairs"
     if cut:
-        force = "cutoff (Hilbert-sorted tile pairs), " + (
+        force = "cutoff (Hilbert-sorted ions), " + (
             "hard: no switching, pairs within FP32 rounding of r_c decided in FP64"
             if ext.get("switch_distance") == 0.0 else "OpenMM switching from 15/16 of r_c")
     return {"workload": f"{name}: {w}", "n_ions": int(sim.N), "grains": len(sim_grains(name)),
@@ -346,18 +359,20 @@ def run_ours(args, dist: Dist):
     n3 = not cutoff and plan["variant"] == 7
     traffic = load_traffic(N, plan, cutoff)
     if cutoff and plan["variant"] == 3:
-        kernel = (f"Hilbert-order sort + tile-pair list + k_pairs_cutn3 (each pair once, {plan['jsplit']}-ion "
-                  "tiles, 64-ion group pairs beyond r_c skipped; pairs inside the cutoff credited)")
+        kernel = ("Hilbert-order sort + k_pairs_cutn3 or, up to 131072 ions, k_cut_lists + "
+                  "k_pairs_cutlist (each pair once, 32-ion blocks beyond r_c skipped; pairs inside "
+                  "the cutoff credited)")
     elif cutoff:
         kernel = "cell-list build + k_pairs_cut (pairs inside the cutoff)"
     elif n3:
-        kernel = (f"k_pairs_n3 + k_n3_take (each unordered pair once, {plan['jsplit']}-ion tiles, "
-                  "fixed-point atomic sums; "
+        kernel = ("k_pairs_n3 (each unordered pair once, one warp per slice of "
+                  f"{32 * plan['targets_per_thread']}-ion target groups, fixed-point atomic sums; "
                   "credited with the N(N-1) directed pair terms it replaces)")
     else:
         kernel = f"k_pairs_x2 variant {plan['variant']} (all-pairs ion-ion)"
     if cutoff:
-        launches = KERNELS_PER_STEP_CUTOFF_TILES if plan["variant"] == 3 else KERNELS_PER_STEP_CUTOFF
+        launches = (kernels_per_step_sorted_cutoff(N, sim.R, sim.H) if plan["variant"] == 3
+                    else KERNELS_PER_STEP_CUTOFF)
     else:
         launches = KERNELS_PER_STEP
 

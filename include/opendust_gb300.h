@@ -270,7 +270,8 @@ od_status od_get_timing(od_handle* h, double* step_ms, int64_t* steps, double* p
 /* Pairs inside the cutoff evaluated by the cutoff force kernel while timing was enabled
  * (0 for the all-pairs method). */
 od_status od_get_cutoff_pairs(od_handle* h, int64_t* pairs);
-/* Use (1, default) or bypass (0) the CUDA-graph replay of a step. */
+/* Let steps replay a CUDA graph where that is faster than single launches (1, default), or never
+ * (0). The results are the same bits. */
 od_status od_set_graph(od_handle* h, int32_t enable);
 /* Work decomposition of the all-pairs force kernel (OpenMM picks its own nonbonded
  * kernel configuration; this exposes ours). variant 0: shared-memory broadcast of each
@@ -281,9 +282,9 @@ od_status od_set_graph(od_handle* h, int32_t enable);
  * pair on the Newton path of variant 4, 7: each unordered pair evaluated once and applied to
  * both ions (threads 256; targets_per_thread = target ions per lane: 2 or 4 with as many source
  * ions, 8 with two; jsplit = tile, 1024, 2048 or 4096 (not 1024 with 8; also 512 with 2), <= 0
- * for the default: it caps the work a warp takes at a time). Variants 2-7 add their sums into 64-bit fixed-point accumulators (24
- * bytes per ion) with integer atomics, so results do not depend on the order of the GPU's
- * blocks. od_create selects variant 7.
+ * for the default: it caps the work a warp takes at a time). Variants 2-7 add their sums into
+ * 64-bit fixed-point accumulators (24 bytes per ion) with integer atomics, so results do not
+ * depend on the order of the GPU's blocks. od_create selects variant 7.
  * jsplit <= 0 picks the source split from the SM count. Takes effect at the next step.
  * Cutoff method (force_method OD_FORCE_CUTOFF): variant 0 or 2 walks a stencil of cells per
  * target cell (scalar or packed); variant 3 (the default) sorts the ions along a Hilbert curve and
@@ -427,7 +428,7 @@ const char* od_batch_last_error(const od_batch* b);
 /* Free and total device memory (admission control of a request server). */
 od_status od_device_memory(int32_t device, int64_t* free_bytes, int64_t* total_bytes);
 /* Device bytes a simulation created by od_create with this configuration allocates, including
- * the fixed-point accumulators and the cutoff's sort and tile-pair list (admission control). */
+ * the fixed-point accumulators and the cutoff's sort and block lists (admission control). */
 od_status od_config_device_bytes(const od_config* cfg, int64_t* bytes);
 
 /* Trajectory dumps of OpenDust.simulate() (opendust.py:1071-1098, which writes them with a Python

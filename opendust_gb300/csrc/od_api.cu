@@ -1098,6 +1098,7 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
     c.take(L->unsorted, (size_t)N);
     c.take(L->count, nc);
     c.take(L->start, nc + 1);
+    c.take(L->totals, nc / 4096 + 1);
     c.take(L->perm, ns);
     c.take(L->xs, ns);
     c.take(L->ys, ns);
@@ -1191,9 +1192,9 @@ extern "C" od_status od_set_pair_plan(od_handle* h, int32_t threads, int32_t tar
                                       int32_t variant, int32_t jsplit) {
   if (!h) return fail(nullptr, OD_ERR_INVALID, "handle is NULL");
   if (h->has_cut) {
-    // cutoff method: variant 0 selects the scalar pair kernel, 2 the packed one, 3 the tile
-    // pairs with each pair once (targets_per_thread 2: 512-ion tiles, 4: 1024-ion tiles; a
-    // positive jsplit must name that tile size)
+    // cutoff method: variant 0 selects the scalar pair kernel, 2 the packed one, 3 the
+    // sorted one with each pair once (targets_per_thread 2: slots padded to 512, 4: to 1024; a
+    // positive jsplit must name that padding)
     if (variant != 0 && variant != 2 && variant != 3)
       return fail(h, OD_ERR_INVALID, "cutoff variants are 0, 2 and 3");
     if (variant == 3) {
@@ -1343,7 +1344,7 @@ extern "C" od_status od_autotune(od_handle* h, int32_t use_cache, double* best_p
 
 extern "C" od_status od_get_pair_plan(const od_handle* h, int32_t* plan5) {
   if (!h || !plan5) return fail(nullptr, OD_ERR_INVALID, "NULL argument");
-  if (h->has_cut) {  // cutoff variant: 3 (tile pairs), 2 (packed cells) or 0 (scalar cells)
+  if (h->has_cut) {  // cutoff variant: 3 (sorted ions), 2 (packed cells) or 0 (scalar cells)
     plan5[0] = 256;
     plan5[1] = h->cut.n3 ? h->cut.n3->ipt : 2;
     plan5[2] = h->cut.n3 ? 3 : (h->cut.packed ? 2 : 0);
@@ -1931,7 +1932,7 @@ extern "C" od_status od_config_device_bytes(const od_config* cfg, int64_t* bytes
   const int64_t Np = ((cfg->n_ions + OD_PAD - 1) / OD_PAD) * OD_PAD;
   const int64_t P = std::max(cfg->n_grains, 1);
   int64_t b = 0;
-  if (cfg->force_method == OD_FORCE_CUTOFF) {  // tile-pair cutoff, as od_create chooses it
+  if (cfg->force_method == OD_FORCE_CUTOFF) {  // sorted cutoff, as od_create chooses it
     const int nc = od_cutn3_grid((int)cfg->n_ions, cfg->R, cfg->H).ncells;
     const size_t c512 = od_cutn3_bytes((int)cfg->n_ions, 512, nc);
     const size_t c1024 = od_cutn3_bytes((int)cfg->n_ions, 1024, nc);

@@ -186,8 +186,8 @@ __device__ __forceinline__ void od_acc2(float& hi, float& lo, float x) {
 }
 
 // ------------------------------------------------------------------ fixed-point sums
-// The each-pair-once kernels add every (tile pair, ion) partial sum to the ion's accumulator
-// with a 64-bit integer atomic: the value in units of 2^-32 (lambda units of the pair sums;
+// The each-pair-once kernels add every partial sum of a warp (16 or 32 lane steps) to the ion's
+// accumulator with a 64-bit integer atomic: the value in units of 2^-32 (lambda units of the pair sums;
 // per-ion sums are 10^0..10^5 and single terms at most ~1/r0^2 = 1e6, far inside the 2^31
 // range). Integer addition is associative, so the result is the same bits for any order of
 // the atomics; each partial (hi + lo) is rounded once per word, 2^-32 at most, against the

@@ -52,26 +52,10 @@ __global__ void k_mc_count(int n, const float4* __restrict__ pos, float lo, floa
   rank_of[i] = atomicAdd(&count[c], 1);
 }
 
-// exclusive scan of in[0..n) into out[0..n], out[n] = total (one 1024-thread block, four entries to a
-// load where the threads' runs allow it)
-__global__ void __launch_bounds__(1024) k_scan_excl(int n, const int32_t* in, int32_t* out) {
+// exclusive scan over the block's 1024 threads
+__device__ __forceinline__ int block_scan_1024(int a) {
   __shared__ int s_w[32];
-  od_pdl_wait();
-  od_pdl_trigger();
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int per = (n + 1023) / 1024;
-  const bool quads = n % 4096 == 0;
-  const int c0 = min(tid * per, n), c1 = min(c0 + per, n);
-  int a = 0;
-  if (quads) {
-#pragma unroll 8
-    for (int c = c0; c < c1; c += 4) {
-      const int4 v = *reinterpret_cast<const int4*>(in + c);
-      a += (v.x + v.y) + (v.z + v.w);
-    }
-  } else {
-    for (int c = c0; c < c1; c++) a += in[c];
-  }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int ia = a;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -91,23 +75,60 @@ __global__ void __launch_bounds__(1024) k_scan_excl(int n, const int32_t* in, in
     s_w[lane] = x - v;
   }
   __syncthreads();
-  int off = s_w[wid] + ia - a;
-  if (quads) {
-#pragma unroll 8
-    for (int c = c0; c < c1; c += 4) {
-      const int4 v = *reinterpret_cast<const int4*>(in + c);
-      *reinterpret_cast<int4*>(out + c) = make_int4(off, off + v.x, off + v.x + v.y,
-                                                    off + v.x + v.y + v.z);
-      off += (v.x + v.y) + (v.z + v.w);
-    }
-  } else {
-    for (int c = c0; c < c1; c++) {
-      const int v = in[c];
-      out[c] = off;
-      off += v;
-    }
+  return s_w[wid] + ia - a;
+}
+
+// exclusive scan of in[0..n) into out[0..n], out[n] = total (one 1024-thread block)
+__global__ void __launch_bounds__(1024) k_scan_excl(int n, const int32_t* in, int32_t* out) {
+  od_pdl_wait();
+  od_pdl_trigger();
+  const int tid = threadIdx.x, per = (n + 1023) / 1024;
+  const int c0 = min(tid * per, n), c1 = min(c0 + per, n);
+  int a = 0;
+  for (int c = c0; c < c1; c++) a += in[c];
+  int off = block_scan_1024(a);
+  for (int c = c0; c < c1; c++) {
+    const int v = in[c];
+    out[c] = off;
+    off += v;
   }
   if (tid == 1023) out[n] = off;
+}
+
+// The same in two kernels where n is a multiple of 4096 (262144 cells at 2^19 ions: 7.6 us, one
+// block 119): blocks of 4096 entries with their totals, then the totals before each block added.
+constexpr int kScanBlock = 4096;
+__global__ void __launch_bounds__(1024) k_scan_blocks(const int32_t* in, int32_t* out,
+                                                      int32_t* __restrict__ totals) {
+  od_pdl_wait();
+  od_pdl_trigger();
+  const int c = blockIdx.x * kScanBlock + 4 * threadIdx.x;
+  const int4 v = *reinterpret_cast<const int4*>(in + c);
+  const int sum = (v.x + v.y) + (v.z + v.w), off = block_scan_1024(sum);
+  *reinterpret_cast<int4*>(out + c) = make_int4(off, off + v.x, off + v.x + v.y, off + v.x + v.y + v.z);
+  if (threadIdx.x == 1023) totals[blockIdx.x] = off + sum;
+}
+__global__ void __launch_bounds__(1024) k_scan_add(int n, const int32_t* totals, int32_t* out) {
+  __shared__ int s_before, s_all;
+  od_pdl_wait();
+  od_pdl_trigger();
+  if (threadIdx.x == 0) s_before = s_all = 0;
+  __syncthreads();
+  int before = 0, all = 0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += 1024) {
+    const int v = totals[b];
+    all += v;
+    if (b < (int)blockIdx.x) before += v;
+  }
+  before = __reduce_add_sync(0xffffffffu, before);
+  all = __reduce_add_sync(0xffffffffu, all);
+  if ((threadIdx.x & 31) == 0) { atomicAdd(&s_before, before); atomicAdd(&s_all, all); }
+  __syncthreads();
+  int4* const o = reinterpret_cast<int4*>(out + blockIdx.x * kScanBlock) + threadIdx.x;
+  int4 v = *o;
+  v.x += s_before; v.y += s_before; v.z += s_before; v.w += s_before;
+  *o = v;
+  if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = s_all;
 }
 
 __global__ void k_mc_scatter(int n, const int32_t* __restrict__ cell_of,
@@ -376,8 +397,8 @@ __device__ __noinline__ void exact_pass(const float* __restrict__ xs, const floa
 }
 
 // MT target blocks tb[0 .. nb) (nb <= MT, the rest empty) against the 64 slots of source group sg:
-// halves [h0, h1) of the 32 lane steps. Reactions are summed in FP32 over 16 lane steps and added to the accumulators of the sources where
-// they stand (shorter chains than the 32 steps they could take: at 2^19 ions the median per-ion
+// halves [h0, h1) of the 32 lane steps. Reactions are summed in FP32 over 16 lane steps and added to
+// the accumulators of the sources where they stand (shorter chains than the 32 steps they could take: at 2^19 ions the median per-ion
 // error is 0.8 of that and the kernel 1 % slower).
 template <int MT, int CUT, bool REACT, bool COUNT, int UNROLL>
 __device__ __forceinline__ void cut_batch(const cut_consts& k, const float* __restrict__ xs,
@@ -571,7 +592,8 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
 // Up to kListBlocks blocks the units above are too coarse: a warp gets a few batches, and the last ones
 // run alone (force chain of 8192 ions at 2 lambda 0.132 ms). Here one warp per source group lists its
 // target blocks first (inner ones from the front of its row, the others from the back), every block of the
-// pair kernel takes the prefix over the groups, and its warps draw runs of equal length from it: half batches where there are fewer than four per warp (8192 ions 0.069 ms; whole batches 0.077), else
+// pair kernel takes the prefix over the groups, and its warps draw runs of equal length from it: half
+// batches where there are fewer than four per warp (8192 ions 0.069 ms; whole batches 0.077), else
 // whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635 with the units).
 constexpr int kListBlocks = 4096;
 __global__ void __launch_bounds__(256) k_cut_lists(int nsg, int nT, const cut_args cut,
@@ -773,7 +795,7 @@ size_t od_cutn3_bytes(int N, int T, int ncells) {
          + sizeof(float4) * 2 * (ns / kBlk + ns / kTile)              // boxes
          + od_cutn3_list_bytes(ns)
          + sizeof(float) * 3 * ns                                     // sorted positions
-         + sizeof(int32_t) * (ns + 3 * (size_t)N + 2 * nc + 1);
+         + sizeof(int32_t) * (ns + 3 * (size_t)N + 2 * nc + 2 + nc / 4096);
 }
 
 bool od_cutn3_supported(int ipt, int T) {
@@ -819,9 +841,17 @@ cudaError_t od_launch_cutoff_n3(const od_cutn3& L, const float4* pos, int n, flo
                              n, L.ncells, (const int32_t*)L.cell_of, (const int32_t*)L.rank_of,
                              (const int32_t*)L.count, L.start, L.unsorted);
   } else {
-    if (e == cudaSuccess)
+    const int sb = L.ncells / kScanBlock;
+    if (e == cudaSuccess && L.ncells % kScanBlock == 0) {
+      e = od_launch_pdl(k_scan_blocks, dim3(sb), dim3(1024), s, (const int32_t*)L.count, L.start,
+                        L.totals);
+      if (e == cudaSuccess)
+        e = od_launch_pdl(k_scan_add, dim3(sb), dim3(1024), s, L.ncells, (const int32_t*)L.totals,
+                          L.start);
+    } else if (e == cudaSuccess) {
       e = od_launch_pdl(k_scan_excl, dim3(1), dim3(1024), s, L.ncells, (const int32_t*)L.count,
                         L.start);
+    }
     if (e == cudaSuccess)
       e = od_launch_pdl(k_mc_scatter, nb, nt, s, n, (const int32_t*)L.cell_of,
                         (const int32_t*)L.rank_of, (const int32_t*)L.start, L.unsorted);

@@ -122,6 +122,7 @@ struct od_cutn3 {
   int T, ipt, nslots;               // plan (the slots are padded to a multiple of T), slots
   int32_t *cell_of, *rank_of, *unsorted;  // [N] cell of each ion, rank in it, ions by cell
   int32_t *count, *start;           // [ncells] (zero between evaluations), [ncells + 1]
+  int32_t* totals;                  // [ncells / 4096 + 1] of the scan's blocks
   int32_t* perm;                    // [nslots] ion of each sorted slot, -1 for sentinels
   float *xs, *ys, *zs;              // [nslots] sorted positions; sentinels in the tail
   float4 *tbox, *bbox;              // [nslots / 512][2], [nslots / 32][2] boxes
@@ -135,7 +136,7 @@ struct od_cutn3 {
   double rc_d;                      // cutoff / r_D_e in FP64 (the hard cutoff's exact test)
   int grid, grid_hard;              // persistent blocks of the pair kernel (switching, hard)
 };
-// cell grid of the tile-pair cutoff for N ions in a cylinder of radius R and height H (any
+// cell grid of the sorted cutoff for N ions in a cylinder of radius R and height H (any
 // unit): nb cubes of side `side` (that unit) along z, G^3 cells each
 struct od_cgrid { int G, nb, ncells; double side; };
 od_cgrid od_cutn3_grid(int N, double R, double H);

@@ -7,7 +7,7 @@
 
 `pairs` steps the small_plain workload with the given all-pairs plan, `cutoff` the field_chain
 workload (cutoff 2 lambda; variants 0 and 2 walk a cell stencil, variant 3 with --plan takes the
-tile pairs over Hilbert-sorted ions), both launching kernel by kernel (no CUDA graph) so that
+Hilbert-sorted 32-ion blocks), both launching kernel by kernel (no CUDA graph) so that
 `ncu -k regex:<kernel>` sees individual launches. `sweep` times every all-pairs plan with CUDA
 events and prints pairs/s (a plan may carry the tile size as a fourth number, e.g. 256,8,7,2048).
 """
