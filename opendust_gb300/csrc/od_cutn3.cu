@@ -13,10 +13,10 @@
 // What bounds it: as the all-pairs kernel, operand fetch of the packed FP32 pipe (17 packed
 // operations per pair of pairs for the plain term, 27 with switching), plus the pairs of the
 // listed blocks that lie beyond the cutoff. field_chain (2^19 ions, 2 lambda): 1.63 pairs
-// evaluated per pair inside, 22.2 ms per evaluation. The tile-pair form this replaces (512-ion
+// listed per pair inside (1.35 evaluated), 21.9 ms per evaluation. The tile-pair form this replaces (512-ion
 // tile pairs, 64 x 64 group lists built by one warp between two block barriers, 2 x 2 ions per
 // lane, sums in shared memory with compare-and-swap atomics) took 32.2 ms there; 65536 ions in
-// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.74 ms, 20011 ions at 2 lambda 0.197 -> 0.077 ms.
+// the 12 lambda tall cylinder at 3.2 lambda 1.28 -> 0.70 ms, 20011 ions at 2 lambda 0.197 -> 0.077 ms.
 #include "od_hilbert.h"
 #include "od_internal.h"
 #include <algorithm>
