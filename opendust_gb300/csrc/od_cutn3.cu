@@ -593,8 +593,10 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
 // run alone (force chain of 8192 ions at 2 lambda 0.132 ms). Here one warp per source group lists its
 // target blocks first (inner ones from the front of its row, the others from the back), every block of the
 // pair kernel takes the prefix over the groups, and its warps draw runs of equal length from it: half
-// batches where there are fewer than four per warp (8192 ions 0.069 ms; whole batches 0.077), else
-// whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635 with the units).
+// batches where there are fewer than six per warp (20011 ions 118.9 us per step, whole batches 121.5;
+// 30000 with 7.2 per warp 195 and 193), else whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635
+// with the units). Ending whole runs with a round of halves: 117.0 us at 20011 ions, but 588 instead of
+// 585 at 65536 and 1864 instead of 1848 at 131072.
 constexpr int kListBlocks = 4096;
 __global__ void __launch_bounds__(256) k_cut_lists(int nsg, int nT, const cut_args cut,
                                                    const float4* __restrict__ tbox,
@@ -694,7 +696,7 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
   const cut_consts k = make_consts(cut);
   unsigned int cnt = 0;
   const int Q = s_prefix[nsg], W = gridDim.x * WARPS;
-  const int run = Q < 4 * W ? 1 : max(2, (Q / (W * 32)) & ~1);
+  const int run = Q < 6 * W ? 1 : max(2, (Q / (W * 32)) & ~1);
   for (;;) {
     int q = 0;
     if (lane == 0) q = (int)min(atomicAdd(next, 1u), (unsigned)Q) * run;
