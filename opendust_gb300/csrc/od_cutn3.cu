@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(cut_traits<CUT>::WARPS * 32, cut_traits<CUT>::
 // target blocks first (inner ones from the front of its row, the others from the back), every block of the
 // pair kernel takes the prefix over the groups, and its warps draw runs of equal length from it: half
 // batches where there are fewer than six per warp (20011 ions 118.9 us per step, whole batches 121.5;
-// 30000 with 7.2 per warp 195 and 193), else whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635
+// 30000, with eight to twelve per warp, 195.0 and 193.1), else whole ones, 32 runs per warp (65536 ions 0.594 ms, 0.635
 // with the units). Ending whole runs with a round of halves: 117.0 us at 20011 ions, but 588 instead of
 // 585 at 65536 and 1864 instead of 1848 at 131072.
 constexpr int kListBlocks = 4096;

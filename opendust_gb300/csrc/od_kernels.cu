@@ -1559,7 +1559,7 @@ __global__ void k_static_pack(const double* __restrict__ pos, int n, int Npad, d
 // Bound by the SFU (three operations per pair, 21 cycles per 32 pairs and sub-partition) and, below
 // 4000 ions, by launches. Directed, not each pair once: the caller's positions may be anywhere, and
 // fixed-point sums would not keep the relative accuracy of a far ion's small force.
-// One call, 700 ions: 18 us (44.5 with up to 8 source chunks and an error word read back), 3001: 24
+// One call, 700 ions: 18 us (44.5 with up to 8 source chunks and an error word read back), 3001: 23
 // (57), 8000: 59 (87), 32768: 641 (763). Two targets per thread: 20.6, 27.1, 62, 758.
 constexpr int kStaticThreads = 256, kStaticTile = 256;
 __global__ void __launch_bounds__(kStaticThreads) k_static_pairs(
@@ -1597,22 +1597,27 @@ __global__ void __launch_bounds__(kStaticThreads) k_static_pairs(
   pl[e] = make_float4(lo.x, lo.y, lo.z, 0.f);
 }
 
-// four lanes to an ion: each sums every fourth slab, then two-float sums over the four
+// LANES lanes to an ion: each sums every LANES-th slab, then two-float sums over them. Bound by latency:
+// above 16 slabs eight lanes (3001 ions, 24 slabs: 4.1 us, four 5.2; the call 22.6 and 23.5), else four
+// (15000 ions, 10 slabs: the call 156, eight 158).
+template <int LANES>
 __global__ void __launch_bounds__(kBlk) k_static_finish(const float4* ph, const float4* pl, int n,
                                                         int Npad, int jsplit, double scale,
                                                         double* __restrict__ force) {
   od_pdl_wait();
-  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e >> 2;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, i = e / LANES, l0 = e % LANES;
   float3 hi = make_float3(0.f, 0.f, 0.f), lo = hi;
-  if (i < n)
-    for (int s = e & 3; s < jsplit; s += 4) {
+  if (i < n) {
+#pragma unroll 4
+    for (int s = l0; s < jsplit; s += LANES) {
       const float4 a = ph[(size_t)s * Npad + i], b = pl[(size_t)s * Npad + i];
       od_acc2(hi.x, lo.x, a.x); lo.x += b.x;
       od_acc2(hi.y, lo.y, a.y); lo.y += b.y;
       od_acc2(hi.z, lo.z, a.z); lo.z += b.z;
     }
+  }
 #pragma unroll
-  for (int o = 1; o < 4; o <<= 1) {
+  for (int o = 1; o < LANES; o <<= 1) {
     float t;
     t = __shfl_xor_sync(0xffffffffu, hi.x, o); lo.x += __shfl_xor_sync(0xffffffffu, lo.x, o);
     od_acc2(hi.x, lo.x, t);
@@ -1621,8 +1626,8 @@ __global__ void __launch_bounds__(kBlk) k_static_finish(const float4* ph, const 
     t = __shfl_xor_sync(0xffffffffu, hi.z, o); lo.z += __shfl_xor_sync(0xffffffffu, lo.z, o);
     od_acc2(hi.z, lo.z, t);
   }
-  if (i >= n || (e & 3) == 3) return;
-  const int c = e & 3;
+  const int c = l0;
+  if (i >= n || c >= 3) return;
   const float h = c == 0 ? hi.x : (c == 1 ? hi.y : hi.z), l = c == 0 ? lo.x : (c == 1 ? lo.y : lo.z);
   force[3 * (size_t)i + c] = scale * ((double)h + (double)l);
 }
@@ -1645,7 +1650,9 @@ cudaError_t od_launch_static_forces(const od_static_view& v, const double* pos, 
                                 (const float*)v.sx, (const float*)v.sy, (const float*)v.sz, Npad,
                                 chunk, (float)(r0 / lam), v.part_hi, v.part_lo);
   if (e != cudaSuccess) return e;
-  e = od_launch_pdl(k_static_finish, dim3((4 * n + kBlk - 1) / kBlk), dim3(kBlk), s,
+  const int lanes = jsplit > 16 ? 8 : 4;
+  e = od_launch_pdl(lanes == 8 ? k_static_finish<8> : k_static_finish<4>,
+                    dim3((lanes * n + kBlk - 1) / kBlk), dim3(kBlk), s,
                     (const float4*)v.part_hi, (const float4*)v.part_lo, n, Npad, jsplit, scale,
                     force);
   return e != cudaSuccess ? e : cudaGetLastError();
