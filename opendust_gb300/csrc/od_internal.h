@@ -66,7 +66,7 @@ struct od_n3_split {
 };
 od_n3_split od_n3_split_of(int Npad, int ipt, int tile);
 long long od_n3_blocks(const od_n3_split& sp);
-constexpr int OD_N3_FORMS = 5;
+constexpr int OD_N3_FORMS = 6;
 int od_n3_form(int ipt, const od_n3_split& sp);  // kernel form of a batch member, < OD_N3_FORMS
 
 // One member of a batch, as the batched kernels see it.

@@ -328,11 +328,13 @@ size_t od_n3_floats(int Npad, int T) {
 
 int od_n3_form(int ipt, const od_n3_split& sp) {
   if (ipt == 8) return 3;
+  if (ipt == 2) return 5;
   return sp.split == 4 ? 2 : (sp.split == 2 ? 1 : (sp.L > 1 ? 4 : 0));
 }
 
 cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, unsigned pairs, cudaStream_t s) {
-  // the forms batch members use (od_n3_batch_plan, od_n3_form)
+  // the forms batch members use: those of od_n3_batch_plan, and 2 x 2, which a member's own handle may
+  // be given (od_set_pair_plan)
   cudaError_t e = cudaSuccess;
 #define OD_B_N3(f, MT, MS, SPLIT, FOLD)                                                      \
   if (v.n3_nitems[f] > 0 && (pairs >> f & 1) && e == cudaSuccess)                            \
@@ -343,6 +345,7 @@ cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, unsigned pairs, cuda
   OD_B_N3(1, 4, 4, 2, false);
   OD_B_N3(2, 4, 4, 4, false);
   OD_B_N3(4, 4, 4, 1, true);
+  OD_B_N3(5, 2, 2, 1, true);
 #undef OD_B_N3
   return e != cudaSuccess ? e : cudaGetLastError();
 }

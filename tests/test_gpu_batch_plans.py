@@ -1,0 +1,51 @@
+"""Batch members whose all-pairs plan is set through their own handle (od_batch_member): the batch steps
+them with that plan. Each-pair-once plans give bitwise the results of the simulation stepped alone with
+the same plans; small, ragged and larger members, beside one that keeps its plan."""
+import numpy as np
+import pytest
+
+from opendust_gb300 import _lib
+from tests._util import case
+
+pytestmark = pytest.mark.gpu
+
+ONCE = [(256, 2, 7, 512), (256, 2, 7, 4096), (256, 4, 7, 4096), (256, 8, 7, 2048), (256, 8, 7, 4096)]
+
+
+def stepped_alone(holder, pos, vel, plan, before, steps):
+    with _lib.Engine(holder) as eng:
+        eng.set_pair_plan(*_lib.batch_pair_plan(eng.n))
+        eng.set_state(pos, vel)
+        eng.step(before)
+        if plan:
+            eng.set_pair_plan(*plan)
+        eng.step(steps)
+        return (*eng.get_state(), eng.series(0, before + steps))
+
+
+def stepped_in_batch(members, before, steps):
+    """members: (holder, pos, vel, plan or None)"""
+    with _lib.Batch() as b:
+        slots = [b.add(*m[:3]) for m in members]
+        if before:
+            b.step(before)
+        for s, (*_, plan) in zip(slots, members):
+            if plan:
+                b.member(s).set_pair_plan(*plan)
+        b.step(steps)
+        return [(*b.member(s).get_state(), b.member(s).series(0, before + steps)) for s in slots]
+
+
+def same(a, b):
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    assert all(np.array_equal(a[2][k], b[2][k]) for k in a[2])
+
+
+@pytest.mark.parametrize("plan", ONCE)
+@pytest.mark.parametrize("N", [300, 9001, 66000])
+def test_plan_set_before_the_first_step(gpu_lib, plan, N):
+    a = case(N=N, n=8, seed=N, trap=np.zeros(15))[:3]
+    c = case(N=2048, n=8, seed=7, trap=np.zeros(15))[:3]
+    got = stepped_in_batch([(*a, plan), (*c, None)], 0, 3)
+    same(got[0], stepped_alone(*a, plan, 0, 3))
+    same(got[1], stepped_alone(*c, None, 0, 3))

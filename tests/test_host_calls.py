@@ -1,0 +1,63 @@
+"""CPU tests of the host code's CUDA calls: the library's objects linked against a CUDA runtime on host
+memory (fake_cudart.cu), which runs what a stream was given as late as CUDA allows, makes calls fail on
+demand, and reports what the host code did wrong on the way. No GPU, no kernel runs."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from opendust_gb300 import _build, _lib, workloads
+from tests._util import case
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake_path(tmp_path_factory):
+    _build.build()
+    objs = [os.path.join(_build.OUT_DIR, s.replace(".cu", ".o")) for s in _build.SOURCES]
+    if not all(os.path.exists(o) for o in objs):
+        _build.build(force=True)
+    d = tmp_path_factory.mktemp("fake_cudart")
+    obj, lib = str(d / "fake.o"), str(d / "libfake.so")
+    # the guard of the device runtime's header: its weak stubs have the names defined here
+    subprocess.run([_build._nvcc(), *_build.NVCC_FLAGS, "-D__CUDA_DEVICE_RUNTIME_API_H__",
+                    "-diag-suppress", "20096", "-cudart", "none", "-I", _build.CSRC, "-c",
+                    os.path.join(HERE, "fake_cudart.cu"), "-o", obj], check=True)
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", lib, *objs, obj, "-lpthread"], check=True)
+    return lib
+
+
+@pytest.fixture
+def fake(fake_path, monkeypatch):
+    monkeypatch.setattr(_lib, "_lib", None)
+    lib = _lib.load(fake_path)
+    lib.fake_log.restype = lib.fake_faults.restype = ctypes.c_char_p
+    lib.fake_reset()
+    yield lib
+    lib.fake_reset()
+
+
+def faults(lib):
+    return lib.fake_faults().decode().splitlines()
+
+
+def log(lib):
+    return lib.fake_log().decode().splitlines()
+
+
+def member_case(N=1500, n=24, **kw):
+    return case(N=N, n=n, builder=workloads.small_plain, trap=np.zeros(15), **kw)[:3]
+
+
+@pytest.mark.parametrize("plan", [(256, 2, 7, 512), (256, 2, 7, 1024), (256, 4, 7, 4096), (256, 8, 7, 4096)])
+def test_batch_member_with_any_each_pair_once_plan(fake, plan):
+    # the batch launches each member's work table with the kernel of that member's shape
+    with _lib.Batch() as b:
+        s = b.add(*member_case())
+        b.add(*member_case(N=600))
+        b.member(s).set_pair_plan(*plan)
+        b.step(2)
+    assert any("k_b_pairs_n3" in x for x in log(fake)) and faults(fake) == []
