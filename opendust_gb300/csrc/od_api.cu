@@ -452,12 +452,15 @@ static void free_all(od_handle* h) {
     if (p) cudaFree(p);
 }
 
+static void drop_graph(od_handle* h);
+
 // Partial-sum slabs: one (the consumers' view of the sums), or jsplit of them for the plans that
-// write each source chunk's sums apart (the scalar variants 0 and 1, and batch members on the
-// directed kernel).
+// write each source chunk's sums apart (the scalar variants 0 and 1, and every directed plan of a
+// batch member: batch_rebuild asks for those). The handle's step graphs hold the slabs' address.
 static int slabs_of(const od_pair_plan& pl) { return pl.variant <= 1 ? pl.jsplit : 1; }
 static od_status ensure_slabs(od_handle* h, int slabs) {
   if (h->slabs >= slabs) return OD_OK;
+  drop_graph(h);
   if (h->b.part_hi) cudaFree(h->b.part_hi);
   h->b.part_hi = h->b.part_lo = nullptr;
   h->slabs = 0;
@@ -1764,6 +1767,10 @@ static od_status batch_rebuild(od_batch* b) {
   std::vector<int2> n3_items[OD_N3_FORMS];
   for (od_handle* h : b->members) {
     if (!h) continue;
+    if (h->plan.variant != 7) {  // the batched directed kernel writes a slab per source chunk
+      const od_status st = ensure_slabs(h, h->plan.jsplit);
+      if (st != OD_OK) return bfail(b, st, h->err);
+    }
     const int m = (int)sims.size();
     od_simdesc d{};
     d.dp = h->dp; d.ds = h->ds; d.b = h->b;

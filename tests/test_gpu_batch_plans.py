@@ -49,3 +49,27 @@ def test_plan_set_before_the_first_step(gpu_lib, plan, N):
     got = stepped_in_batch([(*a, plan), (*c, None)], 0, 3)
     same(got[0], stepped_alone(*a, plan, 0, 3))
     same(got[1], stepped_alone(*c, None, 0, 3))
+
+
+@pytest.mark.parametrize("plan", [(256, 1, 5, 0), (128, 1, 5, 7), (256, 2, 2, 0), (256, 1, 0, 0)])
+@pytest.mark.parametrize("N", [700, 5000, 20000])
+def test_directed_plan_set_before_the_first_step(gpu_lib, plan, N):
+    # the batch's directed kernel sums other chains than the handle alone: FP32 rounding apart. The
+    # forces of the two agree to 1e-5 (the bound of every all-pairs plan) and a step's kick moves an
+    # ion by less than 1e-2 lambda, so the positions agree to 4e-7 lambda after four steps, and to 1e-6
+    # with the rounding of the position words (2.4e-7 at 3 lambda)
+    a = case(N=N, n=8, seed=N, trap=np.zeros(15))
+    plasma = a[3]
+    with _lib.Batch() as b:
+        s = b.add(*a[:3])
+        m = b.member(s)
+        m.set_pair_plan(*plan)
+        b.step(3)
+        p, _ = m.get_state()
+        m.step(1)  # alone, with the same slabs
+        p4, _ = m.get_state()
+    ref = stepped_alone(*a[:3], plan, 0, 3)
+    ref4 = stepped_alone(*a[:3], plan, 0, 4)
+    d, d4 = (np.abs(x - y[0]).max() / plasma.r_D_e for x, y in ((p, ref), (p4, ref4)))
+    print(f"N={N} plan {plan}: {d:.2e} {d4:.2e} lambda")
+    assert d < 1e-6 and d4 < 1e-6

@@ -61,3 +61,31 @@ def test_batch_member_with_any_each_pair_once_plan(fake, plan):
         b.member(s).set_pair_plan(*plan)
         b.step(2)
     assert any("k_b_pairs_n3" in x for x in log(fake)) and faults(fake) == []
+
+
+DIRECTED = [(256, 1, 5, 0), (128, 1, 5, 3), (256, 2, 2, 0), (128, 1, 0, 0)]
+
+
+@pytest.mark.parametrize("plan", DIRECTED)
+def test_batch_member_with_a_directed_plan(fake, plan):
+    # the batched directed kernel writes one slab of partial sums per source chunk
+    with _lib.Batch() as b:
+        s = b.add(*member_case(N=5000))
+        b.member(s).set_pair_plan(*plan)
+        assert b.member(s).pair_plan()["jsplit"] > 1
+        b.step(2)
+    assert any("9k_b_pairsE" in x for x in log(fake)) and faults(fake) == []
+
+
+def test_batch_slabs_leave_no_stale_step_graph(fake):
+    # a member that has stepped alone from its graph, then in a batch that gives it more slabs
+    with _lib.Batch() as b:
+        s = b.add(*member_case(N=3000, n=80))
+        m = b.member(s)
+        m.set_pair_plan(256, 1, 5)
+        m.step(40)
+        assert "cudaGraphLaunch" in log(fake)
+        b.step(1)
+        fake.fake_reset()
+        m.step(1)
+    assert "cudaGraphInstantiate" in log(fake)
