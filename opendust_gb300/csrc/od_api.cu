@@ -49,6 +49,10 @@ struct od_handle {
   cudaGraphExec_t graph_exec_nf = nullptr;
   bool use_graph = true;
   int64_t steps_made = 0;  // by od_step, in all windows
+  // batch member: the batch's "tables are out of date" flag, set when the plan changes, and the pair
+  // launch (bit of batch_pair_mask) whose table holds this member
+  bool* batch_dirty = nullptr;
+  int batch_launch = 0;
   // device timing (events on the handle's stream)
   bool timing = false;
   bool count_pairs = false;  // timing mode 1: the cutoff kernel also counts its pairs
@@ -1126,6 +1130,11 @@ static od_status alloc_cutn3(od_handle* h, int ipt, int T) {
   return OD_OK;
 }
 
+static void plan_changed(od_handle* h) {
+  drop_graph(h);
+  if (h->batch_dirty) *h->batch_dirty = true;
+}
+
 static void drop_graph(od_handle* h) {
   if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
   if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
@@ -1187,7 +1196,7 @@ static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
     OD_CK(h, cudaMemsetAsync(h->b.n3, 0, sizeof(float) * need, h->stream));
   }
   h->plan = pl;  // one partial slab: part_hi/part_lo always hold at least one
-  drop_graph(h);
+  plan_changed(h);
   return OD_OK;
 }
 
@@ -1243,10 +1252,7 @@ extern "C" od_status od_set_pair_plan(od_handle* h, int32_t threads, int32_t tar
   pl.jsplit = (h->Npad + chunk - 1) / chunk;
   if (ensure_slabs(h, slabs_of(pl)) != OD_OK) return OD_ERR_OOM;
   h->plan = pl;
-  if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
-  if (h->graph) { cudaGraphDestroy(h->graph); h->graph = nullptr; }
-  if (h->graph_exec_nf) { cudaGraphExecDestroy(h->graph_exec_nf); h->graph_exec_nf = nullptr; }
-  if (h->graph_nf) { cudaGraphDestroy(h->graph_nf); h->graph_nf = nullptr; }
+  plan_changed(h);
   return OD_OK;
 }
 
@@ -1611,7 +1617,8 @@ extern "C" od_status od_ion_forces_static(const double* pos_dev, int64_t n, doub
 // ============================================================== batches of simulations
 // A batch owns member handles (ordinary od_handle objects) and steps all of them with one set
 // of batch-wide launches per step (od_launch_batch_step), replayed from a CUDA graph for each set of
-// pair launches that a step needs; the graphs are dropped whenever members join or leave.
+// pair launches that a step needs; tables and graphs are rebuilt whenever members join, leave or change
+// their plan (through the batch or through their own handle).
 struct od_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -1701,6 +1708,7 @@ extern "C" od_status od_batch_add(od_batch* b, const od_config* cfg, const doubl
     if (!b->members[k]) { s = (int)k; break; }
   if (s < 0) { s = (int)b->members.size(); b->members.push_back(nullptr); }
   b->members[s] = h;
+  h->batch_dirty = &b->dirty;
   b->dirty = true;
   *slot = s;
   return OD_OK;
@@ -1714,9 +1722,7 @@ extern "C" od_status od_batch_set_plan(od_batch* b, int32_t slot, int32_t ions_p
     return bfail(b, OD_ERR_INVALID, "batch members take (4, 1024) or (8, 2048)");
   od_handle* h = b->members[slot];
   const od_status st = set_plan_n3(h, ions_per_lane, tile);
-  if (st != OD_OK) return bfail(b, st, h->err);
-  b->dirty = true;
-  return OD_OK;
+  return st == OD_OK ? OD_OK : bfail(b, st, h->err);
 }
 
 extern "C" od_status od_batch_remove(od_batch* b, int32_t slot) {
@@ -1781,11 +1787,12 @@ static od_status batch_rebuild(od_batch* b) {
     d.newton_r2 = nr * nr;
     d.n3_tile = h->plan.variant == 7 ? h->plan.tile : 0;
     if (d.n3_tile) d.n3 = od_n3_split_of(d.Npad, h->plan.ipt, d.n3_tile);
+    h->batch_launch = d.n3_tile ? od_n3_form(h->plan.ipt, d.n3) : OD_N3_FORMS;
     sims.push_back(d);
     for (int lb = 0; lb < d.nb; lb++) blk_ion.push_back(make_int2(m, lb));
     if (d.n3_tile) {
       // every block of this member's pair kernel, in the table of its form
-      std::vector<int2>& t = n3_items[od_n3_form(h->plan.ipt, sims.back().n3)];
+      std::vector<int2>& t = n3_items[h->batch_launch];
       for (long long k = 0; k < od_n3_blocks(sims.back().n3); k++) t.push_back(make_int2(m, (int)k));
       continue;
     }
@@ -1827,16 +1834,13 @@ static od_status batch_rebuild(od_batch* b) {
   return OD_OK;
 }
 
-// The pair launches of the batch's step s from now: those with a member that evaluates in it. With a
-// force interval of 16 the pair kernels' blocks, which would find nothing to do and leave, took 126 us
-// of a 230 us step (seven members, 4.5 10^5 ions).
+// The pair launches of the batch's step s from now: those whose tables hold a member that evaluates in
+// it. With a force interval of 16 the pair kernels' blocks, which would find nothing to do and leave,
+// took 126 us of a 230 us step (seven members, 4.5 10^5 ions).
 static unsigned batch_pair_mask(const od_batch* b, int64_t s) {
   unsigned mask = 0;
   for (const od_handle* h : b->members)
-    if (h && step_evaluates(h, h->step + s))
-      mask |= 1u << (h->plan.variant == 7
-                         ? od_n3_form(h->plan.ipt, od_n3_split_of(h->Npad, h->plan.ipt, h->plan.tile))
-                         : OD_N3_FORMS);
+    if (h && step_evaluates(h, h->step + s)) mask |= 1u << h->batch_launch;
   return mask;
 }
 

@@ -73,3 +73,48 @@ def test_directed_plan_set_before_the_first_step(gpu_lib, plan, N):
     d, d4 = (np.abs(x - y[0]).max() / plasma.r_D_e for x, y in ((p, ref), (p4, ref4)))
     print(f"N={N} plan {plan}: {d:.2e} {d4:.2e} lambda")
     assert d < 1e-6 and d4 < 1e-6
+
+
+@pytest.mark.parametrize("plan", ONCE)
+@pytest.mark.parametrize("N", [300, 9001])
+def test_plan_changed_between_steps(gpu_lib, plan, N):
+    a = case(N=N, n=8, seed=N, trap=np.zeros(15))[:3]
+    c = case(N=2048, n=8, seed=7, trap=np.zeros(15))[:3]
+    got = stepped_in_batch([(*a, plan), (*c, None)], 2, 4)
+    same(got[0], stepped_alone(*a, plan, 2, 4))
+    same(got[1], stepped_alone(*c, None, 2, 4))
+
+
+def test_directed_plan_between_steps_and_back(gpu_lib):
+    # bounds as above
+    a = case(N=5000, n=8, seed=3, trap=np.zeros(15))
+    plans = [(256, 8, 7, 2048), (256, 1, 5, 0), (256, 4, 7, 1024)]
+    with _lib.Batch() as b:
+        m = b.member(b.add(*a[:3]))
+        b.step(1)
+        for plan in plans:
+            m.set_pair_plan(*plan)
+            b.step(1)
+        p, _ = m.get_state()
+    with _lib.Engine(a[0]) as eng:
+        eng.set_pair_plan(*_lib.batch_pair_plan(5000))
+        eng.set_state(*a[1:3])
+        eng.step(1)
+        for plan in plans:
+            eng.set_pair_plan(*plan)
+            eng.step(1)
+        ref, _ = eng.get_state()
+    assert np.abs(p - ref).max() / a[3].r_D_e < 1e-6
+
+
+def test_autotuned_member(gpu_lib):
+    # whatever plan the tuner takes, the batch steps the member with it (bounds as above)
+    a = case(N=3000, n=8, seed=4, trap=np.zeros(15))
+    with _lib.Batch() as b:
+        m = b.member(b.add(*a[:3]))
+        b.step(2)
+        m.autotune(use_cache=False)
+        b.step(2)
+        p, _ = m.get_state()
+    ref = stepped_alone(*a[:3], None, 0, 4)
+    assert np.abs(p - ref[0]).max() / a[3].r_D_e < 1e-6

@@ -74,6 +74,10 @@ def test_batch_member_with_a_directed_plan(fake, plan):
         b.member(s).set_pair_plan(*plan)
         assert b.member(s).pair_plan()["jsplit"] > 1
         b.step(2)
+        b.member(s).set_pair_plan(256, 4, 7)
+        b.step(1)
+        b.member(s).set_pair_plan(*plan)
+        b.step(1)
     assert any("9k_b_pairsE" in x for x in log(fake)) and faults(fake) == []
 
 
@@ -89,3 +93,24 @@ def test_batch_slabs_leave_no_stale_step_graph(fake):
         fake.fake_reset()
         m.step(1)
     assert "cudaGraphInstantiate" in log(fake)
+
+
+def test_batch_launches_follow_a_member_that_changes_its_plan(fake):
+    # after the change the member's pairs are launched by the kernel of its new shape, and by no other
+    def pair_kernels(plan):
+        fake.fake_reset()
+        b.member(s).set_pair_plan(*plan)
+        b.step(1)
+        return {x.split("12k_b_pairs_n3ILi")[1][0] if "12k_b_pairs_n3ILi" in x else "directed"
+                for x in log(fake) if "k_b_pairs" in x}
+
+    with _lib.Batch() as b:
+        s = b.add(*member_case(N=9000))
+        b.step(1)
+        for plan, kernel in (((256, 8, 7, 2048), "8"), ((256, 4, 7, 1024), "4"), ((256, 1, 5, 0), "directed"),
+                             ((256, 2, 7, 1024), "2")):
+            assert pair_kernels(plan) == {kernel}
+        fake.fake_reset()
+        b.set_plan(s, 8, 2048)
+        b.step(1)
+        assert any("12k_b_pairs_n3ILi8" in x for x in log(fake)) and faults(fake) == []
