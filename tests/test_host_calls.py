@@ -114,3 +114,27 @@ def test_batch_launches_follow_a_member_that_changes_its_plan(fake):
         b.set_plan(s, 8, 2048)
         b.step(1)
         assert any("12k_b_pairs_n3ILi8" in x for x in log(fake)) and faults(fake) == []
+
+
+def mixed_batch(b):
+    # force intervals 2 and 4: steps with and without the pair launch
+    return [b.add(*member_case(N=9000, force_every=k)) for k in (2, 4)]
+
+
+def test_batch_makes_its_graphs_before_it_steps(fake):
+    with _lib.Batch() as b:
+        slots = mixed_batch(b)
+        fake.fake_reset()
+        b.step(8)
+        calls = log(fake)
+        assert calls.count("cudaGraphInstantiate") == 2 and calls.count("cudaGraphLaunch") == 8
+        assert "cudaGraphInstantiate" not in calls[calls.index("cudaEventRecord"):]
+        # a graph that cannot be made: no step has been launched
+        b.remove(slots[0])
+        slots[0] = b.add(*member_case(N=9000, force_every=2))
+        fake.fake_reset()
+        fake.fake_fail(b"cudaGraphInstantiate", 1)
+        with pytest.raises(_lib.OpenDustError):
+            b.step(8)
+        assert "cudaGraphLaunch" not in log(fake)
+        assert b.member(slots[1]).step_index == 8 and b.member(slots[0]).step_index == 0
