@@ -78,7 +78,9 @@ static od_status fail(od_handle* h, od_status st, const std::string& msg) {
   return st;
 }
 od_status od_fail_nohandle(od_status st, const std::string& msg) { return fail(nullptr, st, msg); }
+// (the thread's last error is read too: a later kernel launch would report it as its own)
 static od_status cuda_fail(od_handle* h, cudaError_t e, const char* what) {
+  cudaGetLastError();
   std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
   return fail(h, e == cudaErrorMemoryAllocation ? OD_ERR_OOM : OD_ERR_CUDA, m);
 }
@@ -1649,9 +1651,11 @@ static od_status bfail(od_batch* b, od_status st, const std::string& msg) {
 #define OD_BCK(b, call)                                                                  \
   do {                                                                                   \
     cudaError_t e_ = (call);                                                             \
-    if (e_ != cudaSuccess)                                                               \
+    if (e_ != cudaSuccess) {                                                             \
+      cudaGetLastError();                                                                \
       return bfail(b, e_ == cudaErrorMemoryAllocation ? OD_ERR_OOM : OD_ERR_CUDA,        \
                    std::string(#call) + ": " + cudaGetErrorString(e_));                  \
+    }                                                                                    \
   } while (0)
 
 extern "C" const char* od_batch_last_error(const od_batch* b) { return b ? b->err.c_str() : g_err.c_str(); }
@@ -1672,6 +1676,7 @@ extern "C" od_status od_batch_create(int32_t device, od_batch** out) {
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     g_err = std::string("od_batch_create: ") + cudaGetErrorString(e);
     if (b->d_next) cudaFree(b->d_next);
     if (b->d_err) cudaFree(b->d_err);
@@ -1853,8 +1858,10 @@ static od_status batch_graph(od_batch* b, unsigned mask) {
   if (e == cudaSuccess) e = e2;
   if (e == cudaSuccess) e = cudaGraphInstantiate(&b->exec[mask], g, 0);
   if (g) cudaGraphDestroy(g);
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();
     return bfail(b, OD_ERR_CUDA, std::string("batch step capture: ") + cudaGetErrorString(e));
+  }
   return OD_OK;
 }
 

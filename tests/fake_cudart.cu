@@ -14,14 +14,14 @@
 
 namespace {
 using op = std::function<void()>;
-struct graph_t { std::vector<op> ops; };
+struct graph_t { std::vector<op> ops; std::string kernels; };
 struct stream_t { std::vector<op> ops; graph_t* capture = nullptr; };
 struct call_t { dim3 grid, block; size_t smem; cudaStream_t s; };
 
 stream_t g_legacy;
 std::map<char*, size_t> g_blocks;            // device allocations
 std::vector<std::string> g_faults;
-std::string g_log;                           // the calls made, one per line
+std::string g_log;                           // the calls made and, indented, the kernels launched
 std::map<std::string, int> g_fail;           // call -> successful calls left before it fails once
 std::vector<call_t> g_calls;
 cudaError_t g_last = cudaSuccess;
@@ -86,7 +86,7 @@ void check_once(const od_simdesc* sims, const int2* items, int n, int targets) {
 cudaError_t launch(const std::string& name, dim3 grid, void** args, cudaStream_t s) {
   const cudaError_t e = call("launch", cudaErrorLaunchFailure);
   if (e != cudaSuccess) return e;
-  g_log += "  " + name + "\n";
+  (st(s).capture ? st(s).capture->kernels : g_log) += "  " + name + "\n";
   if (!g_poke.empty() && name.find(g_poke) != std::string::npos) {
     uint32_t* p = *(uint32_t**)args[g_poke_arg];
     const uint32_t bits = g_poke_bits;
@@ -125,6 +125,7 @@ void fake_reset() {
   g_fail.clear();
   g_poke.clear();
   g_member_bits = 0;
+  g_last = cudaSuccess;
   mallopt(M_PERTURB, 0x5a);  // freed memory is overwritten at once
 }
 void fake_fail(const char* name, int after) { g_fail[name] = after; }
@@ -256,7 +257,10 @@ cudaError_t CUDARTAPI cudaGraphExecDestroy(cudaGraphExec_t x) {
 }
 cudaError_t CUDARTAPI cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) {
   const cudaError_t e = call("cudaGraphLaunch");
-  if (e == cudaSuccess) for (const op& f : reinterpret_cast<graph_t*>(x)->ops) put(s, f);
+  if (e != cudaSuccess) return e;
+  const graph_t& g = *reinterpret_cast<graph_t*>(x);
+  g_log += g.kernels;
+  for (const op& f : g.ops) put(s, f);
   return e;
 }
 

@@ -138,3 +138,21 @@ def test_batch_makes_its_graphs_before_it_steps(fake):
             b.step(8)
         assert "cudaGraphLaunch" not in log(fake)
         assert b.member(slots[1]).step_index == 8 and b.member(slots[0]).step_index == 0
+
+
+def test_a_failed_call_does_not_fail_the_next(fake):
+    # the error of a failed call stays the thread's last error until it is read, and every kernel
+    # launch reports that one: it is read where it is reported
+    holder, pos, vel = member_case()
+    with _lib.Engine(holder) as eng, _lib.Batch() as b:
+        eng.set_state(pos, vel)
+        fake.fake_fail(b"cudaMemcpyAsync", 0)
+        with pytest.raises(_lib.OpenDustError):
+            eng.get_state()
+        eng.get_state()
+        b.add(holder, pos, vel)
+        b.step(1)
+        fake.fake_fail(b"cudaGraphLaunch", 0)
+        with pytest.raises(_lib.OpenDustError):
+            b.step(1)
+        b.step(1)
