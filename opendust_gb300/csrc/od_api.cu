@@ -1884,8 +1884,13 @@ extern "C" od_status od_batch_step(od_batch* b, int64_t nsteps) {
     if (st != OD_OK) return st;
   }
   OD_BCK(b, cudaEventRecord(b->ev0, b->stream));
-  for (int64_t s = 0; s < nsteps; s++)
-    OD_BCK(b, cudaGraphLaunch(b->exec[batch_pair_mask(b, s)], b->stream));
+  for (int64_t s = 0; s < nsteps; s++) {
+    const cudaError_t e = cudaGraphLaunch(b->exec[batch_pair_mask(b, 0)], b->stream);
+    if (e != cudaSuccess) cudaStreamSynchronize(b->stream);  // the steps before are the members' to read
+    OD_BCK(b, e);
+    for (od_handle* h : b->members)  // with every launch: the device counts the steps before a failed one
+      if (h) h->step++;
+  }
   OD_BCK(b, cudaEventRecord(b->ev1, b->stream));
   OD_BCK(b, od_launch_batch_errors(b->view, b->stream));
   uint32_t berr = 0;
@@ -1894,8 +1899,6 @@ extern "C" od_status od_batch_step(od_batch* b, int64_t nsteps) {
   float ms = 0;
   OD_BCK(b, cudaEventElapsedTime(&ms, b->ev0, b->ev1));
   b->last_ms = ms;
-  for (od_handle* h : b->members)
-    if (h) h->step += nsteps;
   if (berr)  // some member's error word, or the batch's own
     for (od_handle* h : b->members) {
       if (!h) continue;

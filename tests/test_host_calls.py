@@ -156,3 +156,20 @@ def test_a_failed_call_does_not_fail_the_next(fake):
         with pytest.raises(_lib.OpenDustError):
             b.step(1)
         b.step(1)
+
+
+def test_batch_launch_that_fails_midway(fake):
+    # the members' step indices count what was launched, as the device's do, so that the next call
+    # launches the pair kernels on the steps that evaluate (the fourth here, of interval 4)
+    with _lib.Batch() as b:
+        s = b.add(*member_case(N=9000, force_every=4))
+        fake.fake_fail(b"cudaGraphLaunch", 2)
+        with pytest.raises(_lib.OpenDustError):
+            b.step(6)
+        assert b.member(s).step_index == 2 and log(fake)[-1] == "cudaStreamSynchronize"
+        pairs = []
+        for _ in range(4):
+            fake.fake_reset()
+            b.step(1)
+            pairs.append(any("k_b_pairs" in x for x in log(fake)))
+        assert b.member(s).step_index == 6 and pairs == [False, True, False, False]
