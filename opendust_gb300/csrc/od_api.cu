@@ -1634,7 +1634,7 @@ struct od_batch {
   int2* d_n3_items[OD_N3_FORMS] = {};
   size_t c_n3_items[OD_N3_FORMS] = {};
   unsigned int* d_next = nullptr;
-  uint32_t* d_err = nullptr;
+  uint32_t* d_err = nullptr;  // [2] of the batch's own waits, of the members (od_launch_batch_errors)
   od_batchview view{};
   // step graphs by the set of pair launches they hold: bit f form f of variant 7, bit OD_N3_FORMS the
   // directed kernel
@@ -1671,8 +1671,8 @@ extern "C" od_status od_batch_create(int32_t device, od_batch** out) {
   cudaError_t e = cudaSetDevice(device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_next, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMalloc(&b->d_err, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_err, 2 * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemset(b->d_err, 0, 2 * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
   if (e != cudaSuccess) {
@@ -1893,19 +1893,19 @@ extern "C" od_status od_batch_step(od_batch* b, int64_t nsteps) {
   }
   OD_BCK(b, cudaEventRecord(b->ev1, b->stream));
   OD_BCK(b, od_launch_batch_errors(b->view, b->stream));
-  uint32_t berr = 0;
-  OD_BCK(b, cudaMemcpyAsync(&berr, b->d_err, sizeof(berr), cudaMemcpyDeviceToHost, b->stream));
+  uint32_t berr[2] = {0, 0};
+  OD_BCK(b, cudaMemcpyAsync(berr, b->d_err, sizeof(berr), cudaMemcpyDeviceToHost, b->stream));
   OD_BCK(b, cudaStreamSynchronize(b->stream));
   float ms = 0;
   OD_BCK(b, cudaEventElapsedTime(&ms, b->ev0, b->ev1));
   b->last_ms = ms;
-  if (berr)  // some member's error word, or the batch's own
+  if (berr[1])  // some member's error word
     for (od_handle* h : b->members) {
       if (!h) continue;
       od_status st = check_device_err(h);
       if (st != OD_OK) return bfail(b, st, h->err);
     }
-  if (berr & OD_DERR_TIMEOUT) return bfail(b, OD_ERR_TIMEOUT, "a bounded device wait ran out");
+  if (berr[0] & OD_DERR_TIMEOUT) return bfail(b, OD_ERR_TIMEOUT, "a bounded device wait ran out");
   return OD_OK;
 }
 

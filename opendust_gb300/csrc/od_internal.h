@@ -91,7 +91,7 @@ struct od_batchview {
   int nblk_corr;
   int pair_grid;         // persistent blocks of the all-pairs stage
   unsigned int* next;    // work counter of the all-pairs stage
-  uint32_t* err;
+  uint32_t* err;         // [2]: of the all-pairs stage's waits; of the members
   // members on variant 7: (member, block of its pair kernel) per kernel form
   const int2* n3_items[OD_N3_FORMS];
   int n3_nitems[OD_N3_FORMS];
@@ -199,7 +199,7 @@ cudaError_t od_launch_snapshot_out(int n, int Npad, int jsplit, const float4* ph
 cudaError_t od_launch_clear_state(int Npad, const od_dbufs& b, cudaStream_t s);
 // series row 0 next, averages restarted, the Philox step counter running on (od_begin_window)
 cudaError_t od_launch_begin_window(od_dstate* ds, cudaStream_t s);
-// *err |= the members' error words
+// err[1] = the members' error words as they are now, or-ed (a member that left is forgotten)
 cudaError_t od_launch_batch_errors(const od_batchview& v, cudaStream_t s);
 cudaError_t od_launch_aos_to_soa(const float4* pos, int Npad, float* sx, float* sy, float* sz,
                                  cudaStream_t s);

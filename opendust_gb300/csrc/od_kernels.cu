@@ -1908,9 +1908,15 @@ __global__ void k_begin_window(od_dstate* __restrict__ ds) {
   for (int k = threadIdx.x; k < OD_MAX_GRAINS * 13; k += blockDim.x) (&ds->avg[0][0])[k] = 0.0;
 }
 
+// one block
 __global__ void k_b_errors(const od_simdesc* __restrict__ sims, int n, uint32_t* __restrict__ err) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m < n && sims[m].ds->err) atomicOr(err, sims[m].ds->err);
+  __shared__ uint32_t s_err;
+  if (threadIdx.x == 0) s_err = 0u;
+  __syncthreads();
+  for (int m = threadIdx.x; m < n; m += blockDim.x)
+    if (sims[m].ds->err) atomicOr(&s_err, sims[m].ds->err);
+  __syncthreads();
+  if (threadIdx.x == 0) err[1] = s_err;
 }
 }  // namespace
 
@@ -1950,7 +1956,7 @@ cudaError_t od_launch_begin_window(od_dstate* ds, cudaStream_t s) {
   return cudaGetLastError();
 }
 cudaError_t od_launch_batch_errors(const od_batchview& v, cudaStream_t s) {
-  k_b_errors<<<(v.nsims + 255) / 256, 256, 0, s>>>(v.sims, v.nsims, v.err);
+  k_b_errors<<<1, 256, 0, s>>>(v.sims, v.nsims, v.err);
   return cudaGetLastError();
 }
 

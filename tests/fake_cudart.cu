@@ -110,7 +110,8 @@ cudaError_t launch(const std::string& name, dim3 grid, void** args, cudaStream_t
     put(s, [=] {
       if (n > 0) sims[0].ds->err |= g_member_bits;
       g_member_bits = 0;
-      for (int m = 0; m < n; m++) *err |= sims[m].ds->err;
+      err[1] = 0u;
+      for (int m = 0; m < n; m++) err[1] |= sims[m].ds->err;
     });
   }
   return cudaSuccess;

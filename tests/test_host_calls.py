@@ -173,3 +173,21 @@ def test_batch_launch_that_fails_midway(fake):
             b.step(1)
             pairs.append(any("k_b_pairs" in x for x in log(fake)))
         assert b.member(s).step_index == 6 and pairs == [False, True, False, False]
+
+
+@pytest.mark.parametrize("bits,status", [(1, 5), (4, 7)])  # a wait that ran out, a crowded cell
+def test_batch_forgets_the_error_of_a_member_that_left(fake, bits, status):
+    with _lib.Batch() as b:
+        first = b.add(*member_case())
+        b.add(*member_case(N=700))
+        b.step(1)
+        fake.fake_member_error(bits)  # of the first member
+        for _ in range(2):            # it stays until the member leaves
+            with pytest.raises(_lib.OpenDustError) as e:
+                b.step(1)
+            assert e.value.status == status
+        b.remove(first)
+        b.step(1)
+        fake.fake_reset()
+        b.step(1)
+        assert log(fake).count("cudaMemcpyAsync") == 1  # the batch's words alone, no member's
