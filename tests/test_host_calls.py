@@ -191,3 +191,16 @@ def test_batch_forgets_the_error_of_a_member_that_left(fake, bits, status):
         fake.fake_reset()
         b.step(1)
         assert log(fake).count("cudaMemcpyAsync") == 1  # the batch's words alone, no member's
+
+
+@pytest.mark.parametrize("builder", [workloads.small_plain, workloads.field_chain])
+def test_force_snapshot_in_place(fake, builder):
+    # the caller's positions are read before anything is written to the forces, also where the upload
+    # runs late (page-locked memory, or a host whose pageable memory the device reads itself)
+    holder, pos, _ = case(N=1500, n=8, builder=builder, trap=np.zeros(15))[:3]
+    with _lib.Engine(holder) as eng:
+        fake.fake_reset()
+        for n in (1500, 1):
+            x = pos[:n].copy()
+            _lib.check(fake.od_force_snapshot(eng.h, _lib._dptr(x), n, _lib._dptr(x)), eng.h)
+    assert faults(fake) == []
