@@ -1482,8 +1482,11 @@ extern "C" od_status od_force_snapshot(od_handle* h, const double* pos, int64_t 
   OD_CK(h, od_launch_snapshot_out((int)n, h->Npad, force_jsplit(h), h->b.part_hi, h->b.part_lo,
                                   fc.acc, F, out, h->stream));
   touch_pages(force, sizeof(double) * 3 * n);  // while the kernels run
+  st = check_device_err(h);
+  if (st != OD_OK) return st;  // the caller's array as it was
   OD_CK(h, cudaMemcpyAsync(force, out, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream));
-  return check_device_err(h);
+  OD_CK(h, cudaStreamSynchronize(h->stream));
+  return OD_OK;
 }
 
 extern "C" od_status od_snapshot_positions(od_handle* h, const double* pos, int64_t n, double* pos_dev) {

@@ -204,3 +204,12 @@ def test_force_snapshot_in_place(fake, builder):
             x = pos[:n].copy()
             _lib.check(fake.od_force_snapshot(eng.h, _lib._dptr(x), n, _lib._dptr(x)), eng.h)
     assert faults(fake) == []
+
+
+def test_force_snapshot_that_fails_leaves_the_output(fake):
+    holder, pos, _ = case(N=1500, n=8, builder=workloads.field_chain, trap=np.zeros(15))[:3]
+    force = np.full_like(pos, 7.0)
+    with _lib.Engine(holder) as eng:
+        fake.fake_poke(b"9k_mc_sort", 10, 4)  # a crowded cell
+        assert fake.od_force_snapshot(eng.h, _lib._dptr(pos), 1500, _lib._dptr(force)) == 7
+    assert (force == 7.0).all()
