@@ -554,6 +554,7 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
     cudaGetLastError();
     h->err.clear();
   }
+  std::vector<int4> stencil;  // uploaded asynchronously: lives until the stream has been waited for
   if (cfg->force_method == OD_FORCE_CUTOFF) {
     // Cells of side c = a power of two not above rc/4 (halved while the mean occupancy exceeds
     // ~800 ions), on a grid whose origin is a multiple of c: cell origins and the shifts between
@@ -573,14 +574,13 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
     g.gx = g.gy = (int)(2 * mx);
     g.gz = (int)(2 * mz);
     g.ncells = g.gx * g.gy * g.gz;
-    std::vector<int4> st;
     for (int dz = -kk - 1; dz <= kk + 1; dz++)
       for (int dy = -kk - 1; dy <= kk + 1; dy++)
         for (int dx = -kk - 1; dx <= kk + 1; dx++) {
           auto m = [&](int d) { double v = std::max(std::abs(d) - 1, 0) * c; return v * v; };
-          if (m(dx) + m(dy) + m(dz) < rc * rc) st.push_back(make_int4(dx, dy, dz, 0));
+          if (m(dx) + m(dy) + m(dz) < rc * rc) stencil.push_back(make_int4(dx, dy, dz, 0));
         }
-    h->cut.nstencil = (int)st.size();
+    h->cut.nstencil = (int)stencil.size();
     h->cut.cap = h->Npad + 8 * g.ncells;
     const size_t nc = g.ncells;
     h->cut.packed = true;
@@ -595,10 +595,10 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
       c.take(h->cut.ox, h->cut.cap);
       c.take(h->cut.oy, h->cut.cap);
       c.take(h->cut.oz, h->cut.cap);
-      c.take(h->cut.stencil, st.size());
+      c.take(h->cut.stencil, stencil.size());
       c.take(h->d_pairs, 1);
     }));
-    OD_CKC(cudaMemcpyAsync(h->cut.stencil, st.data(), sizeof(int4) * st.size(),
+    OD_CKC(cudaMemcpyAsync(h->cut.stencil, stencil.data(), sizeof(int4) * stencil.size(),
                            cudaMemcpyHostToDevice, h->stream));
     OD_CKC(cudaMemsetAsync(h->d_pairs, 0, sizeof(unsigned long long), h->stream));
     h->has_cut = true;

@@ -8,6 +8,7 @@
 #include <string.h>
 #include <functional>
 #include <map>
+#include <set>
 #include <string>
 #include <vector>
 #include "od_internal.h"
@@ -19,6 +20,7 @@ struct stream_t { std::vector<op> ops; graph_t* capture = nullptr; };
 struct call_t { dim3 grid, block; size_t smem; cudaStream_t s; };
 
 stream_t g_legacy;
+std::set<stream_t*> g_streams = {&g_legacy};
 std::map<char*, size_t> g_blocks;            // device allocations
 std::vector<std::string> g_faults;
 std::string g_log;                           // the calls made and, indented, the kernels launched
@@ -186,6 +188,7 @@ cudaError_t CUDARTAPI cudaMalloc(void** p, size_t n) {
 }
 cudaError_t CUDARTAPI cudaFree(void* p) {
   if (!p) return cudaSuccess;
+  for (stream_t* s : g_streams) run(*s);  // cudaFree waits for the device
   if (!g_blocks.erase((char*)p)) fault("cudaFree of something else");
   else free(p);
   return cudaSuccess;
@@ -224,10 +227,17 @@ cudaError_t CUDARTAPI cudaGetSymbolAddress(void**, const void*) { return cudaErr
 
 // ------------------------------------------------------------------ streams, events, graphs
 cudaError_t CUDARTAPI cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
-  *s = reinterpret_cast<cudaStream_t>(new stream_t);
+  stream_t* q = new stream_t;
+  g_streams.insert(q);
+  *s = reinterpret_cast<cudaStream_t>(q);
   return cudaSuccess;
 }
-cudaError_t CUDARTAPI cudaStreamDestroy(cudaStream_t s) { delete &st(s); return cudaSuccess; }
+cudaError_t CUDARTAPI cudaStreamDestroy(cudaStream_t s) {
+  run(st(s));
+  g_streams.erase(&st(s));
+  delete &st(s);
+  return cudaSuccess;
+}
 cudaError_t CUDARTAPI cudaStreamSynchronize(cudaStream_t s) {
   run(st(s));
   return call("cudaStreamSynchronize");

@@ -213,3 +213,20 @@ def test_force_snapshot_that_fails_leaves_the_output(fake):
         fake.fake_poke(b"9k_mc_sort", 10, 4)  # a crowded cell
         assert fake.od_force_snapshot(eng.h, _lib._dptr(pos), 1500, _lib._dptr(force)) == 7
     assert (force == 7.0).all()
+
+
+@pytest.mark.parametrize("cutoff_lambda", [None, 2.0])
+def test_create_keeps_its_upload_sources(fake, cutoff_lambda):
+    # what od_create uploads asynchronously lives until the stream has been waited for
+    kw = {} if cutoff_lambda is None else dict(cutoff_distance=cutoff_lambda * 1.2e-3)
+    holder, pos, vel = member_case(**kw)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        if cutoff_lambda:
+            eng.set_pair_plan(256, 4, 3, 1024)
+            eng.set_pair_plan(256, 2, 2)
+            eng.set_state(pos, vel)
+        eng.step(2)
+        eng.get_state()
+        eng.collect_flags(pos)
+    assert faults(fake) == []
