@@ -466,13 +466,13 @@ static void drop_graph(od_handle* h);
 static int slabs_of(const od_pair_plan& pl) { return pl.variant <= 1 ? pl.jsplit : 1; }
 static od_status ensure_slabs(od_handle* h, int slabs) {
   if (h->slabs >= slabs) return OD_OK;
+  const size_t n = (size_t)slabs * h->Npad;
+  float4* p = nullptr;
+  OD_CK(h, dalloc(&p, 2 * n));  // the present slabs serve the present plan until there are others
   drop_graph(h);
   if (h->b.part_hi) cudaFree(h->b.part_hi);
-  h->b.part_hi = h->b.part_lo = nullptr;
-  h->slabs = 0;
-  const size_t n = (size_t)slabs * h->Npad;
-  OD_CK(h, dalloc(&h->b.part_hi, 2 * n));
-  h->b.part_lo = h->b.part_hi + n;
+  h->b.part_hi = p;
+  h->b.part_lo = p + n;
   h->slabs = slabs;
   return OD_OK;
 }

@@ -95,6 +95,11 @@ cudaError_t launch(const std::string& name, dim3 grid, void** args, cudaStream_t
     put(s, [p, bits] { *p |= bits; });
   }
   const size_t once = name.find("12k_b_pairs_n3ILi");
+  if (name.find("11k_kick_flagE") != std::string::npos) {  // K3 reads part_hi, part_lo
+    const float4 *ph = *(const float4**)args[4], *pl = *(const float4**)args[5];
+    const size_t need = sizeof(float4) * *(int*)args[6];
+    put(s, [=] { if (room(ph) < need || room(pl) < need) fault("no partial sums to take"); });
+  }
   if (name.find("9k_b_pairsE") != std::string::npos) {
     const od_simdesc* sims = *(const od_simdesc**)args[0];
     const int4* items = *(const int4**)args[1];

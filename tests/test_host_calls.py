@@ -230,3 +230,19 @@ def test_create_keeps_its_upload_sources(fake, cutoff_lambda):
         eng.get_state()
         eng.collect_flags(pos)
     assert faults(fake) == []
+
+
+def test_plan_without_memory_keeps_the_present_one(fake):
+    # a plan that needs more partial-sum slabs than there is memory for: an error, and the present plan
+    # with its slabs goes on
+    holder, pos, vel = member_case(N=5000)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        eng.set_pair_plan(256, 1, 0, 2)
+        eng.step(1)
+        fake.fake_fail(b"cudaMalloc", 0)
+        with pytest.raises(_lib.OpenDustError) as e:
+            eng.set_pair_plan(256, 1, 0, 8)
+        assert e.value.status == 3 and eng.pair_plan()["jsplit"] == 2
+        eng.step(1)
+    assert faults(fake) == []
