@@ -1293,26 +1293,33 @@ extern "C" od_status od_autotune(od_handle* h, int32_t use_cache, double* best_p
   OD_CK(h, cudaEventCreate(&e1));
   double best = -1;
   od_pair_plan best_plan = h->plan;
+  const int reps = h->Npad <= 16384 ? 16 : 2;  // launches timed: short ones are a few us each
+  // Launches are timed as a step makes them, the sums of the variants with accumulators left there for
+  // K3; untimed, they are cleared for the next plan. (ms: of `reps` launches.)
+  auto time_launches = [&](auto launch, float* ms) {
+    OD_CK(h, launch());
+    OD_CK(h, cudaEventRecord(e0, h->stream));
+    for (int r = 0; r < reps; r++) OD_CK(h, launch());
+    OD_CK(h, cudaEventRecord(e1, h->stream));
+    if (uses_acc(h))
+      OD_CK(h, cudaMemsetAsync(h->b.n3, 0, sizeof(float) * h->b.n3_len, h->stream));
+    OD_CK(h, cudaEventSynchronize(e1));
+    OD_CK(h, cudaEventElapsedTime(ms, e0, e1));
+    return OD_OK;
+  };
   for (const auto& sh : shapes) {
     if (sh[2] == 7) {
-      // each unordered pair once: timed over a full launch with the default tile, and only
-      // (the pair rate counts directed pairs, as for the others)
-      if (h->Npad < 8192 || od_set_pair_plan(h, sh[0], sh[1], 7, 0) != OD_OK) {
-        cudaGetLastError();
-        continue;
-      }
+      // each unordered pair once: timed over full launches with the default tile (the pair rate
+      // counts directed pairs, as for the others)
+      if (od_set_pair_plan(h, sh[0], sh[1], 7, 0) != OD_OK) continue;
       const od_pair_io io{h->b.pos, h->b.sx, h->b.sy, h->b.sz, h->b.n3};
-      OD_CK(h, od_launch_pairs(h->plan, io, h->Npad, h->b.part_hi, h->b.part_lo, h->hp.rho0,
-                               &h->ds->err, h->stream));
-      OD_CK(h, cudaEventRecord(e0, h->stream));
-      for (int r = 0; r < 2; r++)
-        OD_CK(h, od_launch_pairs(h->plan, io, h->Npad, h->b.part_hi, h->b.part_lo, h->hp.rho0,
-                                 &h->ds->err, h->stream));
-      OD_CK(h, cudaEventRecord(e1, h->stream));
-      OD_CK(h, cudaEventSynchronize(e1));
       float ms = 0;
-      OD_CK(h, cudaEventElapsedTime(&ms, e0, e1));
-      const double rate = 2.0 * (double)h->Npad * h->Npad / (ms * 1e-3);
+      const od_status st = time_launches([&] {
+        return od_launch_pairs(h->plan, io, h->Npad, h->b.part_hi, h->b.part_lo, h->hp.rho0,
+                               &h->ds->err, h->stream, false);
+      }, &ms);
+      if (st != OD_OK) return st;
+      const double rate = reps * (double)h->Npad * h->Npad / (ms * 1e-3);
       if (rate > best) { best = rate; best_plan = h->plan; }
       continue;
     }
@@ -1325,17 +1332,13 @@ extern "C" od_status od_autotune(od_handle* h, int32_t use_cache, double* best_p
       // enough target blocks for ~8 waves of the source split, at most the full grid
       const int limit = std::min(nbx, std::max(1, (sms * 32 + pl.jsplit - 1) / pl.jsplit));
       const od_pair_io io{h->b.pos, h->b.sx, h->b.sy, h->b.sz, h->b.n3};
-      OD_CK(h, od_launch_pairs_probe(pl, io, h->Npad, limit, h->b.part_hi, h->b.part_lo, h->hp.rho0,
-                                     &h->ds->err, h->stream));
-      OD_CK(h, cudaEventRecord(e0, h->stream));
-      for (int r = 0; r < 2; r++)
-        OD_CK(h, od_launch_pairs_probe(pl, io, h->Npad, limit, h->b.part_hi, h->b.part_lo,
-                                       h->hp.rho0, &h->ds->err, h->stream));
-      OD_CK(h, cudaEventRecord(e1, h->stream));
-      OD_CK(h, cudaEventSynchronize(e1));
       float ms = 0;
-      OD_CK(h, cudaEventElapsedTime(&ms, e0, e1));
-      const double pairs = 2.0 * limit * (double)(sh[0] * sh[1]) * h->Npad;
+      const od_status st = time_launches([&] {
+        return od_launch_pairs_probe(pl, io, h->Npad, limit, h->b.part_hi, h->b.part_lo, h->hp.rho0,
+                                     &h->ds->err, h->stream);
+      }, &ms);
+      if (st != OD_OK) return st;
+      const double pairs = (double)reps * limit * (double)(sh[0] * sh[1]) * h->Npad;
       const double rate = pairs / (ms * 1e-3);
       if (rate > best) { best = rate; best_plan = pl; }
     }

@@ -1391,7 +1391,7 @@ cudaError_t od_launch_pairs_probe(const od_pair_plan& pl, const od_pair_io& io, 
                                   int gridx_limit, float4* ph, float4* plo, float rho0,
                                   uint32_t* err, cudaStream_t s) {
   g_gridx_limit = gridx_limit;
-  cudaError_t e = od_launch_pairs(pl, io, Npad, ph, plo, rho0, err, s);
+  cudaError_t e = od_launch_pairs(pl, io, Npad, ph, plo, rho0, err, s, false);
   g_gridx_limit = 0;
   return e;
 }

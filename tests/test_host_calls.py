@@ -246,3 +246,18 @@ def test_plan_without_memory_keeps_the_present_one(fake):
         assert e.value.status == 3 and eng.pair_plan()["jsplit"] == 2
         eng.step(1)
     assert faults(fake) == []
+
+
+@pytest.mark.parametrize("N", [300, 2048, 9000])
+def test_autotuner_times_every_shape(fake, N):
+    # the default (variant 7) among them at every size, without the kernels that a step does not launch
+    holder, pos, vel = member_case(N=N)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        fake.fake_reset()
+        eng.autotune(use_cache=False)
+        calls = log(fake)
+    for mt, ms in ((2, 2), (4, 4), (8, 2)):
+        assert any(f"10k_pairs_n3ILi{mt}ELi{ms}E" in x for x in calls), mt
+    # the sums are taken out of the accumulators once, of the present state with the plan chosen
+    assert sum("k_n3_take" in x or "k_acc_take" in x for x in calls) <= 1
