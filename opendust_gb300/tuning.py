@@ -189,17 +189,22 @@ class PlanCache:
         os.replace(tmp, self.path)
 
 
+# "single" entries without the number came from a tuner that left the default kernel out below 8192
+# ions; they are not read any more, the sizes are measured again.
+SINGLE = "single|2"
+
+
 def tuned_plan(eng: _lib.Engine, device: int = 0, cache: PlanCache | None = None) -> tuple:
     """The autotuner's all-pairs plan for this engine's size, from the persisted cache or, on a
     miss, by od_autotune on the engine's current positions (then stored). Applies it."""
     cache = cache or PlanCache()
     model = gpu_model(device)
-    plan = cache.get("single", model, eng.n)
+    plan = cache.get(SINGLE, model, eng.n)
     if plan is None:
         eng.autotune(use_cache=False)
         p = eng.pair_plan()
         plan = (p["threads"], p["targets_per_thread"], p["variant"], p["jsplit"])
-        cache.put("single", model, eng.n, plan)
+        cache.put(SINGLE, model, eng.n, plan)
     eng.set_pair_plan(*plan)
     return plan
 
