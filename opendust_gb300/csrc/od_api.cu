@@ -42,6 +42,7 @@ struct od_handle {
   float4* snap_pos = nullptr;
   double* snap_counts = nullptr;
   double* stage = nullptr;  // FP64 staging of a shard (other handles use the list block)
+  double* series_out = nullptr;  // [series_stage_rows] rows of a long series, split for the copies
   // CUDA graph of one step (production path)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
@@ -478,6 +479,17 @@ static od_status ensure_slabs(od_handle* h, int slabs) {
   return OD_OK;
 }
 
+// Series reads up to this many bytes take one copy of the rows, split on the host. Longer ones are split
+// on the device, up to OD_SERIES_STAGE bytes at a time, in a block of the handle: 20000 rows of one
+// grain 90 us, 20000 of four 135, into fresh arrays 555 (strided copies straight from the rows, 8 or 24
+// bytes wide: 167, 350, 8700).
+static constexpr size_t OD_SERIES_WHOLE = (size_t)256 << 10, OD_SERIES_STAGE = (size_t)16 << 20;
+// rows of the splitting block of a series of `rows` rows (0: no read is that long)
+static size_t series_stage_rows(size_t rows, size_t P) {
+  const size_t row = sizeof(double) * 13 * P;
+  return rows * row <= OD_SERIES_WHOLE ? 0 : std::min(rows, std::max<size_t>(1, OD_SERIES_STAGE / row));
+}
+
 static od_status create_handle(const od_config* cfg, int32_t device, bool n3_default,
                                od_handle** out);
 static od_status alloc_cutn3(od_handle* h, int ipt, int T);
@@ -538,6 +550,7 @@ static od_status create_handle(const od_config* cfg, int32_t device, bool n3_def
     c.take(h->b.list_old, 3 * Np);
     c.take(h->b.orbit_part, (size_t)h->nb * P * 3);
     c.take(h->b.series, ns * P * 13);
+    c.take(h->series_out, series_stage_rows(ns, P) * P * 13);
     c.take(h->b.cq, OD_MAX_GRAINS);
     c.take(h->b.sx, Np);
     c.take(h->b.sy, Np);
@@ -1425,25 +1438,33 @@ extern "C" od_status od_get_series(od_handle* h, int64_t first, int64_t count, d
   if (P == 0) return OD_OK;
   double* out[5] = {q, f_orbit, f_collect, f_dust, f_field};
   const double* src = h->b.series + first * row;
-  const bool whole = sizeof(double) * row * count <= (256 << 10);
-  std::vector<double> rows;
-  if (whole) {  // one copy of the rows (each copy takes about 9 us), split on the host
-    rows.resize((size_t)count * row);
+  const size_t width[5] = {P, 3 * P, 3 * P, 3 * P, 3 * P};  // of a row
+  if (sizeof(double) * row * count <= OD_SERIES_WHOLE) {  // each copy takes about 9 us
+    std::vector<double> rows((size_t)count * row);
     OD_CK(h, cudaMemcpyAsync(rows.data(), src, sizeof(double) * rows.size(),
                              cudaMemcpyDeviceToHost, h->stream));
     OD_CK(h, cudaStreamSynchronize(h->stream));
+    for (size_t m = 0, at = 0; m < 5; at += width[m++])
+      if (out[m])
+        for (int64_t k = 0; k < count; k++)
+          memcpy(out[m] + (size_t)k * width[m], rows.data() + (size_t)k * row + at,
+                 sizeof(double) * width[m]);
+    return OD_OK;
   }
-  for (int m = 0; m < 5; m++) {
-    if (!out[m]) continue;
-    const size_t w = m ? 3 * P : P, at = m ? P + 3 * P * (m - 1) : 0;
-    if (whole)
-      for (int64_t k = 0; k < count; k++)
-        memcpy(out[m] + (size_t)k * w, rows.data() + (size_t)k * row + at, sizeof(double) * w);
-    else
-      OD_CK(h, cudaMemcpy2DAsync(out[m], sizeof(double) * w, src + at, sizeof(double) * row,
-                                 sizeof(double) * w, (size_t)count, cudaMemcpyDeviceToHost, h->stream));
+  const int64_t most = (int64_t)series_stage_rows((size_t)h->cfg.n_steps, P);
+  for (int64_t k = 0; k < count; k += most) {
+    const int64_t n = std::min(most, count - k);
+    OD_CK(h, od_launch_series_split(src + k * row, n, (int)P, h->series_out, h->stream));
+    const double* from = h->series_out;
+    if (k == 0)
+      for (int m = 0; m < 5; m++)
+        if (out[m]) touch_pages(out[m], sizeof(double) * count * width[m]);
+    for (int m = 0; m < 5; from += (size_t)n * width[m++])
+      if (out[m])
+        OD_CK(h, cudaMemcpyAsync(out[m] + (size_t)k * width[m], from, sizeof(double) * n * width[m],
+                                 cudaMemcpyDeviceToHost, h->stream));
   }
-  if (!whole) OD_CK(h, cudaStreamSynchronize(h->stream));
+  OD_CK(h, cudaStreamSynchronize(h->stream));
   return OD_OK;
 }
 
@@ -1986,6 +2007,7 @@ extern "C" od_status od_config_device_bytes(const od_config* cfg, int64_t* bytes
   b += Np / 32 * 4 + Np * (4 + 4 + 48);  // flags, list, list bits, list positions/velocities
   b += (Np / 256) * P * 3 * 8;      // orbit partials
   b += cfg->n_steps * P * 13 * 8;   // result series
+  b += (int64_t)series_stage_rows((size_t)cfg->n_steps, (size_t)P) * P * 13 * 8;
   b += sizeof(od_dparams) + sizeof(od_dstate) + 4096;
   *bytes = b;
   return OD_OK;

@@ -195,6 +195,9 @@ cudaError_t od_launch_snapshot_in(int n, int Npad, const double* pos, double lam
 cudaError_t od_launch_snapshot_out(int n, int Npad, int jsplit, const float4* ph, const float4* pl,
                                    unsigned long long* acc, double scale, double* force,
                                    cudaStream_t s);
+// rows of the series (13 P doubles each) -> q [rows][P], orbit, collect, dust, field [rows][P][3]
+cudaError_t od_launch_series_split(const double* series, int64_t rows, int P, double* out,
+                                   cudaStream_t s);
 // empty state of a new handle: every position a far-away sentinel
 cudaError_t od_launch_clear_state(int Npad, const od_dbufs& b, cudaStream_t s);
 // series row 0 next, averages restarted, the Philox step counter running on (od_begin_window)

@@ -1899,6 +1899,16 @@ __global__ void __launch_bounds__(kBlk) k_clear_state(int Npad, float4* __restri
   sx[i] = sy[i] = sz[i] = OD_SENTINEL;
 }
 
+__global__ void __launch_bounds__(kBlk) k_series_split(const double* __restrict__ series,
+                                                       unsigned rows, unsigned P,
+                                                       double* __restrict__ out) {
+  const unsigned e = blockIdx.x * kBlk + threadIdx.x, row = 13 * P;  // at most 16 MB of rows
+  if (e >= rows * row) return;
+  const unsigned r = e / row, c = e - r * row, m = c < P ? 0 : 1 + (c - P) / (3 * P);
+  const unsigned at = m ? P + 3 * P * (m - 1) : 0, w = m ? 3 * P : P;
+  out[rows * at + r * w + (c - at)] = series[e];
+}
+
 __global__ void k_begin_window(od_dstate* __restrict__ ds) {
   if (threadIdx.x == 0) {
     ds->rng_base += ds->step;
@@ -1949,6 +1959,11 @@ cudaError_t od_launch_snapshot_out(int n, int Npad, int jsplit, const float4* ph
 }
 cudaError_t od_launch_clear_state(int Npad, const od_dbufs& b, cudaStream_t s) {
   k_clear_state<<<blocks_of(Npad), kBlk, 0, s>>>(Npad, b.pos, b.sx, b.sy, b.sz);
+  return cudaGetLastError();
+}
+cudaError_t od_launch_series_split(const double* series, int64_t rows, int P, double* out,
+                                   cudaStream_t s) {
+  k_series_split<<<blocks_of(rows * 13 * P), kBlk, 0, s>>>(series, (unsigned)rows, (unsigned)P, out);
   return cudaGetLastError();
 }
 cudaError_t od_launch_begin_window(od_dstate* ds, cudaStream_t s) {

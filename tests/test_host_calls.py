@@ -261,3 +261,20 @@ def test_autotuner_times_every_shape(fake, N):
         assert any(f"10k_pairs_n3ILi{mt}ELi{ms}E" in x for x in calls), mt
     # the sums are taken out of the accumulators once, of the present state with the plan chosen
     assert sum("k_n3_take" in x or "k_acc_take" in x for x in calls) <= 1
+
+
+@pytest.mark.parametrize("rows,wanted", [(2000, 5), (2520, 5), (30000, 5), (30000, 1)])
+def test_series_reads_are_few_contiguous_copies(fake, rows, wanted):
+    # up to 256 KB (2520 rows of one grain) one copy, then one per array and 16 MB: no strided ones,
+    # which move 8 or 24 bytes at a time
+    holder, pos, vel = member_case(N=300, n=rows)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        eng.step(rows)
+        fake.fake_reset()
+        a = [np.empty((rows, 3)) for _ in range(5)]
+        ptr = [_lib._dptr(x) if m < wanted else None for m, x in enumerate(a)]
+        _lib.check(fake.od_get_series(eng.h, 0, rows, *ptr), eng.h)
+        calls = log(fake)
+    assert "cudaMemcpy2DAsync" not in calls
+    assert calls.count("cudaMemcpyAsync") == (1 if rows <= 2520 else wanted)
