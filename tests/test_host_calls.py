@@ -278,3 +278,13 @@ def test_series_reads_are_few_contiguous_copies(fake, rows, wanted):
         calls = log(fake)
     assert "cudaMemcpy2DAsync" not in calls
     assert calls.count("cudaMemcpyAsync") == (1 if rows <= 2520 else wanted)
+
+
+@pytest.mark.parametrize("N,copies", [(2, 1), (1365, 1), (1366, 2)])
+def test_small_state_is_one_copy(fake, N, copies):
+    holder, pos, vel = member_case(N=N)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        fake.fake_reset()
+        eng.get_state()
+        assert log(fake).count("cudaMemcpyAsync") == copies
