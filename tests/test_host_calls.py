@@ -284,7 +284,10 @@ def test_series_reads_are_few_contiguous_copies(fake, rows, wanted):
 def test_small_state_is_one_copy(fake, N, copies):
     holder, pos, vel = member_case(N=N)
     with _lib.Engine(holder) as eng:
+        fake.fake_reset()
         eng.set_state(pos, vel)
+        # and the error word; more ions also the word of the device's check
+        assert log(fake).count("cudaMemcpyAsync") == (2 if copies == 1 else 4)
         fake.fake_reset()
         eng.get_state()
-        assert log(fake).count("cudaMemcpyAsync") == copies
+        assert log(fake).count("cudaMemcpyAsync") == copies and faults(fake) == []
