@@ -19,8 +19,8 @@
 //     at most one group pair of work.
 //   * The source groups inside a target group are evaluated as directed pairs (no reaction; the
 //     self pair contributes exactly 0).
-//   * Reactions are summed in FP32 over at most 16 lane steps, target sums over one group pair
-//     (then as two-floats in the warp's shared-memory slice when L > 1); both are then added to
+//   * Reactions are summed in FP32 over at most 16 lane steps, target sums over one group pair or
+//     part of one (then as two-floats in the warp's shared-memory slice when L > 1); both are added to
 //     the ions' 64-bit fixed-point accumulators with integer atomics, so every result bit is
 //     independent of scheduling.
 //
@@ -275,8 +275,13 @@ long long od_n3_blocks(const od_n3_split& sp) { return (sp.units + kSliceWarps -
 //     empty (3040 on 152 SMs; 4656 group pairs at 12000) and a single warp's dependency chain sets
 //     the time, so they are split by lane steps. Steps of 2048, 4096, 5000, 7680, 8192 and 14000
 //     ions in us: whole 29.0, 31.1, 52.4, 54.7, 55.3, 94.5; two parts 24.4, 28.9, 37.5, 44.7, 44.4,
-//     90.7; four 22.8, 27.0, 30.1, 42.6, 46.0, 97.5. Two parts still gain 1.5 % at 2^14, but there
-//     batches would run them apart from their larger members, with a last wave of their own.
+//     90.7; four 22.8, 27.0, 30.1, 42.6, 46.0, 97.5. From 2^14 to 2^15 ions two parts keep the
+//     accuracy of the 2 x 2 shape that was the default there, as their FP32 chains on the target side have 32
+//     terms where a whole group pair's have 64: median relative error per ion at 16385, 20011 and
+//     32768 ions 5.5e-8, 5.2e-8, 4.7e-8 in two parts, 6.0e-8, 5.7e-8, 5.1e-8 whole, 5.8e-8, 5.6e-8,
+//     5.0e-8 with 2 x 2. Steps of 16384, 20011, 25000, 28000 and 32768 ions: 113.5, 162.8, 233.0,
+//     289.4, 385.6 us, whole 115.1, 166.1, 232.5, 285.9, 383.5; batches run them apart from their larger
+//     members, with a last wave of their own (0.2 %; six members of 2^14 to 2^15 ions 1.6 %).
 //   * 8 x 2 (256 x 64 ions) and 2 x 2: a tile names how many group pairs a slice may hold (tile / 64),
 //     at least 16 slices per resident warp. 8 x 2 at 2^18 ions: 21.6 ms with 8 or 16, 22.3 with 1.
 od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
@@ -286,7 +291,7 @@ od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
   sp.split = 1;
   long long L = 1;
   if (ipt == 4) {
-    if (Npad < 16384) sp.split = Npad <= 7680 ? 4 : 2;
+    if (Npad <= 32768) sp.split = Npad <= 7680 ? 4 : 2;
   } else {
     const long long warps = 152ll * kSliceWarps * (ipt == 8 ? 4 : 8);
     L = std::max(1ll, std::min<long long>(tile / 64, sp.pairs / (warps * 16)));
