@@ -746,6 +746,14 @@ static bool all_finite(const double* a, int64_t n) {
   return true;
 }
 
+// Waits for the stream where a call leaves early: no copy of the caller's arrays, or of its own, runs on
+// after it has returned. (done: the call has waited itself)
+struct od_copies {
+  cudaStream_t s;
+  bool done = false;
+  ~od_copies() { if (!done) cudaStreamSynchronize(s); }
+};
+
 // A state up to this many bytes is checked on the host and is one copy (a copy takes about 9 us: 512 ions
 // 56 us to set, with the device's check and two copies 70; 27 us to get, in two copies 35).
 static constexpr size_t OD_STATE_WHOLE = (size_t)64 << 10;
@@ -759,7 +767,8 @@ extern "C" od_status od_set_state(od_handle* h, const double* pos, const double*
   od_status st = staging(h, &st64);
   if (st != OD_OK) return st;
   const size_t bytes = sizeof(double) * 3 * n;
-  std::vector<double> both;  // lives until the stream has been waited for
+  std::vector<double> both;
+  od_copies copies{h->stream};
   if (2 * bytes <= OD_STATE_WHOLE) {
     if (!all_finite(pos, 3 * n) || !all_finite(vel, 3 * n))
       return fail(h, OD_ERR_INVALID, "a position or velocity is not finite");
@@ -780,6 +789,7 @@ extern "C" od_status od_set_state(od_handle* h, const double* pos, const double*
   st = refresh_forces(h);
   if (st != OD_OK) return st;
   OD_CK(h, cudaStreamSynchronize(h->stream));
+  copies.done = true;
   h->state_set = true;
   return check_device_err(h);
 }
@@ -914,12 +924,15 @@ extern "C" od_status od_get_state(od_handle* h, double* pos, double* vel, int64_
   od_status st = staging(h, &st64);
   if (st != OD_OK) return st;
   const size_t bytes = sizeof(double) * 3 * n;
+  std::vector<double> both;
+  od_copies copies{h->stream};
   OD_CK(h, od_launch_state_out(h->dp, h->N, h->b, pos ? st64 : nullptr, vel ? st64 + 3 * n : nullptr,
                                h->stream));
   if (pos && vel && 2 * bytes <= OD_STATE_WHOLE) {
-    std::vector<double> both((size_t)6 * n);
+    both.resize((size_t)6 * n);
     OD_CK(h, cudaMemcpyAsync(both.data(), st64, 2 * bytes, cudaMemcpyDeviceToHost, h->stream));
     OD_CK(h, cudaStreamSynchronize(h->stream));
+    copies.done = true;
     memcpy(pos, both.data(), bytes);
     memcpy(vel, both.data() + 3 * n, bytes);
     return OD_OK;
@@ -929,6 +942,7 @@ extern "C" od_status od_get_state(od_handle* h, double* pos, double* vel, int64_
   if (pos) OD_CK(h, cudaMemcpyAsync(pos, st64, bytes, cudaMemcpyDeviceToHost, h->stream));
   if (vel) OD_CK(h, cudaMemcpyAsync(vel, st64 + 3 * n, bytes, cudaMemcpyDeviceToHost, h->stream));
   OD_CK(h, cudaStreamSynchronize(h->stream));
+  copies.done = true;
   return OD_OK;
 }
 
@@ -1523,6 +1537,7 @@ extern "C" od_status od_force_snapshot(od_handle* h, const double* pos, int64_t 
   if (!pos || !force) return fail(h, OD_ERR_INVALID, "NULL argument");
   if (n < 1 || n > h->N) return fail(h, OD_ERR_INVALID, "n must be in [1, n_ions]");
   OD_CK(h, cudaSetDevice(h->device));
+  od_copies copies{h->stream};
   od_status st = upload_snapshot(h, pos, n, true);
   if (st != OD_OK) return st;
   const od_force_ctx fc = force_ctx(h, false);
@@ -1539,6 +1554,7 @@ extern "C" od_status od_force_snapshot(od_handle* h, const double* pos, int64_t 
   if (st != OD_OK) return st;  // the caller's array as it was
   OD_CK(h, cudaMemcpyAsync(force, out, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, h->stream));
   OD_CK(h, cudaStreamSynchronize(h->stream));
+  copies.done = true;
   return OD_OK;
 }
 
@@ -1560,13 +1576,15 @@ extern "C" od_status od_collect_flags(od_handle* h, const double* pos, int64_t n
   if (!pos || !count || (cap > 0 && !idx_out)) return fail(h, OD_ERR_INVALID, "NULL argument");
   if (n < 1 || n > h->N) return fail(h, OD_ERR_INVALID, "n must be in [1, n_ions]");
   OD_CK(h, cudaSetDevice(h->device));
+  double counts[OD_MAX_GRAINS + 1];
+  od_copies copies{h->stream};
   od_status st = upload_snapshot(h, pos, n, false);
   if (st != OD_OK) return st;
   OD_CK(h, od_launch_snapshot_flags(h->dp, (int)n, h->Npad, h->snap_pos, h->b.flags, h->b.list,
                                     h->b.list_bits, h->snap_counts, h->stream));
-  double counts[OD_MAX_GRAINS + 1];
   OD_CK(h, cudaMemcpyAsync(counts, h->snap_counts, sizeof(counts), cudaMemcpyDeviceToHost, h->stream));
   OD_CK(h, cudaStreamSynchronize(h->stream));
+  copies.done = true;
   const int64_t K = (int64_t)counts[OD_MAX_GRAINS];
   *count = K;
   if (grain_counts)

@@ -305,3 +305,26 @@ def test_short_fp32_chains_up_to_2_15_ions(fake, N):
     names = [x for x in log(fake) if "pairs_n3ILi4ELi4E" in x]
     split = "ILi4ELi4ELi4E" if N <= 7680 else "ILi4ELi4ELi2E"
     assert names and all(split in x for x in names)
+
+
+@pytest.mark.parametrize("N", [1000, 2000])
+@pytest.mark.parametrize("call,fails", [("force_snapshot", b"launch"), ("collect_flags", b"launch"),
+                                        ("set_state", b"launch"), ("get_state", b"cudaMemcpyAsync")])
+def test_failed_call_leaves_no_copy_behind(fake, call, fails, N):
+    # the caller may free its arrays when the call returns, also when it failed after a copy began
+    holder, pos, vel = member_case(N=N)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        for after in range(3):
+            a, b = pos.copy(), vel.copy()
+            fake.fake_reset()
+            fake.fake_fail(fails, after)
+            args = dict(set_state=(a, b), get_state=()).get(call, (a,))
+            try:
+                getattr(eng, call)(*args)
+            except _lib.OpenDustError:
+                assert log(fake)[-1] == "cudaStreamSynchronize"
+            a[:] = b[:] = 0.0
+            fake.fake_fail(fails, 1000)
+            eng.get_state()
+            assert faults(fake) == []
