@@ -282,7 +282,8 @@ od_status od_set_graph(od_handle* h, int32_t enable);
  * pair on the Newton path of variant 4, 7: each unordered pair evaluated once and applied to
  * both ions (threads 256; targets_per_thread = target ions per lane: 2 or 4 with as many source
  * ions, 8 with two; jsplit = tile, 1024, 2048 or 4096 (not 1024 with 8; also 512 with 2), <= 0
- * for the default: it caps the work a warp takes at a time). Variants 2-7 add their sums into
+ * for the default: with 2 and 8 it caps the group pairs that a warp takes at a time, with 4 a warp
+ * takes one or a part of one whatever the tile). Variants 2-7 add their sums into
  * 64-bit fixed-point accumulators (24 bytes per ion) with integer atomics, so results do not
  * depend on the order of the GPU's blocks. od_create selects variant 7.
  * jsplit <= 0 picks the source split from the SM count. Takes effect at the next step.
@@ -459,7 +460,7 @@ od_status od_read_restart(const char* path, int64_t n, double* pos_nm, double* v
  * (n x 3 doubles, metres) and force_dev (n x 3 doubles, newtons, written), the Debye length
  * r_D_e, the softening r_0 and the prefactor kq_sq_s = k q_s^2 (J m, the reference's
  * "kq_sq_s" parameter). The call allocates and frees nothing: its scratch (positions in
- * device units, partial sums, an error word) is one file-scope device array of about 8.8 MB
+ * device units, partial sums) is one file-scope device array of about 8.8 MB
  * that every GPU which loads this library holds until the process exits; it limits n to
  * 2..32768 (larger n returns OD_ERR_INVALID). The call runs on the calling thread's current
  * device and on `stream` (a cudaStream_t, NULL for the default stream) and returns after the

@@ -388,8 +388,8 @@ static void fill_params(const od_config* c, int N, int Npad, od_dparams* p) {
 // 8 x 2); its sums go to 24 bytes of fixed-point accumulators per ion, so it always fits (the
 // budget below only bounds the rule).
 static constexpr size_t OD_N3_BUDGET = (size_t)32 << 30;
-// The cutoff's sorted path (variant 3) needs its sort, boxes and slot accumulators (45 bytes per
-// ion); beyond the budget the cell stencil takes over.
+// The cutoff's sorted path (variant 3) needs its sort, boxes, lists and slot accumulators (od_cutn3_bytes:
+// 53 bytes per ion and 8 per cell without the lists); beyond the budget the cell stencil takes over.
 static constexpr size_t OD_CUTN3_BUDGET = (size_t)64 << 30;
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile);
 
@@ -673,7 +673,7 @@ static od_status check_device_err(od_handle* h) {
   OD_CK(h, cudaStreamSynchronize(h->stream));
   if (err & OD_DERR_TIMEOUT) return fail(h, OD_ERR_TIMEOUT, "a bounded device wait ran out");
   if (err & OD_DERR_CELL)
-    return fail(h, OD_ERR_CAPACITY, "a cutoff cell holds more than 4096 ions (density too high)");
+    return fail(h, OD_ERR_CAPACITY, "a cutoff cell holds more ions than its sort takes (density too high)");
   if (err) return fail(h, OD_ERR_STATE, "device error word set");
   return OD_OK;
 }
@@ -1223,8 +1223,8 @@ static od_status ensure_acc(od_handle* h) {
 }
 
 // Variant 7: `ions_per_lane` targets per lane (2 or 4 with as many sources, 8 with two sources),
-// `tile` caps the work per warp (od_n3_split_of; 1024, 2048, 4096; <= 0: 1024 up to 2^17 ions, else
-// 2048). The pair sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25
+// `tile` caps the work per warp for 2 and 8 (od_n3_split_of; 1024, 2048, 4096; <= 0: 1024 up to 2^17
+// ions, else 2048). The pair sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25
 // MB at 2^20).
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
   if (!plan_supported(256, ions_per_lane, 7))
@@ -2129,7 +2129,7 @@ extern "C" od_status od_shard_create(const od_config* cfg, int64_t first, int64_
     g_err = m;
     return r;
   };
-    const size_t nt = (size_t)h->Npad_total, P = std::max(h->P, 1);
+  const size_t nt = (size_t)h->Npad_total, P = std::max(h->P, 1);
   if (dalloc(&h->ssx, nt) || dalloc(&h->ssy, nt) || dalloc(&h->ssz, nt) ||
       dalloc(&h->g_idx, (size_t)Nt) || dalloc(&h->g_bits, (size_t)Nt) ||
       dalloc(&h->g_old, (size_t)Nt) || dalloc(&h->g_new, (size_t)Nt) ||

@@ -15,7 +15,7 @@ struct od_pair_plan {
   int variant; // 0: shared-memory broadcast, 1: warp-shuffle broadcast, 2: packed f32x2 with
                // SoA tiles (ipt 2), 3: as 2 with Newton reciprocals for half of the targets,
                // 4-6: further packed forms, 7: each unordered pair once (od_n3.cu)
-  int tile;    // variant 7: caps the work per warp (od_n3_split_of); ipt = targets per lane (2, 4:
+  int tile;    // variant 7: caps the work per warp for ipt 2 and 8 (od_n3_split_of); ipt = targets per lane (2, 4:
                // as many sources; 8: two sources)
 };
 

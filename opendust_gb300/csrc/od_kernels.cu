@@ -801,7 +801,7 @@ inline int orbit_per(int nb) { return nb > 2 * 152 ? 4 : 1; }
 
 // ============================================================== FP64 host-tail on device
 // opendust.py:1117-1202 (charge), :1205-1235 (dust–dust), :1237-1331 (orbit + out-of-domain),
-// :1333-1365 (collect), :1367-1383 (field); one 256-thread block, the first of K5, so that its FP64
+// :1333-1365 (collect), :1367-1383 (field); one block of kCT threads, the first of K5, so that its FP64
 // latency (3.5 us: an FP64 instruction takes a GB300 SM 16 cycles per warp, and the chains are short
 // and dependent) passes while the other blocks correct the forces. In the last block of K5 to finish,
 // with the orbit sums before it, it held up every step by 8 us (2048 ions: K3 to K5 19.5 us, now 14).
@@ -1418,7 +1418,7 @@ cudaError_t od_launch_force(const od_force_ctx& fc, const od_pair_io& io, int n,
   return od_launch_pairs(fc.plan, io, Npad, part_hi, part_lo, fc.rho0, err, s, take);
 }
 
-// part 0: K1 (kick/drift); part 1: K2 (ion–ion sums); part 2: K3..K6
+// part 0: K1 (kick/drift); part 1: K2 (ion–ion sums); part 2: K3..K5
 cudaError_t od_launch_step_part(int part, const od_dparams* dp, od_dstate* ds, const od_dbufs& b,
                                 int N, int Npad, int P, const od_force_ctx& fc, int nrec,
                                 cudaStream_t s) {
