@@ -282,8 +282,9 @@ od_status od_set_graph(od_handle* h, int32_t enable);
  * pair on the Newton path of variant 4, 7: each unordered pair evaluated once and applied to
  * both ions (threads 256; targets_per_thread = target ions per lane: 2 or 4 with as many source
  * ions, 8 with two; jsplit = tile, 1024, 2048 or 4096 (not 1024 with 8; also 512 with 2), <= 0
- * for the default: with 2 and 8 it caps the group pairs that a warp takes at a time, with 4 a warp
- * takes one or a part of one whatever the tile). Variants 2-7 add their sums into
+ * for the default: with 2 and 8 it caps the group pairs that a warp takes at a time; with 4 a warp
+ * takes one, or in small systems a part, and from 2048 on adds its target sums after each half of
+ * one, which halves their FP32 chains from 2^14 ions on). Variants 2-7 add their sums into
  * 64-bit fixed-point accumulators (24 bytes per ion) with integer atomics, so results do not
  * depend on the order of the GPU's blocks. od_create selects variant 7.
  * jsplit <= 0 picks the source split from the SM count. Takes effect at the next step.

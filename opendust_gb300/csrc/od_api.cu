@@ -1223,8 +1223,8 @@ static od_status ensure_acc(od_handle* h) {
 }
 
 // Variant 7: `ions_per_lane` targets per lane (2 or 4 with as many sources, 8 with two sources),
-// `tile` caps the work per warp for 2 and 8 (od_n3_split_of; 1024, 2048, 4096; <= 0: 1024 up to 2^17
-// ions, else 2048). The pair sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25
+// `tile` caps the work per warp for 2 and 8, above 1024 its FP32 chains for 4 (od_n3_split_of; 1024,
+// 2048, 4096; <= 0: 1024 up to 2^17 ions, else 2048). The pair sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25
 // MB at 2^20).
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
   if (!plan_supported(256, ions_per_lane, 7))

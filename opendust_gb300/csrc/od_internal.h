@@ -15,7 +15,7 @@ struct od_pair_plan {
   int variant; // 0: shared-memory broadcast, 1: warp-shuffle broadcast, 2: packed f32x2 with
                // SoA tiles (ipt 2), 3: as 2 with Newton reciprocals for half of the targets,
                // 4-6: further packed forms, 7: each unordered pair once (od_n3.cu)
-  int tile;    // variant 7: caps the work per warp for ipt 2 and 8 (od_n3_split_of); ipt = targets per lane (2, 4:
+  int tile;    // variant 7: caps the work per warp, or (ipt 4) its FP32 chains (od_n3_split_of); ipt = targets per lane (2, 4:
                // as many sources; 8: two sources)
 };
 
@@ -63,10 +63,11 @@ cudaError_t od_launch_pairs_n3(const od_pair_plan& pl, const od_pair_io& io, int
 struct od_n3_split {
   long long pairs, units;  // group pairs of the upper triangle, units
   int L, split;
+  bool half;  // target sums of whole 4 x 4 group pairs added after each half
 };
 od_n3_split od_n3_split_of(int Npad, int ipt, int tile);
 long long od_n3_blocks(const od_n3_split& sp);
-constexpr int OD_N3_FORMS = 6;
+constexpr int OD_N3_FORMS = 7;
 int od_n3_form(int ipt, const od_n3_split& sp);  // kernel form of a batch member, < OD_N3_FORMS
 
 // One member of a batch, as the batched kernels see it.

@@ -99,7 +99,8 @@ __device__ __forceinline__ void lane_steps(const pair_consts& k, const od_u64 (&
 // Unit `unit` of one simulation (one warp): group pairs [unit L, unit L + L) of the row-major
 // upper triangle, or (SPLIT > 1, L = 1) part unit % SPLIT of group pair unit / SPLIT.
 // h: this lane's column of the warp's shared-memory slice ([6][GT] floats, used when FOLD).
-template <int MT, int MS, int SPLIT, bool FOLD>
+// HALF: the target sums too are added to the accumulators every 16 lane steps.
+template <int MT, int MS, int SPLIT, bool FOLD, bool HALF>
 __device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const float* __restrict__ sy,
                                          const float* __restrict__ sz, int Npad,
                                          unsigned long long* __restrict__ acc, float rho0,
@@ -107,6 +108,7 @@ __device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const flo
   using TR = slice_traits<MT, MS>;
   constexpr int GT = TR::GT, GS = TR::GS, R = TR::R;
   static_assert(!(FOLD && SPLIT > 1), "a split group pair is one unit");
+  static_assert(!HALF || (SPLIT == 1 && !FOLD), "halves of a whole group pair");
   const int lane = threadIdx.x & 31, src = (lane + 1) & 31;
   constexpr int STEPS = 32 / SPLIT;        // lane steps of a unit's group pairs
   constexpr int PART = STEPS < 16 ? STEPS : 16;  // lane steps between two reaction flushes
@@ -149,6 +151,16 @@ __device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const flo
       }
 #pragma unroll
       for (int t = 0; t < MT; t++) AX[t] = AY[t] = AZ[t] = 0ull;
+      const auto add_targets = [&] {
+#pragma unroll
+        for (int t = 0; t < MT; t++) {
+          unsigned long long* a = acc + g * GT + lane + 32 * t;
+          od_fix_add1(a, sum2(AX[t]));
+          od_fix_add1(a + Npad, sum2(AY[t]));
+          od_fix_add1(a + 2 * (size_t)Npad, sum2(AZ[t]));
+          AX[t] = AY[t] = AZ[t] = 0ull;
+        }
+      };
       if (s >= g * R + R) {
         // each part's reactions are added to the accumulators of the sources where they stand
         // (the force on a source is minus the accumulated terms)
@@ -167,18 +179,19 @@ __device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const flo
             e += Npad;
             od_fix_add1(e, -rz.x); od_fix_add1(e + 32, -rz.y);
           }
+          if (HALF) add_targets();
+        }
+      } else if (HALF) {
+#pragma unroll 1
+        for (int st = PART; st <= STEPS; st += PART) {
+          lane_steps<MT, MS, false, PART>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src);
+          add_targets();
         }
       } else {
         lane_steps<MT, MS, false, STEPS>(k, X, Y, Z, QX, QY, QZ, AX, AY, AZ, RX, RY, RZ, src);
       }
       if (!FOLD) {
-#pragma unroll
-        for (int t = 0; t < MT; t++) {
-          unsigned long long* a = acc + g * GT + lane + 32 * t;
-          od_fix_add1(a, sum2(AX[t]));
-          od_fix_add1(a + Npad, sum2(AY[t]));
-          od_fix_add1(a + 2 * (size_t)Npad, sum2(AZ[t]));
-        }
+        if (!HALF) add_targets();
         return;
       }
 #pragma unroll
@@ -202,7 +215,7 @@ __device__ __forceinline__ void n3_slice(const float* __restrict__ sx, const flo
   }
 }
 
-template <int MT, int MS, int SPLIT, bool FOLD>
+template <int MT, int MS, int SPLIT, bool FOLD, bool HALF>
 __global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_BLOCKS))
     k_pairs_n3(const float* __restrict__ sx, const float* __restrict__ sy,
                const float* __restrict__ sz, int Npad, unsigned long long* __restrict__ acc,
@@ -210,15 +223,16 @@ __global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_B
   __shared__ float sm[FOLD ? kSliceWarps * 6 * slice_traits<MT, MS>::GT : 1];
   const int w = threadIdx.x >> 5;
   od_pdl_trigger();
-  n3_slice<MT, MS, SPLIT, FOLD>(sx, sy, sz, Npad, acc, rho0,
-                                (long long)blockIdx.x * kSliceWarps + w, sp,
-                                sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT + (threadIdx.x & 31)
-                                           : 0));
+  n3_slice<MT, MS, SPLIT, FOLD, HALF>(sx, sy, sz, Npad, acc, rho0,
+                                      (long long)blockIdx.x * kSliceWarps + w, sp,
+                                      sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT +
+                                                       (threadIdx.x & 31)
+                                                 : 0));
 }
 
 // Batched form: block k takes block items[k].y of member items[k].x; the table lists every block of
 // every member using this form.
-template <int MT, int MS, int SPLIT, bool FOLD>
+template <int MT, int MS, int SPLIT, bool FOLD, bool HALF>
 __global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_BLOCKS))
     k_b_pairs_n3(const od_simdesc* __restrict__ sims, const int2* __restrict__ items) {
   __shared__ float sm[FOLD ? kSliceWarps * 6 * slice_traits<MT, MS>::GT : 1];
@@ -230,10 +244,11 @@ __global__ void __launch_bounds__(kSliceWarps * 32, (slice_traits<MT, MS>::MIN_B
     return;
   }
   const int w = threadIdx.x >> 5;
-  n3_slice<MT, MS, SPLIT, FOLD>(d.b.sx, d.b.sy, d.b.sz, d.Npad, d.b.n3, d.rho0,
-                                (long long)it.y * kSliceWarps + w, d.n3,
-                                sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT + (threadIdx.x & 31)
-                                           : 0));
+  n3_slice<MT, MS, SPLIT, FOLD, HALF>(d.b.sx, d.b.sy, d.b.sz, d.Npad, d.b.n3, d.rho0,
+                                      (long long)it.y * kSliceWarps + w, d.n3,
+                                      sm + (FOLD ? w * 6 * slice_traits<MT, MS>::GT +
+                                                       (threadIdx.x & 31)
+                                                 : 0));
 }
 
 // Accumulators -> slab 0 of (ph, pl) as two-float sums, and cleared for the next evaluation.
@@ -247,10 +262,10 @@ __global__ void k_n3_take(unsigned long long* __restrict__ acc, int Npad, float4
   pl[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
 }
 
-template <int MT, int MS, int SPLIT, bool FOLD>
+template <int MT, int MS, int SPLIT, bool FOLD, bool HALF = false>
 cudaError_t launch_n3(const od_pair_io& io, int Npad, float rho0, const od_n3_split& sp,
                       cudaStream_t s) {
-  return od_launch_pdl(k_pairs_n3<MT, MS, SPLIT, FOLD>, dim3((unsigned)od_n3_blocks(sp)),
+  return od_launch_pdl(k_pairs_n3<MT, MS, SPLIT, FOLD, HALF>, dim3((unsigned)od_n3_blocks(sp)),
                        dim3(kSliceWarps * 32), s, io.sx, io.sy, io.sz, Npad, io.n3, rho0, sp);
 }
 
@@ -275,13 +290,12 @@ long long od_n3_blocks(const od_n3_split& sp) { return (sp.units + kSliceWarps -
 //     empty (3040 on 152 SMs; 4656 group pairs at 12000) and a single warp's dependency chain sets
 //     the time, so they are split by lane steps. Steps of 2048, 4096, 5000, 7680, 8192 and 14000
 //     ions in us: whole 29.0, 31.1, 52.4, 54.7, 55.3, 94.5; two parts 24.4, 28.9, 37.5, 44.7, 44.4,
-//     90.7; four 22.8, 27.0, 30.1, 42.6, 46.0, 97.5. From 2^14 to 2^15 ions two parts keep the
-//     accuracy of the 2 x 2 shape that was the default there, as their FP32 chains on the target side have 32
-//     terms where a whole group pair's have 64: median relative error per ion at 16385, 20011 and
-//     32768 ions 5.5e-8, 5.2e-8, 4.7e-8 in two parts, 6.0e-8, 5.7e-8, 5.1e-8 whole, 5.8e-8, 5.6e-8,
-//     5.0e-8 with 2 x 2. Steps of 16384, 20011, 25000, 28000 and 32768 ions: 113.5, 162.8, 233.0,
-//     289.4, 385.6 us, whole 115.1, 166.1, 232.5, 285.9, 383.5; batches run them apart from their larger
-//     members, with a last wave of their own (0.2 %; six members of 2^14 to 2^15 ions 1.6 %).
+//     90.7; four 22.8, 27.0, 30.1, 42.6, 46.0, 97.5. Two parts still gain 1.5 % at 2^14, but there
+//     batches would run them apart from their larger members, with a last wave of their own.
+//     Tiles of 2048 and 4096 ions: the target sums of whole group pairs are added after each half, so
+//     that the FP32 chains have 32 terms instead of 64: median relative error per ion at 16385, 20011 and 32768
+//     ions 5.5e-8, 5.2e-8, 4.7e-8 against 6.0e-8, 5.7e-8, 5.1e-8. No slower for a single simulation (325
+//     us per step at 30000 ions), 2.5 % in batches.
 //   * 8 x 2 (256 x 64 ions) and 2 x 2: a tile names how many group pairs a slice may hold (tile / 64),
 //     at least 16 slices per resident warp. 8 x 2 at 2^18 ions: 21.6 ms with 8 or 16, 22.3 with 1.
 od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
@@ -291,13 +305,14 @@ od_n3_split od_n3_split_of(int Npad, int ipt, int tile) {
   sp.split = 1;
   long long L = 1;
   if (ipt == 4) {
-    if (Npad <= 32768) sp.split = Npad <= 7680 ? 4 : 2;
+    if (Npad < 16384) sp.split = Npad <= 7680 ? 4 : 2;
   } else {
     const long long warps = 152ll * kSliceWarps * (ipt == 8 ? 4 : 8);
     L = std::max(1ll, std::min<long long>(tile / 64, sp.pairs / (warps * 16)));
   }
   while (sp.pairs / L / kSliceWarps >= 0x7fffffff) L *= 2;  // the grid holds 2^31 - 1 blocks
   sp.L = (int)L;
+  sp.half = ipt == 4 && tile > 1024 && sp.split == 1 && L == 1;
   sp.units = sp.split > 1 ? sp.pairs * sp.split : (sp.pairs + L - 1) / L;
   return sp;
 }
@@ -312,6 +327,7 @@ cudaError_t od_launch_pairs_n3(const od_pair_plan& pl, const od_pair_io& io, int
   else if (sp.split == 4) e = launch_n3<4, 4, 4, false>(io, Npad, rho0, sp, s);
   else if (sp.split == 2) e = launch_n3<4, 4, 2, false>(io, Npad, rho0, sp, s);
   else if (sp.L > 1) e = launch_n3<4, 4, 1, true>(io, Npad, rho0, sp, s);
+  else if (sp.half) e = launch_n3<4, 4, 1, false, true>(io, Npad, rho0, sp, s);
   else e = launch_n3<4, 4, 1, false>(io, Npad, rho0, sp, s);
   if (e != cudaSuccess) return e;
   if (take) k_n3_take<<<(Npad + 255) / 256, 256, 0, s>>>(io.n3, Npad, ph, plo);
@@ -319,10 +335,12 @@ cudaError_t od_launch_pairs_n3(const od_pair_plan& pl, const od_pair_io& io, int
 }
 
 int od_n3_default(int Npad, size_t budget_bytes, int* ipt) {
-  // 4 x 4 up to 2^16 ions, 8 x 2 above: 100000 ions 3.33 and 3.22 ms, 50021 ions 0.838 and 0.824 ms,
-  // 16384 ions 0.100 and 0.102 ms (the accumulators fit any budget that holds the ions: 24 bytes
-  // per ion)
-  return od_n3_batch_plan(Npad, budget_bytes, ipt);
+  // as a batch member: 4 x 4 up to 2^16 ions, 8 x 2 above: 100000 ions 3.33 and 3.22 ms, 50021 ions 0.838
+  // and 0.824 ms, 16384 ions 0.100 and 0.102 ms (the accumulators fit any budget that holds the
+  // ions: 24 bytes per ion). From 2^14 to 2^15 ions with halves, as accurate as the 2 x 2 shape
+  // that was the default there (5.8e-8, 5.6e-8 and 5.0e-8 at 16385, 20011 and 32768 ions).
+  const int tile = od_n3_batch_plan(Npad, budget_bytes, ipt);
+  return tile == 1024 && Npad >= 16384 && Npad <= 32768 ? 2048 : tile;
 }
 
 size_t od_n3_floats(int Npad, int T) {
@@ -334,23 +352,25 @@ size_t od_n3_floats(int Npad, int T) {
 int od_n3_form(int ipt, const od_n3_split& sp) {
   if (ipt == 8) return 3;
   if (ipt == 2) return 5;
+  if (sp.half) return 6;
   return sp.split == 4 ? 2 : (sp.split == 2 ? 1 : (sp.L > 1 ? 4 : 0));
 }
 
 cudaError_t od_launch_batch_pairs_n3(const od_batchview& v, unsigned pairs, cudaStream_t s) {
-  // the forms batch members use: those of od_n3_batch_plan, and 2 x 2, which a member's own handle may
-  // be given (od_set_pair_plan)
+  // the forms batch members use: those of od_n3_batch_plan, and 2 x 2 and halves, which a member's own
+  // handle may be given (od_set_pair_plan)
   cudaError_t e = cudaSuccess;
-#define OD_B_N3(f, MT, MS, SPLIT, FOLD)                                                      \
+#define OD_B_N3(f, MT, MS, SPLIT, FOLD, HALF)                                                \
   if (v.n3_nitems[f] > 0 && (pairs >> f & 1) && e == cudaSuccess)                            \
-  e = od_launch_pdl(k_b_pairs_n3<MT, MS, SPLIT, FOLD>, dim3(v.n3_nitems[f]),                 \
+  e = od_launch_pdl(k_b_pairs_n3<MT, MS, SPLIT, FOLD, HALF>, dim3(v.n3_nitems[f]),           \
                     dim3(kSliceWarps * 32), s, v.sims, (const int2*)v.n3_items[f])
-  OD_B_N3(3, 8, 2, 1, true);
-  OD_B_N3(0, 4, 4, 1, false);
-  OD_B_N3(1, 4, 4, 2, false);
-  OD_B_N3(2, 4, 4, 4, false);
-  OD_B_N3(4, 4, 4, 1, true);
-  OD_B_N3(5, 2, 2, 1, true);
+  OD_B_N3(3, 8, 2, 1, true, false);
+  OD_B_N3(0, 4, 4, 1, false, false);
+  OD_B_N3(6, 4, 4, 1, false, true);
+  OD_B_N3(1, 4, 4, 2, false, false);
+  OD_B_N3(2, 4, 4, 4, false, false);
+  OD_B_N3(4, 4, 4, 1, true, false);
+  OD_B_N3(5, 2, 2, 1, true, false);
 #undef OD_B_N3
   return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -293,18 +293,18 @@ def test_small_state_is_one_copy(fake, N, copies):
         assert log(fake).count("cudaMemcpyAsync") == copies and faults(fake) == []
 
 
-@pytest.mark.parametrize("N", [512, 7680, 7681, 16384, 32768])
+@pytest.mark.parametrize("N", [512, 7680, 7681, 15872, 16384, 32768, 33280])
 def test_short_fp32_chains_up_to_2_15_ions(fake, N):
-    # an FP32 chain of target sums has 64 terms in a whole 4 x 4 group pair, 32 in one of two parts
+    # an FP32 chain of target sums has 64 terms in a whole 4 x 4 group pair, 32 in one of two parts or
+    # with sums added after each half
     holder, pos, vel = member_case(N=N)
-    with _lib.Engine(holder) as eng, _lib.Batch() as b:
+    with _lib.Engine(holder) as eng:
         eng.set_state(pos, vel)
         eng.step(1)
-        b.add(holder, pos, vel)
-        b.step(1)
-    names = [x for x in log(fake) if "pairs_n3ILi4ELi4E" in x]
-    split = "ILi4ELi4ELi4E" if N <= 7680 else "ILi4ELi4ELi2E"
-    assert names and all(split in x for x in names)
+    names = [x for x in log(fake) if "10k_pairs_n3I" in x]
+    kernel = ("ILi4ELi4ELi4ELb0ELb0E" if N <= 7680 else "ILi4ELi4ELi2ELb0ELb0E" if N < 16384 else
+              "ILi4ELi4ELi1ELb0ELb1E" if N <= 32768 else "ILi4ELi4ELi1ELb0ELb0E")
+    assert names and all(kernel in x for x in names)
 
 
 @pytest.mark.parametrize("N", [1000, 2000])
