@@ -197,10 +197,10 @@ def test_batch_forgets_the_error_of_a_member_that_left(fake, bits, status):
 def test_force_snapshot_in_place(fake, builder):
     # the caller's positions are read before anything is written to the forces, also where the upload
     # runs late (page-locked memory, or a host whose pageable memory the device reads itself)
-    holder, pos, _ = case(N=1500, n=8, builder=builder, trap=np.zeros(15))[:3]
+    holder, pos, _ = case(N=8000, n=8, builder=builder, trap=np.zeros(15))[:3]
     with _lib.Engine(holder) as eng:
         fake.fake_reset()
-        for n in (1500, 1):
+        for n in (8000, 1500, 1):  # forces above and below 128 KB
             x = pos[:n].copy()
             _lib.check(fake.od_force_snapshot(eng.h, _lib._dptr(x), n, _lib._dptr(x)), eng.h)
     assert faults(fake) == []
