@@ -1225,8 +1225,8 @@ static od_status ensure_acc(od_handle* h) {
 
 // Variant 7: `ions_per_lane` targets per lane (2 or 4 with as many sources, 8 with two sources),
 // `tile` caps the work per warp for 2 and 8, above 1024 its FP32 chains for 4 (od_n3_split_of; 1024,
-// 2048, 4096; <= 0: 1024 up to 2^17 ions, else 2048). The pair sums go to three 64-bit fixed-point accumulators per ion (24 bytes per ion: 25
-// MB at 2^20).
+// 2048, 4096; <= 0: 1024 up to 2^17 ions, else 2048). The pair sums go to three 64-bit fixed-point
+// accumulators per ion (24 bytes per ion: 25 MB at 2^20).
 static od_status set_plan_n3(od_handle* h, int ions_per_lane, int tile) {
   if (!plan_supported(256, ions_per_lane, 7))
     return fail(h, OD_ERR_INVALID, "variant 7 takes 2, 4 or 8 targets per lane");
@@ -1354,12 +1354,13 @@ extern "C" od_status od_autotune(od_handle* h, int32_t use_cache, double* best_p
   // Launches are timed as a step makes them, the sums of the variants with accumulators left there for
   // K3; untimed, they are cleared for the next plan. (ms: of `reps` launches.)
   auto time_launches = [&](auto launch, float* ms) {
-    OD_CK(h, launch());
-    OD_CK(h, cudaEventRecord(e0, h->stream));
-    for (int r = 0; r < reps; r++) OD_CK(h, launch());
-    OD_CK(h, cudaEventRecord(e1, h->stream));
+    cudaError_t e = launch();
+    if (e == cudaSuccess) e = cudaEventRecord(e0, h->stream);
+    for (int r = 0; r < reps && e == cudaSuccess; r++) e = launch();
+    if (e == cudaSuccess) e = cudaEventRecord(e1, h->stream);
     if (uses_acc(h))
       OD_CK(h, cudaMemsetAsync(h->b.n3, 0, sizeof(float) * h->b.n3_len, h->stream));
+    if (e != cudaSuccess) return cuda_fail(h, e, "autotuner launch");
     OD_CK(h, cudaEventSynchronize(e1));
     OD_CK(h, cudaEventElapsedTime(ms, e0, e1));
     return OD_OK;
@@ -1475,11 +1476,14 @@ extern "C" od_status od_get_series(od_handle* h, int64_t first, int64_t count, d
   double* out[5] = {q, f_orbit, f_collect, f_dust, f_field};
   const double* src = h->b.series + first * row;
   const size_t width[5] = {P, 3 * P, 3 * P, 3 * P, 3 * P};  // of a row
+  std::vector<double> rows;
+  od_copies copies{h->stream};
   if (sizeof(double) * row * count <= OD_SERIES_WHOLE) {  // each copy takes about 9 us
-    std::vector<double> rows((size_t)count * row);
+    rows.resize((size_t)count * row);
     OD_CK(h, cudaMemcpyAsync(rows.data(), src, sizeof(double) * rows.size(),
                              cudaMemcpyDeviceToHost, h->stream));
     OD_CK(h, cudaStreamSynchronize(h->stream));
+    copies.done = true;
     for (size_t m = 0, at = 0; m < 5; at += width[m++])
       if (out[m])
         for (int64_t k = 0; k < count; k++)
@@ -1501,6 +1505,7 @@ extern "C" od_status od_get_series(od_handle* h, int64_t first, int64_t count, d
                                  cudaMemcpyDeviceToHost, h->stream));
   }
   OD_CK(h, cudaStreamSynchronize(h->stream));
+  copies.done = true;
   return OD_OK;
 }
 
@@ -1963,8 +1968,11 @@ extern "C" od_status od_batch_step(od_batch* b, int64_t nsteps) {
   OD_BCK(b, cudaEventRecord(b->ev0, b->stream));
   for (int64_t s = 0; s < nsteps; s++) {
     const cudaError_t e = cudaGraphLaunch(b->exec[batch_pair_mask(b, 0)], b->stream);
-    if (e != cudaSuccess) cudaStreamSynchronize(b->stream);  // the steps before are the members' to read
-    OD_BCK(b, e);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      cudaStreamSynchronize(b->stream);  // the steps before are the members' to read
+      return bfail(b, OD_ERR_CUDA, std::string("batch step launch: ") + cudaGetErrorString(e));
+    }
     for (od_handle* h : b->members)  // with every launch: the device counts the steps before a failed one
       if (h) h->step++;
   }

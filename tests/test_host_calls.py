@@ -328,3 +328,31 @@ def test_failed_call_leaves_no_copy_behind(fake, call, fails, N):
             fake.fake_fail(fails, 1000)
             eng.get_state()
             assert faults(fake) == []
+
+
+@pytest.mark.parametrize("rows", [100, 30000])
+def test_failed_series_read_leaves_no_copy_behind(fake, rows):
+    holder, pos, vel = member_case(N=300, n=rows)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        eng.step(rows)
+        for after in range(1 if rows == 100 else 5):
+            fake.fake_reset()
+            fake.fake_fail(b"cudaMemcpyAsync", after)
+            with pytest.raises(_lib.OpenDustError):
+                eng.series(0, rows)
+            assert log(fake)[-1] == "cudaStreamSynchronize"
+
+
+def test_autotuner_that_fails_leaves_clear_accumulators(fake):
+    # K3 would take what a failed timing left there as forces
+    holder, pos, vel = member_case(N=3000)
+    with _lib.Engine(holder) as eng:
+        eng.set_state(pos, vel)
+        for after in (8, 150):
+            fake.fake_reset()
+            fake.fake_fail(b"launch", after)
+            with pytest.raises(_lib.OpenDustError):
+                eng.autotune(use_cache=False)
+            if eng.pair_plan()["variant"] >= 2:
+                assert log(fake)[-1] == "cudaMemsetAsync"
