@@ -349,10 +349,9 @@ def test_autotuner_that_fails_leaves_clear_accumulators(fake):
     holder, pos, vel = member_case(N=3000)
     with _lib.Engine(holder) as eng:
         eng.set_state(pos, vel)
-        for after in (8, 150):
+        for after, variant in ((200, 2), (685, 7)):
             fake.fake_reset()
             fake.fake_fail(b"launch", after)
             with pytest.raises(_lib.OpenDustError):
                 eng.autotune(use_cache=False)
-            if eng.pair_plan()["variant"] >= 2:
-                assert log(fake)[-1] == "cudaMemsetAsync"
+            assert eng.pair_plan()["variant"] == variant and log(fake)[-1] == "cudaMemsetAsync"
